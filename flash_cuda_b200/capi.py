@@ -20,6 +20,7 @@ FA_ERR_BAD_METADATA = 8
 STATIC_SCRATCH_BYTES = 8 << 20
 FA_DT_BF16, FA_DT_FP16, FA_DT_FP8_E4M3, FA_DT_FP32 = 0, 1, 2, 3
 FA_FLAG_WORKSPACE_CLEAN = 1
+FA_FLAG_WORKSPACE_CLEAN_4K = 2
 FA_ROUTE_AUTO, FA_ROUTE_PREFILL_TC, FA_ROUTE_DECODE, FA_ROUTE_GENERAL = 0, 1, 2, 3
 
 EXPORTS = (

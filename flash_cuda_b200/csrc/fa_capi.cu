@@ -26,6 +26,7 @@ int launch_prefill_tc(const KParams& kp, const Plan& pl, int compute_dtype, cuda
 bool prefill_tc_supported(const PlanInput& in);
 bool prefill_tc_single_tile(int hd, int hdv);
 bool decode_supported(const PlanInput& in);
+int decode_line_ctas(int hd, int kv_dtype, int num_sms);
 bool prefill_tc_layout_ok(const FaFwdParams* p);
 
 static thread_local char g_last_cuda_error[256] = "";
@@ -181,6 +182,35 @@ static Plan decode_part_plan(const PlanInput& in, const Plan& pl) {
   return d;
 }
 
+// The decode kernel cuts the batch's key blocks into equal spans, one per CTA (fa_decode.cu), unless
+//   - the caller fixed the split count (1 = one pass per sequence, whatever else is in the batch) or wants fp32 partials;
+//   - there are three or more work items per CTA: longest first they balance by themselves, and one that ends early
+//     makes room (128 sequences x 8 heads: 1420 us as items, 1477 cut; 111 x 8 x 2 row tiles 70 against 81);
+//   - the sequences are so short that most of them would be cut although there are items for half of the CTAs
+//     (10 sequences of 160 .. 376 keys x 16 heads over e4m3: 19.1 us as items, 20.5 cut);
+//   - the scan that finds the spans, which runs in every CTA, would have more than 2048 entries (13 per thread).
+static bool balanced_decode(const FaFwdParams* p, const Plan& decode_plan, bool mixed = false) {
+  const long long entries = (long long)p->batch * decode_plan.max_mtiles, items = entries * p->hkv;
+  const int ctas = decode_line_ctas(p->hd, p->kv_dtype, decode_plan.num_sms);
+  if (decode_plan.route != FA_ROUTE_DECODE || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 ||
+      entries > kBalancedEntriesMax || items * (p->max_seqlen_k / 64 + 2) >= (1ll << 30) || ctas > kWsArrivalWords)
+    return false;
+  if (mixed) return true;      // (four row tiles per sequence in `entries`, nearly all of them empty)
+  return items < 3ll * ctas && !(p->max_seqlen_k <= 512 && items * 2 >= ctas);
+}
+
+// Scratch for the pieces of a balanced call: two pieces of `rows` rows for each CTA.
+struct PartPlan { int rows; size_t ml_bytes, o_bytes; };
+static PartPlan part_plan(const FaFwdParams* p, const Plan& decode_plan) {
+  PartPlan pp;
+  const long long rows = (long long)p->max_seqlen_q * decode_plan.rows_per_token;
+  pp.rows = rows < 16 ? (int)rows : 16;
+  const size_t n = (size_t)decode_line_ctas(p->hd, p->kv_dtype, decode_plan.num_sms) * 2 * pp.rows;
+  pp.ml_bytes = align_up(n * 8, 256);
+  pp.o_bytes = align_up(n * p->hdv * 4, 256);
+  return pp;
+}
+
 // De-paging.  A prefill over pages of 1 .. 16 keys pays for its small copies in every query tile that reads a key
 // block (the tensor-core kernel runs at 500 - 900 TFLOP/s there against ~1150 over contiguous keys).  Where the keys
 // are read often enough - ceil(max_seqlen_q / 256) x (q heads per kv head) tiles per block, at least 4 - and the
@@ -213,12 +243,26 @@ struct WsLayout {
   size_t work2_off, work2_bytes;   // mixed batches: the prefill kernel's list
   size_t lse_off, lse_bytes;
   size_t o_off, o_bytes;
+  PartPlan parts;
+  size_t part_ml_off, part_o_off;   // balanced decode: pieces of cut (sequence, head) triples; part_o_off 0: none
   size_t total;
 };
 static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
   WsLayout w{};
-  w.header = 256;
+  w.header = kWsHeader;
   size_t off = w.header;
+  auto carve_parts = [&](const Plan& pd) {
+    w.parts = part_plan(p, pd);
+    w.part_ml_off = off;
+    off += w.parts.ml_bytes;
+    w.part_o_off = off;
+    off += w.parts.o_bytes;
+  };
+  if (balanced_decode(p, pl)) {
+    carve_parts(pl);
+    w.total = off;
+    return w;
+  }
   w.work_off = off;
   w.work_bytes = (pl.route == FA_ROUTE_DECODE && p->scheduler_metadata == nullptr)
                      ? align_up((size_t)sched_len(pl, p->batch) * 4, 256) : 0;
@@ -227,9 +271,14 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
     // room for the two lists of a mixed batch (whether the call is one is decided from the same facts in fa_b200_fwd)
     const PlanInput in = plan_input(p, pl.num_sms);
     if (mixed_batch(p, in, pl)) {
-      w.work_off = off;
-      w.work_bytes = align_up((size_t)sched_len(decode_part_plan(in, pl), p->batch) * 4, 256);
-      off += w.work_bytes;
+      const Plan pd = decode_part_plan(in, pl);
+      if (balanced_decode(p, pd, true)) {
+        carve_parts(pd);
+      } else {
+        w.work_off = off;
+        w.work_bytes = align_up((size_t)sched_len(pd, p->batch) * 4, 256);
+        off += w.work_bytes;
+      }
       w.work2_off = off;
       w.work2_bytes = align_up((size_t)sched_len(pl, p->batch) * 4, 256);
       off += w.work2_bytes;
@@ -382,9 +431,14 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   // (FA_FLAG_WORKSPACE_CLEAN) saves the memset: the kernels leave the counters at zero when they finish.
   const bool clean = (p->flags & FA_FLAG_WORKSPACE_CLEAN) != 0;
   // (on the decode route without caller metadata the work-list kernel runs first and clears the header itself)
-  const bool sched_first = pl.route == FA_ROUTE_DECODE && p->scheduler_metadata == nullptr;
+  const bool balanced = w.part_o_off > 0;
+  const bool sched_first = pl.route == FA_ROUTE_DECODE && p->scheduler_metadata == nullptr && !balanced;
   if (!clean && !sched_first) {
-    cudaError_t ce = cudaMemsetAsync(ws, 0, w.header, stream);
+    cudaError_t ce = cudaMemsetAsync(ws, 0, balanced ? kWsHeader : kWsArrivalOff, stream);
+    if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(workspace header)");
+  } else if (balanced && !(p->flags & FA_FLAG_WORKSPACE_CLEAN_4K)) {
+    // the caller keeps the first 256 bytes only
+    cudaError_t ce = cudaMemsetAsync(ws + kWsArrivalOff, 0, kWsHeader - kWsArrivalOff, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(workspace header)");
   }
 
@@ -416,13 +470,18 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   kp.out_f32 = p->out_dtype == FA_DT_FP32;
   kp.work_expect = SchedExpect{p->batch, pl.nsplits, pl.tile_m, pl.tile_n, pl.max_mtiles, pl.rows_per_token, pl.route};
   kp.scale = p->softmax_scale; kp.softcap = p->softcap;
-  if (pl.nsplits > 1) { kp.lse_part = (float*)(ws + w.lse_off); kp.o_part = (float*)(ws + w.o_off); }
+  if (balanced) {
+    kp.part_ml = (float*)(ws + w.part_ml_off); kp.part_o = (float*)(ws + w.part_o_off);
+    kp.arrivals = (uint32_t*)(ws + kWsArrivalOff);
+    kp.part_rows = w.parts.rows;
+  }
+  else if (pl.nsplits > 1) { kp.lse_part = (float*)(ws + w.lse_off); kp.o_part = (float*)(ws + w.o_off); }
 
   const int compute_dtype = p->q_dtype == FA_DT_FP16 ? FA_DT_FP16 : FA_DT_BF16;
 
   if (pl.route == FA_ROUTE_DECODE) {
     const int32_t* work = p->scheduler_metadata;
-    if (!work) {
+    if (!work && !balanced) {
       FaSchedParams sp{};
       sp.seqused_k = p->seqused_k; sp.cu_seqlens_q = p->cu_seqlens_q; sp.cu_seqlens_k = p->cu_seqlens_k;
       sp.leftpad_k = p->leftpad_k; sp.batch = p->batch; sp.max_seqlen_q = p->max_seqlen_q;
@@ -445,11 +504,12 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     const Plan pd = decode_part_plan(in, pl);
     int32_t* list_d = (int32_t*)(ws + w.work_off);
     int32_t* list_p = (int32_t*)(ws + w.work2_off);
-    rc = note_cuda_error(launch_sched(sp, pd, list_d, nullptr, stream, 1, kDecodeMaxRows), "sched_kernel");
+    if (!balanced) rc = note_cuda_error(launch_sched(sp, pd, list_d, nullptr, stream, 1, kDecodeMaxRows), "sched_kernel");
     if (rc == FA_OK) rc = note_cuda_error(launch_sched(sp, pl, list_p, nullptr, stream, 2, kDecodeMaxRows), "sched_kernel");
     if (rc != FA_OK) return rc;
     KParams kd = kp;
-    kd.work = list_d;
+    kd.work = balanced ? nullptr : list_d;
+    kd.class_rows = kDecodeMaxRows;
     kd.nsplits = 1;
     kd.work_expect = SchedExpect{p->batch, 1, pd.tile_m, pd.tile_n, pd.max_mtiles, pd.rows_per_token, pd.route};
     rc = note_cuda_error(launch_decode(kd, pd, compute_dtype, stream), "decode kernel");
@@ -478,7 +538,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   }
   if (rc != FA_OK) return rc;
 
-  if (pl.nsplits > 1) {
+  if (pl.nsplits > 1 && !balanced) {
     rc = note_cuda_error(launch_combine(kp.o_part, kp.lse_part, pl.nsplits, p->total_q, p->hq, p->hdv, p->s_aux,
                                         p->out, p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream),
                          "combine kernel");
@@ -489,7 +549,9 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
 // ---- decode without allocation: scratch in a device array that is part of this library's image ----
 // In host code `g_static_scratch` is only a handle for the symbol, not a device address: the address is looked up
 // once per device with cudaGetSymbolAddress and that pointer is what the kernels receive.
-static __device__ __align__(256) unsigned char g_static_scratch[FA_B200_STATIC_SCRATCH_BYTES];
+// (The limit is stated for the scratch behind the header.)
+constexpr size_t kStaticBytes = (size_t)FA_B200_STATIC_SCRATCH_BYTES + kWsHeader;
+static __device__ __align__(256) unsigned char g_static_scratch[kStaticBytes];
 static void* g_static_scratch_addr[64];
 static std::atomic<int> g_static_scratch_ready[64];
 
@@ -501,7 +563,7 @@ int fa_b200_decode_fwd_static(const FaFwdParams* p, fa_stream_t stream) {
   Plan pl = make_plan(plan_input(p, di->sms));
   if (pl.err != FA_OK) return pl.err;
   if (pl.route != FA_ROUTE_DECODE) return FA_ERR_UNSUPPORTED;
-  if (ws_layout(p, pl).total > (size_t)FA_B200_STATIC_SCRATCH_BYTES) return FA_ERR_STATIC_LIMIT;
+  if (ws_layout(p, pl).total > kStaticBytes) return FA_ERR_STATIC_LIMIT;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FA_ERR_NO_DEVICE;
   if (g_static_scratch_ready[dev].load(std::memory_order_acquire) == 0) {
@@ -516,7 +578,7 @@ int fa_b200_decode_fwd_static(const FaFwdParams* p, fa_stream_t stream) {
   }
   FaFwdParams q = *p;
   q.route = FA_ROUTE_DECODE;
-  return fa_b200_fwd(&q, g_static_scratch_addr[dev], (size_t)FA_B200_STATIC_SCRATCH_BYTES, stream);
+  return fa_b200_fwd(&q, g_static_scratch_addr[dev], kStaticBytes, stream);
 }
 
 int fa_b200_scheduler_metadata_len(const FaSchedParams* p) {

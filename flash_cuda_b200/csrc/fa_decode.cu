@@ -29,6 +29,7 @@
 namespace fa {
 namespace dec {
 
+
 constexpr int TN = 64;                 // keys per scheduler block (metadata unit); a stage holds TNS keys
 // Consumer warps per CTA.  A 16-bit cache runs one CTA per SM; an e4m3 cache runs TWO (half-size stages): every
 // consumer warp works on every stage, so one CTA's stage rate is bounded by the latency of one warp's
@@ -38,6 +39,8 @@ constexpr int ncons_for(int) { return 4; }
 constexpr int ctas_per_sm(int esz) { return esz == 1 ? 2 : 1; }
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
+constexpr int kMinSpan = 4;            // balanced kernels: key blocks of a span at least
+constexpr int kPieces = 4;             // mailbox slots between the producer and the consumers
 enum Role : unsigned { ROLE_PRODUCER = 5, ROLE_CONSUMER = 6 };
 enum : int { F_FIRST = 1, F_LAST = 2, F_EMPTY = 4 };
 
@@ -47,6 +50,11 @@ struct DecArgs {
   int box_rows;       // rows per TMA box = min(page_size, 64); 1 in gather mode
   int kv_total_rows;
   int gather;         // pages of 1, 2 or 4 keys: rows are fetched 16 bytes per lane with cp.async
+  // balanced kernels (see LineCut)
+  int use_list;       // kp.work holds the caller's scheduler metadata: its entries are the line, else all (batch, tile)
+  int max_mtiles;     // row tiles per sequence
+  int team;           // CTAs that walk the same keys side by side, one kv head each (a divisor of hkv)
+  int class_rows;     // > 0: only sequences with at most this many packed query rows (the short ones of a mixed batch)
 };
 
 template <int ESZ, int NST, int HD, int HDV, int TNS_>
@@ -61,8 +69,13 @@ struct Smem {
   static constexpr int kMiscOff = kBarOff + 2 * NST * 8;       // abort flags
   static constexpr int kScrOff = (kMiscOff + 16 + 15) / 16 * 16;
   static constexpr int kLdO = HDV + 4;
-  static constexpr int kScrBytes = NC * 16 * kLdO * 4 + 3 * NC * 16 * 4;
-  static constexpr int kBytes = kScrOff + kScrBytes;
+  static constexpr int kScrBytes = NC * 16 * kLdO * 4 + 2 * NC * 16 * 4;
+  // balanced kernels: piece mailbox with its barriers, then the line's prefix sums
+  static constexpr int kPieceOff = kScrOff + kScrBytes;
+  static constexpr int kPieceBarOff = kPieceOff + kPieces * 80;   // full[kPieces], empty[kPieces], flag
+  static constexpr int kPrefOff = kPieceBarOff + 2 * kPieces * 8 + 16;
+  static constexpr int kBytesBalanced = kPrefOff + (kBalancedEntriesMax + 4) * 4;
+  static constexpr int kBytes = kPieceOff;
 };
 
 template <int NC>
@@ -103,6 +116,85 @@ __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
   }
   return it;
 }
+
+// ---------------------------------------------------------------------------------------------------------
+// Balanced kernels.  The key blocks of all (batch, row tile, group of `team` kv heads), one after the other, form a
+// line that is cut into spans of equal length, whatever sequences they cross; the CTAs of a team walk one span side by
+// side, one kv head each.  With one work item per (batch, row tile, kv head) a ragged batch of 16 sequences (128 items)
+// waited for its longest sequence, and few long sequences needed a split count, a work-list kernel before and a merge
+// kernel after: 16 sequences of 1024 .. 16384 keys 174 -> 109 us per call (HBM floor 83), one of 1000 keys 20.5 ->
+// 16.4 us, 24 x 4 queries over 500 .. 8000 keys of head_dim 64 107 -> 84 us.
+// The team keeps the heads of a token, neighbours in memory, together in time: with the heads of a sequence one after
+// the other on the line (every CTA somewhere else, 256-byte rows 2 KB apart) the 16 sequences took 119 us, and 128
+// sequences of 1024 .. 32768 keys fell from 6.25 to 5.4 TB/s.
+// What lies inside one span is written out directly; the pieces of a (batch, row tile, head) that crosses span borders
+// go to `part_*` as unnormalised fp32 rows with their maximum and sum, and the CTA that finishes the last piece merges
+// all of them in the order of the line (the same bits every time).  A cut costs about 3.5 us of a CTA per piece, which
+// is why the line is cut once per CTA and no finer: with half of it handed out in spans of 8 blocks the 16 sequences
+// took 159 us.  Batches with several items per CTA keep the work-item kernels (balanced_decode in fa_capi.cu).
+struct LineCut {
+  int spans, width, extra;       // the first `extra` spans have width + 1 blocks, the others width
+  __device__ __forceinline__ int begin(int c) const { return c * width + min(c, extra); }
+  __device__ __forceinline__ int span_of(int x) const {
+    const int wide = extra * (width + 1);
+    return x < wide ? x / (width + 1) : extra + (x - wide) / width;
+  }
+  __device__ __forceinline__ void plan(int total, int max_spans) {
+    spans = max(1, min(max_spans, (total + kMinSpan - 1) / kMinSpan));
+    width = total / spans;
+    extra = total - width * spans;
+  }
+};
+
+// Entry e of the line: a (batch, row tile), all head groups; `hk` and `split` are left at 0.
+__device__ __forceinline__ WorkItem line_entry(const DecArgs& a, int e) {
+  const KParams& p = a.kp;
+  WorkItem it;
+  it.hk = it.split = 0;
+  it.lo = it.hi = 0;
+  it.seqlen_q = it.seqlen_k = it.q0 = it.k0 = it.leftpad = 0;
+  it.valid = it.bad = false;
+  int n_lo = 0, n_hi = 0;
+  if (a.use_list) {
+    const int32_t* ent = p.work + kSchedHeader + 4 * e;      // (a caller's tensor: 4-byte aligned)
+    it.b = ent[0];
+    it.mt = ent[1] > 0 ? ent[1] : 0;
+    n_lo = ent[2]; n_hi = ent[3];
+    if (it.b < 0) return it;
+    if (it.b >= p.batch || it.mt >= a.max_mtiles) { it.bad = true; return it; }
+  } else {
+    it.b = e / a.max_mtiles;
+    it.mt = e - it.b * a.max_mtiles;
+  }
+  it.q0 = p.cu_q[it.b];
+  it.seqlen_q = p.cu_q[it.b + 1] - it.q0;
+  it.k0 = p.page_table ? 0 : p.cu_k[it.b];
+  it.seqlen_k = p.seqused_k ? p.seqused_k[it.b] : (p.cu_k[it.b + 1] - p.cu_k[it.b]);
+  it.leftpad = p.leftpad_k ? p.leftpad_k[it.b] : 0;
+  const int rows = it.seqlen_q * p.rep;
+  if (it.mt * 16 >= rows || (a.class_rows > 0 && rows > a.class_rows)) return it;
+  if (a.use_list) {
+    if (n_lo < 0 || n_hi < n_lo || (int64_t)n_hi * TN > (int64_t)it.seqlen_k + TN - 1) { it.bad = true; return it; }
+  } else {
+    const int off = it.seqlen_k - it.seqlen_q, row0 = it.mt * 16;
+    nblock_range(it.seqlen_k, it.leftpad, off + row0 / p.rep, off + min(it.seqlen_q - 1, (row0 + 15) / p.rep), p.is_causal,
+                 p.window_left, p.window_right, TN, &n_lo, &n_hi);
+  }
+  it.valid = true;
+  it.lo = n_lo; it.hi = n_hi;
+  return it;
+}
+// Blocks of one head group of an entry; an entry whose rows see no key counts as one, so that some CTA writes its rows.
+__device__ __forceinline__ int line_len(const WorkItem& it) { return it.valid ? max(it.hi - it.lo, 1) : 0; }
+
+// One piece of a (batch, row tile, head), as the producer hands it to the consumers.
+struct Piece {
+  WorkItem it;               // key blocks [it.lo, it.hi); it.b < 0: no more pieces
+  int pieces;                // pieces this (batch, row tile, head) is cut into (1 = not cut)
+  int first, number;         // scratch numbers of its first piece and of this one: member * spans + span
+  int head;                  // 1: this is the first piece
+};
+static_assert(sizeof(Piece) <= 80, "mailbox slot");
 
 // The cp.async producer's copies of one operand (K or V) of a stage: TNS rows of CPR 16-byte chunks, row r from
 // pool row yr[r / 32] of lane r % 32, written where a 128-byte-swizzled TMA box would have put them (column block
@@ -159,7 +251,7 @@ __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* sr
 }
 
 // T = MMA element type (bf16 / fp16); KV8 = the cache holds e4m3 bytes.
-template <typename T, bool KV8, int NST, int HD, int HDV, int CPS, int TNS_>
+template <typename T, bool KV8, int NST, int HD, int HDV, int CPS, int TNS_, bool BAL>
 __global__ void __launch_bounds__((ncons_for(KV8 ? 1 : 2) + 1) * 32, CPS)
 fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v) {
   constexpr int ESZ = KV8 ? 1 : 2;
@@ -188,7 +280,6 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   float* s_o = reinterpret_cast<float*>(sm + SM::kScrOff);
   float* s_m = s_o + NC * 16 * SM::kLdO;
   float* s_l = s_m + NC * 16;
-  float* s_lr = s_l + NC * 16;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
@@ -197,6 +288,56 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     for (int s = 0; s < NST; ++s) { mbar_init(bar_full + 8 * s, a.gather ? 33 : 1); mbar_init(bar_empty + 8 * s, NC); }
     s_abort[0] = 0; s_abort[1] = 0;
     mbar_fence_init();
+  }
+  Piece* s_piece = reinterpret_cast<Piece*>(sm + SM::kPieceOff);
+  const uint32_t bar_pc_full = base + SM::kPieceBarOff, bar_pc_empty = bar_pc_full + 8 * kPieces;
+  volatile int* s_last = reinterpret_cast<volatile int*>(sm + SM::kPieceBarOff + 2 * kPieces * 8);
+  int* s_pref = reinterpret_cast<int*>(sm + SM::kPrefOff);      // blocks before entry e (one head group)
+  LineCut cut{};
+  int groups = 1;
+  if constexpr (BAL) {
+    // ---- the line: lengths summed per thread over consecutive entries, then a block scan ----
+    int* s_sum = reinterpret_cast<int*>(s_o);      // the merge area is not in use yet
+    int E = p.batch * a.max_mtiles;
+    if (a.use_list) {
+      // the list's header must describe this call before any entry is read
+      const bool good = sched_header_matches(p.work, p.work_expect);
+      if (!good && tid == 0) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
+      E = good ? p.work[6] : 0;
+    }
+    if (tid == 0) {
+      for (int i = 0; i < kPieces; ++i) { mbar_init(bar_pc_full + 8 * i, 1); mbar_init(bar_pc_empty + 8 * i, NC); }
+      mbar_fence_init();
+    }
+    constexpr int NTH = (NC + 1) * 32;
+    const int per = (E + NTH - 1) / NTH, e_lo = min(E, tid * per), e_hi = min(E, e_lo + per);
+    int mine = 0;
+    bool bad = false;
+    for (int e = e_lo; e < e_hi; ++e) {
+      const WorkItem it = line_entry(a, e);
+      bad |= it.bad;
+      s_pref[e] = mine;
+      mine += line_len(it);
+    }
+    if (bad) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
+    int incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    int total = 0, before = incl - mine;
+#pragma unroll
+    for (int w = 0; w <= NC; ++w) {
+      if (w < warp) before += s_sum[w];
+      total += s_sum[w];
+    }
+    for (int e = e_lo; e < e_hi; ++e) s_pref[e] += before;
+    if (tid == 0) s_pref[E] = total;
+    groups = p.hkv / a.team;
+    cut.plan(total * groups, (int)gridDim.x / a.team);
   }
   __syncthreads();
 
@@ -210,7 +351,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     const int boxes = TNS / a.box_rows;         // TMA boxes per stage and 128-byte column block
     // the list's header must describe this call before any entry is read
     int total_work = a.total_work;
-    if (!sched_header_matches(p.work, p.work_expect)) {
+    if (!BAL && !sched_header_matches(p.work, p.work_expect)) {
       if (lane == 0) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
       total_work = 0;
     }
@@ -220,19 +361,62 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       if (a.gather) mbar_arrive(bar_full + 8 * s);
       if (lane == 0) mbar_arrive(bar_full + 8 * s);
     };
+    // balanced kernels: the rest [x, x_end) of this CTA's span and the entry that x lies in
+    const int span = BAL ? (int)blockIdx.x / a.team : 0, member = BAL ? (int)blockIdx.x - span * a.team : 0;
+    int x = 0, x_end = 0, ent = 0;
+    uint32_t pcnt = 0;
+    if constexpr (BAL) {
+      if (span < cut.spans) { x = cut.begin(span); x_end = cut.begin(span + 1); }
+      if (x < x_end) {
+        int hi_e = a.use_list ? p.work[6] : p.batch * a.max_mtiles;    // the last entry with groups * s_pref[e] <= x
+        while (hi_e - ent > 1) {
+          const int mid = (ent + hi_e) >> 1;
+          if (s_pref[mid] * groups <= x) ent = mid; else hi_e = mid;
+        }
+      }
+    }
     while (ok) {
       int w = 0;
-      if (first_ticket) w = (int)blockIdx.x;     // a CTA's first work id is its block index, later ones are tickets
-      else if (lane == 0) w = (int)gridDim.x + atomicAdd(p.counters, 1);
-      if (!first_ticket) w = __shfl_sync(0xffffffffu, w, 0);
-      first_ticket = false;
-      if (w >= total_work) break;
-      const WorkItem it = decode_work(p, w);
-      if (it.bad) {
-        if (lane == 0) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
-        break;
+      WorkItem it;
+      if constexpr (BAL) {
+        if (x >= x_end) break;
+        while (x >= s_pref[ent + 1] * groups) ++ent;      // (entries without blocks are passed over)
+        const int len = s_pref[ent + 1] - s_pref[ent], off = x - s_pref[ent] * groups;
+        const int hg = off / len, pos = off - hg * len, n = min(len - pos, x_end - x);
+        it = line_entry(a, ent);
+        it.hk = hg * a.team + member;
+        if (it.hi > it.lo) { it.lo += pos; it.hi = it.lo + n; }
+        const uint32_t slot = pcnt % kPieces;
+        ok = wait_or_abort(bar_pc_empty + 8 * slot, ((pcnt / kPieces) & 1) ^ 1, s_abort);
+        if (!ok) break;
+        if (lane == 0) {
+          Piece& pc = s_piece[slot];
+          pc.it = it;
+          pc.pieces = 1;
+          pc.first = pc.number = member * cut.spans + span;
+          pc.head = pos == 0;
+          if (n != len) {
+            const int s0 = cut.span_of(x - pos);
+            pc.pieces = cut.span_of(x - pos + len - 1) - s0 + 1;
+            pc.first = member * cut.spans + s0;
+          }
+          mbar_arrive(bar_pc_full + 8 * slot);
+        }
+        ++pcnt;
+        x += n;
+      } else {
+        if (first_ticket) w = (int)blockIdx.x;     // a CTA's first work id is its block index, later ones are tickets
+        else if (lane == 0) w = (int)gridDim.x + atomicAdd(p.counters, 1);
+        if (!first_ticket) w = __shfl_sync(0xffffffffu, w, 0);
+        first_ticket = false;
+        if (w >= total_work) break;
+        it = decode_work(p, w);
+        if (it.bad) {
+          if (lane == 0) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
+          break;
+        }
+        if (!it.valid) continue;
       }
-      if (!it.valid) continue;
       if (it.lo >= it.hi) {   // nothing to stream: one descriptor-only stage so that the output still gets written
         const uint32_t s = cnt % NST;
         ok = wait_or_abort(bar_empty + 8 * s, ((cnt / NST) & 1) ^ 1, s_abort);
@@ -335,7 +519,14 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       }
     }
     if (!ok) { if (lane == 0) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_PRODUCER); s_abort[0] = 1; } }
-    if (ok) {   // end-of-stream marker
+    if (BAL && ok) {
+      const uint32_t slot = pcnt % kPieces;
+      if (wait_or_abort(bar_pc_empty + 8 * slot, ((pcnt / kPieces) & 1) ^ 1, s_abort) && lane == 0) {
+        s_piece[slot].it.b = -1;
+        mbar_arrive(bar_pc_full + 8 * slot);
+      }
+    }
+    if (!BAL && ok) {   // end-of-stream marker
       const uint32_t s = cnt % NST;
       if (wait_or_abort(bar_empty + 8 * s, ((cnt / NST) & 1) ^ 1, s_abort)) {
         if (lane == 0) s_info[4 * s] = -1;
@@ -347,7 +538,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     if (lane == 0) {
       for (uint32_t s = 0; s < (uint32_t)NST; ++s)
         if (cnt > s) wait_or_abort(bar_full + 8 * s, ((cnt - 1 - s) / NST) & 1, s_abort + 1);
-      counters_release(p.counters);   // this CTA takes no more tickets
+      if constexpr (!BAL) counters_release(p.counters);   // this CTA takes no more tickets
     }
   } else {
     // ============================================ consumers ===========================================
@@ -359,21 +550,42 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     float qs_a = 1.f, qs_b = 1.f;   // e4m3 Q: 1 / (row quantisation scale), folded into the logit scale
     float o[HDV / 8][4];
     float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
-    float lr_a = 0.f, lr_b = 0.f;   // e4m3 cache: sums of the ROUNDED probabilities (normalise O); l_* stay exact for the LSE
     int lo_a = 0, hi_a = -1, lo_b = 0, hi_b = -1, lo_max = 0, hi_min = -1;
     float c_mul = 0.f, cap_in = 0.f, vds = 1.f;
-    WorkItem it{};
+    WorkItem it_reg{};
+    uint32_t pcnt = 0;
     const bool has_cap = p.softcap > 0.f;
 
+    int bal_key = 0, bal_flags = F_LAST;     // balanced kernels: position inside the piece
     while (true) {
       const uint32_t s = cnt % NST;
-      ok = wait_or_abort(bar_full + 8 * s, (cnt / NST) & 1, s_abort);
-      if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_CONSUMER); s_abort[0] = 1; break; }
-      const int4 info = make_int4(s_info[4 * s], s_info[4 * s + 1], s_info[4 * s + 2], 0);
-      if (info.x < 0) break;
-      const int key0 = info.y, flags = info.z;
+      // balanced kernels: the piece stays in its mailbox slot until its rows are written
+      const Piece& cur = s_piece[pcnt % kPieces];
+      const WorkItem& it = BAL ? cur.it : it_reg;
+      int key0, flags, wid = 0;
+      if constexpr (BAL) {
+        if (bal_flags & F_LAST) {
+          ok = wait_or_abort(bar_pc_full + 8 * (pcnt % kPieces), (pcnt / kPieces) & 1, s_abort);
+          if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_CONSUMER); s_abort[0] = 1; break; }
+          if (cur.it.b < 0) break;
+          bal_flags = F_FIRST;
+          if (cur.it.lo >= cur.it.hi) bal_flags |= F_EMPTY;
+          bal_key = cur.it.lo * TN;
+        } else {
+          bal_flags = 0;
+          bal_key += TNS;
+        }
+        if (bal_key + TNS >= cur.it.hi * TN) bal_flags |= F_LAST;
+        key0 = bal_key; flags = bal_flags;
+      } else {
+        ok = wait_or_abort(bar_full + 8 * s, (cnt / NST) & 1, s_abort);
+        if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_CONSUMER); s_abort[0] = 1; break; }
+        wid = s_info[4 * s];
+        if (wid < 0) break;
+        key0 = s_info[4 * s + 1]; flags = s_info[4 * s + 2];
+      }
       if (flags & F_FIRST) {
-        it = decode_work(p, info.x);
+        if constexpr (!BAL) it_reg = decode_work(p, wid);
         const int rows_total = it.seqlen_q * rep;
         // Q fragments straight from global memory (rows g and g+8 of the packed tile)
         if constexpr (!KV8) {
@@ -461,11 +673,15 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         if (p.is_causal) hi_min = min(hi_min, qp_lo);
         if (p.window_right >= 0) hi_min = min(hi_min, qp_lo + p.window_right);
         if (p.window_left >= 0) lo_max = max(lo_max, qp_hi - p.window_left);
-        m_a = m_b = -INFINITY; l_a = l_b = 0.f; lr_a = lr_b = 0.f;
+        m_a = m_b = -INFINITY; l_a = l_b = 0.f;
 #pragma unroll
         for (int i = 0; i < HDV / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
       }
 
+      if constexpr (BAL) {      // (the queries above are fetched while the first stage is on its way)
+        ok = wait_or_abort(bar_full + 8 * s, (cnt / NST) & 1, s_abort);
+        if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_CONSUMER); s_abort[0] = 1; break; }
+      }
       if (!(flags & F_EMPTY)) {
         const uint32_t kb = base + s * SM::kStage, vb = kb + SM::kKBytes;
         const int mat = lane >> 3, l7 = lane & 7;
@@ -542,7 +758,6 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         }
         l_a = l_a * corr_a + ps_a;
         l_b = l_b * corr_b + ps_b;
-        if constexpr (KV8) { lr_a = l_a; lr_b = l_b; }   // P is fp16: one sum serves the LSE and the normalisation
         if (__any_sync(0xffffffffu, corr_a != 1.f || corr_b != 1.f)) {
 #pragma unroll
           for (int i = 0; i < HDV / 8; ++i) { o[i][0] *= corr_a; o[i][1] *= corr_a; o[i][2] *= corr_b; o[i][3] *= corr_b; }
@@ -606,8 +821,6 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         // ---- merge the four warps' partial results and write the output rows ----
         l_a += __shfl_xor_sync(0xffffffffu, l_a, 1); l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
         l_b += __shfl_xor_sync(0xffffffffu, l_b, 1); l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-        lr_a += __shfl_xor_sync(0xffffffffu, lr_a, 1); lr_a += __shfl_xor_sync(0xffffffffu, lr_a, 2);
-        lr_b += __shfl_xor_sync(0xffffffffu, lr_b, 1); lr_b += __shfl_xor_sync(0xffffffffu, lr_b, 2);
         float* so = s_o + warp * 16 * SM::kLdO;
         if (!KV8) {
 #pragma unroll
@@ -627,7 +840,6 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         if (tq == 0) {
           s_m[warp * 16 + g] = m_a; s_m[warp * 16 + g + 8] = m_b;
           s_l[warp * 16 + g] = l_a; s_l[warp * 16 + g + 8] = l_b;
-          s_lr[warp * 16 + g] = lr_a; s_lr[warp * 16 + g + 8] = lr_b;
         }
         bar_consumers<NC>();
         {
@@ -639,14 +851,13 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           float mw[NC], M = -INFINITY;
 #pragma unroll
           for (int wi = 0; wi < NC; ++wi) { mw[wi] = s_m[wi * 16 + Rl]; M = fmaxf(M, mw[wi]); }
-          float L = 0.f, Lr = 0.f, acc[CPT];
+          float L = 0.f, acc[CPT];
 #pragma unroll
           for (int j = 0; j < CPT; ++j) acc[j] = 0.f;
 #pragma unroll
           for (int wi = 0; wi < NC; ++wi) {
             const float e = mw[wi] == -INFINITY ? 0.f : ex2(mw[wi] - M);
             L += e * s_l[wi * 16 + Rl];
-            Lr += e * s_lr[wi * 16 + Rl];
             const float* src = s_o + (wi * 16 + Rl) * SM::kLdO + c0;
 #pragma unroll
             for (int j = 0; j < CPT; j += 4) {
@@ -654,12 +865,77 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
               acc[j] += e * v4.x; acc[j + 1] += e * v4.y; acc[j + 2] += e * v4.z; acc[j + 3] += e * v4.w;
             }
           }
-          if (R < rows_total) {
+          bool is_piece = false;
+          if constexpr (BAL) is_piece = cur.pieces > 1;
+          if (BAL && is_piece) {
+            if constexpr (BAL) {
+              // one piece: rows as they are, with their maximum and sum; the CTA that arrives last merges
+              const int64_t slot = (int64_t)cur.number * 2 + cur.head;
+              if (R < rows_total && Rl < p.part_rows) {
+                float* po = p.part_o + (slot * p.part_rows + Rl) * HDV + c0;
+#pragma unroll
+                for (int j = 0; j < CPT; j += 4)
+                  *reinterpret_cast<float4*>(po + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+                if (tid % GPR == 0) reinterpret_cast<float2*>(p.part_ml)[slot * p.part_rows + Rl] = make_float2(M, L);
+              }
+              bar_consumers<NC>();       // (thread 0's fence then covers the rows of all four warps)
+              if (tid == 0) {
+                __threadfence();
+                unsigned* word = p.arrivals + cur.first;
+                const bool last = atomicAdd(word, 1u) == (unsigned)cur.pieces - 1u;
+                if (last) *word = 0u;        // zero again for the next call
+                __threadfence();
+                *s_last = last ? 1 : 0;
+              }
+              bar_consumers<NC>();
+              if (*s_last) {
+                const int live = min(p.part_rows, rows_total - it.mt * 16), np = cur.pieces;
+                const int64_t s0 = (int64_t)cur.first * 2;
+                for (int u = tid; u < live * (HDV / 4); u += NC * 32) {
+                  const int r = u / (HDV / 4), c4 = (u - r * (HDV / 4)) * 4;
+                  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + r;
+                  const float* pr = p.part_o + (int64_t)r * HDV + c4;
+                  // piece j lies in slot 2 (first + j) + (j == 0)
+                  float Mx = -INFINITY;
+#pragma unroll 8
+                  for (int j = 0; j < np; ++j) Mx = fmaxf(Mx, __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows).x);
+                  float Ls = 0.f;
+                  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                  if (Mx > -INFINITY) {
+#pragma unroll 8
+                    for (int j = 0; j < np; ++j) {
+                      const int64_t sl = (s0 + 2 * j + (j == 0)) * p.part_rows;
+                      const float2 q2 = __ldcg(ml + sl);
+                      const float4 w4 = __ldcg(reinterpret_cast<const float4*>(pr + sl * HDV));
+                      const float e = ex2(q2.x - Mx);      // (a piece without visible keys: exactly 0, its rows are 0)
+                      Ls += e * q2.y;
+                      v.x += e * w4.x; v.y += e * w4.y; v.z += e * w4.z; v.w += e * w4.w;
+                    }
+                  }
+                  const int Rg = it.mt * 16 + r, token = Rg / rep, head = it.hk * rep + Rg % rep;
+                  const int64_t qi = it.q0 + token;
+                  float osc = 1.f;
+                  if (p.s_aux) {
+                    const float ys = p.s_aux[head] * kLog2e, mn = fmaxf(Mx, ys);
+                    osc = Mx == -INFINITY ? 0.f : ex2(Mx - mn);
+                    Ls = Ls * osc + ex2(ys - mn);
+                    Mx = mn;
+                  }
+                  const float inv = Ls > 0.f ? osc * vds / Ls : 0.f;
+                  T* op = reinterpret_cast<T*>(p.out) + qi * p.o_row_stride + (int64_t)head * p.o_head_stride + c4;
+                  uint2 w2;
+                  w2.x = pack2<T>(v.x * inv, v.y * inv);
+                  w2.y = pack2<T>(v.z * inv, v.w * inv);
+                  *reinterpret_cast<uint2*>(op) = w2;
+                  if (c4 == 0) p.lse[(int64_t)head * p.total_q + qi] = Ls > 0.f ? (Mx + lg2(Ls)) * kLn2 : -INFINITY;
+                }
+              }
+            }
+          } else if (R < rows_total) {
             const int token = R / rep, head = it.hk * rep + R % rep;
             const int64_t qi = it.q0 + token;
-            if (p.nsplits > 1) {
-              const float Ln = KV8 ? Lr : L;   // e4m3: divide by the sum of the rounded probabilities
-              const float inv = Ln > 0.f ? vds / Ln : 0.f;
+            if (!BAL && p.nsplits > 1) {
+              const float inv = L > 0.f ? vds / L : 0.f;
               float* op = p.o_part + (((int64_t)it.split * p.total_q + qi) * p.hq + head) * p.hdv + c0;
 #pragma unroll
               for (int j = 0; j < CPT; j += 4)
@@ -673,11 +949,9 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
                 const float mn = fmaxf(M, ys);
                 osc = M == -INFINITY ? 0.f : ex2(M - mn);
                 L = L * osc + ex2(ys - mn);
-                Lr = Lr * osc + ex2(ys - mn);
                 M = mn;
               }
-              const float Ln = KV8 ? Lr : L;
-              const float inv = Ln > 0.f ? osc * vds / Ln : 0.f;
+              const float inv = L > 0.f ? osc * vds / L : 0.f;
               if (p.out_f32) {
                 float* of = reinterpret_cast<float*>(p.out) + qi * p.o_row_stride + (int64_t)head * p.o_head_stride + c0;
 #pragma unroll
@@ -698,6 +972,10 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           }
         }
         bar_consumers<NC>();   // the scratch area is free again
+        if constexpr (BAL) {
+          if (lane == 0) mbar_arrive(bar_pc_empty + 8 * (pcnt % kPieces));
+          ++pcnt;
+        }
       }
     }
   }
@@ -739,12 +1017,24 @@ static bool make_map(CUtensorMap* m, const void* ptr, int dtype, uint64_t rows, 
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename T, bool KV8, int NST, int HD, int HDV, int CPS = ctas_per_sm(KV8 ? 1 : 2), int TNS_ = 64>
+// Heads that walk the line together: the largest divisor of hkv, up to 16 (4 KB of every token), that leaves at most
+// one CTA in twenty without work.
+static int line_team(int hkv, int ctas) {
+  int team = 1;
+  for (int g = 2; g <= 16 && g <= ctas; ++g)
+    if (hkv % g == 0 && ctas / g * g * 20 >= ctas * 19) team = g;
+  return team;
+}
+
+template <typename T, bool KV8, int NST, int HD, int HDV, bool BAL, int CPS = ctas_per_sm(KV8 ? 1 : 2), int TNS_ = 64>
 static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaStream_t stream) {
   using SM = Smem<KV8 ? 1 : 2, NST, HD, HDV, TNS_>;
   DecArgs a;
   a.kp = kp;
   a.total_work = num_work_slots * kp.hkv * kp.nsplits;
+  a.use_list = kp.work != nullptr;
+  a.max_mtiles = pl.max_mtiles;
+  a.class_rows = kp.class_rows;
   constexpr int TNS = SM::TNS;
   const bool paged = kp.page_table != nullptr;
   // (the cp.async producer takes any power-of-two page; measured, pages of 8 and 16 keys are faster as TMA boxes:
@@ -760,8 +1050,8 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
   CUtensorMap mk, mv;
   if (!make_map(&mk, kp.k, kvdt, rows, (uint64_t)kp.hkv * HD, (uint64_t)kp.k_row_stride, a.box_rows)) return -1;
   if (!make_map(&mv, kp.v, kvdt, rows, (uint64_t)kp.hkv * HDV, (uint64_t)kp.v_row_stride, a.box_rows)) return -1;
-  auto kern = fwd_decode_kernel<T, KV8, NST, HD, HDV, CPS, TNS_>;
-  const int smem = SM::kBytes + 1024;
+  auto kern = fwd_decode_kernel<T, KV8, NST, HD, HDV, CPS, TNS_, BAL>;
+  const int smem = (BAL ? SM::kBytesBalanced : SM::kBytes) + 1024;
   static std::atomic<unsigned long long> attr_done{0};   // one bit per device
   int dev = 0;
   cudaGetDevice(&dev);
@@ -772,6 +1062,13 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
   }
   const int ctas = pl.num_sms * CPS;
   int grid = a.total_work < ctas ? a.total_work : ctas;
+  if constexpr (BAL) {
+    a.team = line_team(kp.hkv, ctas);      // (8 heads: 18 teams, 144 of 148 SMs)
+    // no more CTAs than spans of the least length there can be (from the longest sequence; the kernel knows better)
+    const long long blocks = (long long)num_work_slots * (kp.hkv / a.team) * ((kp.max_seqlen_k + TN - 1) / TN + 1);
+    const long long spans = (blocks + kMinSpan - 1) / kMinSpan;
+    grid = (int)(spans < ctas / a.team ? spans : ctas / a.team) * a.team;
+  }
   if (grid <= 0) return 0;
   kern<<<grid, (SM::NC + 1) * 32, smem, stream>>>(a, mk, mv);
   return (int)cudaGetLastError();
@@ -783,6 +1080,11 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
 // (head_dim 128) of e4m3 bytes, K/V contiguous or in pages of 1, 2, 4, 8, 16, 32 or a multiple of 64 keys (the small
 // pages row by row, as the reference's cp.async producer does for page size 1, kernels/fa4_blackwell.cu:8936-8947).  These are the
 // head dims of the reference's paged kernel (kernels/fa4_blackwell.cu:9958-9983).
+// CTAs of a balanced launch at most: each has scratch for two pieces and one arrival counter.
+int decode_line_ctas(int hd, int kv_dtype, int num_sms) {
+  return num_sms * (hd == 64 || kv_dtype == FA_DT_FP8_E4M3 ? 2 : 1);
+}
+
 bool decode_supported(const PlanInput& in) {
   if (in.q_dtype == FA_DT_FP8_E4M3) return false;
   if (in.kv_dtype != in.q_dtype && in.kv_dtype != FA_DT_FP8_E4M3) return false;
@@ -796,21 +1098,24 @@ bool decode_supported(const PlanInput& in) {
   return in.hkv > 0 && in.hq % in.hkv == 0 && in.tc_layout_ok;
 }
 
-template <typename T>
+template <typename T, bool BAL>
 static int launch_decode_t(const KParams& kp, const Plan& pl, int slots, cudaStream_t stream) {
   // e4m3 cache: 128-key stages (32 keys = two independent 16-key chains per consumer warp: the chains hide each
   // other's fixed latencies; 0.80 -> 0.92 of the HBM peak against 64-key stages), two stages, two CTAs per SM
-  if (kp.kv_fp8) return dec::launch_t<T, true, 2, 128, 128, 2, 128>(kp, pl, slots, stream);
-  if (kp.hd == 64) return dec::launch_t<T, false, 5, 64, 64, 2>(kp, pl, slots, stream);   // 16 KB stages: two CTAs per SM
-  if (kp.hd == 192) return dec::launch_t<T, false, 4, 192, 128>(kp, pl, slots, stream);
-  return dec::launch_t<T, false, 5, 128, 128>(kp, pl, slots, stream);
+  if (kp.kv_fp8) return dec::launch_t<T, true, 2, 128, 128, BAL, 2, 128>(kp, pl, slots, stream);
+  if (kp.hd == 64) return dec::launch_t<T, false, 5, 64, 64, BAL, 2>(kp, pl, slots, stream);   // 16 KB stages: two CTAs per SM
+  if (kp.hd == 192) return dec::launch_t<T, false, 4, 192, 128, BAL>(kp, pl, slots, stream);
+  return dec::launch_t<T, false, 5, 128, 128, BAL>(kp, pl, slots, stream);
 }
 
 int launch_decode(const KParams& kp, const Plan& pl, int compute_dtype, cudaStream_t stream) {
   // every (batch, m_tile) slot of the metadata may hold a work entry
   const int slots = kp.batch * pl.max_mtiles;
-  return compute_dtype != FA_DT_FP16 ? launch_decode_t<__nv_bfloat16>(kp, pl, slots, stream)
-                                     : launch_decode_t<__half>(kp, pl, slots, stream);
+  if (kp.part_o != nullptr)
+    return compute_dtype != FA_DT_FP16 ? launch_decode_t<__nv_bfloat16, true>(kp, pl, slots, stream)
+                                       : launch_decode_t<__half, true>(kp, pl, slots, stream);
+  return compute_dtype != FA_DT_FP16 ? launch_decode_t<__nv_bfloat16, false>(kp, pl, slots, stream)
+                                     : launch_decode_t<__half, false>(kp, pl, slots, stream);
 }
 
 }  // namespace fa

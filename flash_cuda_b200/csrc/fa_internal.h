@@ -10,6 +10,13 @@ namespace fa {
 
 struct DeviceStatus;
 
+// The front of the workspace that is zero whenever no call runs: status word at 0, work counters at 64, and (balanced
+// decode) arrival counters from 256 on.
+constexpr int kWsHeader = 4096;
+constexpr int kWsArrivalOff = 256;
+constexpr int kWsArrivalWords = (kWsHeader - kWsArrivalOff) / 4;
+constexpr int kBalancedEntriesMax = 2048;   // (sequence, row tile) entries a balanced decode call may have
+
 // Kernel-side view of one problem: FaFwdParams plus what the planner derived.
 struct KParams {
   const void* q;
@@ -19,6 +26,9 @@ struct KParams {
   float* lse;
   float* o_part;      // (nsplits, total_q, hq, hdv) fp32 when nsplits > 1
   float* lse_part;    // (nsplits, hq, total_q) fp32 when nsplits > 1
+  float* part_o;      // balanced decode: rows of cut pieces (fa_decode.cu), else null
+  float* part_ml;     //                  their (maximum, sum) pairs
+  uint32_t* arrivals; //                  one counter per CTA, zero at kernel start and again when it ends
   const int32_t* cu_q;
   const int32_t* cu_k;
   const int32_t* seqused_k;
@@ -44,6 +54,8 @@ struct KParams {
   int32_t q_fp8, kv_fp8;
   int32_t is_causal, window_left, window_right;
   int32_t nsplits;
+  int32_t part_rows;   // balanced decode: rows of a piece
+  int32_t class_rows;  // balanced decode: > 0 = only sequences with at most this many packed query rows
   int32_t out_f32;     // `out` is fp32 (FA_DT_FP32) instead of the 16-bit type of the kernel
   float scale;         // softmax_scale
   float softcap;       // 0 = off

@@ -53,7 +53,7 @@ const EnvConfig& env_config() {
   return cfg;
 }
 
-// Scratch for fa_b200_fwd, kept per (device, stream) and reused: its 256-byte header is zeroed once when the
+// Scratch for fa_b200_fwd, kept per (device, stream) and reused: its 4 KB header is zeroed once when the
 // buffer is made and every call leaves it zero again (FA_FLAG_WORKSPACE_CLEAN), so a call costs neither an
 // allocation nor a memset.  Calls on one stream run one after the other, which is what sharing a buffer needs.
 // Requests above kCacheLimit are served by a plain allocation instead.
@@ -300,7 +300,7 @@ std::vector<at::Tensor> mha_fwd(
   auto stream = at::cuda::getCurrentCUDAStream();
   bool clean = false;
   at::Tensor ws = cached_workspace(q, stream.stream(), (int64_t)ws_bytes, &clean);
-  if (clean) p.flags |= FA_FLAG_WORKSPACE_CLEAN;
+  if (clean) p.flags |= FA_FLAG_WORKSPACE_CLEAN | FA_FLAG_WORKSPACE_CLEAN_4K;
   const int rc = fa_b200_fwd(&p, ws.data_ptr(), (size_t)ws.numel(), (fa_stream_t)stream.stream());
   if (rc == FA_ERR_UNSUPPORTED) {
     TORCH_CHECK(false, "fa_b200: unsupported config (hd=", p.hd, " hdv=", p.hdv, " paged=", paged,

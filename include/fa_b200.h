@@ -43,7 +43,10 @@ enum {
   /* The caller promises that the first 256 bytes of `workspace` are zero when the call runs on its stream:
    * zeroed once after allocation and since then used only by this library, one call at a time (every
    * successful call leaves them zero again).  The library then issues no memset for them. */
-  FA_FLAG_WORKSPACE_CLEAN = 1
+  FA_FLAG_WORKSPACE_CLEAN = 1,
+  /* The same promise for the first 4096 bytes (with FA_FLAG_WORKSPACE_CLEAN): decode calls then need no memset for
+   * their arrival counters either. */
+  FA_FLAG_WORKSPACE_CLEAN_4K = 2
 };
 
 /* Which kernel family to use. AUTO routes by shape; the others force one family (testing, A/B). */
@@ -210,7 +213,7 @@ int fa_b200_selftest_timeout(void* workspace, int64_t max_cycles, fa_stream_t st
  * (status word, work counter, work list, split partials) living in an array compiled into this library
  * instead of a caller-supplied workspace.  The caller still passes inputs and outputs in `p`.
  *   - The array is FA_B200_STATIC_SCRATCH_BYTES (8 MiB) per GPU, held by every GPU that loads the library
- *     until the process exits.  A problem whose scratch (fa_b200_fwd_workspace_bytes) exceeds it returns
+ *     until the process exits.  A problem whose work list and partial results exceed it returns
  *     FA_ERR_STATIC_LIMIT; a shape the decode route does not take returns FA_ERR_UNSUPPORTED.
  *   - The first call on each device looks the array's device address up (with that device current); make that
  *     first call before any stream capture begins.

@@ -1,0 +1,59 @@
+"""The balanced decode kernel: spans of key blocks that cross sequences, pieces merged by the CTA that finishes last.
+Against the CPU oracle with the benchmark's tolerances (16-bit 2e-2, e4m3 cache 6e-2, LSE 5e-3) and against the uncut
+form of the same call (num_splits = 1)."""
+import pytest
+import torch
+
+from flash_cuda_b200 import capi, ops, workloads as W
+from oracle.ref_attention import ref_attention
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(p, dev, tol, check_ref=True, **kw):
+    pd = p.to(dev)
+    out, lse, _ = capi.fwd(pd.q, pd.k, pd.v, check=True, **dict(pd.capi_kw(), **kw))
+    assert torch.isfinite(out.float()).all(), p.name
+    if check_ref:
+        ref_out, ref_lse = ref_attention(p.q, p.k, p.v, **p.oracle_kw())
+        assert (out.float().cpu() - ref_out).abs().max().item() <= tol, p.name
+        fin = torch.isfinite(ref_lse)
+        assert torch.equal(torch.isfinite(lse.cpu()), fin), p.name
+        torch.testing.assert_close(lse.cpu()[fin], ref_lse[fin], atol=5e-3, rtol=1e-2)
+    return out, lse
+
+
+DECODE = {   # (q_len, k_len) per sequence and options: one key; a border of a block and of a span; more sequences than
+             # CTAs; one long sequence among short ones; several row tiles; keyless and rowless sequences; one kv head
+    "one_key": ([(1, 1)], dict(hq=8, hkv=2, hd=128, page_size=16)),
+    "block_borders": ([(1, 63), (1, 64), (1, 65), (1, 255), (1, 257)], dict(hq=32, hkv=8, hd=128, page_size=64)),
+    "many": ([(1, 1 + 37 * i % 700) for i in range(200)], dict(hq=8, hkv=4, hd=128, page_size=32)),
+    "one_long": ([(1, 30000), (1, 5), (1, 700), (1, 1)], dict(hq=8, hkv=2, hd=128, page_size=64, sink=True)),
+    "row_tiles": ([(13, 5000), (16, 900), (1, 3000), (4, 4)], dict(hq=8, hkv=2, hd=64, page_size=16, window_left=700)),
+    "empty": ([(1, 0), (0, 500), (1, 900), (2, 0), (0, 0)], dict(hq=4, hkv=4, hd=128, page_size=64, sink=True)),
+    "one_head": ([(8, 9000), (8, 100)], dict(hq=8, hkv=1, hd=192, hdv=128, page_size=1)),
+    "odd_heads": ([(1, 6000), (1, 3000)], dict(hq=15, hkv=5, hd=128, page_size=128, softcap=20.0)),
+    "leftpad": ([(1, 4100), (1, 300)], dict(hq=8, hkv=2, hd=128, page_size=64, leftpad=[60, 290])),
+    "contiguous": ([(1, 7000), (1, 130)], dict(hq=16, hkv=16, hd=64, page_size=0)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(DECODE))
+@pytest.mark.parametrize("dtype,kv_dtype", [("bf16", None), ("fp16", None), ("bf16", "fp8")])
+def test_balanced_decode(name, dtype, kv_dtype, cuda_device):
+    reqs, kw = DECODE[name]
+    if kv_dtype and kw["hd"] != 128:
+        pytest.skip("the decode kernel takes an e4m3 cache at head_dim 128")
+    p = W.make_problem("bal_" + name, reqs, dtype=dtype, kv_dtype=kv_dtype, seed=91, **kw)
+    tol = 6e-2 if kv_dtype else 2e-2
+    out, lse = _run(p, cuda_device, tol)
+    uncut, uncut_lse = _run(p, cuda_device, tol, check_ref=False, num_splits=1)
+    assert (out.float() - uncut.float()).abs().max().item() <= 2 ** -7      # one rounding to 16 bits of |values| < 2
+    # the op keeps one workspace per stream: its counters must be zero again after every call, and the merge order
+    # does not depend on which CTA took which span
+    pd = p.to(cuda_device)
+    first, first_lse = ops.call_fwd(pd.q, pd.k, pd.v, **pd.capi_kw())
+    for _ in range(3):
+        again, again_lse = ops.call_fwd(pd.q, pd.k, pd.v, **pd.capi_kw())
+        assert torch.equal(first, again) and torch.equal(first_lse, again_lse)
+    assert torch.equal(first, out)
