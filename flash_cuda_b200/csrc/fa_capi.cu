@@ -171,6 +171,7 @@ static PlanInput plan_input(const FaSchedParams* p, int num_sms) {
 static bool mixed_batch(const FaFwdParams* p, const PlanInput& in, const Plan& pl) {
   if (p->route != FA_ROUTE_AUTO || pl.route != FA_ROUTE_PREFILL_TC || p->scheduler_metadata != nullptr) return false;
   if (p->batch < 2 || !decode_supported(in) || p->out_dtype == FA_DT_FP32) return false;
+  if ((long long)p->batch * pl.max_mtiles > kSchedSortMax) return false;   // (the filtered lists are sorted lists)
   return (long long)p->total_q * 4 < (long long)p->batch * p->max_seqlen_q;
 }
 static Plan decode_part_plan(const PlanInput& in, const Plan& pl) {
@@ -225,6 +226,8 @@ static bool depage_plan(const FaFwdParams* p, const Plan& pl, int* kpad, size_t*
   if (!(ps == 1 || ps == 2 || ps == 4 || ps == 8 || ps == 16)) return false;
   if ((long long)ceil_div(p->max_seqlen_q, 256) * (p->hq / p->hkv) < 4) return false;
   const size_t esz = p->kv_dtype == FA_DT_FP8_E4M3 ? 1 : 2;
+  // (16-byte copies: 8-bit rows may start at a multiple of 8 bytes, which the tensor maps refuse as well)
+  if (p->k_row_stride * (int64_t)esz % 16 || p->v_row_stride * (int64_t)esz % 16) return false;
   const size_t rows = (size_t)p->batch * (size_t)((p->max_seqlen_k + 127) / 128 * 128);
   const size_t kb = rows * p->hkv * p->hd * esz, vb = rows * p->hkv * p->hdv * esz;
   if (kb + vb > kDepageMaxBytes) return false;
@@ -232,6 +235,35 @@ static bool depage_plan(const FaFwdParams* p, const Plan& pl, int* kpad, size_t*
   *k_bytes = align_up(kb, 256);
   *v_bytes = align_up(vb, 256);
   return true;
+}
+
+// Key-range parts per work item of the tensor-core prefill kernel (1 = none), from a model of its time: items of
+// `tile_m` rows run in whole waves over the SMs, 1.8 us per key block of 2 x 128 rows at 256 columns; parts leave as
+// fp32 and are merged (a launch, and 8 bytes per row and column through memory).  A chunk of 512 rows over 24500
+// keys has 64 items for 148 SMs.  Taken where the model says a tenth is saved.
+static int tc_splits(const FaFwdParams* p, const PlanInput& in, const Plan& pl) {
+  if (pl.route != FA_ROUTE_PREFILL_TC || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 || p->total_q <= 0) return 1;
+  const long long n = (long long)p->hq * ceil_div(p->total_q, pl.tile_m);
+  if (n >= 2 * pl.num_sms || p->hdv % 4) return 1;
+  // (max_seqlen_k may be a loose bound: a packed K/V says how many keys a sequence has on average)
+  double keys = p->max_seqlen_k;
+  if (!p->page_table && (double)p->total_k / p->batch < keys) keys = (double)p->total_k / p->batch;
+  if (p->page_table && (double)p->num_pages * p->page_size < keys) keys = (double)p->num_pages * p->page_size;
+  double blocks = (keys - (in.is_causal ? 0.5 * (p->max_seqlen_q < keys ? p->max_seqlen_q : keys) : 0.0)) / 128.0;
+  if (in.window_left >= 0 && (in.is_causal || in.window_right >= 0)) {
+    const double w = (in.window_left + (in.window_right > 0 ? in.window_right : 0) + pl.tile_m) / 128.0 + 1.0;
+    if (w < blocks) blocks = w;
+  }
+  const double t_block = 1.8 * (p->hd + p->hdv) / 256.0 * pl.tile_m / 256.0;
+  const double part_us = (double)p->total_q * p->hq * p->hdv * 8.0 / 4.0e6;
+  double best = 0.9 * (double)((n + pl.num_sms - 1) / pl.num_sms) * blocks * t_block;
+  int s = 1;
+  for (int c = 2; c <= 16 && blocks / c >= 4.0; ++c) {
+    if ((size_t)c * p->total_q * p->hq * (p->hdv + 1) * 4 > ((size_t)128 << 20)) break;
+    const double t = (double)((n * c + pl.num_sms - 1) / pl.num_sms) * (blocks / c * t_block + 1.5) + 4.0 + c * part_us;
+    if (t < best) { best = t; s = c; }
+  }
+  return s;
 }
 
 // ---- workspace layout ----
@@ -243,6 +275,7 @@ struct WsLayout {
   size_t work2_off, work2_bytes;   // mixed batches: the prefill kernel's list
   size_t lse_off, lse_bytes;
   size_t o_off, o_bytes;
+  int tc_splits;      // tensor-core prefill: key-range parts per item; their partials lie at lse_off / o_off
   PartPlan parts;
   size_t part_ml_off, part_o_off;   // balanced decode: pieces of cut (sequence, head) triples; part_o_off 0: none
   size_t total;
@@ -258,6 +291,15 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
     w.part_o_off = off;
     off += w.parts.o_bytes;
   };
+  auto carve_splits = [&](int nsplits) {
+    w.lse_off = off;
+    w.lse_bytes = align_up((size_t)nsplits * p->hq * p->total_q * 4, 256);
+    off += w.lse_bytes;
+    w.o_off = off;
+    w.o_bytes = align_up((size_t)nsplits * p->total_q * p->hq * p->hdv * 4, 256);
+    off += w.o_bytes;
+  };
+  w.tc_splits = 1;
   if (balanced_decode(p, pl)) {
     carve_parts(pl);
     w.total = off;
@@ -298,14 +340,9 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
       off += vb;
     }
   }
-  if (pl.nsplits > 1) {
-    w.lse_off = off;
-    w.lse_bytes = align_up((size_t)pl.nsplits * p->hq * p->total_q * 4, 256);
-    off += w.lse_bytes;
-    w.o_off = off;
-    w.o_bytes = align_up((size_t)pl.nsplits * p->total_q * p->hq * p->hdv * 4, 256);
-    off += w.o_bytes;
-  }
+  if (pl.route == FA_ROUTE_PREFILL_TC)
+    w.tc_splits = tc_splits(p, plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0)), pl);
+  if (pl.nsplits > 1 || w.tc_splits > 1) carve_splits(pl.nsplits > 1 ? pl.nsplits : w.tc_splits);
   w.total = off;
   return w;
 }
@@ -467,6 +504,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   kp.q_fp8 = p->q_dtype == FA_DT_FP8_E4M3; kp.kv_fp8 = p->kv_dtype == FA_DT_FP8_E4M3;
   kp.is_causal = in.is_causal; kp.window_left = in.window_left; kp.window_right = in.window_right;
   kp.nsplits = pl.nsplits;
+  kp.tc_splits = 1;
   kp.out_f32 = p->out_dtype == FA_DT_FP32;
   kp.work_expect = SchedExpect{p->batch, pl.nsplits, pl.tile_m, pl.tile_n, pl.max_mtiles, pl.rows_per_token, pl.route};
   kp.scale = p->softmax_scale; kp.softcap = p->softcap;
@@ -475,18 +513,46 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     kp.arrivals = (uint32_t*)(ws + kWsArrivalOff);
     kp.part_rows = w.parts.rows;
   }
-  else if (pl.nsplits > 1) { kp.lse_part = (float*)(ws + w.lse_off); kp.o_part = (float*)(ws + w.o_off); }
+  if (pl.nsplits > 1 && !balanced) { kp.lse_part = (float*)(ws + w.lse_off); kp.o_part = (float*)(ws + w.o_off); }
 
   const int compute_dtype = p->q_dtype == FA_DT_FP16 ? FA_DT_FP16 : FA_DT_BF16;
+
+  FaSchedParams sp{};
+  sp.seqused_k = p->seqused_k; sp.cu_seqlens_q = p->cu_seqlens_q; sp.cu_seqlens_k = p->cu_seqlens_k;
+  sp.leftpad_k = p->leftpad_k; sp.batch = p->batch; sp.max_seqlen_q = p->max_seqlen_q;
+  sp.max_seqlen_k = p->max_seqlen_k; sp.hq = p->hq; sp.hkv = p->hkv; sp.hd = p->hd; sp.hdv = p->hdv;
+  sp.is_causal = in.is_causal; sp.window_left = in.window_left; sp.window_right = in.window_right;
+
+  // the tensor-core kernel over `kt`, in key-range parts with their merge where the plan says so (the merge writes
+  // every row of the call: what other kernels of the call own is launched after it)
+  auto run_prefill = [&](KParams kt, const Plan& plt) -> int {
+    if (w.tc_splits <= 1) return note_cuda_error(launch_prefill_tc(kt, plt, compute_dtype, stream), "tcgen05 prefill kernel");
+    float* o_part = (float*)(ws + w.o_off);
+    float* lse_part = (float*)(ws + w.lse_off);
+    kt.tc_splits = w.tc_splits;
+    kt.out = o_part; kt.lse = lse_part; kt.out_f32 = 1; kt.s_aux = nullptr;
+    kt.o_row_stride = (int64_t)p->hq * p->hdv; kt.o_head_stride = p->hdv;
+    kt.o_split_stride = (int64_t)p->total_q * p->hq * p->hdv;
+    kt.lse_split_stride = (int64_t)p->hq * p->total_q;
+    int r = note_cuda_error(launch_prefill_tc(kt, plt, compute_dtype, stream), "tcgen05 prefill kernel");
+    if (r != FA_OK) return r;
+    return note_cuda_error(launch_combine(o_part, lse_part, w.tc_splits, p->total_q, p->hq, p->hdv, p->s_aux, p->out,
+                                          p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream), "combine kernel");
+  };
+  // the decode kernel over the short sequences of a batch that also holds long ones
+  auto run_short = [&](const int32_t* list) -> int {
+    const Plan pd = decode_part_plan(in, pl);
+    KParams kd = kp;
+    kd.work = list;
+    kd.class_rows = kDecodeMaxRows;
+    kd.nsplits = 1;
+    kd.work_expect = SchedExpect{p->batch, 1, pd.tile_m, pd.tile_n, pd.max_mtiles, pd.rows_per_token, pd.route};
+    return note_cuda_error(launch_decode(kd, pd, compute_dtype, stream), "decode kernel");
+  };
 
   if (pl.route == FA_ROUTE_DECODE) {
     const int32_t* work = p->scheduler_metadata;
     if (!work && !balanced) {
-      FaSchedParams sp{};
-      sp.seqused_k = p->seqused_k; sp.cu_seqlens_q = p->cu_seqlens_q; sp.cu_seqlens_k = p->cu_seqlens_k;
-      sp.leftpad_k = p->leftpad_k; sp.batch = p->batch; sp.max_seqlen_q = p->max_seqlen_q;
-      sp.max_seqlen_k = p->max_seqlen_k; sp.hq = p->hq; sp.hkv = p->hkv; sp.hd = p->hd; sp.hdv = p->hdv;
-      sp.is_causal = in.is_causal; sp.window_left = in.window_left; sp.window_right = in.window_right;
       rc = note_cuda_error(launch_sched(sp, pl, (int32_t*)(ws + w.work_off), clean ? nullptr : (int32_t*)ws, stream),
                            "sched_kernel");
       if (rc != FA_OK) return rc;
@@ -495,27 +561,17 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     kp.work = work;
     rc = note_cuda_error(launch_decode(kp, pl, compute_dtype, stream), "decode kernel");
   } else if (pl.route == FA_ROUTE_PREFILL_TC && w.work2_bytes > 0) {
-    // mixed batch: two work lists, the decode kernel over the short sequences, then the prefill kernel over the rest
-    FaSchedParams sp{};
-    sp.seqused_k = p->seqused_k; sp.cu_seqlens_q = p->cu_seqlens_q; sp.cu_seqlens_k = p->cu_seqlens_k;
-    sp.leftpad_k = p->leftpad_k; sp.batch = p->batch; sp.max_seqlen_q = p->max_seqlen_q;
-    sp.max_seqlen_k = p->max_seqlen_k; sp.hq = p->hq; sp.hkv = p->hkv; sp.hd = p->hd; sp.hdv = p->hdv;
-    sp.is_causal = in.is_causal; sp.window_left = in.window_left; sp.window_right = in.window_right;
-    const Plan pd = decode_part_plan(in, pl);
-    int32_t* list_d = (int32_t*)(ws + w.work_off);
+    // mixed batch: the prefill kernel over its work list, the decode kernel over the short sequences
+    int32_t* list_d = balanced ? nullptr : (int32_t*)(ws + w.work_off);
     int32_t* list_p = (int32_t*)(ws + w.work2_off);
-    if (!balanced) rc = note_cuda_error(launch_sched(sp, pd, list_d, nullptr, stream, 1, kDecodeMaxRows), "sched_kernel");
+    if (!balanced)
+      rc = note_cuda_error(launch_sched(sp, decode_part_plan(in, pl), list_d, nullptr, stream, 1, kDecodeMaxRows), "sched_kernel");
     if (rc == FA_OK) rc = note_cuda_error(launch_sched(sp, pl, list_p, nullptr, stream, 2, kDecodeMaxRows), "sched_kernel");
     if (rc != FA_OK) return rc;
-    KParams kd = kp;
-    kd.work = balanced ? nullptr : list_d;
-    kd.class_rows = kDecodeMaxRows;
-    kd.nsplits = 1;
-    kd.work_expect = SchedExpect{p->batch, 1, pd.tile_m, pd.tile_n, pd.max_mtiles, pd.rows_per_token, pd.route};
-    rc = note_cuda_error(launch_decode(kd, pd, compute_dtype, stream), "decode kernel");
-    if (rc != FA_OK) return rc;
-    kp.work = list_p;
-    rc = note_cuda_error(launch_prefill_tc(kp, pl, compute_dtype, stream), "tcgen05 prefill kernel");
+    KParams kt = kp;
+    kt.work = list_p;
+    rc = run_prefill(kt, pl);
+    if (rc == FA_OK) rc = run_short(list_d);
   } else if (pl.route == FA_ROUTE_PREFILL_TC) {
     kp.work = p->scheduler_metadata;   // optional: the sorted (batch, tile) list replaces the arithmetic order
     if (w.dp_k_bytes > 0) {
@@ -532,7 +588,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
       kp.cu_k = cu;                              // slab b starts at row b * kpad; lengths still come from seqused_k
       kp.total_k = p->batch * w.dp_kpad;
     }
-    rc = note_cuda_error(launch_prefill_tc(kp, pl, compute_dtype, stream), "tcgen05 prefill kernel");
+    rc = run_prefill(kp, pl);
   } else {
     rc = note_cuda_error(launch_general(kp, compute_dtype, p->out_dtype, pl.num_sms, stream), "general kernel");
   }

@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
   float g = -INFINITY;
   const int64_t lse_idx = (int64_t)h * total_q + qi;
   const int64_t o_idx = (qi * hq + h) * hdv + dv;
+#pragma unroll 4
   for (int s = 0; s < nsplits; ++s) g = fmaxf(g, lse_part[s * lse_split_stride + lse_idx]);
   const bool has_sink = s_aux != nullptr;
   const float sk = has_sink ? s_aux[h] : -INFINITY;
@@ -45,13 +46,23 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
   }
   float L = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s = 0; s < nsplits; ++s) {
-    const float ls = lse_part[s * lse_split_stride + lse_idx];
-    if (ls > -INFINITY) {
-      const float w = ex2((ls - g) * kLog2eC);
-      const float4 o = *reinterpret_cast<const float4*>(o_part + s * o_split_stride + o_idx);
+  // four splits at a time, so that their loads are in flight together (the kernel is bound by memory latency: a thread
+  // has two dependent loads per split)
+  for (int s0 = 0; s0 < nsplits; s0 += 4) {
+    float ls[4];
+    float4 o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ls[j] = s0 + j < nsplits ? lse_part[(s0 + j) * lse_split_stride + lse_idx] : -INFINITY;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      o[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (ls[j] > -INFINITY) o[j] = *reinterpret_cast<const float4*>(o_part + (s0 + j) * o_split_stride + o_idx);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float w = ls[j] > -INFINITY ? ex2((ls[j] - g) * kLog2eC) : 0.f;
       L += w;
-      acc.x += w * o.x; acc.y += w * o.y; acc.z += w * o.z; acc.w += w * o.w;
+      acc.x += w * o[j].x; acc.y += w * o[j].y; acc.z += w * o[j].z; acc.w += w * o[j].w;
     }
   }
   if (has_sink) L += ex2((sk - g) * kLog2eC);

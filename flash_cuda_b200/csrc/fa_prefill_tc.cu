@@ -111,7 +111,7 @@ struct Smem {
 
 // One work item, decoded once by the TMA thread and handed to every role through shared memory (64 bytes).
 struct alignas(16) Item {
-  int b, h, pair, q0;
+  int b, h, pair, q0;   // h: head | key-range part << kPartShift (one word: the epilogue has no register for two)
   int seqlen_q, seqlen_k, k0, leftpad;
   int lo[2], hi[2];   // key-block range per tile
   int ulo, uhi;       // union
@@ -119,6 +119,7 @@ struct alignas(16) Item {
   int w;              // work id; kEndOfWork ends the role loops
 };
 static_assert(sizeof(Item) == 64, "mailbox slot");
+constexpr int kPartShift = 24, kHeadMask = (1 << kPartShift) - 1;
 
 template <int NTL>
 __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_entry) {
@@ -126,6 +127,13 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
   const KParams& p = a.kp;
   Item it;
   it.w = w;
+  // the key-range parts of an item are consecutive work ids
+  int part = 0;
+  if (p.tc_splits > 1) {
+    const int q = w / p.tc_splits;
+    part = w - q * p.tc_splits;
+    w = q;
+  }
   if (a.use_list) {
     // entry e of the sorted list = (batch, tile of item_rows rows); all q heads of one entry are consecutive work
     // ids, or (K/V larger than L2) the kv head is the slowest index and the list is walked once per kv head
@@ -183,6 +191,20 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
                    p.is_causal, p.window_left, p.window_right, TN, &it.lo[t], &it.hi[t]);
     }
     if (it.hi[t] > it.lo[t]) { it.ulo = min(it.ulo, it.lo[t]); it.uhi = max(it.uhi, it.hi[t]); }
+  }
+  if (p.tc_splits > 1 && it.valid) {
+    int plo, phi;
+    split_range(it.ulo, max(it.uhi, it.ulo), part, p.tc_splits, &plo, &phi);
+    it.ulo = 0x7fffffff;
+    it.uhi = 0;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      it.lo[t] = max(it.lo[t], plo);
+      it.hi[t] = min(it.hi[t], phi);
+      if (it.hi[t] > it.lo[t]) { it.ulo = min(it.ulo, it.lo[t]); it.uhi = max(it.uhi, it.hi[t]); }
+      else it.lo[t] = it.hi[t] = 0;
+    }
+    it.h |= part << kPartShift;
   }
   if (it.uhi <= it.ulo) { it.ulo = it.uhi = 0; }
   return it;
@@ -425,7 +447,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       int num_items = a.num_items;
       if (a.use_list) {
         if (sched_header_matches(p.work, p.work_expect)) {
-          num_items = p.work[6] * p.hq;
+          num_items = p.work[6] * p.hq * p.tc_splits;
         } else {
           if (leader) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_TMA);
           num_items = 0;
@@ -488,14 +510,14 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
             mbar_expect_tx(bar_q_full + 8 * t, TM * HD * ESZ);
 #pragma unroll
             for (int cb = 0; cb < HD / EPB; ++cb)
-              tma_load_3d(sQ + t * (TM * HD * ESZ) + cb * (TM * 128), &map_q, cb * EPB, it.h,
+              tma_load_3d(sQ + t * (TM * HD * ESZ) + cb * (TM * 128), &map_q, cb * EPB, it.h & kHeadMask,
                           it.q0 + it.pair * (NTL * TM) + t * TM, bar_q_full + 8 * t);
           }
           return true;
         };
         ok = load_q(0);
         if (!ok) { if (leader) report_error(p.status, DEV_ERR_TIMEOUT, ROLE_TMA); break; }
-        const int hk = it.h / p.rep;
+        const int hk = (it.h & kHeadMask) / p.rep;
         // one K or V tile of key block nb into `dst`, completing on `bar`
         const int pj0 = wide ? lane : 0, pjs = wide ? 32 : 1;
         // first row of this lane's first box and the distance to its next one
@@ -831,7 +853,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       const int row0 = it.pair * (NTL * TM) + t * TM;
       if (row0 >= it.seqlen_q) continue;           // this tile owns no row
       const int row = row0 + r;
-      const int hk = it.h / p.rep;
+      const int hk = (it.h & kHeadMask) / p.rep;
       float sc = p.scale, vds = 1.f;
       {
         const int di = it.b * p.descale_batch_stride + hk * p.descale_head_stride;
@@ -1153,9 +1175,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
               }
             }
           }
-        } else if (row_ok) {
+        } else if (row_ok && (had_blocks || p.tc_splits == 1)) {   // (the merge does not read an empty part's rows)
           if (p.out_f32) {
-            float* op = reinterpret_cast<float*>(p.out) + (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)it.h * p.o_head_stride;
+            float* op = reinterpret_cast<float*>(p.out) + (int64_t)(it.h >> kPartShift) * p.o_split_stride +
+                        (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(it.h & kHeadMask) * p.o_head_stride;
   #pragma unroll
             for (int c = 0; c < HDV / 32; ++c) {
               if (c * 32 < a.out_cols) {
@@ -1185,7 +1208,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           }
         }
         if (row_ok)
-          p.lse[(int64_t)it.h * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
+          p.lse[(int64_t)(it.h >> kPartShift) * p.lse_split_stride + (int64_t)(it.h & kHeadMask) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
       } else {
         // HDV > 128 (one tile per item): the O row is read 64 columns at a time; O_t is released as soon as its last
         // column has been read.  Each 64-column group leaves like a half row of the two-tile form: staged + one TMA
@@ -1256,9 +1279,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
                 bulk_commit_group();
               }
             }
-          } else if (row_ok) {
+          } else if (row_ok && (had_blocks || p.tc_splits == 1)) {
             if (p.out_f32) {
-              float* op = reinterpret_cast<float*>(p.out) + (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)it.h * p.o_head_stride + g * 64;
+              float* op = reinterpret_cast<float*>(p.out) + (int64_t)(it.h >> kPartShift) * p.o_split_stride +
+                        (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(it.h & kHeadMask) * p.o_head_stride + g * 64;
 #pragma unroll
               for (int c = 0; c < 2; ++c)
 #pragma unroll
@@ -1283,7 +1307,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           }
         }
         if (row_ok)
-          p.lse[(int64_t)it.h * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
+          p.lse[(int64_t)(it.h >> kPartShift) * p.lse_split_stride + (int64_t)(it.h & kHeadMask) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
       }
     }
     if constexpr (SM::kStageOut) {
@@ -1383,7 +1407,7 @@ static int launch_prod(const KParams& kp, const Plan& pl, int dtype, uint64_t kv
   a.kp = kp;
   a.item_rows = NTL * TM;
   a.max_pairs = (kp.max_seqlen_q + a.item_rows - 1) / a.item_rows;
-  a.num_items = kp.batch * kp.hq * a.max_pairs;
+  a.num_items = kp.batch * kp.hq * a.max_pairs * kp.tc_splits;
   a.use_list = kp.work != nullptr;
   // bytes of K and V the batch can touch, against the L2 capacity the tiles of concurrently running heads share
   {

@@ -1,6 +1,7 @@
-"""The balanced decode kernel: spans of key blocks that cross sequences, pieces merged by the CTA that finishes last.
-Against the CPU oracle with the benchmark's tolerances (16-bit 2e-2, e4m3 cache 6e-2, LSE 5e-3) and against the uncut
-form of the same call (num_splits = 1)."""
+"""Work that is cut along the keys: the balanced decode kernel (spans that cross sequences, pieces merged by the CTA
+that finishes last) and key-range parts of the tensor-core prefill kernel.  Each against the CPU oracle with the
+benchmark's tolerances (16-bit 2e-2, e4m3 cache 6e-2, LSE 5e-3) and against the uncut form of the same call
+(num_splits = 1)."""
 import pytest
 import torch
 
@@ -57,3 +58,26 @@ def test_balanced_decode(name, dtype, kv_dtype, cuda_device):
         again, again_lse = ops.call_fwd(pd.q, pd.k, pd.v, **pd.capi_kw())
         assert torch.equal(first, again) and torch.equal(first_lse, again_lse)
     assert torch.equal(first, out)
+
+
+PARTS = {    # few query tiles over many keys: the key range of an item goes to several CTAs
+    "chunk": ([(300, 9000)], dict(hq=8, hkv=2, hd=128, page_size=64)),
+    "chunk_packed": ([(130, 7000)], dict(hq=8, hkv=8, hd=128, page_size=0)),
+    "ragged": ([(200, 6000), (17, 900), (90, 6100)], dict(hq=8, hkv=2, hd=64, page_size=16, sink=True)),
+    "window": ([(400, 9000)], dict(hq=4, hkv=4, hd=128, page_size=128, window_left=5000, softcap=15.0)),
+    "hd192": ([(256, 8000)], dict(hq=4, hkv=4, hd=192, hdv=128, page_size=64)),
+    "hd256": ([(129, 5000)], dict(hq=4, hkv=2, hd=256, page_size=0, causal=False)),
+    "mixed": ([(1, 3000)] * 6 + [(200, 9000)], dict(hq=8, hkv=2, hd=128, page_size=64)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(PARTS))
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+def test_prefill_in_key_range_parts(name, dtype, cuda_device):
+    reqs, kw = PARTS[name]
+    p = W.make_problem("parts_" + name, reqs, dtype=dtype, seed=92, **kw)
+    out, lse = _run(p, cuda_device, 2e-2)
+    whole, whole_lse = _run(p, cuda_device, 2e-2, check_ref=False, num_splits=1)
+    assert not torch.equal(lse, whole_lse)                     # the call was cut
+    assert (out.float() - whole.float()).abs().max().item() <= 2 ** -7
+    torch.testing.assert_close(lse, whole_lse, atol=1e-4, rtol=1e-5)
