@@ -220,6 +220,146 @@ __global__ void __launch_bounds__(256) depage_kernel(const DepageArgs a) {
   }
 }
 
+// ------------------------------------------------------------------------------------------------------
+// Widening: the e4m3 keys and values of the sequences that the tensor-core prefill kernel is to take with 16-bit
+// queries, as 16-bit rows in contiguous slabs (exact: bf16 and fp16 hold every e4m3 value; the descales stay with the
+// attention kernel).  widen_plan_kernel lays the slabs out, `cap_rows` rows in all: sequence b gets the rows
+// [cu[b], cu[b + 1]), a multiple of 128, or none if it is short (at most class_rows packed query rows: the decode
+// kernel's) or does not fit any more; then take[b] = 1 and the general kernel runs it from the cache.
+// widen_kernel is bound by memory: 1 byte in and 2 out per element, 16 bytes per load.
+struct WidenArgs {
+  const unsigned char* k;
+  const unsigned char* v;
+  unsigned char* k_out;
+  unsigned char* v_out;
+  const int32_t* page_table;
+  const int32_t* seqused_k;
+  const int32_t* cu_k;
+  const int32_t* cu_q;
+  int32_t* cu;        // batch + 1
+  int32_t* take;      // batch + 1
+  int32_t* lens;      // batch: key counts (the slabs are padded, so their offsets do not say)
+  int64_t k_page, k_row, k_head, v_page, v_row, v_head;   // bytes
+  int batch, hkv, rep, class_rows, cap_rows, page_size, page_table_stride, k_chunks, v_chunks;   // 16-byte chunks per head
+};
+
+__device__ __forceinline__ int widen_len(const WidenArgs& a, int b) {
+  return a.seqused_k ? a.seqused_k[b] : a.cu_k[b + 1] - a.cu_k[b];
+}
+
+__global__ void __launch_bounds__(256) widen_plan_kernel(const WidenArgs a) {
+  __shared__ int s_warp[8];
+  __shared__ int s_run, s_left;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) { s_run = 0; s_left = 0; }
+  __syncthreads();
+  for (int b0 = 0; b0 < a.batch; b0 += 256) {
+    const int b = b0 + tid;
+    int need = 0;
+    bool mine = false;
+    if (b < a.batch) {
+      const int rows = (a.cu_q[b + 1] - a.cu_q[b]) * a.rep;
+      mine = rows > a.class_rows;
+      if (mine) need = min((max(widen_len(a, b), 0) + 127) / 128, 1 << 20) * 128;
+    }
+    // (in blocks of 128 rows, so that the sum of many long sequences stays far from 2^31)
+    const int blocks = need >> 7;
+    int incl = blocks;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int before = s_run;
+    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    const int cap = a.cap_rows >> 7;
+    const int at = before + incl - blocks, end = before + incl;
+    if (b < a.batch) {
+      const bool fits = end <= cap;
+      a.cu[b] = min(at, cap) << 7;
+      a.take[b] = mine && !fits ? 1 : 0;
+      a.lens[b] = widen_len(a, b);
+      if (mine && !fits) atomicAdd(&s_left, 1);
+    }
+    __syncthreads();
+    if (tid == 255) s_run = min(end, cap + 1);      // (past the capacity nothing fits, whatever the sum)
+    __syncthreads();
+  }
+  if (tid == 0) { a.cu[a.batch] = min(s_run, a.cap_rows >> 7) << 7; a.take[a.batch] = s_left; }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {
+  constexpr int RB = 8;                       // slab rows per turn (slabs are multiples of 128 rows)
+  const int rows = a.cu[a.batch];
+  const int kc = a.hkv * a.k_chunks, vc = a.hkv * a.v_chunks, rc = kc + vc;
+  for (int r0 = blockIdx.x * RB; r0 < rows; r0 += gridDim.x * RB) {
+    int lo = 0, hi = a.batch;                 // the sequence whose slab holds r0: the last one with cu[b] <= r0
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (a.cu[mid] <= r0) lo = mid; else hi = mid;
+    }
+    const int b = lo, s0 = r0 - a.cu[b];
+    if (a.take[b]) continue;                  // (what is left of the capacity before a sequence that did not fit)
+    const int used = widen_len(a, b);
+    const int first = a.page_table ? 0 : a.cu_k[b];
+    const int32_t* pt = a.page_table ? a.page_table + (int64_t)b * a.page_table_stride : nullptr;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < RB * rc; i += 256) {
+      const int rr = i / rc, c = i - rr * rc, r = s0 + rr;
+      const bool is_v = c >= kc;
+      const int cc = is_v ? c - kc : c, hch = is_v ? a.v_chunks : a.k_chunks;
+      const int h = cc / hch, w = cc - h * hch;
+      uint4 val = make_uint4(0u, 0u, 0u, 0u);
+      if (r < used) {
+        int64_t off;
+        if (pt) {
+          const int lp = r / a.page_size;
+          off = (int64_t)pt[lp] * (is_v ? a.v_page : a.k_page) + (int64_t)(r - lp * a.page_size) * (is_v ? a.v_row : a.k_row);
+        } else {
+          off = (int64_t)(first + r) * (is_v ? a.v_row : a.k_row);
+        }
+        off += (int64_t)h * (is_v ? a.v_head : a.k_head) + w * 16;
+        val = *reinterpret_cast<const uint4*>((is_v ? a.v : a.k) + off);
+      }
+      uint4 o0, o1;
+      e4m3x4_to<T>(val.x, o0.x, o0.y);
+      e4m3x4_to<T>(val.y, o0.z, o0.w);
+      e4m3x4_to<T>(val.z, o1.x, o1.y);
+      e4m3x4_to<T>(val.w, o1.z, o1.w);
+      uint4* dst = reinterpret_cast<uint4*>((is_v ? a.v_out + (int64_t)(r0 + rr) * vc * 32 : a.k_out + (int64_t)(r0 + rr) * kc * 32) +
+                                            (int64_t)cc * 32);
+      dst[0] = o0;
+      dst[1] = o1;
+    }
+  }
+}
+
+int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_rows, void* k_out, void* v_out, int32_t* cu,
+                 int32_t* take, int32_t* lens, int num_sms, cudaStream_t stream) {
+  if (kp.hd % 16 || kp.hdv % 16 || kp.batch <= 0) return (int)cudaErrorInvalidValue;
+  WidenArgs a;
+  a.k = reinterpret_cast<const unsigned char*>(kp.k);
+  a.v = reinterpret_cast<const unsigned char*>(kp.v);
+  a.k_out = reinterpret_cast<unsigned char*>(k_out);
+  a.v_out = reinterpret_cast<unsigned char*>(v_out);
+  a.page_table = kp.page_table; a.seqused_k = kp.seqused_k; a.cu_k = kp.cu_k; a.cu_q = kp.cu_q;
+  a.cu = cu; a.take = take; a.lens = lens;
+  a.k_page = kp.k_page_stride; a.k_row = kp.k_row_stride; a.k_head = kp.k_head_stride;
+  a.v_page = kp.v_page_stride; a.v_row = kp.v_row_stride; a.v_head = kp.v_head_stride;
+  a.batch = kp.batch; a.hkv = kp.hkv; a.rep = kp.rep; a.class_rows = class_rows; a.cap_rows = cap_rows;
+  a.page_size = kp.page_size; a.page_table_stride = kp.page_table_stride;
+  a.k_chunks = kp.hd / 16; a.v_chunks = kp.hdv / 16;
+  widen_plan_kernel<<<1, 256, 0, stream>>>(a);
+  int blocks = (cap_rows + 7) / 8;
+  if (blocks > num_sms * 8) blocks = num_sms * 8;
+  if (compute_dtype == FA_DT_FP16) widen_kernel<__half><<<blocks, 256, 0, stream>>>(a);
+  else widen_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(a);
+  return (int)cudaGetLastError();
+}
+
 int launch_depage(const KParams& kp, int kpad, void* k_out, void* v_out, int32_t* cu_out, int num_sms, cudaStream_t stream) {
   const int esz = kp.kv_fp8 ? 1 : 2;
   DepageArgs a;

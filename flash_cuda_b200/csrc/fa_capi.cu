@@ -14,7 +14,9 @@
 namespace fa {
 
 int launch_sched(const FaSchedParams& sp, const Plan& pl, int32_t* out_dev, int32_t* zero_words, cudaStream_t stream,
-                 int row_class = 0, int class_rows = 0);
+                 int row_class = 0, int class_rows = 0, const int32_t* skip = nullptr);
+int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_rows, void* k_out, void* v_out, int32_t* cu,
+                 int32_t* take, int32_t* lens, int num_sms, cudaStream_t stream);
 int launch_selftest_timeout(DeviceStatus* status, long long max_cycles, cudaStream_t stream);
 int launch_append_kv(const FaAppendParams& p, int num_sms, cudaStream_t stream);
 int launch_depage(const KParams& kp, int kpad, void* k_out, void* v_out, int32_t* cu_out, int num_sms, cudaStream_t stream);
@@ -237,6 +239,44 @@ static bool depage_plan(const FaFwdParams* p, const Plan& pl, int* kpad, size_t*
   return true;
 }
 
+// 16-bit queries over an e4m3 cache with more rows than the decode kernel takes: the tensor-core kernel wants both
+// operands of one type, so the keys of the prefill-shaped sequences are widened into 16-bit slabs first (fa_append.cu)
+// and the decode kernel runs the others.  The general kernel, which ran all of it before, runs at about 80 TFLOP/s
+// and packs every decode row alone into a tile of 64.
+struct WidenPlan {
+  bool on;
+  Plan tc;            // plan of the prefill part
+  int class_rows;     // > 0: sequences with at most this many packed rows go to the decode kernel
+  int cap_rows;       // rows of the slabs
+  bool may_overflow;  // not every batch of these bounds fits them
+};
+static WidenPlan widen_plan(const FaFwdParams* p, const PlanInput& in, const Plan& pl) {
+  WidenPlan wp{};
+  if (p->route != FA_ROUTE_AUTO || pl.route != FA_ROUTE_GENERAL || p->kv_dtype != FA_DT_FP8_E4M3 ||
+      p->q_dtype == FA_DT_FP8_E4M3 || p->out_dtype == FA_DT_FP32 || p->num_splits > 0 || !in.tc_layout_ok)
+    return wp;
+  PlanInput tin = in;
+  tin.kv_dtype = in.q_dtype;
+  tin.page_size = 0;
+  tin.route = FA_ROUTE_PREFILL_TC;
+  // (16-byte loads of 8-bit rows)
+  if (p->hd % 16 || p->hdv % 16 || p->k_row_stride % 16 || p->v_row_stride % 16 || !prefill_tc_supported(tin)) return wp;
+  wp.tc = make_plan(tin);
+  if (wp.tc.err != FA_OK || (long long)p->batch * wp.tc.max_mtiles > kSchedSortMax) return wp;
+  if (p->batch > 1) {
+    if (!decode_supported(in) || p->batch * (kDecodeMaxRows / 16) > kBalancedEntriesMax) return wp;
+    wp.class_rows = kDecodeMaxRows;
+  }
+  const size_t row = (size_t)p->hkv * (p->hd + p->hdv) * 2;
+  const size_t want = (size_t)p->batch * (size_t)((p->max_seqlen_k + 127) / 128 * 128);
+  const size_t cap = kDepageMaxBytes / row / 128 * 128;
+  wp.may_overflow = want > cap;
+  if (wp.may_overflow && pl.nsplits > 1) return wp;     // few long sequences: the general kernel in split form
+  wp.cap_rows = (int)(want < cap ? want : cap);
+  wp.on = wp.cap_rows > 0 && p->max_seqlen_k > 0;
+  return wp;
+}
+
 // Key-range parts per work item of the tensor-core prefill kernel (1 = none), from a model of its time: items of
 // `tile_m` rows run in whole waves over the SMs, 1.8 us per key block of 2 x 128 rows at 256 columns; parts leave as
 // fp32 and are merged (a launch, and 8 bytes per row and column through memory).  A chunk of 512 rows over 24500
@@ -276,6 +316,8 @@ struct WsLayout {
   size_t lse_off, lse_bytes;
   size_t o_off, o_bytes;
   int tc_splits;      // tensor-core prefill: key-range parts per item; their partials lie at lse_off / o_off
+  WidenPlan widen;
+  size_t wd_cu_off, wd_take_off, wd_lens_off, wd_k_off, wd_v_off;
   PartPlan parts;
   size_t part_ml_off, part_o_off;   // balanced decode: pieces of cut (sequence, head) triples; part_o_off 0: none
   size_t total;
@@ -300,6 +342,30 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
     off += w.o_bytes;
   };
   w.tc_splits = 1;
+  if (pl.route == FA_ROUTE_GENERAL) {
+    const PlanInput in = plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0));
+    w.widen = widen_plan(p, in, pl);
+    if (w.widen.on) {
+      w.wd_cu_off = off;
+      off += align_up((size_t)(p->batch + 1) * 4, 256);
+      w.wd_take_off = off;
+      off += align_up((size_t)(p->batch + 1) * 4, 256);
+      w.wd_lens_off = off;
+      off += align_up((size_t)p->batch * 4, 256);
+      w.work2_off = off;
+      w.work2_bytes = align_up((size_t)sched_len(w.widen.tc, p->batch) * 4, 256);
+      off += w.work2_bytes;
+      if (w.widen.class_rows > 0) carve_parts(decode_part_plan(in, pl));
+      w.tc_splits = tc_splits(p, in, w.widen.tc);
+      if (w.tc_splits > 1) carve_splits(w.tc_splits);
+      w.wd_k_off = off;
+      off += align_up((size_t)w.widen.cap_rows * p->hkv * p->hd * 2, 256);
+      w.wd_v_off = off;
+      off += align_up((size_t)w.widen.cap_rows * p->hkv * p->hdv * 2, 256);
+      w.total = off;
+      return w;
+    }
+  }
   if (balanced_decode(p, pl)) {
     carve_parts(pl);
     w.total = off;
@@ -572,6 +638,37 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     kt.work = list_p;
     rc = run_prefill(kt, pl);
     if (rc == FA_OK) rc = run_short(list_d);
+  } else if (w.widen.on) {
+    // 16-bit queries over an e4m3 cache: see widen_plan
+    const WidenPlan& wp = w.widen;
+    int32_t* cu = (int32_t*)(ws + w.wd_cu_off);
+    int32_t* take = (int32_t*)(ws + w.wd_take_off);
+    int32_t* list = (int32_t*)(ws + w.work2_off);
+    KParams kt = kp;
+    rc = note_cuda_error(launch_widen(kp, compute_dtype, wp.class_rows, wp.cap_rows, ws + w.wd_k_off, ws + w.wd_v_off, cu,
+                                      take, (int32_t*)(ws + w.wd_lens_off), pl.num_sms, stream), "widening kernel");
+    if (rc == FA_OK)
+      rc = note_cuda_error(launch_sched(sp, wp.tc, list, nullptr, stream, wp.class_rows > 0 ? 2 : 0, wp.class_rows, take), "sched_kernel");
+    if (rc != FA_OK) return rc;
+    kt.work = list;
+    kt.work_expect = SchedExpect{p->batch, 1, wp.tc.tile_m, wp.tc.tile_n, wp.tc.max_mtiles, wp.tc.rows_per_token, wp.tc.route};
+    kt.nsplits = 1;
+    kt.k = ws + w.wd_k_off; kt.v = ws + w.wd_v_off;
+    kt.kv_fp8 = 0;
+    kt.k_row_stride = (int64_t)p->hkv * p->hd; kt.k_head_stride = p->hd; kt.k_page_stride = 0;
+    kt.v_row_stride = (int64_t)p->hkv * p->hdv; kt.v_head_stride = p->hdv; kt.v_page_stride = 0;
+    kt.page_table = nullptr; kt.page_size = 0; kt.page_shift = -1; kt.page_table_stride = 0; kt.num_pages = 0;
+    kt.cu_k = cu;
+    kt.seqused_k = (const int32_t*)(ws + w.wd_lens_off);
+    kt.total_k = wp.cap_rows;
+    rc = run_prefill(kt, wp.tc);
+    if (rc == FA_OK && wp.may_overflow) {
+      KParams kg = kp;
+      kg.take = take;
+      kg.nsplits = 1;
+      rc = note_cuda_error(launch_general(kg, compute_dtype, p->out_dtype, pl.num_sms, stream), "general kernel");
+    }
+    if (rc == FA_OK && wp.class_rows > 0) rc = run_short(nullptr);
   } else if (pl.route == FA_ROUTE_PREFILL_TC) {
     kp.work = p->scheduler_metadata;   // optional: the sorted (batch, tile) list replaces the arithmetic order
     if (w.dp_k_bytes > 0) {
@@ -594,7 +691,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   }
   if (rc != FA_OK) return rc;
 
-  if (pl.nsplits > 1 && !balanced) {
+  if (pl.nsplits > 1 && !balanced && !w.widen.on) {
     rc = note_cuda_error(launch_combine(kp.o_part, kp.lse_part, pl.nsplits, p->total_q, p->hq, p->hdv, p->s_aux,
                                         p->out, p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream),
                          "combine kernel");

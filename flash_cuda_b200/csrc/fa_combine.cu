@@ -118,6 +118,7 @@ struct SchedArgs {
   int32_t* zero_words;     // when not null: 64 words (a workspace header) this kernel clears for the kernel after it
   int32_t row_class;       // 0: every sequence; 1: only sequences with at most class_rows packed query rows per kv head
   int32_t class_rows;      //    (the decode kernel's share of a mixed batch); 2: only the others (the prefill kernel's)
+  const int32_t* skip;     // when not null: sequences with a nonzero word are left out
   int32_t class_rep;       // q heads per kv head, for the row count of the class test
 };
 
@@ -135,6 +136,7 @@ __device__ __forceinline__ bool sched_entry(const SchedArgs& a, int e, int* b_ou
     const bool small = seqlen_q * a.class_rep <= a.class_rows;
     if (small != (a.row_class == 1)) { *lo = 0; *hi = 0; return false; }
   }
+  if (a.skip != nullptr && a.skip[b] != 0) { *lo = 0; *hi = 0; return false; }
   const int tok_min = row0 / a.rows_per_token;
   const int tok_max = min(seqlen_q - 1, (row0 + a.tile_m - 1) / a.rows_per_token);
   nblock_range(seqlen_k, leftpad, seqlen_k - seqlen_q + tok_min, seqlen_k - seqlen_q + tok_max, a.is_causal,
@@ -243,8 +245,9 @@ int launch_selftest_timeout(DeviceStatus* status, long long max_cycles, cudaStre
 }
 
 int launch_sched(const FaSchedParams& sp, const Plan& pl, int32_t* out_dev, int32_t* zero_words, cudaStream_t stream,
-                 int row_class, int class_rows) {
+                 int row_class, int class_rows, const int32_t* skip) {
   SchedArgs a;
+  a.skip = skip;
   a.seqused_k = sp.seqused_k; a.cu_q = sp.cu_seqlens_q; a.cu_k = sp.cu_seqlens_k; a.leftpad_k = sp.leftpad_k;
   a.batch = sp.batch; a.max_seqlen_q = sp.max_seqlen_q; a.max_seqlen_k = sp.max_seqlen_k;
   a.is_causal = sp.is_causal; a.window_left = sp.window_left; a.window_right = sp.window_right;

@@ -34,20 +34,20 @@ __device__ __forceinline__ uint4 load8(const void* base, int64_t elem_off, bool 
 }
 
 template <typename T, int HD, int HDV>
-__global__ void __launch_bounds__(NTHREADS) fwd_general_kernel(const KParams p) {
+__device__ __forceinline__ void general_tile(const KParams& p, unsigned char* smem_raw, unsigned tile) {
   constexpr int LDQ = HD + PAD, LDV = HDV + PAD;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sQ = reinterpret_cast<T*>(smem_raw);
   T* sK = sQ + BM * LDQ;
   T* sV = sK + BN * LDQ;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // grid: x = (split * batch + b) * mtiles + m tile (x has the 2^31 range; y and z stop at 65535), y = kv head
+  // tile = (split * batch + b) * mtiles + m tile (grid x has the 2^31 range; y and z stop at 65535); y = kv head
   const int mtiles = (p.max_seqlen_q * p.rep + BM - 1) / BM;
-  const int mt = blockIdx.x % mtiles, hk = blockIdx.y;
-  const int bz = blockIdx.x / mtiles;
+  const int mt = tile % mtiles, hk = blockIdx.y;
+  const int bz = tile / mtiles;
   const int b = bz % p.batch, split = bz / p.batch;
   const int rep = p.rep;
+  if (p.take && !p.take[b]) return;
 
   const int q0 = p.cu_q[b];
   const int seqlen_q = p.cu_q[b + 1] - q0;
@@ -278,6 +278,16 @@ __global__ void __launch_bounds__(NTHREADS) fwd_general_kernel(const KParams p) 
 }
 
 template <typename T, int HD, int HDV>
+__global__ void __launch_bounds__(NTHREADS) fwd_general_kernel(const KParams p, unsigned tiles) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (p.take && p.take[p.batch] == 0) return;      // (usual: nothing was left over for this kernel)
+  for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    general_tile<T, HD, HDV>(p, smem_raw, tile);
+    __syncthreads();
+  }
+}
+
+template <typename T, int HD, int HDV>
 static int launch_t(const KParams& kp, cudaStream_t stream) {
   const size_t smem = (size_t)(BM * (HD + PAD) + BN * (HD + PAD) + BN * (HDV + PAD)) * sizeof(T);
   auto kern = fwd_general_kernel<T, HD, HDV>;
@@ -285,8 +295,10 @@ static int launch_t(const KParams& kp, cudaStream_t stream) {
   if (e != cudaSuccess) return (int)e;
   const int mtiles = (kp.max_seqlen_q * kp.rep + BM - 1) / BM;
   if (kp.hkv > 65535 || (long long)mtiles * kp.batch * kp.nsplits > 2147483647ll) return -1;
-  dim3 grid((unsigned)(mtiles * kp.batch * kp.nsplits), kp.hkv, 1);
-  kern<<<grid, NTHREADS, smem, stream>>>(kp);
+  const unsigned tiles = (unsigned)(mtiles * kp.batch * kp.nsplits);
+  // one block per tile; where usually no tile is this kernel's, few blocks that look for theirs
+  dim3 grid(kp.take && tiles > 64u ? 64u : tiles, kp.hkv, 1);
+  kern<<<grid, NTHREADS, smem, stream>>>(kp, tiles);
   return (int)cudaGetLastError();
 }
 

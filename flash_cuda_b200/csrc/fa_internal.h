@@ -57,6 +57,7 @@ struct KParams {
   int32_t tc_splits;                 // tensor-core prefill: key-range parts per work item; part s > 0 of `out` and `lse`
   int64_t o_split_stride, lse_split_stride;   //             lies this many floats behind part s - 1 (out_f32 then)
   int32_t part_rows;   // balanced decode: rows of a piece
+  const int32_t* take; // general kernel: per sequence 1 = this kernel's, and at [batch] how many are; null = all
   int32_t class_rows;  // balanced decode: > 0 = only sequences with at most this many packed query rows
   int32_t out_f32;     // `out` is fp32 (FA_DT_FP32) instead of the 16-bit type of the kernel
   float scale;         // softmax_scale

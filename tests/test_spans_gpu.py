@@ -1,7 +1,7 @@
 """Work that is cut along the keys: the balanced decode kernel (spans that cross sequences, pieces merged by the CTA
-that finishes last) and key-range parts of the tensor-core prefill kernel.  Each against the CPU oracle with the
-benchmark's tolerances (16-bit 2e-2, e4m3 cache 6e-2, LSE 5e-3) and against the uncut form of the same call
-(num_splits = 1)."""
+that finishes last), key-range parts of the tensor-core prefill kernel, and the widening of an e4m3 cache for 16-bit
+queries.  Each against the CPU oracle with the benchmark's tolerances (16-bit 2e-2, e4m3 cache 6e-2, LSE 5e-3) and
+against the uncut form of the same call (num_splits = 1, or the general kernel)."""
 import pytest
 import torch
 
@@ -81,3 +81,50 @@ def test_prefill_in_key_range_parts(name, dtype, cuda_device):
     assert not torch.equal(lse, whole_lse)                     # the call was cut
     assert (out.float() - whole.float()).abs().max().item() <= 2 ** -7
     torch.testing.assert_close(lse, whole_lse, atol=1e-4, rtol=1e-5)
+
+
+WIDEN = {    # 16-bit queries over an e4m3 cache, more rows than the decode kernel takes
+    "chunk": ([(200, 3000)], dict(hq=8, hkv=2, hd=128, page_size=16)),
+    "mixed": ([(1, 900), (70, 2000), (3, 65), (33, 33), (1, 1), (0, 40)], dict(hq=8, hkv=2, hd=128, page_size=64, sink=True)),
+    "packed": ([(150, 1500), (129, 129)], dict(hq=4, hkv=4, hd=128, page_size=0, window_left=500)),
+    "leftpad": ([(100, 1000), (1, 500)], dict(hq=8, hkv=1, hd=128, page_size=8, leftpad=[70, 3], softcap=25.0)),
+    "hd64": ([(100, 1000)], dict(hq=8, hkv=2, hd=64, page_size=32)),
+    "hd256": ([(140, 700)], dict(hq=4, hkv=2, hd=256, page_size=64, causal=False)),
+    "keyless": ([(100, 0), (90, 300), (1, 0)], dict(hq=8, hkv=2, hd=128, page_size=64)),
+    "odd_page": ([(100, 1000)], dict(hq=8, hkv=2, hd=128, page_size=24)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(WIDEN))
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+def test_wide_queries_over_an_e4m3_cache(name, dtype, cuda_device):
+    reqs, kw = WIDEN[name]
+    p = W.make_problem("widen_" + name, reqs, dtype=dtype, kv_dtype="fp8", seed=93, **kw)
+    out, _ = _run(p, cuda_device, 6e-2)
+    gen, _ = _run(p, cuda_device, 6e-2, check_ref=False, route=capi.FA_ROUTE_GENERAL)
+    assert (out.float() - gen.float()).abs().max().item() <= 2 ** -6        # two roundings of P and one of the result
+
+
+def test_wide_queries_over_more_keys_than_the_slabs_hold(cuda_device):
+    """Sequences that do not fit the 256 MB of slabs are left to the general kernel, inside the same call."""
+    g = torch.Generator(device=cuda_device).manual_seed(94)
+    lens, hkv = [30000, 20000, 25000, 700], 8
+    pages = [(n + 63) // 64 for n in lens]
+    k = torch.randn(sum(pages), 64, hkv, 128, generator=g, device=cuda_device, dtype=torch.bfloat16).to(torch.float8_e4m3fn)
+    v = torch.randn(sum(pages), 64, hkv, 128, generator=g, device=cuda_device, dtype=torch.bfloat16).to(torch.float8_e4m3fn)
+    table = torch.zeros(4, max(pages), dtype=torch.int32)
+    at = 0
+    for b, n in enumerate(pages):
+        table[b, :n] = torch.arange(at, at + n, dtype=torch.int32)
+        at += n
+    q_lens = [80, 70, 90, 1]
+    q = torch.randn(sum(q_lens), 16, 128, generator=g, device=cuda_device, dtype=torch.bfloat16)
+    cu = torch.tensor([0, 80, 150, 240, 241], dtype=torch.int32, device=cuda_device)
+    kw = dict(cu_seqlens_q=cu, seqused_k=torch.tensor(lens, dtype=torch.int32, device=cuda_device),
+              page_table=table.to(cuda_device), max_seqlen_q=90, max_seqlen_k=30000, softmax_scale=128 ** -0.5, causal=True)
+    out, lse, _ = capi.fwd(q, k, v, check=True, **kw)
+    gen, gen_lse, _ = capi.fwd(q, k, v, check=True, route=capi.FA_ROUTE_GENERAL, **kw)
+    assert (out.float() - gen.float()).abs().max().item() <= 2 ** -8        # values of about 0.01 over 20000 keys
+    torch.testing.assert_close(lse, gen_lse, atol=1e-3, rtol=1e-4)
+
+
