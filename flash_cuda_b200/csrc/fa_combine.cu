@@ -145,7 +145,7 @@ __device__ __forceinline__ bool sched_entry(const SchedArgs& a, int e, int* b_ou
 }
 
 __global__ void __launch_bounds__(1024) sched_kernel(const SchedArgs a, int32_t* __restrict__ out) {
-  extern __shared__ uint32_t s_key[];   // sort keys, sort_n of them
+  extern __shared__ __align__(16) uint32_t s_key[];   // sort keys, sort_n of them (a multiple of four)
   __shared__ int s_valid;
   const int E = a.batch * a.max_mtiles;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -161,6 +161,35 @@ __global__ void __launch_bounds__(1024) sched_kernel(const SchedArgs a, int32_t*
       out[kSchedHeader + 4 * e + 1] = ok ? mt : -1;
       out[kSchedHeader + 4 * e + 2] = lo;
       out[kSchedHeader + 4 * e + 3] = hi;
+    }
+  } else if (a.sort_n <= (int)blockDim.x) {
+    // One slot per thread: a slot's place is the number of smaller keys, counted over all of them in shared memory
+    // (broadcast reads, four keys each).  No barriers between steps, and the entry stays in registers: with the sorting
+    // network a list of 132 slots took 10.1 us, nearly all of it barriers and the second look at the lengths.
+    int b = -1, mt = -1, lo = 0, hi = 0;
+    uint32_t key = 0xffffffffu;
+    if (tid < E && sched_entry(a, tid, &b, &mt, &lo, &hi)) {
+      key = ((uint32_t)(kSchedCountMax - (hi - lo)) << kSchedSlotBits) | (uint32_t)tid;
+      atomicAdd(&s_valid, 1);
+    }
+    if (tid < a.sort_n) s_key[tid] = key;
+    __syncthreads();
+    if (tid < E) {
+      if (key != 0xffffffffu) {
+        int place = 0;
+        const uint4* k4 = reinterpret_cast<const uint4*>(s_key);
+#pragma unroll 4
+        for (int i = 0; i < a.sort_n / 4; ++i) {
+          const uint4 k = k4[i];
+          place += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
+        }
+        int32_t* ent = out + kSchedHeader + 4 * place;
+        ent[0] = b; ent[1] = mt; ent[2] = lo; ent[3] = hi;
+      }
+      if (tid >= s_valid) {
+        int32_t* ent = out + kSchedHeader + 4 * tid;
+        ent[0] = -1; ent[1] = -1; ent[2] = 0; ent[3] = 0;
+      }
     }
   } else {
     const int N = a.sort_n;
@@ -255,7 +284,7 @@ int launch_sched(const FaSchedParams& sp, const Plan& pl, int32_t* out_dev, int3
   a.max_mtiles = pl.max_mtiles; a.nsplits = pl.nsplits; a.route = pl.route;
   const int E = sp.batch * pl.max_mtiles;
   a.sorted = sched_is_sorted(E, sp.max_seqlen_k, pl.tile_n) ? 1 : 0;
-  a.sort_n = 1;
+  a.sort_n = 4;
   while (a.sort_n < E) a.sort_n <<= 1;
   a.zero_words = zero_words;
   a.row_class = row_class; a.class_rows = class_rows; a.class_rep = sp.hkv > 0 ? sp.hq / sp.hkv : 1;
