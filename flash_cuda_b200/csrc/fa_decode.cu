@@ -39,7 +39,7 @@ constexpr int ncons_for(int) { return 4; }
 constexpr int ctas_per_sm(int esz) { return esz == 1 ? 2 : 1; }
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
-constexpr int kMinSpan = 4;            // balanced kernels: key blocks of a span at least
+constexpr int kMinSpan = 2;            // balanced kernels: key blocks of a span at least (one sequence of 1000 keys: 16.1 us at 4, 14.4 at 2)
 constexpr int kPieces = 4;             // mailbox slots between the producer and the consumers
 enum Role : unsigned { ROLE_PRODUCER = 5, ROLE_CONSUMER = 6 };
 enum : int { F_FIRST = 1, F_LAST = 2, F_EMPTY = 4 };
@@ -123,7 +123,7 @@ __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
 // side, one kv head each.  With one work item per (batch, row tile, kv head) a ragged batch of 16 sequences (128 items)
 // waited for its longest sequence, and few long sequences needed a split count, a work-list kernel before and a merge
 // kernel after: 16 sequences of 1024 .. 16384 keys 174 -> 109 us per call (HBM floor 83), one of 1000 keys 20.5 ->
-// 16.4 us, 24 x 4 queries over 500 .. 8000 keys of head_dim 64 107 -> 84 us.
+// 14.4 us, 24 x 4 queries over 500 .. 8000 keys of head_dim 64 107 -> 84 us.
 // The team keeps the heads of a token, neighbours in memory, together in time: with the heads of a sequence one after
 // the other on the line (every CTA somewhere else, 256-byte rows 2 KB apart) the 16 sequences took 119 us, and 128
 // sequences of 1024 .. 32768 keys fell from 6.25 to 5.4 TB/s.
