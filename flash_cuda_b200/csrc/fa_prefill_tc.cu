@@ -121,7 +121,7 @@ struct alignas(16) Item {
 static_assert(sizeof(Item) == 64, "mailbox slot");
 constexpr int kPartShift = 24, kHeadMask = (1 << kPartShift) - 1;
 
-template <int NTL>
+template <int NTL, bool PARTS>
 __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_entry) {
   constexpr int kItemRows = NTL * TM;
   const KParams& p = a.kp;
@@ -129,7 +129,7 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
   it.w = w;
   // the key-range parts of an item are consecutive work ids
   int part = 0;
-  if (p.tc_splits > 1) {
+  if constexpr (PARTS) {
     const int q = w / p.tc_splits;
     part = w - q * p.tc_splits;
     w = q;
@@ -192,7 +192,7 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
     }
     if (it.hi[t] > it.lo[t]) { it.ulo = min(it.ulo, it.lo[t]); it.uhi = max(it.uhi, it.hi[t]); }
   }
-  if (p.tc_splits > 1 && it.valid) {
+  if (PARTS && it.valid) {
     int plo, phi;
     split_range(it.ulo, max(it.uhi, it.ulo), part, p.tc_splits, &plo, &phi);
     it.ulo = 0x7fffffff;
@@ -332,10 +332,12 @@ __device__ __forceinline__ void copy_tile_rows(uint32_t dst0, const unsigned cha
 // second softmax warpgroup stays idle and softmax and MMAs of the tile alternate instead of overlapping.
 // CAP: the logit soft cap is compiled in (the host picks the instantiation by softcap > 0, so that the common
 // kernel carries none of its code: the softmax loop's time follows its instruction count).
+// PARTS: an item is one of kp.tc_splits parts of its key range (the code for it, in the decoding of items and in the
+// epilogue, cost the calls without parts 1 - 3 %).
 // PROD: the form of the TMA producer: 0 = contiguous K/V, lane 0 alone; 1 = paged, lane 0 alone; 2 = paged, the whole
 // warp (see the TMA role).  Template arguments rather than run-time flags for the same reason as CAP: code that a
 // launch never runs still moved the time of the code it does run by a few per cent.
-template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD>
+template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD, bool PARTS>
 __global__ void __launch_bounds__(NTHREADS, 1)
 fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -447,7 +449,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       int num_items = a.num_items;
       if (a.use_list) {
         if (sched_header_matches(p.work, p.work_expect)) {
-          num_items = p.work[6] * p.hq * p.tc_splits;
+          num_items = p.work[6] * p.hq * (PARTS ? p.tc_splits : 1);
         } else {
           if (leader) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_TMA);
           num_items = 0;
@@ -477,7 +479,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
             first_ticket = false;
             if (w >= num_items) { it.w = kEndOfWork; break; }
             bool bad = false;
-            it = decode_item<NTL>(a, w, &bad);   // sequence bounds are read from global memory once per item
+            it = decode_item<NTL, PARTS>(a, w, &bad);   // sequence bounds are read from global memory once per item
             if (bad) { report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_TMA); num_items = 0; it.w = kEndOfWork; break; }
             if (it.valid) break;
           }
@@ -510,14 +512,14 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
             mbar_expect_tx(bar_q_full + 8 * t, TM * HD * ESZ);
 #pragma unroll
             for (int cb = 0; cb < HD / EPB; ++cb)
-              tma_load_3d(sQ + t * (TM * HD * ESZ) + cb * (TM * 128), &map_q, cb * EPB, it.h & kHeadMask,
+              tma_load_3d(sQ + t * (TM * HD * ESZ) + cb * (TM * 128), &map_q, cb * EPB, PARTS ? it.h & kHeadMask : it.h,
                           it.q0 + it.pair * (NTL * TM) + t * TM, bar_q_full + 8 * t);
           }
           return true;
         };
         ok = load_q(0);
         if (!ok) { if (leader) report_error(p.status, DEV_ERR_TIMEOUT, ROLE_TMA); break; }
-        const int hk = (it.h & kHeadMask) / p.rep;
+        const int hk = (PARTS ? it.h & kHeadMask : it.h) / p.rep;
         // one K or V tile of key block nb into `dst`, completing on `bar`
         const int pj0 = wide ? lane : 0, pjs = wide ? 32 : 1;
         // first row of this lane's first box and the distance to its next one
@@ -853,7 +855,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       const int row0 = it.pair * (NTL * TM) + t * TM;
       if (row0 >= it.seqlen_q) continue;           // this tile owns no row
       const int row = row0 + r;
-      const int hk = (it.h & kHeadMask) / p.rep;
+      const int hk = (PARTS ? it.h & kHeadMask : it.h) / p.rep;
       float sc = p.scale, vds = 1.f;
       {
         const int di = it.b * p.descale_batch_stride + hk * p.descale_head_stride;
@@ -1175,10 +1177,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
               }
             }
           }
-        } else if (row_ok && (had_blocks || p.tc_splits == 1)) {   // (the merge does not read an empty part's rows)
+        } else if (row_ok && (!PARTS || had_blocks)) {   // (the merge does not read an empty part's rows)
           if (p.out_f32) {
-            float* op = reinterpret_cast<float*>(p.out) + (int64_t)(it.h >> kPartShift) * p.o_split_stride +
-                        (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(it.h & kHeadMask) * p.o_head_stride;
+            float* op = reinterpret_cast<float*>(p.out) + (PARTS ? (int64_t)(it.h >> kPartShift) * p.o_split_stride : 0) +
+                        (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.o_head_stride;
   #pragma unroll
             for (int c = 0; c < HDV / 32; ++c) {
               if (c * 32 < a.out_cols) {
@@ -1208,7 +1210,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           }
         }
         if (row_ok)
-          p.lse[(int64_t)(it.h >> kPartShift) * p.lse_split_stride + (int64_t)(it.h & kHeadMask) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
+          p.lse[(PARTS ? (int64_t)(it.h >> kPartShift) * p.lse_split_stride : 0) +
+                (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
       } else {
         // HDV > 128 (one tile per item): the O row is read 64 columns at a time; O_t is released as soon as its last
         // column has been read.  Each 64-column group leaves like a half row of the two-tile form: staged + one TMA
@@ -1279,10 +1282,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
                 bulk_commit_group();
               }
             }
-          } else if (row_ok && (had_blocks || p.tc_splits == 1)) {
+          } else if (row_ok && (!PARTS || had_blocks)) {
             if (p.out_f32) {
-              float* op = reinterpret_cast<float*>(p.out) + (int64_t)(it.h >> kPartShift) * p.o_split_stride +
-                        (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(it.h & kHeadMask) * p.o_head_stride + g * 64;
+              float* op = reinterpret_cast<float*>(p.out) + (PARTS ? (int64_t)(it.h >> kPartShift) * p.o_split_stride : 0) +
+                        (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.o_head_stride + g * 64;
 #pragma unroll
               for (int c = 0; c < 2; ++c)
 #pragma unroll
@@ -1307,7 +1310,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           }
         }
         if (row_ok)
-          p.lse[(int64_t)(it.h >> kPartShift) * p.lse_split_stride + (int64_t)(it.h & kHeadMask) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
+          p.lse[(PARTS ? (int64_t)(it.h >> kPartShift) * p.lse_split_stride : 0) +
+                (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
       }
     }
     if constexpr (SM::kStageOut) {
@@ -1400,8 +1404,8 @@ static bool producer_is_wide(const KParams& kp) {
   return kp.page_size <= 32 || (KST == VST && kp.page_size <= 64);
 }
 
-template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD>
-static int launch_prod(const KParams& kp, const Plan& pl, int dtype, uint64_t kv_rows, cudaStream_t stream) {
+template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD, bool PARTS>
+static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t kv_rows, cudaStream_t stream) {
   using SM = Smem<Elem<T>::kSize, HD, HDV, KST, VST, NTL>;
   TcArgs a;
   a.kp = kp;
@@ -1434,7 +1438,7 @@ static int launch_prod(const KParams& kp, const Plan& pl, int dtype, uint64_t kv
                     (uint64_t)kp.o_row_stride, 32))
       a.stage_out = 1;
   }
-  auto kern = fwd_prefill_tc_kernel<T, HD, HDV, KST, VST, NTL, CAP, PROD>;
+  auto kern = fwd_prefill_tc_kernel<T, HD, HDV, KST, VST, NTL, CAP, PROD, PARTS>;
   int smem = SM::kBytes + 1024;
   if (smem < 120 * 1024) smem = 120 * 1024;   // one CTA per SM: the CTA owns all 512 TMEM columns
   static std::atomic<unsigned long long> attr_done{0};   // one bit per device
@@ -1449,6 +1453,12 @@ static int launch_prod(const KParams& kp, const Plan& pl, int dtype, uint64_t kv
   if (grid <= 0) return 0;
   kern<<<grid, NTHREADS, smem, stream>>>(a, mq, mk, mv, mo);
   return (int)cudaGetLastError();
+}
+
+template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD>
+static int launch_prod(const KParams& kp, const Plan& pl, int dtype, uint64_t kv_rows, cudaStream_t stream) {
+  return kp.tc_splits > 1 ? launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, true>(kp, pl, dtype, kv_rows, stream)
+                          : launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, false>(kp, pl, dtype, kv_rows, stream);
 }
 
 template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP>
