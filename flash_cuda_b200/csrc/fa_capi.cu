@@ -22,7 +22,8 @@ int launch_append_kv(const FaAppendParams& p, int num_sms, cudaStream_t stream);
 int launch_depage(const KParams& kp, int kpad, void* k_out, void* v_out, int32_t* cu_out, int num_sms, cudaStream_t stream);
 int launch_combine_strided(const float* o_part, const float* lse_part, int64_t o_split_stride, int64_t lse_split_stride,
                            int nsplits, int total_q, int hq, int hdv, const float* s_aux, void* out,
-                           int64_t o_row_stride, int64_t o_head_stride, int out_dtype, float* lse, cudaStream_t stream);
+                           int64_t o_row_stride, int64_t o_head_stride, int out_dtype, float* lse, cudaStream_t stream,
+                           const int32_t* rows_end = nullptr);
 int launch_decode(const KParams& kp, const Plan& pl, int compute_dtype, cudaStream_t stream);
 int launch_prefill_tc(const KParams& kp, const Plan& pl, int compute_dtype, cudaStream_t stream);
 bool prefill_tc_supported(const PlanInput& in);
@@ -603,7 +604,8 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     int r = note_cuda_error(launch_prefill_tc(kt, plt, compute_dtype, stream), "tcgen05 prefill kernel");
     if (r != FA_OK) return r;
     return note_cuda_error(launch_combine(o_part, lse_part, w.tc_splits, p->total_q, p->hq, p->hdv, p->s_aux, p->out,
-                                          p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream), "combine kernel");
+                                          p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream,
+                                          p->cu_seqlens_q + p->batch), "combine kernel");
   };
   // the decode kernel over the short sequences of a batch that also holds long ones
   auto run_short = [&](const int32_t* list) -> int {
@@ -693,7 +695,8 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
 
   if (pl.nsplits > 1 && !balanced && !w.widen.on) {
     rc = note_cuda_error(launch_combine(kp.o_part, kp.lse_part, pl.nsplits, p->total_q, p->hq, p->hdv, p->s_aux,
-                                        p->out, p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream),
+                                        p->out, p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream,
+                                        p->cu_seqlens_q + p->batch),
                          "combine kernel");
   }
   return rc;

@@ -14,6 +14,8 @@ constexpr float kLn2C = 0.6931471805599453f;
 // A split whose lse is -inf contributes exactly 0 even if its partial was never written.
 // Split s starts o_split_stride / lse_split_stride floats after split s-1, so partials can be merged where a
 // gather left them (one packed [O | LSE] buffer per rank).
+// rows_end, when not null, points at the number of rows that have partials (cu_seqlens_q[batch]): where total_q is
+// larger, no kernel wrote partials of the rows behind, and the caller's rows there stay as they are.
 // ------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ o_part,
@@ -21,7 +23,8 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
                                                       int64_t lse_split_stride, int nsplits, int total_q,
                                                       int hq, int hdv, const float* __restrict__ s_aux,
                                                       T* __restrict__ out, int64_t o_row_stride,
-                                                      int64_t o_head_stride, float* __restrict__ lse) {
+                                                      int64_t o_head_stride, float* __restrict__ lse,
+                                                      const int32_t* __restrict__ rows_end) {
   const int vec = hdv >> 2;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)total_q * hq * vec) return;
@@ -29,6 +32,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
   const int64_t qh = idx / vec;
   const int h = (int)(qh % hq);
   const int64_t qi = qh / hq;
+  const int64_t end = rows_end != nullptr ? *rows_end : total_q;      // (looked at where the row is written: one wait less)
 
   float g = -INFINITY;
   const int64_t lse_idx = (int64_t)h * total_q + qi;
@@ -40,6 +44,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
   g = fmaxf(g, sk);
   T* op = out + qi * o_row_stride + (int64_t)h * o_head_stride + dv;
   if (g == -INFINITY) {
+    if (qi >= end) return;
     *reinterpret_cast<uint2*>(op) = make_uint2(0u, 0u);
     if (dv == 0) lse[(int64_t)h * total_q + qi] = -INFINITY;
     return;
@@ -70,13 +75,15 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
   uint2 packed;
   packed.x = pack2<T>(acc.x * inv, acc.y * inv);
   packed.y = pack2<T>(acc.z * inv, acc.w * inv);
+  if (qi >= end) return;
   *reinterpret_cast<uint2*>(op) = packed;
   if (dv == 0) lse[(int64_t)h * total_q + qi] = g + lg2(L) * kLn2C;
 }
 
 int launch_combine_strided(const float* o_part, const float* lse_part, int64_t o_split_stride, int64_t lse_split_stride,
                            int nsplits, int total_q, int hq, int hdv, const float* s_aux, void* out,
-                           int64_t o_row_stride, int64_t o_head_stride, int out_dtype, float* lse, cudaStream_t stream) {
+                           int64_t o_row_stride, int64_t o_head_stride, int out_dtype, float* lse, cudaStream_t stream,
+                           const int32_t* rows_end) {
   if (hdv % 4 != 0) return -1;
   const int64_t n = (int64_t)total_q * hq * (hdv / 4);
   if (n == 0) return 0;
@@ -85,19 +92,20 @@ int launch_combine_strided(const float* o_part, const float* lse_part, int64_t o
   if (out_dtype == FA_DT_FP16)
     combine_kernel<__half><<<blocks, threads, 0, stream>>>(o_part, lse_part, o_split_stride, lse_split_stride, nsplits,
                                                             total_q, hq, hdv, s_aux, (__half*)out, o_row_stride,
-                                                            o_head_stride, lse);
+                                                            o_head_stride, lse, rows_end);
   else
     combine_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>(o_part, lse_part, o_split_stride, lse_split_stride,
                                                                    nsplits, total_q, hq, hdv, s_aux,
-                                                                   (__nv_bfloat16*)out, o_row_stride, o_head_stride, lse);
+                                                                   (__nv_bfloat16*)out, o_row_stride, o_head_stride, lse,
+                                                                   rows_end);
   return (int)cudaGetLastError();
 }
 
 int launch_combine(const float* o_part, const float* lse_part, int nsplits, int total_q, int hq, int hdv,
                    const float* s_aux, void* out, int64_t o_row_stride, int64_t o_head_stride, int out_dtype,
-                   float* lse, cudaStream_t stream) {
+                   float* lse, cudaStream_t stream, const int32_t* rows_end) {
   return launch_combine_strided(o_part, lse_part, (int64_t)total_q * hq * hdv, (int64_t)hq * total_q, nsplits, total_q,
-                                hq, hdv, s_aux, out, o_row_stride, o_head_stride, out_dtype, lse, stream);
+                                hq, hdv, s_aux, out, o_row_stride, o_head_stride, out_dtype, lse, stream, rows_end);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -103,6 +103,6 @@ int launch_general(const KParams& kp, int dtype /*FA_DT_BF16|FP16 compute type*/
                    cudaStream_t stream);
 int launch_combine(const float* o_part, const float* lse_part, int nsplits, int total_q, int hq, int hdv,
                    const float* s_aux, void* out, int64_t o_row_stride, int64_t o_head_stride, int out_dtype,
-                   float* lse, cudaStream_t stream);
+                   float* lse, cudaStream_t stream, const int32_t* rows_end = nullptr);
 
 }  // namespace fa

@@ -68,7 +68,8 @@ typedef struct FaFwdParams {
   int64_t k_row_stride, k_head_stride, k_page_stride; /* row = one token; page stride only when paged */
   int64_t v_row_stride, v_head_stride, v_page_stride;
   int64_t o_row_stride, o_head_stride;
-  const int32_t* cu_seqlens_q;  /* (batch+1), required */
+  const int32_t* cu_seqlens_q;  /* (batch+1), required; rows of q, out and lse from cu_seqlens_q[batch] on (a batch
+                                 * padded to a larger total_q) belong to no sequence and are not written */
   const int32_t* cu_seqlens_k;  /* (batch+1), non-paged */
   const int32_t* seqused_k;     /* (batch), paged (optional override when non-paged) */
   const int32_t* page_table;    /* (batch, page_table_stride) physical page of each logical page, or NULL */

@@ -1,0 +1,39 @@
+"""What a call that is cut along the keys must leave as an uncut call does: rows that no sequence owns, results after an
+earlier call that failed, precision, key pages outside the window, workspaces sized for the plain form, loose bounds."""
+import ctypes as C
+
+import pytest
+import torch
+
+from flash_cuda_b200 import capi, workloads as W
+from oracle.ref_attention import ref_attention
+
+pytestmark = pytest.mark.gpu
+
+PARTS = dict(reqs=[(200, 9000)], hq=8, hkv=2, hd=128, page_size=64)             # key-range parts of the prefill kernel
+MIXED = dict(reqs=[(1, 3000)] * 6 + [(200, 9000)], hq=8, hkv=2, hd=128, page_size=64)
+DECODE = dict(reqs=[(1, 5000), (1, 300), (1, 2500)], hq=8, hkv=2, hd=128, page_size=64)
+WIDEN = dict(reqs=[(1, 900), (200, 9000), (3, 65)], hq=8, hkv=2, hd=128, page_size=64, kv_dtype="fp8")
+
+
+def _problem(spec, dev, **kw):
+    spec = dict(spec, **kw)
+    return W.make_problem("cut", spec.pop("reqs"), seed=301, **spec).to(dev)
+
+
+@pytest.mark.parametrize("spec,kw", [(PARTS, {}), (MIXED, {}), (WIDEN, {}), (DECODE, {}), (DECODE, dict(num_splits=4)),
+                                     (PARTS, dict(route=capi.FA_ROUTE_GENERAL, num_splits=3))],
+                         ids=["parts", "mixed", "widened", "decode", "decode_split", "general_split"])
+def test_rows_past_the_last_sequence_stay_as_they_are(spec, kw, cuda_device):
+    """A batch padded for a captured graph: total_q is larger than cu_seqlens_q[batch]."""
+    p = _problem(spec, cuda_device)
+    n, pad = p.q.shape[0], 37
+    q = torch.cat([p.q, p.q[:1].expand(pad, -1, -1)])
+    out = torch.full((n + pad, *p.q.shape[1:]), 7.0, device=cuda_device, dtype=p.q.dtype)
+    lse = torch.full((p.q.shape[1], n + pad), 7.0, device=cuda_device)
+    capi.fwd(q, p.k, p.v, out=out, lse=lse, check=True, **dict(p.capi_kw(), **kw))
+    tight, tight_lse, _ = capi.fwd(p.q, p.k, p.v, check=True, **dict(p.capi_kw(), **kw))
+    assert (out[n:] == 7.0).all() and (lse[:, n:] == 7.0).all()
+    # (the padding is part of total_q and may move the cuts: one rounding to 16 bits of values below 2)
+    assert (out[:n].float() - tight.float()).abs().max().item() <= 2 ** -7
+    torch.testing.assert_close(lse[:, :n], tight_lse, atol=1e-4, rtol=1e-5)
