@@ -129,9 +129,12 @@ __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
 // sequences of 1024 .. 32768 keys fell from 6.25 to 5.4 TB/s.
 // What lies inside one span is written out directly; the pieces of a (batch, row tile, head) that crosses span borders
 // go to `part_*` as unnormalised fp32 rows with their maximum and sum, and the CTA that finishes the last piece merges
-// all of them in the order of the line (the same bits every time).  A cut costs about 3.5 us of a CTA per piece, which
-// is why the line is cut once per CTA and no finer: with half of it handed out in spans of 8 blocks the 16 sequences
-// took 159 us.  Batches with several items per CTA keep the work-item kernels (balanced_decode in fa_capi.cu).
+// all of them in the order of the line (the same bits every time).  The counters of the arriving pieces are zero again
+// after every call whose waits did not run out; a CTA that gave up leaves some of them behind.  The status word, which
+// the caller then still has, says so: a call that finds it set cuts nothing and needs no counter.
+// A cut costs about 3.5 us of a CTA per piece, which is why the line is cut once per CTA and no finer: with half of it
+// handed out in spans of 8 blocks the 16 sequences took 159 us.  Batches with several items per CTA keep the work-item
+// kernels (balanced_decode in fa_capi.cu).
 struct LineCut {
   int spans, width, extra;       // the first `extra` spans have width + 1 blocks, the others width
   __device__ __forceinline__ int begin(int c) const { return c * width + min(c, extra); }
@@ -295,7 +298,9 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   int* s_pref = reinterpret_cast<int*>(sm + SM::kPrefOff);      // blocks before entry e (one head group)
   LineCut cut{};
   int groups = 1;
+  bool uncut = false;
   if constexpr (BAL) {
+    uncut = __ldcg(&p.status->error) != 0u;
     // ---- the line: lengths summed per thread over consecutive entries, then a block scan ----
     int* s_sum = reinterpret_cast<int*>(s_o);      // the merge area is not in use yet
     int E = p.batch * a.max_mtiles;
@@ -366,14 +371,27 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     int x = 0, x_end = 0, ent = 0;
     uint32_t pcnt = 0;
     if constexpr (BAL) {
-      if (span < cut.spans) { x = cut.begin(span); x_end = cut.begin(span + 1); }
-      if (x < x_end) {
-        int hi_e = a.use_list ? p.work[6] : p.batch * a.max_mtiles;    // the last entry with groups * s_pref[e] <= x
-        while (hi_e - ent > 1) {
-          const int mid = (ent + hi_e) >> 1;
-          if (s_pref[mid] * groups <= x) ent = mid; else hi_e = mid;
+      // the last entry with groups * s_pref[e] <= y
+      auto entry_of = [&](int y) {
+        int lo_e = 0, hi_e = a.use_list ? p.work[6] : p.batch * a.max_mtiles;
+        while (hi_e - lo_e > 1) {
+          const int mid = (lo_e + hi_e) >> 1;
+          if (s_pref[mid] * groups <= y) lo_e = mid; else hi_e = mid;
         }
+        return lo_e;
+      };
+      if (span < cut.spans) { x = cut.begin(span); x_end = cut.begin(span + 1); }
+      if (uncut) {      // what begins in the span, whole
+        const int line = cut.begin(cut.spans);
+        auto border_from = [&](int y) {
+          if (y >= line) return line;
+          const int e = entry_of(y), s0 = s_pref[e] * groups, len = s_pref[e + 1] - s_pref[e];
+          return s0 + (y - s0 + len - 1) / len * len;
+        };
+        x = border_from(x);
+        x_end = border_from(x_end);
       }
+      if (x < x_end) ent = entry_of(x);
     }
     while (ok) {
       int w = 0;

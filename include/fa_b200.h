@@ -45,7 +45,8 @@ enum {
    * successful call leaves them zero again).  The library then issues no memset for them. */
   FA_FLAG_WORKSPACE_CLEAN = 1,
   /* The same promise for the first 4096 bytes (with FA_FLAG_WORKSPACE_CLEAN): decode calls then need no memset for
-   * their arrival counters either. */
+   * their arrival counters either.  (A call whose waits ran out leaves counters behind and its error in the status
+   * word, the first of these bytes; calls that find an error there do without counters.) */
   FA_FLAG_WORKSPACE_CLEAN_4K = 2
 };
 

@@ -37,3 +37,21 @@ def test_rows_past_the_last_sequence_stay_as_they_are(spec, kw, cuda_device):
     # (the padding is part of total_q and may move the cuts: one rounding to 16 bits of values below 2)
     assert (out[:n].float() - tight.float()).abs().max().item() <= 2 ** -7
     torch.testing.assert_close(lse[:, :n], tight_lse, atol=1e-4, rtol=1e-5)
+
+
+@pytest.mark.parametrize("failed", [False, True])
+def test_decode_does_not_depend_on_what_an_earlier_call_left(failed, cuda_device):
+    """Counters between byte 256 and 4095 are not zero: the caller keeps the first 256 bytes only, or a call whose
+    waits ran out left them (its status word says so) and the caller goes on with the buffer."""
+    p = _problem(DECODE, cuda_device)
+    want, want_lse, ws = capi.fwd(p.q, p.k, p.v, check=True, **p.capi_kw())
+    ws.zero_()
+    ws[256:4096] = 1
+    flags = capi.FA_FLAG_WORKSPACE_CLEAN
+    if failed:
+        ws.view(torch.int32)[0] = 1
+        flags |= capi.FA_FLAG_WORKSPACE_CLEAN_4K
+    out, lse = torch.zeros_like(want), torch.zeros_like(want_lse)
+    capi.fwd(p.q, p.k, p.v, out=out, lse=lse, workspace=ws, flags=flags, **p.capi_kw())
+    assert (out.float() - want.float()).abs().max().item() <= 2 ** -7      # (another cut: one rounding to 16 bits)
+    torch.testing.assert_close(lse, want_lse, atol=1e-4, rtol=1e-5)
