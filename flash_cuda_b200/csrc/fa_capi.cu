@@ -256,6 +256,9 @@ static WidenPlan widen_plan(const FaFwdParams* p, const PlanInput& in, const Pla
   if (p->route != FA_ROUTE_AUTO || pl.route != FA_ROUTE_GENERAL || p->kv_dtype != FA_DT_FP8_E4M3 ||
       p->q_dtype == FA_DT_FP8_E4M3 || p->out_dtype == FA_DT_FP32 || p->num_splits > 0 || !in.tc_layout_ok)
     return wp;
+  // (the tensor-core and decode kernels take an approximate tanh, off by up to 2^-11 of the cap; these calls always
+  // had tanhf)
+  if (in.has_softcap) return wp;
   PlanInput tin = in;
   tin.kv_dtype = in.q_dtype;
   tin.page_size = 0;

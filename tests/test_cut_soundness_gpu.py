@@ -55,3 +55,22 @@ def test_decode_does_not_depend_on_what_an_earlier_call_left(failed, cuda_device
     capi.fwd(p.q, p.k, p.v, out=out, lse=lse, workspace=ws, flags=flags, **p.capi_kw())
     assert (out.float() - want.float()).abs().max().item() <= 2 ** -7      # (another cut: one rounding to 16 bits)
     torch.testing.assert_close(lse, want_lse, atol=1e-4, rtol=1e-5)
+
+
+@pytest.mark.parametrize("reqs", [[(90, 1500)], [(90, 1500), (1, 700), (4, 300)]], ids=["chunk", "mixed"])
+def test_softcap_over_an_e4m3_cache_keeps_the_exact_tanh(reqs, cuda_device):
+    """More rows than the decode kernel takes: the LSE is as far from 64 bits as 32-bit sums and tanhf (2 ulp of values
+    up to the cap, 30 * 2^-22) make it; the approximate tanh alone is off by up to 2^-11 of the cap, 0.015."""
+    p = W.make_problem("cap", reqs, hq=8, hkv=2, hd=128, page_size=64, kv_dtype="fp8", softcap=30.0, seed=302)
+    p.softmax_scale *= 12.0              # logits of the size of the cap
+    pd = p.to(cuda_device)
+    _, lse, _ = capi.fwd(pd.q, pd.k, pd.v, check=True, **pd.capi_kw())
+    q0 = 0
+    for b, (ql, kl) in enumerate(reqs):
+        k = p.k[p.page_table[b].long()].flatten(0, 1)[:kl].double()
+        seen = torch.arange(kl)[None] <= torch.arange(kl - ql, kl)[:, None]
+        for h in range(8):
+            s = p.q[q0:q0 + ql, h].double() @ k[:, h // 4].t() * p.k_descale[b, h // 4].double() * p.softmax_scale
+            z = (30.0 * torch.tanh(s / 30.0)).masked_fill(~seen, -float("inf")).logsumexp(1)
+            assert (lse[h, q0:q0 + ql].cpu().double() - z).abs().max().item() <= 1e-4
+        q0 += ql
