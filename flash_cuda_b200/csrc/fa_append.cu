@@ -241,6 +241,8 @@ struct WidenArgs {
   int32_t* lens;      // batch: key counts (the slabs are padded, so their offsets do not say)
   int64_t k_page, k_row, k_head, v_page, v_row, v_head;   // bytes
   int batch, hkv, rep, class_rows, cap_rows, page_size, page_table_stride, k_chunks, v_chunks;   // 16-byte chunks per head
+  const int32_t* leftpad_k;
+  int window_left;
 };
 
 __device__ __forceinline__ int widen_len(const WidenArgs& a, int b) {
@@ -304,6 +306,12 @@ __global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {
     const int b = lo, s0 = r0 - a.cu[b];
     if (a.take[b]) continue;                  // (what is left of the capacity before a sequence that did not fit)
     const int used = widen_len(a, b);
+    // The keys below vis_lo (leftpad, or in front of the first row's window) are seen by no row, and the page table need
+    // not say where they are: they are not read.  The attention kernel loads no 128-key block that lies below vis_lo
+    // as a whole; in the block that holds it the rows below become zeros (weight zero, finite).
+    int vis_lo = a.leftpad_k ? a.leftpad_k[b] : 0;
+    if (a.window_left >= 0) vis_lo = max(vis_lo, used - (a.cu_q[b + 1] - a.cu_q[b]) - a.window_left);
+    if (s0 + RB <= vis_lo / 128 * 128) continue;
     const int first = a.page_table ? 0 : a.cu_k[b];
     const int32_t* pt = a.page_table ? a.page_table + (int64_t)b * a.page_table_stride : nullptr;
 #pragma unroll 4
@@ -313,7 +321,7 @@ __global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {
       const int cc = is_v ? c - kc : c, hch = is_v ? a.v_chunks : a.k_chunks;
       const int h = cc / hch, w = cc - h * hch;
       uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (r < used) {
+      if (r >= vis_lo && r < used) {
         int64_t off;
         if (pt) {
           const int lp = r / a.page_size;
@@ -352,6 +360,7 @@ int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_r
   a.batch = kp.batch; a.hkv = kp.hkv; a.rep = kp.rep; a.class_rows = class_rows; a.cap_rows = cap_rows;
   a.page_size = kp.page_size; a.page_table_stride = kp.page_table_stride;
   a.k_chunks = kp.hd / 16; a.v_chunks = kp.hdv / 16;
+  a.leftpad_k = kp.leftpad_k; a.window_left = kp.window_left;
   widen_plan_kernel<<<1, 256, 0, stream>>>(a);
   int blocks = (cap_rows + 7) / 8;
   if (blocks > num_sms * 8) blocks = num_sms * 8;

@@ -74,3 +74,17 @@ def test_softcap_over_an_e4m3_cache_keeps_the_exact_tanh(reqs, cuda_device):
             z = (30.0 * torch.tanh(s / 30.0)).masked_fill(~seen, -float("inf")).logsumexp(1)
             assert (lse[h, q0:q0 + ql].cpu().double() - z).abs().max().item() <= 1e-4
         q0 += ql
+
+
+@pytest.mark.parametrize("page_size", [16, 64])
+def test_pages_that_no_row_sees_need_no_entry(page_size, cuda_device):
+    """A serving program gives pages back that have left the window; their entries may then hold anything."""
+    reqs, window, leftpad = [(90, 3000), (1, 700), (100, 1111)], 500, [0, 3, 900]
+    p = _problem(dict(reqs=reqs, hq=8, hkv=2, hd=128, page_size=page_size, kv_dtype="fp8", window_left=window,
+                      leftpad=leftpad), cuda_device)
+    want, want_lse, _ = capi.fwd(p.q, p.k, p.v, check=True, **p.capi_kw())
+    for b, (ql, kl) in enumerate(reqs):
+        first = max(kl - ql - window, leftpad[b])              # the first key that a row sees
+        p.page_table[b, :first // page_size] = -1
+    out, lse, _ = capi.fwd(p.q, p.k, p.v, check=True, **p.capi_kw())
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)
