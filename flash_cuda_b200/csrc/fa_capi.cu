@@ -326,9 +326,12 @@ struct WsLayout {
   size_t part_ml_off, part_o_off;   // balanced decode: pieces of cut (sequence, head) triples; part_o_off 0: none
   size_t total;
 };
-static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
+// `plain`: without the forms that a call is only faster with and that take scratch of their own (balanced decode, key-range
+// parts, widening): what fa_b200_fwd falls back to in a workspace that has no room for them.  `header` is the front of the
+// workspace that the layout leaves alone.
+static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = false, size_t header = kWsHeader) {
   WsLayout w{};
-  w.header = kWsHeader;
+  w.header = header;
   size_t off = w.header;
   auto carve_parts = [&](const Plan& pd) {
     w.parts = part_plan(p, pd);
@@ -346,7 +349,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
     off += w.o_bytes;
   };
   w.tc_splits = 1;
-  if (pl.route == FA_ROUTE_GENERAL) {
+  if (pl.route == FA_ROUTE_GENERAL && !plain) {
     const PlanInput in = plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0));
     w.widen = widen_plan(p, in, pl);
     if (w.widen.on) {
@@ -370,7 +373,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
       return w;
     }
   }
-  if (balanced_decode(p, pl)) {
+  if (!plain && balanced_decode(p, pl)) {
     carve_parts(pl);
     w.total = off;
     return w;
@@ -384,7 +387,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
     const PlanInput in = plan_input(p, pl.num_sms);
     if (mixed_batch(p, in, pl)) {
       const Plan pd = decode_part_plan(in, pl);
-      if (balanced_decode(p, pd, true)) {
+      if (!plain && balanced_decode(p, pd, true)) {
         carve_parts(pd);
       } else {
         w.work_off = off;
@@ -410,7 +413,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl) {
       off += vb;
     }
   }
-  if (pl.route == FA_ROUTE_PREFILL_TC)
+  if (pl.route == FA_ROUTE_PREFILL_TC && !plain)
     w.tc_splits = tc_splits(p, plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0)), pl);
   if (pl.nsplits > 1 || w.tc_splits > 1) carve_splits(pl.nsplits > 1 ? pl.nsplits : w.tc_splits);
   w.total = off;
@@ -521,7 +524,10 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   Plan pl = make_plan(in);
   if (pl.err != FA_OK) return pl.err;
   WsLayout w = ws_layout(p, pl);
-  if (!workspace || workspace_bytes < w.total || ((uintptr_t)workspace % 256)) return FA_ERR_WORKSPACE;
+  if (!workspace || ((uintptr_t)workspace % 256)) return FA_ERR_WORKSPACE;
+  if (workspace_bytes < w.total)
+    w = ws_layout(p, pl, true, (p->flags & FA_FLAG_WORKSPACE_CLEAN_4K) ? kWsHeader : kWsArrivalOff);
+  if (workspace_bytes < w.total) return FA_ERR_WORKSPACE;
   if (p->total_q == 0 || p->batch == 0) return FA_OK;
 
   // Only the decode and the tensor-core prefill kernels read the metadata; the general kernel has no use for it, and

@@ -296,10 +296,20 @@ std::vector<at::Tensor> mha_fwd(
   const EnvConfig& env = env_config();
   p.route = env.route;
 
-  const size_t ws_bytes = fa_b200_fwd_workspace_bytes(&p);
   auto stream = at::cuda::getCurrentCUDAStream();
   bool clean = false;
-  at::Tensor ws = cached_workspace(q, stream.stream(), (int64_t)ws_bytes, &clean);
+  at::Tensor ws;
+  try {
+    ws = cached_workspace(q, stream.stream(), (int64_t)fa_b200_fwd_workspace_bytes(&p), &clean);
+  } catch (const c10::OutOfMemoryError&) {
+    // no memory for the scratch that makes the call faster: the uncut form needs next to none (a work list made for
+    // splits does not fit it)
+    if (p.num_splits == 1) throw;
+    p.num_splits = 1;
+    p.scheduler_metadata = nullptr;
+    p.scheduler_metadata_len = 0;
+    ws = cached_workspace(q, stream.stream(), (int64_t)fa_b200_fwd_workspace_bytes(&p), &clean);
+  }
   if (clean) p.flags |= FA_FLAG_WORKSPACE_CLEAN | FA_FLAG_WORKSPACE_CLEAN_4K;
   const int rc = fa_b200_fwd(&p, ws.data_ptr(), (size_t)ws.numel(), (fa_stream_t)stream.stream());
   if (rc == FA_ERR_UNSUPPORTED) {

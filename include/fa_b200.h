@@ -108,6 +108,9 @@ typedef struct FaFwdParams {
 
 /* Bytes of scratch fa_b200_fwd needs for `p` (split partials, work list, status word). Host-only
  * arithmetic. The caller allocates it (256-byte aligned) and may reuse it across calls on one stream.
+ * A smaller workspace is enough as long as the plain form of the call fits it (no key range cut for balance, no widened
+ * copy of an e4m3 cache): 256 bytes, the work lists and the partials of fa_b200_num_splits splits; the call is then
+ * slower.
  * Replaces the per-call `at::empty` scratch of `launch_ws_paged` (kernels/fa4_blackwell.cu:9737-9738). */
 size_t fa_b200_fwd_workspace_bytes(const FaFwdParams* p);
 

@@ -5,7 +5,7 @@ import ctypes as C
 import pytest
 import torch
 
-from flash_cuda_b200 import capi, workloads as W
+from flash_cuda_b200 import capi, ops, workloads as W
 from oracle.ref_attention import ref_attention
 
 pytestmark = pytest.mark.gpu
@@ -88,3 +88,51 @@ def test_pages_that_no_row_sees_need_no_entry(page_size, cuda_device):
         p.page_table[b, :first // page_size] = -1
     out, lse, _ = capi.fwd(p.q, p.k, p.v, check=True, **p.capi_kw())
     assert torch.equal(out, want) and torch.equal(lse, want_lse)
+
+
+@pytest.mark.parametrize("spec", [PARTS, MIXED, WIDEN, DECODE], ids=["parts", "mixed", "widened", "decode"])
+def test_a_workspace_for_the_plain_form_is_enough(spec, cuda_device):
+    """What only makes a call faster is left out where the workspace has no room for it."""
+    p = _problem(spec, cuda_device)
+    want, want_lse, _ = capi.fwd(p.q, p.k, p.v, check=True, **p.capi_kw())
+    lib = capi.load()
+    out, lse = torch.zeros_like(want), torch.zeros_like(want_lse)
+    fp, keep = capi.make_params(p.q, p.k, p.v, out, lse, **p.capi_kw())
+    # header, one work list of 16-byte entries per kernel, and the split partials that num_splits = 0 stands for
+    splits = lib.fa_b200_num_splits(C.byref(fp))
+    rows = p.q.shape[0] * p.q.shape[1]
+    need = 256 + 2 * 4096 + (0 if splits == 1 else splits * rows * (p.v.shape[-1] + 1) * 4 + 512)
+    assert lib.fa_b200_fwd_workspace_bytes(C.byref(fp)) > need
+    ws = torch.full((need + (1 << 20),), 7, device=cuda_device, dtype=torch.uint8)
+    rc = lib.fa_b200_fwd(C.byref(fp), ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream)
+    assert rc == capi.FA_OK, rc
+    capi.check_status(ws)
+    assert (ws[need:] == 7).all()
+    tol = 2 ** -6 if spec is WIDEN else 2 ** -7       # one rounding of the result; over e4m3 also of P in another kernel
+    assert (out.float() - want.float()).abs().max().item() <= tol
+    torch.testing.assert_close(lse, want_lse, atol=1e-3, rtol=1e-4)
+    del keep
+    assert lib.fa_b200_fwd(C.byref(fp), ws.data_ptr(), 128, torch.cuda.current_stream().cuda_stream) == capi.FA_ERR_WORKSPACE
+
+
+def test_the_op_runs_without_memory_for_its_scratch(cuda_device):
+    """The memory limit of the allocator leaves no room for the partial results of a prefill in parts (70 MB here)."""
+    p = _problem(dict(PARTS, reqs=[(600, 16000)], hq=32, hkv=8), cuda_device)
+    out = torch.empty_like(p.q)
+    want, _ = ops.call_fwd(p.q, p.k, p.v, num_splits=1, **p.capi_kw())
+    fp, keep = capi.make_params(p.q, p.k, p.v, out, torch.empty(32, 600, device=cuda_device), **p.capi_kw())
+    scratch = capi.load().fa_b200_fwd_workspace_bytes(C.byref(fp))
+    assert scratch > 16 << 20
+    stream = torch.cuda.Stream()         # (its workspace is not there yet)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(cuda_device).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (8 << 20)) / total)
+    try:
+        with torch.cuda.stream(stream):
+            got, _ = ops.call_fwd(p.q, p.k, p.v, out=out, **p.capi_kw())
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got, want)
+    del keep
