@@ -281,15 +281,30 @@ static WidenPlan widen_plan(const FaFwdParams* p, const PlanInput& in, const Pla
   return wp;
 }
 
-// Key-range parts per work item of the tensor-core prefill kernel (1 = none), from a model of its time: items of
-// `tile_m` rows run in whole waves over the SMs, 1.8 us per key block of 2 x 128 rows at 256 columns; parts leave as
-// fp32 and are merged (a launch, and 8 bytes per row and column through memory).  A chunk of 512 rows over 24500
-// keys has 64 items for 148 SMs.  Taken where the model says a tenth is saved.
-static int tc_splits(const FaFwdParams* p, const PlanInput& in, const Plan& pl) {
-  if (pl.route != FA_ROUTE_PREFILL_TC || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 || p->total_q <= 0) return 1;
-  const long long n = (long long)p->hq * ceil_div(p->total_q, pl.tile_m);
-  if (n >= 2 * pl.num_sms || p->hdv % 4) return 1;
-  // (max_seqlen_k may be a loose bound: a packed K/V says how many keys a sequence has on average)
+// Key-range parts per work item of the tensor-core prefill kernel (most = 1: none).  A chunk of 512 rows over 24500 keys
+// has 64 items for 148 SMs; parts fill the others.  Only as many as fit on the SMs at once: over shapes of 128 .. 2048
+// rows x 1000 .. 24500 keys, 8 .. 32 heads and head_dim 64 .. 256 the best count was always num_sms / items, and a second
+// wave of shorter parts lost what it was to balance (those 64 items: whole 322 us, 2 parts 191, 3 parts 251, 4 parts 201,
+// 8 parts 224), since every part pays for filling its pipeline and for its fp32 rows.  `classed`: the short sequences of
+// the batch are another kernel's.
+static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, bool classed) {
+  TcCut t{1, 0, 0};
+  if (pl.route != FA_ROUTE_PREFILL_TC || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 || p->total_q <= 0) return t;
+  if (p->hdv % 4 || (long long)p->hq * p->hdv > (1ll << 25)) return t;
+  if ((long long)p->batch * p->hq * pl.max_mtiles * 16 > 0x7fffffff) return t;
+  // items: sequences of equal length (the batch's tokens are all that is known), without the one-token ones if those are
+  // not this kernel's
+  long long seqs = p->batch, rows = p->total_q;
+  if (classed && p->max_seqlen_q > 1 && rows > seqs) {
+    const long long other = p->max_seqlen_q - 1, n_long = (rows - seqs + other - 1) / other;
+    if (n_long < seqs) { rows -= seqs - n_long; seqs = n_long; }
+  }
+  const long long per_seq = (rows + seqs - 1) / seqs, n = p->hq * seqs * ((per_seq + pl.tile_m - 1) / pl.tile_m);
+  long long most = pl.num_sms / n;
+  if (most > 16) most = 16;
+  if (most < 2) return t;
+  // (max_seqlen_k may be a loose bound: a packed K/V says how many keys a sequence has on average; the kernel cuts an
+  // item by its true keys)
   double keys = p->max_seqlen_k;
   if (!p->page_table && (double)p->total_k / p->batch < keys) keys = (double)p->total_k / p->batch;
   if (p->page_table && (double)p->num_pages * p->page_size < keys) keys = (double)p->num_pages * p->page_size;
@@ -298,16 +313,14 @@ static int tc_splits(const FaFwdParams* p, const PlanInput& in, const Plan& pl) 
     const double w = (in.window_left + (in.window_right > 0 ? in.window_right : 0) + pl.tile_m) / 128.0 + 1.0;
     if (w < blocks) blocks = w;
   }
-  const double t_block = 1.8 * (p->hd + p->hdv) / 256.0 * pl.tile_m / 256.0;
-  const double part_us = (double)p->total_q * p->hq * p->hdv * 8.0 / 4.0e6;
-  double best = 0.9 * (double)((n + pl.num_sms - 1) / pl.num_sms) * blocks * t_block;
-  int s = 1;
-  for (int c = 2; c <= 16 && blocks / c >= 4.0; ++c) {
-    if ((size_t)c * p->total_q * p->hq * (p->hdv + 1) * 4 > ((size_t)128 << 20)) break;
-    const double t = (double)((n * c + pl.num_sms - 1) / pl.num_sms) * (blocks / c * t_block + 1.5) + 4.0 + c * part_us;
-    if (t < best) { best = t; s = c; }
-  }
-  return s;
+  // 1.8 us per key block of 2 x 128 rows at 256 columns; 8 bytes per row and column of a part through memory
+  t.block_ns = (int)(1800.0 * (p->hd + p->hdv) / 256.0 * pl.tile_m / 256.0);
+  t.part_ns = (int)((double)rows * p->hq * p->hdv * 8.0 / 4.0e3);
+  const size_t part_bytes = (size_t)p->total_q * p->hq * (p->hdv + 1) * 4;
+  while (most > 1 && most * part_bytes > ((size_t)128 << 20)) --most;
+  t.most = (int)most;
+  t.most = tc_item_parts((int)blocks, t);
+  return t;
 }
 
 // ---- workspace layout ----
@@ -319,7 +332,7 @@ struct WsLayout {
   size_t work2_off, work2_bytes;   // mixed batches: the prefill kernel's list
   size_t lse_off, lse_bytes;
   size_t o_off, o_bytes;
-  int tc_splits;      // tensor-core prefill: key-range parts per item; their partials lie at lse_off / o_off
+  TcCut cut;          // tensor-core prefill: key-range parts per item; their partials lie at lse_off / o_off
   WidenPlan widen;
   size_t wd_cu_off, wd_take_off, wd_lens_off, wd_k_off, wd_v_off;
   PartPlan parts;
@@ -348,7 +361,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = fal
     w.o_bytes = align_up((size_t)nsplits * p->total_q * p->hq * p->hdv * 4, 256);
     off += w.o_bytes;
   };
-  w.tc_splits = 1;
+  w.cut = TcCut{1, 0, 0};
   if (pl.route == FA_ROUTE_GENERAL && !plain) {
     const PlanInput in = plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0));
     w.widen = widen_plan(p, in, pl);
@@ -363,8 +376,8 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = fal
       w.work2_bytes = align_up((size_t)sched_len(w.widen.tc, p->batch) * 4, 256);
       off += w.work2_bytes;
       if (w.widen.class_rows > 0) carve_parts(decode_part_plan(in, pl));
-      w.tc_splits = tc_splits(p, in, w.widen.tc);
-      if (w.tc_splits > 1) carve_splits(w.tc_splits);
+      w.cut = tc_cut(p, in, w.widen.tc, w.widen.class_rows > 0);
+      if (w.cut.most > 1) carve_splits(w.cut.most);
       w.wd_k_off = off;
       off += align_up((size_t)w.widen.cap_rows * p->hkv * p->hd * 2, 256);
       w.wd_v_off = off;
@@ -414,8 +427,8 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = fal
     }
   }
   if (pl.route == FA_ROUTE_PREFILL_TC && !plain)
-    w.tc_splits = tc_splits(p, plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0)), pl);
-  if (pl.nsplits > 1 || w.tc_splits > 1) carve_splits(pl.nsplits > 1 ? pl.nsplits : w.tc_splits);
+    w.cut = tc_cut(p, plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0)), pl, w.work2_bytes > 0);
+  if (pl.nsplits > 1 || w.cut.most > 1) carve_splits(pl.nsplits > 1 ? pl.nsplits : w.cut.most);
   w.total = off;
   return w;
 }
@@ -580,7 +593,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   kp.q_fp8 = p->q_dtype == FA_DT_FP8_E4M3; kp.kv_fp8 = p->kv_dtype == FA_DT_FP8_E4M3;
   kp.is_causal = in.is_causal; kp.window_left = in.window_left; kp.window_right = in.window_right;
   kp.nsplits = pl.nsplits;
-  kp.tc_splits = 1;
+  kp.tc_cut = TcCut{1, 0, 0};
   kp.out_f32 = p->out_dtype == FA_DT_FP32;
   kp.work_expect = SchedExpect{p->batch, pl.nsplits, pl.tile_m, pl.tile_n, pl.max_mtiles, pl.rows_per_token, pl.route};
   kp.scale = p->softmax_scale; kp.softcap = p->softcap;
@@ -599,22 +612,22 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   sp.max_seqlen_k = p->max_seqlen_k; sp.hq = p->hq; sp.hkv = p->hkv; sp.hd = p->hd; sp.hdv = p->hdv;
   sp.is_causal = in.is_causal; sp.window_left = in.window_left; sp.window_right = in.window_right;
 
-  // the tensor-core kernel over `kt`, in key-range parts with their merge where the plan says so (the merge writes
-  // every row of the call: what other kernels of the call own is launched after it)
-  auto run_prefill = [&](KParams kt, const Plan& plt) -> int {
-    if (w.tc_splits <= 1) return note_cuda_error(launch_prefill_tc(kt, plt, compute_dtype, stream), "tcgen05 prefill kernel");
-    float* o_part = (float*)(ws + w.o_off);
-    float* lse_part = (float*)(ws + w.lse_off);
-    kt.tc_splits = w.tc_splits;
-    kt.out = o_part; kt.lse = lse_part; kt.out_f32 = 1; kt.s_aux = nullptr;
-    kt.o_row_stride = (int64_t)p->hq * p->hdv; kt.o_head_stride = p->hdv;
-    kt.o_split_stride = (int64_t)p->total_q * p->hq * p->hdv;
-    kt.lse_split_stride = (int64_t)p->hq * p->total_q;
+  // the tensor-core kernel over `kt`, in key-range parts with their merge where the plan says so; `class_rows` and `skip`
+  // say which sequences are other kernels'
+  auto run_prefill = [&](KParams kt, const Plan& plt, int class_rows, const int32_t* skip) -> int {
+    if (w.cut.most > 1) {
+      kt.tc_cut = w.cut;
+      kt.whole_out = kt.out; kt.whole_lse = kt.lse; kt.whole_s_aux = kt.s_aux;
+      kt.whole_row_stride = kt.o_row_stride; kt.whole_head_stride = kt.o_head_stride;
+      kt.out = ws + w.o_off; kt.lse = (float*)(ws + w.lse_off); kt.out_f32 = 1; kt.s_aux = nullptr;
+      kt.o_row_stride = (int64_t)p->hq * p->hdv; kt.o_head_stride = p->hdv;
+      kt.o_split_stride = (int64_t)p->total_q * p->hq * p->hdv;
+      kt.lse_split_stride = (int64_t)p->hq * p->total_q;
+    }
     int r = note_cuda_error(launch_prefill_tc(kt, plt, compute_dtype, stream), "tcgen05 prefill kernel");
-    if (r != FA_OK) return r;
-    return note_cuda_error(launch_combine(o_part, lse_part, w.tc_splits, p->total_q, p->hq, p->hdv, p->s_aux, p->out,
-                                          p->o_row_stride, p->o_head_stride, p->out_dtype, p->lse, stream,
-                                          p->cu_seqlens_q + p->batch), "combine kernel");
+    if (r == FA_OK && w.cut.most > 1)
+      r = note_cuda_error(launch_merge_parts(kt, plt.tile_m, class_rows, skip, p->out_dtype, stream), "merge kernel");
+    return r;
   };
   // the decode kernel over the short sequences of a batch that also holds long ones
   auto run_short = [&](const int32_t* list) -> int {
@@ -647,7 +660,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     if (rc != FA_OK) return rc;
     KParams kt = kp;
     kt.work = list_p;
-    rc = run_prefill(kt, pl);
+    rc = run_prefill(kt, pl, kDecodeMaxRows, nullptr);
     if (rc == FA_OK) rc = run_short(list_d);
   } else if (w.widen.on) {
     // 16-bit queries over an e4m3 cache: see widen_plan
@@ -672,7 +685,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     kt.cu_k = cu;
     kt.seqused_k = (const int32_t*)(ws + w.wd_lens_off);
     kt.total_k = wp.cap_rows;
-    rc = run_prefill(kt, wp.tc);
+    rc = run_prefill(kt, wp.tc, wp.class_rows, take);
     if (rc == FA_OK && wp.may_overflow) {
       KParams kg = kp;
       kg.take = take;
@@ -696,7 +709,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
       kp.cu_k = cu;                              // slab b starts at row b * kpad; lengths still come from seqused_k
       kp.total_k = p->batch * w.dp_kpad;
     }
-    rc = run_prefill(kp, pl);
+    rc = run_prefill(kp, pl, 0, nullptr);
   } else {
     rc = note_cuda_error(launch_general(kp, compute_dtype, p->out_dtype, pl.num_sms, stream), "general kernel");
   }

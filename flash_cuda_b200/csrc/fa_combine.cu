@@ -18,22 +18,11 @@ constexpr float kLn2C = 0.6931471805599453f;
 // larger, no kernel wrote partials of the rows behind, and the caller's rows there stay as they are.
 // ------------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ o_part,
-                                                      const float* __restrict__ lse_part, int64_t o_split_stride,
-                                                      int64_t lse_split_stride, int nsplits, int total_q,
-                                                      int hq, int hdv, const float* __restrict__ s_aux,
-                                                      T* __restrict__ out, int64_t o_row_stride,
-                                                      int64_t o_head_stride, float* __restrict__ lse,
-                                                      const int32_t* __restrict__ rows_end) {
-  const int vec = hdv >> 2;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)total_q * hq * vec) return;
-  const int dv = (int)(idx % vec) * 4;
-  const int64_t qh = idx / vec;
-  const int h = (int)(qh % hq);
-  const int64_t qi = qh / hq;
-  const int64_t end = rows_end != nullptr ? *rows_end : total_q;      // (looked at where the row is written: one wait less)
-
+__device__ __forceinline__ void combine_unit(const float* __restrict__ o_part, const float* __restrict__ lse_part,
+                                             int64_t o_split_stride, int64_t lse_split_stride, int nsplits, int total_q,
+                                             int hq, int hdv, const float* __restrict__ s_aux, T* __restrict__ out,
+                                             int64_t o_row_stride, int64_t o_head_stride, float* __restrict__ lse,
+                                             int64_t qi, int h, int dv, int64_t end) {
   float g = -INFINITY;
   const int64_t lse_idx = (int64_t)h * total_q + qi;
   const int64_t o_idx = (qi * hq + h) * hdv + dv;
@@ -78,6 +67,69 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
   if (qi >= end) return;
   *reinterpret_cast<uint2*>(op) = packed;
   if (dv == 0) lse[(int64_t)h * total_q + qi] = g + lg2(L) * kLn2C;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ o_part,
+                                                      const float* __restrict__ lse_part, int64_t o_split_stride,
+                                                      int64_t lse_split_stride, int nsplits, int total_q,
+                                                      int hq, int hdv, const float* __restrict__ s_aux,
+                                                      T* __restrict__ out, int64_t o_row_stride,
+                                                      int64_t o_head_stride, float* __restrict__ lse,
+                                                      const int32_t* __restrict__ rows_end) {
+  const int vec = hdv >> 2;
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (int64_t)total_q * hq * vec) return;
+  const int dv = (int)(idx % vec) * 4;
+  const int64_t qh = idx / vec;
+  const int64_t end = rows_end != nullptr ? *rows_end : total_q;      // (looked at where the row is written: one wait less)
+  combine_unit<T>(o_part, lse_part, o_split_stride, lse_split_stride, nsplits, total_q, hq, hdv, s_aux, out, o_row_stride,
+                  o_head_stride, lse, qh / hq, (int)(qh % hq), dv, end);
+}
+
+// The merge behind a tensor-core prefill in key-range parts: the same arithmetic, over the parts that the item of a row
+// really has.  Rows of an item with a single part, of sequences that another kernel of the call runs and behind the last
+// sequence are left alone.  Block x = query row, y = 256 units of (head, 4 columns).
+template <typename T>
+__global__ void __launch_bounds__(256) merge_parts_kernel(const KParams p, int tile_m, int class_rows, const int32_t* skip) {
+  __shared__ int s_parts;
+  const int qi = blockIdx.x, vec = p.hdv >> 2;
+  if (threadIdx.x == 0) {
+    int parts = 0;
+    if (qi < p.cu_q[p.batch]) {
+      int b = 0, hi = p.batch;              // the sequence that owns the row: the last one with cu_q[b] <= qi
+      while (hi - b > 1) {
+        const int mid = (b + hi) >> 1;
+        if (p.cu_q[mid] <= qi) b = mid; else hi = mid;
+      }
+      const int q0 = p.cu_q[b], seqlen_q = p.cu_q[b + 1] - q0;
+      if (seqlen_q * p.rep > class_rows && !(skip && skip[b])) {
+        const int seqlen_k = p.seqused_k ? p.seqused_k[b] : p.cu_k[b + 1] - p.cu_k[b];
+        int lo, end;
+        tc_item_range(seqlen_q, seqlen_k, p.leftpad_k ? p.leftpad_k[b] : 0, (qi - q0) / tile_m * tile_m, tile_m, p.is_causal,
+                      p.window_left, p.window_right, &lo, &end);
+        parts = tc_item_parts(end - lo, p.tc_cut);
+      }
+    }
+    s_parts = parts;
+  }
+  __syncthreads();
+  const int u = blockIdx.y * 256 + threadIdx.x, parts = s_parts;
+  if (parts < 2 || u >= p.hq * vec) return;
+  combine_unit<T>(reinterpret_cast<const float*>(p.out), p.lse, p.o_split_stride, p.lse_split_stride, parts, p.total_q, p.hq,
+                  p.hdv, p.whole_s_aux, reinterpret_cast<T*>(p.whole_out), p.whole_row_stride, p.whole_head_stride,
+                  p.whole_lse, qi, u / vec, (u % vec) * 4, p.total_q);
+}
+
+int launch_merge_parts(const KParams& kp, int tile_m, int class_rows, const int32_t* skip, int out_dtype, cudaStream_t stream) {
+  if (kp.hdv % 4 != 0) return -1;
+  const int units = kp.hq * (kp.hdv / 4), y = (units + 255) / 256;
+  if (y > 65535) return -1;
+  if (kp.total_q <= 0 || y == 0) return 0;
+  const dim3 grid((unsigned)kp.total_q, (unsigned)y);
+  if (out_dtype == FA_DT_FP16) merge_parts_kernel<__half><<<grid, 256, 0, stream>>>(kp, tile_m, class_rows, skip);
+  else merge_parts_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(kp, tile_m, class_rows, skip);
+  return (int)cudaGetLastError();
 }
 
 int launch_combine_strided(const float* o_part, const float* lse_part, int64_t o_split_stride, int64_t lse_split_stride,

@@ -17,6 +17,23 @@ constexpr int kWsArrivalOff = 256;
 constexpr int kWsArrivalWords = (kWsHeader - kWsArrivalOff) / 4;
 constexpr int kBalancedEntriesMax = 2048;   // (sequence, row tile) entries a balanced decode call may have
 
+// Tensor-core prefill in key-range parts: into how many parts (at most `most`) an item of that many key blocks is cut.
+// The least of blocks / c blocks of block_ns each plus what c parts cost: 5.5 us, and part_ns for writing one as fp32
+// and reading it back; uncut where that saves less than a tenth.  Asked on the host with what it knows of the key count,
+// which may be no more than a loose bound, and on the device with the true range, by the attention kernel and the merge
+// behind it: integers, so that both get the same answer.
+struct TcCut { int most, block_ns, part_ns; };
+__host__ __device__ inline int tc_item_parts(int blocks, const TcCut& t) {
+  const long long whole = (long long)blocks * t.block_ns;
+  long long best = whole * 9 / 10;
+  int parts = 1;
+  for (int c = 2; c <= t.most && c * 2 <= blocks; ++c) {
+    const long long cost = whole / c + 5500 + (long long)c * t.part_ns;
+    if (cost < best) { best = cost; parts = c; }
+  }
+  return parts;
+}
+
 // Kernel-side view of one problem: FaFwdParams plus what the planner derived.
 struct KParams {
   const void* q;
@@ -54,8 +71,12 @@ struct KParams {
   int32_t q_fp8, kv_fp8;
   int32_t is_causal, window_left, window_right;
   int32_t nsplits;
-  int32_t tc_splits;                 // tensor-core prefill: key-range parts per work item; part s > 0 of `out` and `lse`
-  int64_t o_split_stride, lse_split_stride;   //             lies this many floats behind part s - 1 (out_f32 then)
+  TcCut tc_cut;                      // tensor-core prefill: most > 1 = work items in key-range parts; part s > 0 of `out`
+  int64_t o_split_stride, lse_split_stride;   //             and `lse` lies this many floats behind part s - 1 (out_f32 then);
+  void* whole_out;                   //             items of one part go to the caller's tensors
+  float* whole_lse;
+  const float* whole_s_aux;
+  int64_t whole_row_stride, whole_head_stride;
   int32_t part_rows;   // balanced decode: rows of a piece
   const int32_t* take; // general kernel: per sequence 1 = this kernel's, and at [batch] how many are; null = all
   int32_t class_rows;  // balanced decode: > 0 = only sequences with at most this many packed query rows
@@ -89,6 +110,20 @@ __host__ __device__ inline void nblock_range(int seqlen_k, int leftpad, int qp_m
   *hi = n_hi;
 }
 
+// Key blocks (of 128) that the rows [row0, row0 + rows) of one sequence see: the union over tiles of 128 rows.
+__host__ __device__ inline void tc_item_range(int seqlen_q, int seqlen_k, int leftpad, int row0, int rows, int is_causal,
+                                              int win_l, int win_r, int* lo, int* hi) {
+  *lo = 0x7fffffff;
+  *hi = 0;
+  for (int r = row0; r < row0 + rows && r < seqlen_q; r += 128) {
+    const int last = r + 127 < seqlen_q ? r + 127 : seqlen_q - 1, off = seqlen_k - seqlen_q;
+    int l, h;
+    nblock_range(seqlen_k, leftpad, off + r, off + last, is_causal, win_l, win_r, 128, &l, &h);
+    if (h > l) { *lo = l < *lo ? l : *lo; *hi = h > *hi ? h : *hi; }
+  }
+  if (*hi <= *lo) *lo = *hi = 0;
+}
+
 // Sub-range of [lo, hi) owned by split `s` of `nsplits`: contiguous chunks of ceil(total / nsplits).
 __host__ __device__ inline void split_range(int lo, int hi, int s, int nsplits, int* slo, int* shi) {
   int tot = hi - lo;
@@ -104,5 +139,8 @@ int launch_general(const KParams& kp, int dtype /*FA_DT_BF16|FP16 compute type*/
 int launch_combine(const float* o_part, const float* lse_part, int nsplits, int total_q, int hq, int hdv,
                    const float* s_aux, void* out, int64_t o_row_stride, int64_t o_head_stride, int out_dtype,
                    float* lse, cudaStream_t stream, const int32_t* rows_end = nullptr);
+// Merge of the key-range parts that launch_prefill_tc left with `kp` (items of tile_m rows): rows of sequences with more
+// than class_rows packed rows whose word in `skip` (may be null) is zero.
+int launch_merge_parts(const KParams& kp, int tile_m, int class_rows, const int32_t* skip, int out_dtype, cudaStream_t stream);
 
 }  // namespace fa

@@ -111,7 +111,7 @@ struct Smem {
 
 // One work item, decoded once by the TMA thread and handed to every role through shared memory (64 bytes).
 struct alignas(16) Item {
-  int b, h, pair, q0;   // h: head | key-range part << kPartShift (one word: the epilogue has no register for two)
+  int b, h, pair, q0;   // h: head | key-range part (or kWhole) << kPartShift (one word: the epilogue has no register for two)
   int seqlen_q, seqlen_k, k0, leftpad;
   int lo[2], hi[2];   // key-block range per tile
   int ulo, uhi;       // union
@@ -119,7 +119,7 @@ struct alignas(16) Item {
   int w;              // work id; kEndOfWork ends the role loops
 };
 static_assert(sizeof(Item) == 64, "mailbox slot");
-constexpr int kPartShift = 24, kHeadMask = (1 << kPartShift) - 1;
+constexpr int kPartShift = 24, kHeadMask = (1 << kPartShift) - 1, kWhole = 127;
 
 template <int NTL, bool PARTS>
 __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_entry) {
@@ -127,12 +127,13 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
   const KParams& p = a.kp;
   Item it;
   it.w = w;
-  // the key-range parts of an item are consecutive work ids
+  // the first parts of all items come first: what an item has no part for, the id's owner passes over, and where the
+  // keys turn out to be few those ids lie behind all the work
   int part = 0;
   if constexpr (PARTS) {
-    const int q = w / p.tc_splits;
-    part = w - q * p.tc_splits;
-    w = q;
+    const int items = a.use_list ? p.work[6] * p.hq : a.num_items / p.tc_cut.most;
+    part = w / items;
+    w -= part * items;
   }
   if (a.use_list) {
     // entry e of the sorted list = (batch, tile of item_rows rows); all q heads of one entry are consecutive work
@@ -193,18 +194,25 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
     if (it.hi[t] > it.lo[t]) { it.ulo = min(it.ulo, it.lo[t]); it.uhi = max(it.uhi, it.hi[t]); }
   }
   if (PARTS && it.valid) {
-    int plo, phi;
-    split_range(it.ulo, max(it.uhi, it.ulo), part, p.tc_splits, &plo, &phi);
-    it.ulo = 0x7fffffff;
-    it.uhi = 0;
+    const int parts = tc_item_parts(max(it.uhi - it.ulo, 0), p.tc_cut);
+    if (part >= parts) {
+      it.valid = 0;
+    } else if (parts == 1) {
+      it.h |= kWhole << kPartShift;
+    } else {
+      int plo, phi;
+      split_range(it.ulo, it.uhi, part, parts, &plo, &phi);
+      it.ulo = 0x7fffffff;
+      it.uhi = 0;
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      it.lo[t] = max(it.lo[t], plo);
-      it.hi[t] = min(it.hi[t], phi);
-      if (it.hi[t] > it.lo[t]) { it.ulo = min(it.ulo, it.lo[t]); it.uhi = max(it.uhi, it.hi[t]); }
-      else it.lo[t] = it.hi[t] = 0;
+      for (int t = 0; t < 2; ++t) {
+        it.lo[t] = max(it.lo[t], plo);
+        it.hi[t] = min(it.hi[t], phi);
+        if (it.hi[t] > it.lo[t]) { it.ulo = min(it.ulo, it.lo[t]); it.uhi = max(it.uhi, it.hi[t]); }
+        else it.lo[t] = it.hi[t] = 0;
+      }
+      it.h |= part << kPartShift;
     }
-    it.h |= part << kPartShift;
   }
   if (it.uhi <= it.ulo) { it.ulo = it.uhi = 0; }
   return it;
@@ -332,7 +340,7 @@ __device__ __forceinline__ void copy_tile_rows(uint32_t dst0, const unsigned cha
 // second softmax warpgroup stays idle and softmax and MMAs of the tile alternate instead of overlapping.
 // CAP: the logit soft cap is compiled in (the host picks the instantiation by softcap > 0, so that the common
 // kernel carries none of its code: the softmax loop's time follows its instruction count).
-// PARTS: an item is one of kp.tc_splits parts of its key range (the code for it, in the decoding of items and in the
+// PARTS: an item is one of kp.tc_cut.most parts of its key range (the code for it, in the decoding of items and in the
 // epilogue, cost the calls without parts 1 - 3 %).
 // PROD: the form of the TMA producer: 0 = contiguous K/V, lane 0 alone; 1 = paged, lane 0 alone; 2 = paged, the whole
 // warp (see the TMA role).  Template arguments rather than run-time flags for the same reason as CAP: code that a
@@ -449,7 +457,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       int num_items = a.num_items;
       if (a.use_list) {
         if (sched_header_matches(p.work, p.work_expect)) {
-          num_items = p.work[6] * p.hq * (PARTS ? p.tc_splits : 1);
+          num_items = p.work[6] * p.hq * (PARTS ? p.tc_cut.most : 1);
         } else {
           if (leader) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_TMA);
           num_items = 0;
@@ -1028,8 +1036,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
               for (int j = 0; j < 32; j += 2) {
                 const float2 x = fmul2(make_float2(__uint_as_float(sreg[c][j]), __uint_as_float(sreg[c][j + 1])), ci2);
                 const float2 y = ffma2(make_float2(tanh_fast(x.x), tanh_fast(x.y)), c2, nm2);
-                // tanh and exp2 share the special-function unit, which bounds this loop: every fourth pair
-                // takes its exponential on the FMA pipe
+                // tanh and exp2 share the special-function unit, which bounds this loop: half of the pairs
+                // take their exponential on the FMA pipe
                 const float2 pp = (((j >> 1) & 3) < kCapEmuPairs) ? ex2_poly2(y) : make_float2(ex2(y.x), ex2(y.y));
                 psum[(j >> 1) & 3] = fadd2(psum[(j >> 1) & 3], pp);
                 pk[j >> 1] = pack2<TO>(pp.x, pp.y);
@@ -1133,8 +1141,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         }
         float m_fin = m_used, l_fin = l, osc = 1.f;
         float l_norm = F8 ? lr : l;          // what O is divided by
-        if (p.s_aux) {
-          const float ys = p.s_aux[it.h] * kLog2e;
+        const bool whole = PARTS && (it.h >> kPartShift) == kWhole;      // (the only part: written like an uncut item)
+        const float* s_aux = PARTS ? (whole ? p.whole_s_aux : nullptr) : p.s_aux;
+        if (s_aux) {
+          const float ys = s_aux[PARTS ? it.h & kHeadMask : it.h] * kLog2e;
           const float mn = fmaxf(m_used, ys);
           osc = (m_used == -INFINITY) ? 0.f : ex2(m_used - mn);
           const float sink = ex2(ys - mn);
@@ -1177,8 +1187,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
               }
             }
           }
-        } else if (row_ok && (!PARTS || had_blocks)) {   // (the merge does not read an empty part's rows)
-          if (p.out_f32) {
+        } else if (row_ok && (!PARTS || had_blocks || whole)) {   // (the merge does not read an empty part's rows)
+          if (p.out_f32 && !whole) {
             float* op = reinterpret_cast<float*>(p.out) + (PARTS ? (int64_t)(it.h >> kPartShift) * p.o_split_stride : 0) +
                         (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.o_head_stride;
   #pragma unroll
@@ -1192,7 +1202,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
               }
             }
           } else {
-            TO* op = reinterpret_cast<TO*>(p.out) + (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)it.h * p.o_head_stride;
+            TO* op = PARTS ? reinterpret_cast<TO*>(p.whole_out) + (int64_t)(it.q0 + row) * p.whole_row_stride + (int64_t)(it.h & kHeadMask) * p.whole_head_stride
+                           : reinterpret_cast<TO*>(p.out) + (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)it.h * p.o_head_stride;
   #pragma unroll
             for (int c = 0; c < HDV / 32; ++c) {
               if (c * 32 < a.out_cols) {
@@ -1210,8 +1221,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           }
         }
         if (row_ok)
-          p.lse[(PARTS ? (int64_t)(it.h >> kPartShift) * p.lse_split_stride : 0) +
-                (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
+          (PARTS ? (whole ? p.whole_lse : p.lse + (int64_t)(it.h >> kPartShift) * p.lse_split_stride)
+                 : p.lse)[(int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
       } else {
         // HDV > 128 (one tile per item): the O row is read 64 columns at a time; O_t is released as soon as its last
         // column has been read.  Each 64-column group leaves like a half row of the two-tile form: staged + one TMA
@@ -1226,8 +1237,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         }
         float m_fin = m_used, l_fin = l, osc = 1.f;
         float l_norm = F8 ? lr : l;          // what O is divided by
-        if (p.s_aux) {
-          const float ys = p.s_aux[it.h] * kLog2e;
+        const bool whole = PARTS && (it.h >> kPartShift) == kWhole;      // (the only part: written like an uncut item)
+        const float* s_aux = PARTS ? (whole ? p.whole_s_aux : nullptr) : p.s_aux;
+        if (s_aux) {
+          const float ys = s_aux[PARTS ? it.h & kHeadMask : it.h] * kLog2e;
           const float mn = fmaxf(m_used, ys);
           osc = (m_used == -INFINITY) ? 0.f : ex2(m_used - mn);
           const float sink = ex2(ys - mn);
@@ -1282,8 +1295,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
                 bulk_commit_group();
               }
             }
-          } else if (row_ok && (!PARTS || had_blocks)) {
-            if (p.out_f32) {
+          } else if (row_ok && (!PARTS || had_blocks || whole)) {
+            if (p.out_f32 && !whole) {
               float* op = reinterpret_cast<float*>(p.out) + (PARTS ? (int64_t)(it.h >> kPartShift) * p.o_split_stride : 0) +
                         (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.o_head_stride + g * 64;
 #pragma unroll
@@ -1294,7 +1307,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
                       make_float4(__uint_as_float(o[c][j]) * inv, __uint_as_float(o[c][j + 1]) * inv,
                                   __uint_as_float(o[c][j + 2]) * inv, __uint_as_float(o[c][j + 3]) * inv);
             } else {
-              TO* op = reinterpret_cast<TO*>(p.out) + (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)it.h * p.o_head_stride + g * 64;
+              TO* op = PARTS ? reinterpret_cast<TO*>(p.whole_out) + (int64_t)(it.q0 + row) * p.whole_row_stride + (int64_t)(it.h & kHeadMask) * p.whole_head_stride + g * 64
+                             : reinterpret_cast<TO*>(p.out) + (int64_t)(it.q0 + row) * p.o_row_stride + (int64_t)it.h * p.o_head_stride + g * 64;
 #pragma unroll
               for (int c = 0; c < 2; ++c)
 #pragma unroll
@@ -1310,8 +1324,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           }
         }
         if (row_ok)
-          p.lse[(PARTS ? (int64_t)(it.h >> kPartShift) * p.lse_split_stride : 0) +
-                (int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
+          (PARTS ? (whole ? p.whole_lse : p.lse + (int64_t)(it.h >> kPartShift) * p.lse_split_stride)
+                 : p.lse)[(int64_t)(PARTS ? it.h & kHeadMask : it.h) * p.total_q + it.q0 + row] = l_fin > 0.f ? (m_fin + lg2(l_fin)) * kLn2 : -INFINITY;
       }
     }
     if constexpr (SM::kStageOut) {
@@ -1411,7 +1425,7 @@ static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t k
   a.kp = kp;
   a.item_rows = NTL * TM;
   a.max_pairs = (kp.max_seqlen_q + a.item_rows - 1) / a.item_rows;
-  a.num_items = kp.batch * kp.hq * a.max_pairs * kp.tc_splits;
+  a.num_items = kp.batch * kp.hq * a.max_pairs * kp.tc_cut.most;
   a.use_list = kp.work != nullptr;
   // bytes of K and V the batch can touch, against the L2 capacity the tiles of concurrently running heads share
   {
@@ -1457,7 +1471,7 @@ static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t k
 
 template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD>
 static int launch_prod(const KParams& kp, const Plan& pl, int dtype, uint64_t kv_rows, cudaStream_t stream) {
-  return kp.tc_splits > 1 ? launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, true>(kp, pl, dtype, kv_rows, stream)
+  return kp.tc_cut.most > 1 ? launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, true>(kp, pl, dtype, kv_rows, stream)
                           : launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, false>(kp, pl, dtype, kv_rows, stream);
 }
 

@@ -136,3 +136,16 @@ def test_the_op_runs_without_memory_for_its_scratch(cuda_device):
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert torch.equal(got, want)
     del keep
+
+
+@pytest.mark.parametrize("kw", [{}, dict(sink=True, window_left=300), dict(hd=192, hdv=128), dict(hd=256)],
+                         ids=["plain", "sink_window", "hd192", "hd256"])
+def test_few_keys_under_a_loose_bound_are_not_cut(kw, cuda_device):
+    """max_seqlen_k may be any upper bound: 600 keys in a table for 131072 give the bits of the uncut call."""
+    p = _problem(dict(PARTS, reqs=[(150, 600), (129, 700)]), cuda_device, **kw)
+    args = dict(p.capi_kw(), max_seqlen_k=131072)
+    pool = torch.zeros(2048 - p.k.shape[0], *p.k.shape[1:], device=cuda_device, dtype=p.k.dtype)     # (a pool of 131072 keys)
+    k, v = torch.cat([p.k, pool]), torch.cat([p.v, pool[..., :p.v.shape[-1]]])
+    out, lse, _ = capi.fwd(p.q, k, v, check=True, **args)
+    whole, whole_lse, _ = capi.fwd(p.q, k, v, check=True, num_splits=1, **args)
+    assert torch.equal(out, whole) and torch.equal(lse, whole_lse)
