@@ -39,8 +39,15 @@ constexpr int ncons_for(int) { return 4; }
 constexpr int ctas_per_sm(int esz) { return esz == 1 ? 2 : 1; }
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
-constexpr int kMinSpan = 2;            // balanced kernels: key blocks of a span at least (one sequence of 1000 keys: 16.1 us at 4, 14.4 at 2)
 constexpr int kPieces = 4;             // mailbox slots between the producer and the consumers
+// Balanced kernels, see LineCut (key blocks, about 0.65 us each with all SMs busy):
+constexpr int kMinSpan = 2;            // a piece has at least so many
+constexpr int kCutCost = 6;            // what cutting a triple costs the CTAs that share it: rows out, fence, atomic, merge
+constexpr int kCrossCost = 12;         // what a CTA pays for a span that begins and ends inside triples
+constexpr int kSnap = 8;               // a span border this close to the end of a triple moves there
+constexpr int kMaxPieces = 64;         // pieces of a triple at most ...
+constexpr int kMaxLinePieces = 96;     // ... and where spans cross sequences (what one CTA merges)
+constexpr int kMaxMerge = 104;         // (those, and a few more where borders moved)
 enum Role : unsigned { ROLE_PRODUCER = 5, ROLE_CONSUMER = 6 };
 enum : int { F_FIRST = 1, F_LAST = 2, F_EMPTY = 4 };
 
@@ -70,6 +77,7 @@ struct Smem {
   static constexpr int kScrOff = (kMiscOff + 16 + 15) / 16 * 16;
   static constexpr int kLdO = HDV + 4;
   static constexpr int kScrBytes = NC * 16 * kLdO * 4 + 2 * NC * 16 * 4;
+  static_assert(NC * 16 * kLdO >= 16 * kMaxMerge, "the merge's weights lie in the merge area");
   // balanced kernels: piece mailbox with its barriers, then the line's prefix sums
   static constexpr int kPieceOff = kScrOff + kScrBytes;
   static constexpr int kPieceBarOff = kPieceOff + kPieces * 80;   // full[kPieces], empty[kPieces], flag
@@ -127,23 +135,31 @@ __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
 // The team keeps the heads of a token, neighbours in memory, together in time: with the heads of a sequence one after
 // the other on the line (every CTA somewhere else, 256-byte rows 2 KB apart) the 16 sequences took 119 us, and 128
 // sequences of 1024 .. 32768 keys fell from 6.25 to 5.4 TB/s.
-// What lies inside one span is written out directly; the pieces of a (batch, row tile, head) that crosses span borders
-// go to `part_*` as unnormalised fp32 rows with their maximum and sum, and the CTA that finishes the last piece merges
-// all of them in the order of the line (the same bits every time).  The counters of the arriving pieces are zero again
-// after every call whose waits did not run out; a CTA that gave up leaves some of them behind.  The status word, which
-// the caller then still has, says so: a call that finds it set cuts nothing and needs no counter.
-// A cut costs about 3.5 us of a CTA per piece, which is why the line is cut once per CTA and no finer: with half of it
-// handed out in spans of 8 blocks the 16 sequences took 159 us.  Batches with several items per CTA keep the work-item
-// kernels (balanced_decode in fa_capi.cu).
+// What lies inside one span is written out directly; the pieces of a (batch, row tile, head) triple that several CTAs
+// share go to `part_*` as unnormalised fp32 rows with their maximum and sum, and the CTA that finishes the last piece
+// merges all of them in the order of the line (the same bits every time).  The counters of the arriving pieces are zero
+// again after every call whose waits did not run out; a CTA that gave up leaves some of them behind.  The status word,
+// which the caller then still has, says so: a call that finds it set cuts nothing and needs no counter.
+//
+// Where the line is cut.  Only the kernel knows the lengths, so every CTA plans the same from them:
+//   - no more (row tile, head group) triples than teams: each triple gets teams of its own, ceil(blocks / width) of them
+//     with the smallest width that the teams suffice for, unless that saves less than the cut costs (kCutCost: nothing
+//     of up to 8 blocks is cut).  No CTA then works on two triples: with equal spans over the line two sequences of 300
+//     keys took 17.7 us, since nearly every CTA had two halves to open, write out and merge.
+//   - otherwise, or where the lengths are so uneven that this leaves the longest piece above the line's mean by more than
+//     kCrossCost: equal spans over the whole line.  Borders that fall near the end of a triple move there.
+// A triple is never cut into more pieces than one CTA merges in a few microseconds.
 struct LineCut {
-  int spans, width, extra;       // the first `extra` spans have width + 1 blocks, the others width
+  int spans, width, extra;       // the first `extra` spans have width + 1 units, the others width
+  int total, snap;               // units of the line; borders move by at most this much (-1: always to the next triple)
   __device__ __forceinline__ int begin(int c) const { return c * width + min(c, extra); }
   __device__ __forceinline__ int span_of(int x) const {
     const int wide = extra * (width + 1);
     return x < wide ? x / (width + 1) : extra + (x - wide) / width;
   }
-  __device__ __forceinline__ void plan(int total, int max_spans) {
-    spans = max(1, min(max_spans, (total + kMinSpan - 1) / kMinSpan));
+  __device__ __forceinline__ void plan(int total_, int spans_) {
+    total = total_;
+    spans = max(1, spans_);
     width = total / spans;
     extra = total - width * spans;
   }
@@ -298,11 +314,10 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   int* s_pref = reinterpret_cast<int*>(sm + SM::kPrefOff);      // blocks before entry e (one head group)
   LineCut cut{};
   int groups = 1;
-  bool uncut = false;
+  bool own = false;      // every triple has teams of its own: a unit of the line is a piece; else a unit is a key block
   if constexpr (BAL) {
-    uncut = __ldcg(&p.status->error) != 0u;
-    // ---- the line: lengths summed per thread over consecutive entries, then a block scan ----
     int* s_sum = reinterpret_cast<int*>(s_o);      // the merge area is not in use yet
+    if (tid == 0) s_sum[30] = __ldcg(&p.status->error) != 0u;      // (one read: the CTA's threads must agree on the plan)
     int E = p.batch * a.max_mtiles;
     if (a.use_list) {
       // the list's header must describe this call before any entry is read
@@ -314,35 +329,93 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       for (int i = 0; i < kPieces; ++i) { mbar_init(bar_pc_full + 8 * i, 1); mbar_init(bar_pc_empty + 8 * i, NC); }
       mbar_fence_init();
     }
+    // ---- lengths: consecutive entries per thread; their sum, number and maximum ----
     constexpr int NTH = (NC + 1) * 32;
     const int per = (E + NTH - 1) / NTH, e_lo = min(E, tid * per), e_hi = min(E, e_lo + per);
-    int mine = 0;
+    int sum = 0, num = 0, longest = 0;
     bool bad = false;
     for (int e = e_lo; e < e_hi; ++e) {
       const WorkItem it = line_entry(a, e);
+      const int len = line_len(it);
       bad |= it.bad;
-      s_pref[e] = mine;
-      mine += line_len(it);
+      s_pref[e] = len;
+      sum += len; num += len > 0; longest = max(longest, len);
     }
     if (bad) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    num = __reduce_add_sync(0xffffffffu, num);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (lane == 0) { s_sum[warp] = sum; s_sum[8 + warp] = num; s_sum[16 + warp] = longest; }
+    __syncthreads();
+    const bool whole = s_sum[30] != 0;
+    sum = num = longest = 0;
+#pragma unroll
+    for (int w = 0; w <= NC; ++w) { sum += s_sum[w]; num += s_sum[8 + w]; longest = max(longest, s_sum[16 + w]); }
+    // ---- the plan ----
+    groups = p.hkv / a.team;
+    const int teams = (int)gridDim.x / a.team;
+    const int mean = (sum * groups + teams - 1) / teams;
+    int width = longest;             // blocks of a piece where triples have teams of their own
+    own = num * groups <= teams;
+    if (own && !whole && longest > kMinSpan + kCutCost) {
+      // the smallest of eight widths, from the least possible to 2.5 times that, for which the teams suffice
+      const int least = max(max(kMinSpan, mean), (longest + kMaxPieces - 1) / kMaxPieces);
+      constexpr int kTries = 8;
+      int need[kTries];
+#pragma unroll
+      for (int k = 0; k < kTries; ++k) need[k] = 0;
+      for (int e = e_lo; e < e_hi; ++e) {
+        const int len = s_pref[e];
+        int wd = least;
+#pragma unroll
+        for (int k = 0; k < kTries; ++k) { need[k] += (len + wd - 1) / wd; wd += (wd + 7) / 8; }
+      }
+#pragma unroll
+      for (int k = 0; k < kTries; ++k) need[k] = __reduce_add_sync(0xffffffffu, need[k]);
+      if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < kTries; ++k) s_sum[32 + warp * kTries + k] = need[k];
+      }
+      __syncthreads();
+      int wd = least, found = longest;
+#pragma unroll
+      for (int k = 0; k < kTries; ++k) {
+        int n = 0;
+#pragma unroll
+        for (int w = 0; w <= NC; ++w) n += s_sum[32 + w * kTries + k];
+        if (n * groups <= teams) found = min(found, wd);
+        wd += (wd + 7) / 8;
+      }
+      if (found + kCutCost < longest) width = found;
+      if (mean + kCrossCost < width + (width < longest ? kCutCost : 0)) own = false;
+    }
+    // ---- units of the line before each entry: blocks, or pieces ----
+    int mine = 0;
+    for (int e = e_lo; e < e_hi; ++e) {
+      const int len = s_pref[e];
+      s_pref[e] = mine;
+      mine += own ? (len + width - 1) / max(width, 1) : len;
+    }
     int incl = mine;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += v;
     }
-    if (lane == 31) s_sum[warp] = incl;
+    if (lane == 31) s_sum[24 + warp] = incl;
     __syncthreads();
     int total = 0, before = incl - mine;
 #pragma unroll
     for (int w = 0; w <= NC; ++w) {
-      if (w < warp) before += s_sum[w];
-      total += s_sum[w];
+      if (w < warp) before += s_sum[24 + w];
+      total += s_sum[24 + w];
     }
     for (int e = e_lo; e < e_hi; ++e) s_pref[e] += before;
     if (tid == 0) s_pref[E] = total;
-    groups = p.hkv / a.team;
-    cut.plan(total * groups, (int)gridDim.x / a.team);
+    total *= groups;
+    const int min_width = max(kMinSpan, (longest + kMaxLinePieces - 1) / kMaxLinePieces);
+    cut.plan(total, own ? total : min(teams, total / min_width));
+    cut.snap = whole ? -1 : min(kSnap, (cut.width - 1) / 2);
   }
   __syncthreads();
 
@@ -370,27 +443,26 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     const int span = BAL ? (int)blockIdx.x / a.team : 0, member = BAL ? (int)blockIdx.x - span * a.team : 0;
     int x = 0, x_end = 0, ent = 0;
     uint32_t pcnt = 0;
-    if constexpr (BAL) {
-      // the last entry with groups * s_pref[e] <= y
-      auto entry_of = [&](int y) {
-        int lo_e = 0, hi_e = a.use_list ? p.work[6] : p.batch * a.max_mtiles;
-        while (hi_e - lo_e > 1) {
-          const int mid = (lo_e + hi_e) >> 1;
-          if (s_pref[mid] * groups <= y) lo_e = mid; else hi_e = mid;
-        }
-        return lo_e;
-      };
-      if (span < cut.spans) { x = cut.begin(span); x_end = cut.begin(span + 1); }
-      if (uncut) {      // what begins in the span, whole
-        const int line = cut.begin(cut.spans);
-        auto border_from = [&](int y) {
-          if (y >= line) return line;
-          const int e = entry_of(y), s0 = s_pref[e] * groups, len = s_pref[e + 1] - s_pref[e];
-          return s0 + (y - s0 + len - 1) / len * len;
-        };
-        x = border_from(x);
-        x_end = border_from(x_end);
+    // the last entry with groups * s_pref[e] <= y
+    auto entry_of = [&](int y) {
+      int lo_e = 0, hi_e = a.use_list ? p.work[6] : p.batch * a.max_mtiles;
+      while (hi_e - lo_e > 1) {
+        const int mid = (lo_e + hi_e) >> 1;
+        if (s_pref[mid] * groups <= y) lo_e = mid; else hi_e = mid;
       }
+      return lo_e;
+    };
+    // where span c begins
+    auto line_begin = [&](int c) {
+      const int y = cut.begin(c);
+      if (own || cut.snap == 0 || y >= cut.total) return y;
+      const int e = entry_of(y), len = s_pref[e + 1] - s_pref[e], over = (y - s_pref[e] * groups) % len;
+      if (over == 0) return y;
+      if (cut.snap < 0) return y - over + len;
+      return over <= cut.snap ? y - over : len - over <= cut.snap ? y - over + len : y;
+    };
+    if constexpr (BAL) {
+      if (span < cut.spans) { x = line_begin(span); x_end = line_begin(span + 1); }
       if (x < x_end) ent = entry_of(x);
     }
     while (ok) {
@@ -400,24 +472,42 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         if (x >= x_end) break;
         while (x >= s_pref[ent + 1] * groups) ++ent;      // (entries without blocks are passed over)
         const int len = s_pref[ent + 1] - s_pref[ent], off = x - s_pref[ent] * groups;
-        const int hg = off / len, pos = off - hg * len, n = min(len - pos, x_end - x);
+        const int hg = off / len, pos = off - hg * len, n = own ? 1 : min(len - pos, x_end - x);
         it = line_entry(a, ent);
         it.hk = hg * a.team + member;
-        if (it.hi > it.lo) { it.lo += pos; it.hi = it.lo + n; }
+        int pieces = 1, first = span;      // of this triple, and the span that holds its first piece
+        if (own) {
+          const int lo = it.lo, blocks = it.hi - it.lo;
+          pieces = len;
+          first = span - pos;
+          it.lo = lo + (int)((int64_t)blocks * pos / len);
+          it.hi = lo + (int)((int64_t)blocks * (pos + 1) / len);
+        } else if (n != len) {
+          if (pos > 0) {
+            first = cut.span_of(x - pos);
+            while (first + 1 < cut.spans && line_begin(first + 1) <= x - pos) ++first;
+            while (line_begin(first) > x - pos) --first;
+          }
+          const int end = x - pos + len - 1;
+          int last = span;
+          if (end >= x_end) {
+            last = cut.span_of(end);
+            while (last + 1 < cut.spans && line_begin(last + 1) <= end) ++last;
+            while (line_begin(last) > end) --last;
+          }
+          pieces = last - first + 1;
+          it.lo += pos; it.hi = it.lo + n;
+        }
         const uint32_t slot = pcnt % kPieces;
         ok = wait_or_abort(bar_pc_empty + 8 * slot, ((pcnt / kPieces) & 1) ^ 1, s_abort);
         if (!ok) break;
         if (lane == 0) {
           Piece& pc = s_piece[slot];
           pc.it = it;
-          pc.pieces = 1;
-          pc.first = pc.number = member * cut.spans + span;
+          pc.pieces = pieces;
+          pc.number = member * cut.spans + span;
+          pc.first = member * cut.spans + first;
           pc.head = pos == 0;
-          if (n != len) {
-            const int s0 = cut.span_of(x - pos);
-            pc.pieces = cut.span_of(x - pos + len - 1) - s0 + 1;
-            pc.first = member * cut.spans + s0;
-          }
           mbar_arrive(bar_pc_full + 8 * slot);
         }
         ++pcnt;
@@ -907,28 +997,38 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
               }
               bar_consumers<NC>();
               if (*s_last) {
+                // piece j lies in slot 2 (first + j) + (j == 0).  Weights first, a warp per row and a lane per piece (the
+                // merge area is free: every warp has written its piece); then all threads over (row, 4 columns).  With
+                // every thread reading the pairs by itself, twice and one after the other, 148 pieces took some 20 us.
                 const int live = min(p.part_rows, rows_total - it.mt * 16), np = cur.pieces;
                 const int64_t s0 = (int64_t)cur.first * 2;
+                const float2* ml = reinterpret_cast<const float2*>(p.part_ml);
+                for (int r = warp; r < live; r += NC) {
+                  float Mx = -INFINITY, Ls = 0.f;
+                  for (int j = lane; j < np; j += 32) Mx = fmaxf(Mx, __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows + r).x);
+#pragma unroll
+                  for (int d = 16; d > 0; d >>= 1) Mx = fmaxf(Mx, __shfl_xor_sync(0xffffffffu, Mx, d));
+                  for (int j = lane; j < np; j += 32) {
+                    const float2 q2 = __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows + r);
+                    const float e = Mx > -INFINITY ? ex2(q2.x - Mx) : 0.f;   // (a piece without visible keys: exactly 0, its rows are 0)
+                    s_o[r * kMaxMerge + j] = e;
+                    Ls += e * q2.y;
+                  }
+#pragma unroll
+                  for (int d = 16; d > 0; d >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, d);
+                  if (lane == 0) { s_m[r] = Mx; s_l[r] = Ls; }
+                }
+                bar_consumers<NC>();
                 for (int u = tid; u < live * (HDV / 4); u += NC * 32) {
                   const int r = u / (HDV / 4), c4 = (u - r * (HDV / 4)) * 4;
-                  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + r;
                   const float* pr = p.part_o + (int64_t)r * HDV + c4;
-                  // piece j lies in slot 2 (first + j) + (j == 0)
-                  float Mx = -INFINITY;
-#pragma unroll 8
-                  for (int j = 0; j < np; ++j) Mx = fmaxf(Mx, __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows).x);
-                  float Ls = 0.f;
+                  float Mx = s_m[r], Ls = s_l[r];
                   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                  if (Mx > -INFINITY) {
 #pragma unroll 8
-                    for (int j = 0; j < np; ++j) {
-                      const int64_t sl = (s0 + 2 * j + (j == 0)) * p.part_rows;
-                      const float2 q2 = __ldcg(ml + sl);
-                      const float4 w4 = __ldcg(reinterpret_cast<const float4*>(pr + sl * HDV));
-                      const float e = ex2(q2.x - Mx);      // (a piece without visible keys: exactly 0, its rows are 0)
-                      Ls += e * q2.y;
-                      v.x += e * w4.x; v.y += e * w4.y; v.z += e * w4.z; v.w += e * w4.w;
-                    }
+                  for (int j = 0; j < np; ++j) {
+                    const float4 w4 = __ldcg(reinterpret_cast<const float4*>(pr + (s0 + 2 * j + (j == 0)) * p.part_rows * HDV));
+                    const float e = s_o[r * kMaxMerge + j];
+                    v.x += e * w4.x; v.y += e * w4.y; v.z += e * w4.z; v.w += e * w4.w;
                   }
                   const int Rg = it.mt * 16 + r, token = Rg / rep, head = it.hk * rep + Rg % rep;
                   const int64_t qi = it.q0 + token;
@@ -1094,15 +1194,15 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
 
 }  // namespace dec
 
-// Shapes the decode route takes: head_dim 64, 128 or 192 (values 128), 16-bit queries, a cache of the same type or
-// (head_dim 128) of e4m3 bytes, K/V contiguous or in pages of 1, 2, 4, 8, 16, 32 or a multiple of 64 keys (the small
-// pages row by row, as the reference's cp.async producer does for page size 1, kernels/fa4_blackwell.cu:8936-8947).  These are the
-// head dims of the reference's paged kernel (kernels/fa4_blackwell.cu:9958-9983).
 // CTAs of a balanced launch at most: each has scratch for two pieces and one arrival counter.
 int decode_line_ctas(int hd, int kv_dtype, int num_sms) {
   return num_sms * (hd == 64 || kv_dtype == FA_DT_FP8_E4M3 ? 2 : 1);
 }
 
+// Shapes the decode route takes: head_dim 64, 128 or 192 (values 128), 16-bit queries, a cache of the same type or
+// (head_dim 128) of e4m3 bytes, K/V contiguous or in pages of 1, 2, 4, 8, 16, 32 or a multiple of 64 keys (the small
+// pages row by row, as the reference's cp.async producer does for page size 1, kernels/fa4_blackwell.cu:8936-8947).  These are the
+// head dims of the reference's paged kernel (kernels/fa4_blackwell.cu:9958-9983).
 bool decode_supported(const PlanInput& in) {
   if (in.q_dtype == FA_DT_FP8_E4M3) return false;
   if (in.kv_dtype != in.q_dtype && in.kv_dtype != FA_DT_FP8_E4M3) return false;

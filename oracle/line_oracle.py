@@ -1,0 +1,85 @@
+"""CPU restatement of how the balanced decode kernel cuts a batch (`LineCut` and the plan in flash_cuda_b200/csrc/
+fa_decode.cu): from the key blocks of every (sequence, row tile) entry to the pieces each team of CTAs walks."""
+from __future__ import annotations
+
+from typing import Iterator, List, NamedTuple
+
+MIN_SPAN, CUT_COST, CROSS_COST, SNAP, MAX_PIECES, MAX_LINE_PIECES, MAX_MERGE = 2, 6, 12, 8, 64, 96, 104
+
+
+class Piece(NamedTuple):
+    span: int      # the team that walks it
+    entry: int
+    group: int     # of kv heads
+    lo: int        # key blocks [lo, hi) of the entry
+    hi: int
+    pieces: int    # of this (entry, group)
+    first: int     # the team with its first piece
+    head: bool     # this is the first piece
+
+
+def _up(a: int, b: int) -> int:
+    return -(-a // b)
+
+
+class Line:
+    def __init__(self, lens: List[int], groups: int, teams: int, whole: bool = False):
+        self.lens, self.groups = lens, groups
+        total, num, longest = sum(lens), sum(n > 0 for n in lens), max(lens, default=0)
+        mean, width = _up(total * groups, teams), longest
+        self.own = num * groups <= teams
+        if self.own and not whole and longest > MIN_SPAN + CUT_COST:
+            least = max(MIN_SPAN, mean, _up(longest, MAX_PIECES))
+            found, w = longest, least
+            for _ in range(8):
+                if sum(_up(n, w) for n in lens) * groups <= teams:
+                    found = min(found, w)
+                w += (w + 7) // 8
+            if found + CUT_COST < longest:
+                width = found
+            if mean + CROSS_COST < width + (CUT_COST if width < longest else 0):
+                self.own = False
+        self.pref = [0]
+        for n in lens:
+            self.pref.append(self.pref[-1] + (_up(n, max(width, 1)) if self.own else n))
+        self.total = self.pref[-1] * groups
+        least = max(MIN_SPAN, _up(longest, MAX_LINE_PIECES))
+        self.spans = max(1, self.total if self.own else min(teams, self.total // least))
+        self.width = self.total // self.spans
+        self.extra = self.total - self.width * self.spans
+        self.snap = -1 if whole else min(SNAP, max(self.width - 1, 0) // 2)
+
+    def _entry(self, y: int) -> int:
+        return max(e for e in range(len(self.lens)) if self.pref[e] * self.groups <= y)
+
+    def begin(self, c: int) -> int:
+        y = c * self.width + min(c, self.extra)
+        if self.own or self.snap == 0 or y >= self.total:
+            return y
+        e = self._entry(y)
+        n = self.pref[e + 1] - self.pref[e]
+        over = (y - self.pref[e] * self.groups) % n
+        if over == 0:
+            return y
+        if self.snap < 0 or (over > self.snap and n - over <= self.snap):
+            return y - over + n
+        return y - over if over <= self.snap else y
+
+    def pieces(self) -> Iterator[Piece]:
+        begins = [self.begin(c) for c in range(self.spans + 1)]
+        for span in range(self.spans):
+            x, end = begins[span], begins[span + 1]
+            while x < end:
+                e = self._entry(x)
+                n = self.pref[e + 1] - self.pref[e]
+                group, pos = divmod(x - self.pref[e] * self.groups, n)
+                if self.own:
+                    blocks = self.lens[e]
+                    yield Piece(span, e, group, blocks * pos // n, blocks * (pos + 1) // n, n, span - pos, pos == 0)
+                    x += 1
+                    continue
+                step = min(n - pos, end - x)
+                first = max(c for c in range(self.spans) if begins[c] <= x - pos)
+                last = max(c for c in range(self.spans) if begins[c] <= x - pos + n - 1)
+                yield Piece(span, e, group, pos, pos + step, last - first + 1, first, pos == 0)
+                x += step

@@ -1,0 +1,51 @@
+"""How the balanced decode kernel cuts a batch, on its CPU restatement: every key block is walked once, a team has
+scratch for the pieces it writes, and whoever merges knows all of them."""
+import random
+
+import pytest
+
+from oracle.line_oracle import CUT_COST, MAX_MERGE, MIN_SPAN, Line
+
+
+@pytest.mark.parametrize("seed", range(40))
+def test_every_block_once_and_every_piece_in_its_place(seed):
+    rng = random.Random(seed)
+    for _ in range(12):
+        n, groups = rng.choice([1, 2, 3, 8, 18, 20, 60]), rng.choice([1, 1, 2, 5])
+        teams, most = rng.choice([1, 2, 9, 18, 37, 148, 296]), rng.choice([1, 2, 5, 10, 20, 80, 400])
+        kind = rng.randrange(3)
+        lens = [most if kind == 0 else rng.randint(0, most) if kind == 1 else
+                rng.randint(0, 3) if rng.random() < 0.9 else rng.randint(1, 10 * most) for _ in range(n)]
+        whole = rng.random() < 0.2
+        line = Line(lens, groups, teams, whole)
+        assert line.spans <= teams
+        found, slots = {}, set()
+        for p in line.pieces():
+            found.setdefault((p.entry, p.group), []).append(p)
+            if p.pieces > 1:
+                assert not whole and (p.span, p.head) not in slots      # two rows of scratch per team
+                slots.add((p.span, p.head))
+        assert set(found) == {(e, g) for e in range(n) if lens[e] for g in range(groups)}
+        counters = [ps[0].first for ps in found.values() if len(ps) > 1]
+        assert len(set(counters)) == len(counters)                      # an arrival counter belongs to one triple
+        for (e, _), ps in found.items():
+            assert [p.lo for p in ps] + [lens[e]] == [0] + [p.hi for p in ps]
+            assert [p.span for p in ps] == [ps[0].span + j for j in range(len(ps))]
+            assert all(p.hi > p.lo and p.pieces == len(ps) and p.first == ps[0].span for p in ps)
+            assert len(ps) <= MAX_MERGE
+            assert len(ps) == 1 or lens[e] >= MIN_SPAN
+
+
+def test_short_sequences_are_not_cut_and_no_team_works_on_two_of_few():
+    for batch in range(1, 19):
+        for blocks in (1, 5, 8):
+            assert all(p.pieces == 1 for p in Line([blocks] * batch, 1, 18).pieces())
+    for lens in ([10] * 4, [313], [79] * 8):
+        spans = [p.span for p in Line(lens, 1, 18).pieces()]
+        assert len(set(spans)) == len(spans)
+    assert all(p.pieces == 1 for p in Line([MIN_SPAN + CUT_COST] * 3, 1, 148).pieces())
+
+
+def test_a_very_long_sequence_is_merged_in_few_pieces():
+    assert max(p.pieces for p in Line([2000], 1, 296).pieces()) <= MAX_MERGE
+    assert max(p.pieces for p in Line([2000] + [1] * 300, 1, 296).pieces()) <= MAX_MERGE
