@@ -3,6 +3,8 @@
 #include "fa_sched.h"
 #include "ptx.cuh"
 
+#include <type_traits>
+
 namespace fa {
 
 constexpr float kLog2eC = 1.4426950408889634f;
@@ -26,7 +28,7 @@ __device__ __forceinline__ void combine_unit(const float* __restrict__ o_part, c
   float g = -INFINITY;
   const int64_t lse_idx = (int64_t)h * total_q + qi;
   const int64_t o_idx = (qi * hq + h) * hdv + dv;
-#pragma unroll 4
+#pragma unroll 8
   for (int s = 0; s < nsplits; ++s) g = fmaxf(g, lse_part[s * lse_split_stride + lse_idx]);
   const bool has_sink = s_aux != nullptr;
   const float sk = has_sink ? s_aux[h] : -INFINITY;
@@ -40,25 +42,32 @@ __device__ __forceinline__ void combine_unit(const float* __restrict__ o_part, c
   }
   float L = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  // four splits at a time, so that their loads are in flight together (the kernel is bound by memory latency: a thread
-  // has two dependent loads per split)
-  for (int s0 = 0; s0 < nsplits; s0 += 4) {
-    float ls[4];
-    float4 o[4];
+  // several splits at a time and without looking at a split's LSE first, so that their loads are in flight together: a
+  // small merge is bound by the latency of its chain (eight rows over 64 splits: 38 us for the call with two dependent
+  // loads per split, 29 so)
+  auto add = [&](float ls, float4 o) {
+    if (!(ls > -INFINITY)) return;            // (a partial without keys may never have been written)
+    const float w = ex2((ls - g) * kLog2eC);
+    L += w;
+    acc.x += w * o.x; acc.y += w * o.y; acc.z += w * o.z; acc.w += w * o.w;
+  };
+  auto batch = [&](int s0, auto n) {
+    constexpr int N = decltype(n)::value;
+    float ls[N];
+    float4 o[N];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ls[j] = s0 + j < nsplits ? lse_part[(s0 + j) * lse_split_stride + lse_idx] : -INFINITY;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      o[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ls[j] > -INFINITY) o[j] = *reinterpret_cast<const float4*>(o_part + (s0 + j) * o_split_stride + o_idx);
+    for (int j = 0; j < N; ++j) {
+      ls[j] = lse_part[(s0 + j) * lse_split_stride + lse_idx];
+      o[j] = *reinterpret_cast<const float4*>(o_part + (s0 + j) * o_split_stride + o_idx);
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float w = ls[j] > -INFINITY ? ex2((ls[j] - g) * kLog2eC) : 0.f;
-      L += w;
-      acc.x += w * o[j].x; acc.y += w * o[j].y; acc.z += w * o[j].z; acc.w += w * o[j].w;
-    }
-  }
+    for (int j = 0; j < N; ++j) add(ls[j], o[j]);
+  };
+  int s0 = 0;
+  for (; s0 + 8 <= nsplits; s0 += 8) batch(s0, std::integral_constant<int, 8>());
+  if (s0 + 4 <= nsplits) { batch(s0, std::integral_constant<int, 4>()); s0 += 4; }
+  if (s0 + 2 <= nsplits) { batch(s0, std::integral_constant<int, 2>()); s0 += 2; }
+  if (s0 < nsplits) batch(s0, std::integral_constant<int, 1>());
   if (has_sink) L += ex2((sk - g) * kLog2eC);
   const float inv = L > 0.f ? 1.f / L : 0.f;
   uint2 packed;
