@@ -186,21 +186,32 @@ static Plan decode_part_plan(const PlanInput& in, const Plan& pl) {
   return d;
 }
 
-// The decode kernel cuts the batch's key blocks into equal spans, one per CTA (fa_decode.cu), unless
-//   - the caller fixed the split count (1 = one pass per sequence, whatever else is in the batch) or wants fp32 partials;
-//   - there are three or more work items per CTA: longest first they balance by themselves, and one that ends early
-//     makes room (128 sequences x 8 heads: 1420 us as items, 1477 cut; 111 x 8 x 2 row tiles 70 against 81);
-//   - the sequences are so short that most of them would be cut although there are items for half of the CTAs
-//     (10 sequences of 160 .. 376 keys x 16 heads over e4m3: 19.1 us as items, 20.5 cut);
-//   - the scan that finds the spans, which runs in every CTA, would have more than 2048 entries (13 per thread).
+// The decode kernel cuts the batch's key blocks by itself (LineCut in fa_decode.cu), or runs work items, longest first,
+// with a split count from here.  Measured side by side over batches of 1 .. 100 x 300 .. 20000 keys, equal and ragged, 8 / 1
+// .. 64 / 8 heads (time as items / time balanced, per class of items per CTA):
+//   - items for every CTA to have one at most: balanced 1.06 .. 1.5 (bf16), up to 2.5 (two CTAs per SM) without a caller's
+//     work list.  With one, the launch that makes the list is saved anyway: 0.85 - 0.92 up to 4096 keys, 1.02 - 1.5 above
+//     8192 (bf16).
+//   - up to 1.5 items per CTA: longest first balances short ragged batches better than cuts do (0.76 - 0.95 up to 2048
+//     keys), and loses above (4096 .. 8192 keys 1.09, longer 1.2 - 1.5; two CTAs per SM from 2048 on 1.10 - 1.5).
+//   - up to 3: 0.82 - 0.99, above 16384 keys 1.08 (two CTAs per SM: above 8192 1.13); more: items always.
+// Never with a split count of the caller's (1 = one pass per sequence, whatever else is in the batch), for fp32 partials,
+// or where the scan over the lengths, which every CTA makes, would have more than 2048 entries (13 per thread).
 static bool balanced_decode(const FaFwdParams* p, const Plan& decode_plan, bool mixed = false) {
   const long long entries = (long long)p->batch * decode_plan.max_mtiles, items = entries * p->hkv;
   const int ctas = decode_line_ctas(p->hd, p->kv_dtype, decode_plan.num_sms);
   if (decode_plan.route != FA_ROUTE_DECODE || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 ||
       entries > kBalancedEntriesMax || items * (p->max_seqlen_k / 64 + 2) >= (1ll << 30) || ctas > kWsArrivalWords)
     return false;
-  if (mixed) return true;      // (four row tiles per sequence in `entries`, nearly all of them empty)
-  return items < 3ll * ctas && !(p->max_seqlen_k <= 512 && items * 2 >= ctas);
+  // (a mixed batch has four row tiles per sequence in `items`, nearly all of them empty)
+  const long long n = mixed ? (long long)p->batch * p->hkv : items;
+  const bool two = ctas > decode_plan.num_sms, list = p->scheduler_metadata != nullptr;
+  int above;
+  if (n * 100 <= 98ll * ctas) above = !list ? 0 : two ? 4096 : 8192;      // (8 heads: 18 teams, 144 of 148 CTAs)
+  else if (n * 2 <= 3ll * ctas) above = list ? 8192 : two ? 2048 : 4096;
+  else if (n < 3ll * ctas) above = two ? 8192 : 16384;
+  else return false;
+  return p->max_seqlen_k > above;
 }
 
 // Scratch for the pieces of a balanced call: two pieces of `rows` rows for each CTA.

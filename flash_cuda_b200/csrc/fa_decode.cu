@@ -41,11 +41,13 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr int kPieces = 4;             // mailbox slots between the producer and the consumers
 // Balanced kernels, see LineCut (key blocks, about 0.65 us each with all SMs busy):
-constexpr int kMinSpan = 2;            // a piece has at least so many
-constexpr int kCutCost = 6;            // what cutting a triple costs the CTAs that share it: rows out, fence, atomic, merge
+// (an e4m3 cache: a stage holds two blocks and a block passes in half the time, so cuts are dearer in blocks; with
+// pieces of 2 blocks and 63 of them a head over 5000 / 20000 keys took 25 / 36 us against 19 / 28 as split work items)
+constexpr int min_span(bool kv8) { return kv8 ? 4 : 2; }       // a piece has at least so many
+constexpr int cut_cost(bool kv8) { return kv8 ? 10 : 6; }      // what cutting a triple costs the CTAs that share it: rows out, fence, atomic, merge
+constexpr int max_pieces(bool kv8) { return kv8 ? 24 : 64; }   // pieces of a triple at most ...
 constexpr int kCrossCost = 12;         // what a CTA pays for a span that begins and ends inside triples
 constexpr int kSnap = 8;               // a span border this close to the end of a triple moves there
-constexpr int kMaxPieces = 64;         // pieces of a triple at most ...
 constexpr int kMaxLinePieces = 96;     // ... and where spans cross sequences (what one CTA merges)
 constexpr int kMaxMerge = 104;         // (those, and a few more where borders moved)
 enum Role : unsigned { ROLE_PRODUCER = 5, ROLE_CONSUMER = 6 };
@@ -143,7 +145,7 @@ __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
 //
 // Where the line is cut.  Only the kernel knows the lengths, so every CTA plans the same from them:
 //   - no more (row tile, head group) triples than teams: each triple gets teams of its own, ceil(blocks / width) of them
-//     with the smallest width that the teams suffice for, unless that saves less than the cut costs (kCutCost: nothing
+//     with the smallest width that the teams suffice for, unless that saves less than the cut costs (cut_cost: nothing
 //     of up to 8 blocks is cut).  No CTA then works on two triples: with equal spans over the line two sequences of 300
 //     keys took 17.7 us, since nearly every CTA had two halves to open, write out and merge.
 //   - otherwise, or where the lengths are so uneven that this leaves the longest piece above the line's mean by more than
@@ -329,6 +331,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       for (int i = 0; i < kPieces; ++i) { mbar_init(bar_pc_full + 8 * i, 1); mbar_init(bar_pc_empty + 8 * i, NC); }
       mbar_fence_init();
     }
+    constexpr int kMinSpan = min_span(KV8), kCutCost = cut_cost(KV8), kMaxPieces = max_pieces(KV8);
     // ---- lengths: consecutive entries per thread; their sum, number and maximum ----
     constexpr int NTH = (NC + 1) * 32;
     const int per = (E + NTH - 1) / NTH, e_lo = min(E, tid * per), e_hi = min(E, e_lo + per);
@@ -1184,7 +1187,7 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
     a.team = line_team(kp.hkv, ctas);      // (8 heads: 18 teams, 144 of 148 SMs)
     // no more CTAs than spans of the least length there can be (from the longest sequence; the kernel knows better)
     const long long blocks = (long long)num_work_slots * (kp.hkv / a.team) * ((kp.max_seqlen_k + TN - 1) / TN + 1);
-    const long long spans = (blocks + kMinSpan - 1) / kMinSpan;
+    const long long spans = (blocks + min_span(KV8) - 1) / min_span(KV8);
     grid = (int)(spans < ctas / a.team ? spans : ctas / a.team) * a.team;
   }
   if (grid <= 0) return 0;

@@ -4,7 +4,8 @@ from __future__ import annotations
 
 from typing import Iterator, List, NamedTuple
 
-MIN_SPAN, CUT_COST, CROSS_COST, SNAP, MAX_PIECES, MAX_LINE_PIECES, MAX_MERGE = 2, 6, 12, 8, 64, 96, 104
+CROSS_COST, SNAP, MAX_LINE_PIECES, MAX_MERGE = 12, 8, 96, 104
+MIN_SPAN, CUT_COST, MAX_PIECES = (2, 4), (6, 10), (64, 24)      # cache of 16 bits, of 8
 
 
 class Piece(NamedTuple):
@@ -23,27 +24,28 @@ def _up(a: int, b: int) -> int:
 
 
 class Line:
-    def __init__(self, lens: List[int], groups: int, teams: int, whole: bool = False):
+    def __init__(self, lens: List[int], groups: int, teams: int, whole: bool = False, kv8: bool = False):
+        min_span, cut_cost, max_pieces = MIN_SPAN[kv8], CUT_COST[kv8], MAX_PIECES[kv8]
         self.lens, self.groups = lens, groups
         total, num, longest = sum(lens), sum(n > 0 for n in lens), max(lens, default=0)
         mean, width = _up(total * groups, teams), longest
         self.own = num * groups <= teams
-        if self.own and not whole and longest > MIN_SPAN + CUT_COST:
-            least = max(MIN_SPAN, mean, _up(longest, MAX_PIECES))
+        if self.own and not whole and longest > min_span + cut_cost:
+            least = max(min_span, mean, _up(longest, max_pieces))
             found, w = longest, least
             for _ in range(8):
                 if sum(_up(n, w) for n in lens) * groups <= teams:
                     found = min(found, w)
                 w += (w + 7) // 8
-            if found + CUT_COST < longest:
+            if found + cut_cost < longest:
                 width = found
-            if mean + CROSS_COST < width + (CUT_COST if width < longest else 0):
+            if mean + CROSS_COST < width + (cut_cost if width < longest else 0):
                 self.own = False
         self.pref = [0]
         for n in lens:
             self.pref.append(self.pref[-1] + (_up(n, max(width, 1)) if self.own else n))
         self.total = self.pref[-1] * groups
-        least = max(MIN_SPAN, _up(longest, MAX_LINE_PIECES))
+        least = max(min_span, _up(longest, MAX_LINE_PIECES))
         self.spans = max(1, self.total if self.own else min(teams, self.total // least))
         self.width = self.total // self.spans
         self.extra = self.total - self.width * self.spans

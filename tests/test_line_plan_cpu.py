@@ -16,8 +16,8 @@ def test_every_block_once_and_every_piece_in_its_place(seed):
         kind = rng.randrange(3)
         lens = [most if kind == 0 else rng.randint(0, most) if kind == 1 else
                 rng.randint(0, 3) if rng.random() < 0.9 else rng.randint(1, 10 * most) for _ in range(n)]
-        whole = rng.random() < 0.2
-        line = Line(lens, groups, teams, whole)
+        whole, kv8 = rng.random() < 0.2, rng.random() < 0.5
+        line = Line(lens, groups, teams, whole, kv8)
         assert line.spans <= teams
         found, slots = {}, set()
         for p in line.pieces():
@@ -33,7 +33,7 @@ def test_every_block_once_and_every_piece_in_its_place(seed):
             assert [p.span for p in ps] == [ps[0].span + j for j in range(len(ps))]
             assert all(p.hi > p.lo and p.pieces == len(ps) and p.first == ps[0].span for p in ps)
             assert len(ps) <= MAX_MERGE
-            assert len(ps) == 1 or lens[e] >= MIN_SPAN
+            assert len(ps) == 1 or lens[e] >= MIN_SPAN[kv8]
 
 
 def test_short_sequences_are_not_cut_and_no_team_works_on_two_of_few():
@@ -43,9 +43,9 @@ def test_short_sequences_are_not_cut_and_no_team_works_on_two_of_few():
     for lens in ([10] * 4, [313], [79] * 8):
         spans = [p.span for p in Line(lens, 1, 18).pieces()]
         assert len(set(spans)) == len(spans)
-    assert all(p.pieces == 1 for p in Line([MIN_SPAN + CUT_COST] * 3, 1, 148).pieces())
+    assert all(p.pieces == 1 for kv8 in (False, True) for p in Line([MIN_SPAN[kv8] + CUT_COST[kv8]] * 3, 1, 148, kv8=kv8).pieces())
 
 
 def test_a_very_long_sequence_is_merged_in_few_pieces():
-    assert max(p.pieces for p in Line([2000], 1, 296).pieces()) <= MAX_MERGE
+    assert max(p.pieces for p in Line([2000], 1, 296, kv8=True).pieces()) <= MAX_MERGE
     assert max(p.pieces for p in Line([2000] + [1] * 300, 1, 296).pieces()) <= MAX_MERGE
