@@ -51,7 +51,7 @@ def test_balanced_decode(name, dtype, kv_dtype, cuda_device):
     uncut, uncut_lse = _run(p, cuda_device, tol, check_ref=False, num_splits=1)
     assert (out.float() - uncut.float()).abs().max().item() <= 2 ** -7      # one rounding to 16 bits of |values| < 2
     if max(k for _, k in reqs) >= 4000:
-        assert not torch.equal(lse, uncut_lse)                              # the call was cut
+        assert not (torch.equal(out, uncut) and torch.equal(lse, uncut_lse))      # the call was cut
     # the op keeps one workspace per stream: its counters must be zero again after every call, and the merge order
     # does not depend on which CTA took which span
     pd = p.to(cuda_device)
