@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) depage_kernel(const DepageArgs a) {
 // queries, as 16-bit rows in contiguous slabs (exact: bf16 and fp16 hold every e4m3 value; the descales stay with the
 // attention kernel).  widen_plan_kernel lays the slabs out, `cap_rows` rows in all: sequence b gets the rows
 // [cu[b], cu[b + 1]), a multiple of 128, or none if it is short (at most class_rows packed query rows: the decode
-// kernel's) or does not fit any more; then take[b] = 1 and the general kernel runs it from the cache.
+// kernel's) or does not fit; then take[b] = 1 and the general kernel runs it from the cache.
 // widen_kernel is bound by memory: 1 byte in and 2 out per element, 16 bytes per load.
 struct WidenArgs {
   const unsigned char* k;
@@ -249,47 +249,40 @@ __device__ __forceinline__ int widen_len(const WidenArgs& a, int b) {
   return a.seqused_k ? a.seqused_k[b] : a.cu_k[b + 1] - a.cu_k[b];
 }
 
+constexpr int kWidenBatchMax = 512;
+
+// One block.  The sequences are taken in order; one that does not fit what is left of the slabs takes nothing of them,
+// so that a later, shorter one still may.
 __global__ void __launch_bounds__(256) widen_plan_kernel(const WidenArgs a) {
-  __shared__ int s_warp[8];
-  __shared__ int s_run, s_left;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) { s_run = 0; s_left = 0; }
-  __syncthreads();
-  for (int b0 = 0; b0 < a.batch; b0 += 256) {
-    const int b = b0 + tid;
-    int need = 0;
-    bool mine = false;
-    if (b < a.batch) {
-      const int rows = (a.cu_q[b + 1] - a.cu_q[b]) * a.rep;
-      mine = rows > a.class_rows;
-      if (mine) need = min((max(widen_len(a, b), 0) + 127) / 128, 1 << 20) * 128;
-    }
-    // (in blocks of 128 rows, so that the sum of many long sequences stays far from 2^31)
-    const int blocks = need >> 7;
-    int incl = blocks;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += v;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    int before = s_run;
-    for (int w = 0; w < warp; ++w) before += s_warp[w];
-    const int cap = a.cap_rows >> 7;
-    const int at = before + incl - blocks, end = before + incl;
-    if (b < a.batch) {
-      const bool fits = end <= cap;
-      a.cu[b] = min(at, cap) << 7;
-      a.take[b] = mine && !fits ? 1 : 0;
-      a.lens[b] = widen_len(a, b);
-      if (mine && !fits) atomicAdd(&s_left, 1);
-    }
-    __syncthreads();
-    if (tid == 255) s_run = min(end, cap + 1);      // (past the capacity nothing fits, whatever the sum)
-    __syncthreads();
+  __shared__ int s_blocks[kWidenBatchMax];      // 128-row blocks a sequence needs, then its first block, -1 - that if left out
+  __shared__ int s_rows, s_left;
+  for (int b = threadIdx.x; b < a.batch; b += 256) {
+    const int len = widen_len(a, b);
+    s_blocks[b] = (a.cu_q[b + 1] - a.cu_q[b]) * a.rep > a.class_rows ? (max(len, 0) + 127) / 128 : 0;
+    a.lens[b] = len;
   }
-  if (tid == 0) { a.cu[a.batch] = min(s_run, a.cap_rows >> 7) << 7; a.take[a.batch] = s_left; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int cap = a.cap_rows >> 7;
+    int run = 0, left = 0;
+#pragma unroll 8
+    for (int b = 0; b < a.batch; ++b) {
+      const int n = s_blocks[b];
+      const bool fits = n <= cap - run;
+      s_blocks[b] = fits ? run : -1 - run;
+      left += !fits;
+      run += fits ? n : 0;
+    }
+    s_rows = run << 7;
+    s_left = left;
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < a.batch; b += 256) {
+    const int at = s_blocks[b];
+    a.cu[b] = (at < 0 ? -1 - at : at) << 7;
+    a.take[b] = at < 0;
+  }
+  if (threadIdx.x == 0) { a.cu[a.batch] = s_rows; a.take[a.batch] = s_left; }
 }
 
 template <typename T>
@@ -304,7 +297,6 @@ __global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {
       if (a.cu[mid] <= r0) lo = mid; else hi = mid;
     }
     const int b = lo, s0 = r0 - a.cu[b];
-    if (a.take[b]) continue;                  // (what is left of the capacity before a sequence that did not fit)
     const int used = widen_len(a, b);
     // The keys below vis_lo (leftpad, or in front of the first row's window) are seen by no row, and the page table need
     // not say where they are: they are not read.  The attention kernel loads no 128-key block that lies below vis_lo
@@ -347,7 +339,7 @@ __global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {
 
 int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_rows, void* k_out, void* v_out, int32_t* cu,
                  int32_t* take, int32_t* lens, int num_sms, cudaStream_t stream) {
-  if (kp.hd % 16 || kp.hdv % 16 || kp.batch <= 0) return (int)cudaErrorInvalidValue;
+  if (kp.hd % 16 || kp.hdv % 16 || kp.batch <= 0 || kp.batch > kWidenBatchMax) return (int)cudaErrorInvalidValue;
   WidenArgs a;
   a.k = reinterpret_cast<const unsigned char*>(kp.k);
   a.v = reinterpret_cast<const unsigned char*>(kp.v);

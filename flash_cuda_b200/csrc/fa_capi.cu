@@ -174,7 +174,9 @@ static PlanInput plan_input(const FaSchedParams* p, int num_sms) {
 static bool mixed_batch(const FaFwdParams* p, const PlanInput& in, const Plan& pl) {
   if (p->route != FA_ROUTE_AUTO || pl.route != FA_ROUTE_PREFILL_TC || p->scheduler_metadata != nullptr) return false;
   if (p->batch < 2 || !decode_supported(in) || p->out_dtype == FA_DT_FP32) return false;
-  if ((long long)p->batch * pl.max_mtiles > kSchedSortMax) return false;   // (the filtered lists are sorted lists)
+  if ((long long)p->batch * pl.max_mtiles > kSchedSortMax ||      // (the filtered lists are sorted lists)
+      !sched_is_sorted(p->batch * pl.max_mtiles, p->max_seqlen_k, pl.tile_n))
+    return false;
   return (long long)p->total_q * 4 < (long long)p->batch * p->max_seqlen_q;
 }
 static Plan decode_part_plan(const PlanInput& in, const Plan& pl) {
@@ -270,6 +272,9 @@ static WidenPlan widen_plan(const FaFwdParams* p, const PlanInput& in, const Pla
   // (the tensor-core and decode kernels take an approximate tanh, off by up to 2^-11 of the cap; these calls always
   // had tanhf)
   if (in.has_softcap) return wp;
+  // (few rows over few keys of head_dim 64, where a copied cache saves least: 4 rows over 1000 keys 23 us on the general
+  // kernel, 28 widened; from 16000 keys on 101 against 72, and at head_dim 96 36 against 30 already at 1000)
+  if (p->hd <= 64 && p->max_seqlen_k <= 4096 && p->max_seqlen_q * (p->hq / p->hkv) <= 200) return wp;
   PlanInput tin = in;
   tin.kv_dtype = in.q_dtype;
   tin.page_size = 0;
@@ -277,9 +282,11 @@ static WidenPlan widen_plan(const FaFwdParams* p, const PlanInput& in, const Pla
   // (16-byte loads of 8-bit rows)
   if (p->hd % 16 || p->hdv % 16 || p->k_row_stride % 16 || p->v_row_stride % 16 || !prefill_tc_supported(tin)) return wp;
   wp.tc = make_plan(tin);
-  if (wp.tc.err != FA_OK || (long long)p->batch * wp.tc.max_mtiles > kSchedSortMax) return wp;
+  if (wp.tc.err != FA_OK || (long long)p->batch * wp.tc.max_mtiles > kSchedSortMax ||
+      !sched_is_sorted(p->batch * wp.tc.max_mtiles, p->max_seqlen_k, wp.tc.tile_n))
+    return wp;
   if (p->batch > 1) {
-    if (!decode_supported(in) || p->batch * (kDecodeMaxRows / 16) > kBalancedEntriesMax) return wp;
+    if (!decode_supported(in) || (long long)p->batch * (kDecodeMaxRows / 16) > kBalancedEntriesMax) return wp;
     wp.class_rows = kDecodeMaxRows;
   }
   const size_t row = (size_t)p->hkv * (p->hd + p->hdv) * 2;

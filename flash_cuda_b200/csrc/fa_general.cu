@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(NTHREADS) fwd_general_kernel(const KParams p, 
 }
 
 template <typename T, int HD, int HDV>
-static int launch_t(const KParams& kp, cudaStream_t stream) {
+static int launch_t(const KParams& kp, int num_sms, cudaStream_t stream) {
   const size_t smem = (size_t)(BM * (HD + PAD) + BN * (HD + PAD) + BN * (HDV + PAD)) * sizeof(T);
   auto kern = fwd_general_kernel<T, HD, HDV>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -296,28 +296,29 @@ static int launch_t(const KParams& kp, cudaStream_t stream) {
   const int mtiles = (kp.max_seqlen_q * kp.rep + BM - 1) / BM;
   if (kp.hkv > 65535 || (long long)mtiles * kp.batch * kp.nsplits > 2147483647ll) return -1;
   const unsigned tiles = (unsigned)(mtiles * kp.batch * kp.nsplits);
-  // one block per tile; where usually no tile is this kernel's, few blocks that look for theirs
-  dim3 grid(kp.take && tiles > 64u ? 64u : tiles, kp.hkv, 1);
+  // one block per tile; where usually no tile is this kernel's, no more blocks than run at once, which look for theirs
+  const unsigned some = (unsigned)((4 * num_sms + kp.hkv - 1) / kp.hkv);
+  dim3 grid(kp.take && tiles > some ? some : tiles, kp.hkv, 1);
   kern<<<grid, NTHREADS, smem, stream>>>(kp, tiles);
   return (int)cudaGetLastError();
 }
 
 template <typename T>
-static int launch_hd(const KParams& kp, cudaStream_t stream) {
+static int launch_hd(const KParams& kp, int num_sms, cudaStream_t stream) {
   const int hd = kp.hd, hdv = kp.hdv;
-  if (hd <= 64 && hdv <= 64) return launch_t<T, 64, 64>(kp, stream);
-  if (hd <= 128 && hdv <= 128) return launch_t<T, 128, 128>(kp, stream);
-  if (hd <= 192 && hdv <= 128) return launch_t<T, 192, 128>(kp, stream);
-  if (hd <= 256 && hdv <= 256) return launch_t<T, 256, 256>(kp, stream);
+  if (hd <= 64 && hdv <= 64) return launch_t<T, 64, 64>(kp, num_sms, stream);
+  if (hd <= 128 && hdv <= 128) return launch_t<T, 128, 128>(kp, num_sms, stream);
+  if (hd <= 192 && hdv <= 128) return launch_t<T, 192, 128>(kp, num_sms, stream);
+  if (hd <= 256 && hdv <= 256) return launch_t<T, 256, 256>(kp, num_sms, stream);
   return -1;
 }
 
 }  // namespace general
 
 // compute type: fp16 inputs -> fp16 MMA; bf16 and fp8 inputs -> bf16 MMA (fp8 values are exact in bf16)
-int launch_general(const KParams& kp, int dtype, int /*out_dtype*/, int /*num_sms*/, cudaStream_t stream) {
-  if (dtype == FA_DT_FP16) return general::launch_hd<__half>(kp, stream);
-  return general::launch_hd<__nv_bfloat16>(kp, stream);
+int launch_general(const KParams& kp, int dtype, int /*out_dtype*/, int num_sms, cudaStream_t stream) {
+  if (dtype == FA_DT_FP16) return general::launch_hd<__half>(kp, num_sms, stream);
+  return general::launch_hd<__nv_bfloat16>(kp, num_sms, stream);
 }
 
 }  // namespace fa

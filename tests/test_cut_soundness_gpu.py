@@ -149,3 +149,33 @@ def test_few_keys_under_a_loose_bound_are_not_cut(kw, cuda_device):
     out, lse, _ = capi.fwd(p.q, k, v, check=True, **args)
     whole, whole_lse, _ = capi.fwd(p.q, k, v, check=True, num_splits=1, **args)
     assert torch.equal(out, whole) and torch.equal(lse, whole_lse)
+
+
+def test_few_rows_over_few_keys_of_an_e4m3_cache_stay_on_the_general_kernel(cuda_device):
+    """At head_dim 64 a widened copy of the cache costs more than it saves there."""
+    for ql, kl in ((1, 3000), (8, 1000), (50, 4096)):
+        p = _problem(dict(reqs=[(ql, kl)], hq=8, hkv=2, hd=64, page_size=64, kv_dtype="fp8"), cuda_device)
+        out, lse, _ = capi.fwd(p.q, p.k, p.v, check=True, **p.capi_kw())
+        gen, gen_lse, _ = capi.fwd(p.q, p.k, p.v, check=True, route=capi.FA_ROUTE_GENERAL, **p.capi_kw())
+        assert torch.equal(out, gen) and torch.equal(lse, gen_lse)
+
+
+def test_a_sequence_that_does_not_fit_the_slabs_leaves_them_to_the_others(cuda_device):
+    """The first of two sequences has more keys than 256 MB of slabs hold (65536 at 8 kv heads of 2 x 128 columns): it
+    gets the general kernel's bits, the second one the tensor-core kernel's."""
+    g = torch.Generator(device=cuda_device).manual_seed(303)
+    lens, q_lens = [66000, 900], [17, 100]
+    pages = [(n + 63) // 64 for n in lens]
+    k, v = (torch.randn(sum(pages), 64, 8, 128, generator=g, device=cuda_device, dtype=torch.bfloat16).to(torch.float8_e4m3fn)
+            for _ in range(2))
+    table = torch.zeros(2, max(pages), dtype=torch.int32)
+    table[0, :pages[0]] = torch.arange(pages[0], dtype=torch.int32)
+    table[1, :pages[1]] = torch.arange(pages[0], sum(pages), dtype=torch.int32)
+    q = torch.randn(117, 32, 128, generator=g, device=cuda_device, dtype=torch.bfloat16)
+    kw = dict(cu_seqlens_q=torch.tensor([0, 17, 117], dtype=torch.int32, device=cuda_device), page_table=table.to(cuda_device),
+              seqused_k=torch.tensor(lens, dtype=torch.int32, device=cuda_device), max_seqlen_q=100, max_seqlen_k=66000,
+              softmax_scale=128 ** -0.5, causal=True)
+    out, _, _ = capi.fwd(q, k, v, check=True, **kw)
+    gen, _, _ = capi.fwd(q, k, v, check=True, route=capi.FA_ROUTE_GENERAL, num_splits=1, **kw)
+    assert torch.equal(out[:17], gen[:17]) and not torch.equal(out[17:], gen[17:])
+    assert (out[17:].float() - gen[17:].float()).abs().max().item() <= 2 ** -6
