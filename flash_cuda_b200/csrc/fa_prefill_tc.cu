@@ -50,7 +50,13 @@ constexpr float kLn2 = 0.6931471805599453f;
 #define FA_CAP_EMU_PAIRS 2
 #endif
 constexpr int kCapEmuPairs = FA_CAP_EMU_PAIRS;   // of every four pairs in the fused softcap loop
+// tanh(u) = u (c0 + c1 u^2 + c2 u^4 + c3 u^6) for |u| <= 0.6, relative error 2.2e-6 (least maximum, fitted numerically;
+// tanh.approx.f32: up to 2^-11).  Up to |u| = 1 the same four terms would be off by 8.2e-5 everywhere, and the LSE of
+// ordinary scores, which lie far below the cap, by more than with tanh.approx.
+__device__ constexpr float kTanhC[4] = {0.99999785f, -0.33314040f, 0.13057856f, -0.04092942f};
+constexpr float kTanhMax = 0.6f;
 constexpr float kRescaleThreshold = 8.0f;   // log2 units
+constexpr float kFastShift = 14.f;         // log2 units: largest probability of a fast block of capped scores
 constexpr float kFastSumLimit = 16384.f;    // 2^14: row sum of a block above which the fast softmax form is redone
 enum Role : unsigned { ROLE_TMA = 1, ROLE_MMA = 2, ROLE_SOFTMAX = 3, ROLE_EPILOGUE = 4 };
 
@@ -873,6 +879,17 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       }
       const float c_mul = has_cap ? p.softcap * kLog2e : sc * kLog2e;
       const float cap_in = has_cap ? sc / p.softcap : 0.f;
+      // capped scores on the FMA pipe: c_mul * tanh(cap_in * s) = s * (cap_a[0] + s^2 (cap_a[1] + ..)), see kTanhC
+      float cap_a[4];
+      if constexpr (CAP && !F8) {
+        const float i2 = cap_in * cap_in;
+        cap_a[0] = kTanhC[0] * c_mul * cap_in;
+        cap_a[1] = kTanhC[1] * c_mul * cap_in * i2;
+        cap_a[2] = kTanhC[2] * c_mul * cap_in * i2 * i2;
+        cap_a[3] = kTanhC[3] * c_mul * cap_in * i2 * i2 * i2;
+      }
+      const float cap_s_max = kTanhMax / cap_in;      // largest |s| the polynomial is good for
+      bool cap_poly = CAP && !F8;     // until a block of this item has shown a score beyond that
       const int qp = it.seqlen_k - it.seqlen_q + row;
       int lo = it.leftpad, hi = it.seqlen_k - 1;
       if (p.is_causal) hi = min(hi, qp);
@@ -898,6 +915,68 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         tc_fence_after_sync();
         const int n0 = i * TN;
         const bool full = (n0 >= lo_max) && (n0 + TN - 1 <= hi_min);
+        // The fast form of a capped block (no masked column, a reference point already taken).  tanh is an odd polynomial
+        // on the FMA pipe, which leaves the special-function unit the exp2 alone (tanh and exp2 on that one unit, half of the
+        // exp2 emulated on the FMA pipe, bounded the capped kernel).  First the largest |s| of the row's block: it says
+        // whether the polynomial's range holds and bounds the probabilities by 2^14, as in the plain kernel's fast
+        // form; a block where either fails sends the rest of the item to the general form.  S comes in quarters, the
+        // next one on its way while one is worked on: the registers of a whole row are those that keep the
+        // exponentials' chains apart.  16 sequences of 128 .. 8192 queries, window 4096, cap 30, sinks: 4860 -> 4230 us
+        // sustained (power-limited), 4440 -> 3680 in a burst; with the whole row held and the range checked afterwards,
+        // 4470 sustained; P held back in registers until a check afterwards, 4160 - 4270 but a redo to code for.
+        bool cap_done = false;
+        if constexpr (CAP && !F8) {
+          if (__all_sync(0xffffffffu, full && cap_poly && m_used != -INFINITY)) {
+            uint32_t sp[2][32];
+            tmem_ld32(tS, sp[0]);
+            tmem_ld32(tS + 32, sp[1]);
+            tmem_wait_ld32(sp[0]);
+            tmem_wait_ld32(sp[1]);
+            float am[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              uint32_t (&sq)[32] = sp[c & 1];
+              if (c >= 2) tmem_wait_ld32(sq);
+#pragma unroll
+              for (int j = 0; j < 32; j += 2)
+                am[(j >> 1) & 3] = fmax3_abs(am[(j >> 1) & 3], __uint_as_float(sq[j]), __uint_as_float(sq[j + 1]));
+              tmem_ld32(tS + ((c + 2) & 3) * 32, sq);     // (the last two: the first quarters again, for the second pass)
+            }
+            const float amax = fmaxf(fmaxf(am[0], am[1]), fmaxf(am[2], am[3]));
+            const float ub = cap_a[0] * amax;              // c_mul * tanh(cap_in * amax) is no larger
+            cap_poly = __all_sync(0xffffffffu, amax <= cap_s_max && ub - m_used <= kFastShift);
+            tmem_wait_ld32(sp[0]);
+            tmem_wait_ld32(sp[1]);
+            if (cap_poly) {
+              const float2 nm2 = make_float2(-m_used, -m_used);
+              const float2 a0 = make_float2(cap_a[0], cap_a[0]), a1 = make_float2(cap_a[1], cap_a[1]);
+              const float2 a2 = make_float2(cap_a[2], cap_a[2]), a3 = make_float2(cap_a[3], cap_a[3]);
+              float2 fs[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                uint32_t (&sq)[32] = sp[c & 1];
+                if (c >= 2) tmem_wait_ld32(sq);
+                uint32_t pk[16];
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                  const float2 x = make_float2(__uint_as_float(sq[j]), __uint_as_float(sq[j + 1]));
+                  const float2 x2 = fmul2(x, x);
+                  const float2 y = ffma2(x, ffma2(ffma2(ffma2(a3, x2, a2), x2, a1), x2, a0), nm2);
+                  const float2 pp = make_float2(ex2(y.x), ex2(y.y));
+                  fs[(j >> 1) & 3] = fadd2(fs[(j >> 1) & 3], pp);
+                  pk[j >> 1] = pack2<TO>(pp.x, pp.y);
+                }
+                if (c + 2 < 4) tmem_ld32(tS + (c + 2) * 32, sq);
+                tmem_st16(tS + c * 16, pk);               // (columns of quarters that have been read)
+              }
+              const float2 s01 = fadd2(fs[0], fs[1]), s23 = fadd2(fs[2], fs[3]);
+              const float2 s4 = fadd2(s01, s23);
+              l += s4.x + s4.y;
+              cap_done = true;
+            }
+          }
+        }
+        if (!cap_done) {
         uint32_t sreg[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, sreg[c]);
@@ -1108,6 +1187,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           l += s4.x + s4.y;
         }
         }   // general form
+        }   // not the capped fast form
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
