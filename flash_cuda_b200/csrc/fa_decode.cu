@@ -50,6 +50,10 @@ constexpr int kCrossCost = 12;         // what a CTA pays for a span that begins
 constexpr int kSnap = 8;               // a span border this close to the end of a triple moves there
 constexpr int kMaxLinePieces = 96;     // ... and where spans cross sequences (what one CTA merges)
 constexpr int kMaxMerge = 104;         // (those, and a few more where borders moved)
+constexpr int kFewPieces = 8;          // ... of which a thread loads so many at once
+constexpr int kMaxBorders = 304;       // spans of a line at most, and its end (CTAs of a launch: two per SM)
+constexpr int kSmallLine = 160;        // entries of a line whose records stay in shared memory (one per thread)
+constexpr int kRecordOff = 256;        // ... behind the prefix sums of as many, words
 enum Role : unsigned { ROLE_PRODUCER = 5, ROLE_CONSUMER = 6 };
 enum : int { F_FIRST = 1, F_LAST = 2, F_EMPTY = 4 };
 
@@ -79,12 +83,14 @@ struct Smem {
   static constexpr int kScrOff = (kMiscOff + 16 + 15) / 16 * 16;
   static constexpr int kLdO = HDV + 4;
   static constexpr int kScrBytes = NC * 16 * kLdO * 4 + 2 * NC * 16 * 4;
-  static_assert(NC * 16 * kLdO >= 16 * kMaxMerge, "the merge's weights lie in the merge area");
+  static_assert(NC * 16 * kLdO >= 2 * 16 * kMaxMerge, "the merge's pairs lie in the merge area");
   // balanced kernels: piece mailbox with its barriers, then the line's prefix sums
   static constexpr int kPieceOff = kScrOff + kScrBytes;
   static constexpr int kPieceBarOff = kPieceOff + kPieces * 80;   // full[kPieces], empty[kPieces], flag
   static constexpr int kPrefOff = kPieceBarOff + 2 * kPieces * 8 + 16;
-  static constexpr int kBytesBalanced = kPrefOff + (kBalancedEntriesMax + 4) * 4;
+  static constexpr int kBorderOff = kPrefOff + (kBalancedEntriesMax + 4) * 4;
+  static constexpr int kBytesBalanced = kBorderOff + kMaxBorders * 4;
+  static_assert(kRecordOff + kSmallLine * 8 <= kBalancedEntriesMax + 4 && kSmallLine < kRecordOff && kRecordOff % 4 == 0, "records of a small line");
   static constexpr int kBytes = kPieceOff;
 };
 
@@ -155,10 +161,6 @@ struct LineCut {
   int spans, width, extra;       // the first `extra` spans have width + 1 units, the others width
   int total, snap;               // units of the line; borders move by at most this much (-1: always to the next triple)
   __device__ __forceinline__ int begin(int c) const { return c * width + min(c, extra); }
-  __device__ __forceinline__ int span_of(int x) const {
-    const int wide = extra * (width + 1);
-    return x < wide ? x / (width + 1) : extra + (x - wide) / width;
-  }
   __device__ __forceinline__ void plan(int total_, int spans_) {
     total = total_;
     spans = max(1, spans_);
@@ -166,6 +168,17 @@ struct LineCut {
     extra = total - width * spans;
   }
 };
+
+// The last of E entries with groups * pref[e] <= y.
+__device__ __forceinline__ int entry_of(const int* pref, int E, int groups, int y) {
+  int lo = 0, hi = E;
+#pragma unroll 1
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (pref[mid] * groups <= y) lo = mid; else hi = mid;
+  }
+  return lo;
+}
 
 // Entry e of the line: a (batch, row tile), all head groups; `hk` and `split` are left at 0.
 __device__ __forceinline__ WorkItem line_entry(const DecArgs& a, int e) {
@@ -207,6 +220,25 @@ __device__ __forceinline__ WorkItem line_entry(const DecArgs& a, int e) {
 }
 // Blocks of one head group of an entry; an entry whose rows see no key counts as one, so that some CTA writes its rows.
 __device__ __forceinline__ int line_len(const WorkItem& it) { return it.valid ? max(it.hi - it.lo, 1) : 0; }
+
+// The entries of a small line, read once while the line is planned, stay in shared memory (8 words each): the producer
+// had read its own a second time, in code that every CTA ran cold.
+__device__ __forceinline__ void keep_entry(int* rec, const WorkItem& it) {
+  int4* r4 = reinterpret_cast<int4*>(rec);
+  r4[0] = make_int4(it.b | it.mt << 16, it.q0, it.seqlen_q, it.seqlen_k);      // (b, mt < 160)
+  r4[1] = make_int4(it.k0, it.leftpad, it.lo, it.hi);
+}
+__device__ __forceinline__ WorkItem kept_entry(const int* rec) {
+  const int4 x = reinterpret_cast<const int4*>(rec)[0], y = reinterpret_cast<const int4*>(rec)[1];
+  WorkItem it;
+  it.b = x.x & 0xffff; it.mt = x.x >> 16;
+  it.q0 = x.y; it.seqlen_q = x.z; it.seqlen_k = x.w;
+  it.k0 = y.x; it.leftpad = y.y; it.lo = y.z; it.hi = y.w;
+  it.hk = it.split = 0;
+  it.valid = true;
+  it.bad = false;
+  return it;
+}
 
 // One piece of a (batch, row tile, head), as the producer hands it to the consumers.
 struct Piece {
@@ -303,7 +335,10 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   float* s_l = s_m + NC * 16;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
+  // (set up by the producer warp: the first threads have the entries of a short line to read)
+  if (warp == NC && lane == 0) {
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
     // cp.async stages complete on 33 arrivals: one per producer lane when its copies have landed, one from lane 0
     // after it has written the stage's descriptor
     for (int s = 0; s < NST; ++s) { mbar_init(bar_full + 8 * s, a.gather ? 33 : 1); mbar_init(bar_empty + 8 * s, NC); }
@@ -314,12 +349,14 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   const uint32_t bar_pc_full = base + SM::kPieceBarOff, bar_pc_empty = bar_pc_full + 8 * kPieces;
   volatile int* s_last = reinterpret_cast<volatile int*>(sm + SM::kPieceBarOff + 2 * kPieces * 8);
   int* s_pref = reinterpret_cast<int*>(sm + SM::kPrefOff);      // blocks before entry e (one head group)
+  int* s_border = reinterpret_cast<int*>(sm + SM::kBorderOff);  // where span c of the line begins
+  bool small = false;    // a line of at most kSmallLine entries
   LineCut cut{};
   int groups = 1;
   bool own = false;      // every triple has teams of its own: a unit of the line is a piece; else a unit is a key block
   if constexpr (BAL) {
     int* s_sum = reinterpret_cast<int*>(s_o);      // the merge area is not in use yet
-    if (tid == 0) s_sum[30] = __ldcg(&p.status->error) != 0u;      // (one read: the CTA's threads must agree on the plan)
+    if (tid == NC * 32 + 31) s_sum[30] = __ldcg(&p.status->error) != 0u;      // (one read: the CTA's threads must agree on the plan)
     int E = p.batch * a.max_mtiles;
     if (a.use_list) {
       // the list's header must describe this call before any entry is read
@@ -327,20 +364,24 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       if (!good && tid == 0) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
       E = good ? p.work[6] : 0;
     }
-    if (tid == 0) {
+    if (tid == NC * 32) {
       for (int i = 0; i < kPieces; ++i) { mbar_init(bar_pc_full + 8 * i, 1); mbar_init(bar_pc_empty + 8 * i, NC); }
       mbar_fence_init();
     }
     constexpr int kMinSpan = min_span(KV8), kCutCost = cut_cost(KV8), kMaxPieces = max_pieces(KV8);
     // ---- lengths: consecutive entries per thread; their sum, number and maximum ----
     constexpr int NTH = (NC + 1) * 32;
+    static_assert(NTH <= kSmallLine, "the prefix sums of a small line end before its records");
     const int per = (E + NTH - 1) / NTH, e_lo = min(E, tid * per), e_hi = min(E, e_lo + per);
+    small = E <= NTH;
     int sum = 0, num = 0, longest = 0;
     bool bad = false;
+#pragma unroll 1
     for (int e = e_lo; e < e_hi; ++e) {
       const WorkItem it = line_entry(a, e);
       const int len = line_len(it);
       bad |= it.bad;
+      if (small && it.valid) keep_entry(s_pref + kRecordOff + 8 * e, it);
       s_pref[e] = len;
       sum += len; num += len > 0; longest = max(longest, len);
     }
@@ -356,44 +397,35 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     for (int w = 0; w <= NC; ++w) { sum += s_sum[w]; num += s_sum[8 + w]; longest = max(longest, s_sum[16 + w]); }
     // ---- the plan ----
     groups = p.hkv / a.team;
-    const int teams = (int)gridDim.x / a.team;
+    const int teams = min((int)gridDim.x / a.team, kMaxBorders - 1);
     const int mean = (sum * groups + teams - 1) / teams;
     int width = longest;             // blocks of a piece where triples have teams of their own
     own = num * groups <= teams;
     if (own && !whole && longest > kMinSpan + kCutCost) {
-      // the smallest of eight widths, from the least possible to 2.5 times that, for which the teams suffice
+      // the smallest of eight widths, from the least possible to 2.5 times that, for which the teams suffice: a lane
+      // counts the pieces that width number (lane & 7) makes of every 20th entry.  (Rolled, like the rest of the plan: a
+      // CTA runs it once, and cold code costs by its size.)
       const int least = max(max(kMinSpan, mean), (longest + kMaxPieces - 1) / kMaxPieces);
-      constexpr int kTries = 8;
-      int need[kTries];
-#pragma unroll
-      for (int k = 0; k < kTries; ++k) need[k] = 0;
-      for (int e = e_lo; e < e_hi; ++e) {
-        const int len = s_pref[e];
-        int wd = least;
-#pragma unroll
-        for (int k = 0; k < kTries; ++k) { need[k] += (len + wd - 1) / wd; wd += (wd + 7) / 8; }
-      }
-#pragma unroll
-      for (int k = 0; k < kTries; ++k) need[k] = __reduce_add_sync(0xffffffffu, need[k]);
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < kTries; ++k) s_sum[32 + warp * kTries + k] = need[k];
-      }
+      int wd = least, n = 0;
+#pragma unroll 1
+      for (int k = lane & 7; k > 0; --k) wd += (wd + 7) / 8;
+#pragma unroll 1
+      for (int e = tid >> 3; e < E; e += NTH / 8) n += (s_pref[e] + wd - 1) / wd;
+      n += __shfl_xor_sync(0xffffffffu, n, 8);
+      n += __shfl_xor_sync(0xffffffffu, n, 16);
+      if (lane < 8) s_sum[32 + warp * 8 + lane] = n;
       __syncthreads();
-      int wd = least, found = longest;
+      n = 0;
 #pragma unroll
-      for (int k = 0; k < kTries; ++k) {
-        int n = 0;
-#pragma unroll
-        for (int w = 0; w <= NC; ++w) n += s_sum[32 + w * kTries + k];
-        if (n * groups <= teams) found = min(found, wd);
-        wd += (wd + 7) / 8;
-      }
+      for (int w = 0; w <= NC; ++w) n += s_sum[32 + w * 8 + (lane & 7)];
+      const int found = __reduce_min_sync(0xffffffffu, n * groups <= teams ? min(wd, longest) : longest);
       if (found + kCutCost < longest) width = found;
+      __syncthreads();       // (every thread has read the lengths that the prefix sums replace)
       if (mean + kCrossCost < width + (width < longest ? kCutCost : 0)) own = false;
     }
     // ---- units of the line before each entry: blocks, or pieces ----
     int mine = 0;
+#pragma unroll 1
     for (int e = e_lo; e < e_hi; ++e) {
       const int len = s_pref[e];
       s_pref[e] = mine;
@@ -413,18 +445,33 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       if (w < warp) before += s_sum[24 + w];
       total += s_sum[24 + w];
     }
+#pragma unroll 1
     for (int e = e_lo; e < e_hi; ++e) s_pref[e] += before;
     if (tid == 0) s_pref[E] = total;
     total *= groups;
     const int min_width = max(kMinSpan, (longest + kMaxLinePieces - 1) / kMaxLinePieces);
     cut.plan(total, own ? total : min(teams, total / min_width));
     cut.snap = whole ? -1 : min(kSnap, (cut.width - 1) / 2);
+    __syncthreads();
+    // ---- where each span begins: a thread per border ----
+#pragma unroll 1
+    for (int c = tid; c <= cut.spans; c += NTH) {
+      int y = cut.begin(c);
+      if (!own && cut.snap != 0 && y < cut.total) {
+        const int e = entry_of(s_pref, E, groups, y), len = s_pref[e + 1] - s_pref[e], over = (y - s_pref[e] * groups) % len;
+        if (over != 0) {
+          if (cut.snap < 0) y += len - over;
+          else if (over <= cut.snap) y -= over;
+          else if (len - over <= cut.snap) y += len - over;
+        }
+      }
+      s_border[c] = y;
+    }
   }
   __syncthreads();
 
   if (warp == NC) {
     // ============================================ producer ============================================
-    if (lane == 0) { tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
     uint32_t cnt = 0;
     bool ok = true;
     const bool paged = p.page_table != nullptr;
@@ -446,27 +493,16 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     const int span = BAL ? (int)blockIdx.x / a.team : 0, member = BAL ? (int)blockIdx.x - span * a.team : 0;
     int x = 0, x_end = 0, ent = 0;
     uint32_t pcnt = 0;
-    // the last entry with groups * s_pref[e] <= y
-    auto entry_of = [&](int y) {
-      int lo_e = 0, hi_e = a.use_list ? p.work[6] : p.batch * a.max_mtiles;
-      while (hi_e - lo_e > 1) {
-        const int mid = (lo_e + hi_e) >> 1;
-        if (s_pref[mid] * groups <= y) lo_e = mid; else hi_e = mid;
-      }
-      return lo_e;
-    };
-    // where span c begins
-    auto line_begin = [&](int c) {
-      const int y = cut.begin(c);
-      if (own || cut.snap == 0 || y >= cut.total) return y;
-      const int e = entry_of(y), len = s_pref[e + 1] - s_pref[e], over = (y - s_pref[e] * groups) % len;
-      if (over == 0) return y;
-      if (cut.snap < 0) return y - over + len;
-      return over <= cut.snap ? y - over : len - over <= cut.snap ? y - over + len : y;
+    // the span that unit y of the line lies in
+    auto span_at = [&](int y) {
+      int n = 0;
+#pragma unroll 1
+      for (int c = lane; c - lane < cut.spans; c += 32) n += __popc(__ballot_sync(0xffffffffu, c < cut.spans && s_border[c] <= y));
+      return n - 1;
     };
     if constexpr (BAL) {
-      if (span < cut.spans) { x = line_begin(span); x_end = line_begin(span + 1); }
-      if (x < x_end) ent = entry_of(x);
+      if (span < cut.spans) { x = s_border[span]; x_end = s_border[span + 1]; }
+      if (x < x_end) ent = entry_of(s_pref, a.use_list ? p.work[6] : p.batch * a.max_mtiles, groups, x);
     }
     while (ok) {
       int w = 0;
@@ -476,7 +512,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         while (x >= s_pref[ent + 1] * groups) ++ent;      // (entries without blocks are passed over)
         const int len = s_pref[ent + 1] - s_pref[ent], off = x - s_pref[ent] * groups;
         const int hg = off / len, pos = off - hg * len, n = own ? 1 : min(len - pos, x_end - x);
-        it = line_entry(a, ent);
+        it = small ? kept_entry(s_pref + kRecordOff + 8 * ent) : line_entry(a, ent);
         it.hk = hg * a.team + member;
         int pieces = 1, first = span;      // of this triple, and the span that holds its first piece
         if (own) {
@@ -486,19 +522,9 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           it.lo = lo + (int)((int64_t)blocks * pos / len);
           it.hi = lo + (int)((int64_t)blocks * (pos + 1) / len);
         } else if (n != len) {
-          if (pos > 0) {
-            first = cut.span_of(x - pos);
-            while (first + 1 < cut.spans && line_begin(first + 1) <= x - pos) ++first;
-            while (line_begin(first) > x - pos) --first;
-          }
           const int end = x - pos + len - 1;
-          int last = span;
-          if (end >= x_end) {
-            last = cut.span_of(end);
-            while (last + 1 < cut.spans && line_begin(last + 1) <= end) ++last;
-            while (line_begin(last) > end) --last;
-          }
-          pieces = last - first + 1;
+          if (pos > 0) first = span_at(x - pos);
+          pieces = (end >= x_end ? span_at(end) : span) - first + 1;
           it.lo += pos; it.hi = it.lo + n;
         }
         const uint32_t slot = pcnt % kPieces;
@@ -655,6 +681,9 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     // ============================================ consumers ===========================================
     const int g = lane >> 2, tq = lane & 3;
     const int rep = p.rep;
+    // R / rep for rows of a sequence: R < 2^21 keeps the rounded product on the right side of every multiple
+    const float inv_rep = __frcp_rn((float)rep);
+    auto token_of = [&](int R) { return (int)(((float)R + 0.5f) * inv_rep); };
     uint32_t cnt = 0;
     bool ok = true;
     uint32_t qf[HD / 16][4];   // A operand of 8 k-steps of 16
@@ -667,7 +696,19 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     uint32_t pcnt = 0;
     const bool has_cap = p.softcap > 0.f;
 
-    int bal_key = 0, bal_flags = F_LAST;     // balanced kernels: position inside the piece
+    // Balanced kernels clear accumulators and queries where an item ends, not where one begins: their registers are then
+    // free during the merge (an e4m3 kernel has 168).
+    auto clear_o = [&]() {
+#pragma unroll
+      for (int i = 0; i < HDV / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
+    };
+    auto clear = [&]() {
+      clear_o();
+#pragma unroll
+      for (int i = 0; i < HD / 16; ++i) { qf[i][0] = qf[i][1] = qf[i][2] = qf[i][3] = 0u; }
+    };
+    if constexpr (BAL) clear();
+    int bal_key = 0, bal_end = 0, bal_flags = F_LAST;     // balanced kernels: position inside the piece
     while (true) {
       const uint32_t s = cnt % NST;
       // balanced kernels: the piece stays in its mailbox slot until its rows are written
@@ -682,11 +723,12 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           bal_flags = F_FIRST;
           if (cur.it.lo >= cur.it.hi) bal_flags |= F_EMPTY;
           bal_key = cur.it.lo * TN;
+          bal_end = cur.it.hi * TN;
         } else {
           bal_flags = 0;
           bal_key += TNS;
         }
-        if (bal_key + TNS >= cur.it.hi * TN) bal_flags |= F_LAST;
+        if (bal_key + TNS >= bal_end) bal_flags |= F_LAST;
         key0 = bal_key; flags = bal_flags;
       } else {
         ok = wait_or_abort(bar_full + 8 * s, (cnt / NST) & 1, s_abort);
@@ -698,22 +740,22 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       if (flags & F_FIRST) {
         if constexpr (!BAL) it_reg = decode_work(p, wid);
         const int rows_total = it.seqlen_q * rep;
+        const int di = it.b * p.descale_batch_stride + it.hk * p.descale_head_stride;
+        const float ds_q = p.q_descale ? p.q_descale[di] : 1.f, ds_k = p.k_descale ? p.k_descale[di] : 1.f;
+        vds = p.v_descale ? p.v_descale[di] : 1.f;
         // Q fragments straight from global memory (rows g and g+8 of the packed tile)
         if constexpr (!KV8) {
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
+          for (int rr = 0; rr < 2; ++rr) {       // A operand of m16n8k16: columns ks*16 + 2*tq (+8)
+            const int R = it.mt * 16 + g + rr * 8;
+            const bool live = R < rows_total;
+            const int token = live ? token_of(R) : 0, head = it.hk * rep + (live ? R - token * rep : 0);
+            const T* qrow = reinterpret_cast<const T*>(p.q) + (int64_t)(it.q0 + token) * p.q_row_stride +
+                            (int64_t)head * p.q_head_stride + 2 * tq;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {      // A operand of m16n8k16: columns ks*16 + 2*tq (+8)
-              const int R = it.mt * 16 + g + (e & 1) * 8;
-              const int c = ks * 16 + 2 * tq + (e >> 1) * 8;
-              uint32_t v = 0;
-              if (R < rows_total) {
-                const int token = R / rep, head = it.hk * rep + R % rep;
-                v = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(p.q) +
-                                                       (int64_t)(it.q0 + token) * p.q_row_stride +
-                                                       (int64_t)head * p.q_head_stride + c);
-              }
-              qf[ks][e] = v;
+            for (int ks = 0; ks < HD / 16; ++ks) {
+              qf[ks][rr] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16) : 0u;
+              qf[ks][rr + 2] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8) : 0u;
             }
           }
         } else {
@@ -721,34 +763,39 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           // (see the QK loop), so k-step ks contracts positions 16ks + {4tq, 4tq+1 | 4tq+2, 4tq+3} in its two halves;
           // Q is gathered in the same order (a sum does not care about the order of its terms).  Each row is
           // scaled so that its largest magnitude is 256 before conversion to fp16.
-          float qv[2][HD / 16][4];
+          // (both rows' loads go out before the first is used)
+          uint2 raw[2][HD / 16];
           float amax[2] = {0.f, 0.f};
+          auto widen = [](uint2 rw, float (&f)[4]) {
+            if (std::is_same<T, __nv_bfloat16>::value) {
+              f[0] = __uint_as_float(rw.x << 16); f[1] = __uint_as_float(rw.x & 0xffff0000u);
+              f[2] = __uint_as_float(rw.y << 16); f[3] = __uint_as_float(rw.y & 0xffff0000u);
+            } else {
+              const float2 lo2 = __half22float2(*reinterpret_cast<const __half2*>(&rw.x));
+              const float2 hi2 = __half22float2(*reinterpret_cast<const __half2*>(&rw.y));
+              f[0] = lo2.x; f[1] = lo2.y; f[2] = hi2.x; f[3] = hi2.y;
+            }
+          };
 #pragma unroll
           for (int rr = 0; rr < 2; ++rr) {
             const int R = it.mt * 16 + g + rr * 8;
             const bool live = R < rows_total;
-            const int token = R / rep, head = it.hk * rep + R % rep;
-            const T* qrow = reinterpret_cast<const T*>(p.q) + (int64_t)(it.q0 + (live ? token : 0)) * p.q_row_stride +
-                            (int64_t)(live ? head : 0) * p.q_head_stride;
+            const int token = live ? token_of(R) : 0, head = live ? it.hk * rep + R - token * rep : 0;
+            const T* qrow = reinterpret_cast<const T*>(p.q) + (int64_t)(it.q0 + token) * p.q_row_stride +
+                            (int64_t)head * p.q_head_stride;
 #pragma unroll
-            for (int ks = 0; ks < HD / 16; ++ks) {
-              uint2 raw = make_uint2(0u, 0u);
-              if (live) raw = *reinterpret_cast<const uint2*>(qrow + ks * 16 + 4 * tq);
-              float f[4];
-              if (std::is_same<T, __nv_bfloat16>::value) {
-                f[0] = __uint_as_float(raw.x << 16); f[1] = __uint_as_float(raw.x & 0xffff0000u);
-                f[2] = __uint_as_float(raw.y << 16); f[3] = __uint_as_float(raw.y & 0xffff0000u);
-              } else {
-                const float2 lo2 = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-                const float2 hi2 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-                f[0] = lo2.x; f[1] = lo2.y; f[2] = hi2.x; f[3] = hi2.y;
-              }
-#pragma unroll
-              for (int j = 0; j < 4; ++j) { qv[rr][ks][j] = f[j]; amax[rr] = fmaxf(amax[rr], fabsf(f[j])); }
-            }
+            for (int ks = 0; ks < HD / 16; ++ks)
+              raw[rr][ks] = live ? *reinterpret_cast<const uint2*>(qrow + ks * 16 + 4 * tq) : make_uint2(0u, 0u);
           }
 #pragma unroll
           for (int rr = 0; rr < 2; ++rr) {
+#pragma unroll
+            for (int ks = 0; ks < HD / 16; ++ks) {
+              float f[4];
+              widen(raw[rr][ks], f);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) amax[rr] = fmaxf(amax[rr], fabsf(f[j]));
+            }
             amax[rr] = fmaxf(amax[rr], __shfl_xor_sync(0xffffffffu, amax[rr], 1));
             amax[rr] = fmaxf(amax[rr], __shfl_xor_sync(0xffffffffu, amax[rr], 2));
           }
@@ -756,37 +803,34 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           qs_a = 1.f / sq_a; qs_b = 1.f / sq_b;
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks) {
-            qf[ks][0] = pack2<__half>(qv[0][ks][0] * sq_a, qv[0][ks][1] * sq_a);
-            qf[ks][1] = pack2<__half>(qv[1][ks][0] * sq_b, qv[1][ks][1] * sq_b);
-            qf[ks][2] = pack2<__half>(qv[0][ks][2] * sq_a, qv[0][ks][3] * sq_a);
-            qf[ks][3] = pack2<__half>(qv[1][ks][2] * sq_b, qv[1][ks][3] * sq_b);
+            float fa_[4], fb_[4];
+            widen(raw[0][ks], fa_);
+            widen(raw[1][ks], fb_);
+            qf[ks][0] = pack2<__half>(fa_[0] * sq_a, fa_[1] * sq_a);
+            qf[ks][1] = pack2<__half>(fb_[0] * sq_b, fb_[1] * sq_b);
+            qf[ks][2] = pack2<__half>(fa_[2] * sq_a, fa_[3] * sq_a);
+            qf[ks][3] = pack2<__half>(fb_[2] * sq_b, fb_[3] * sq_b);
           }
         }
-        float sc = p.scale;
-        vds = 1.f;
-        const int di = it.b * p.descale_batch_stride + it.hk * p.descale_head_stride;
-        if (p.q_descale) sc *= p.q_descale[di];
-        if (p.k_descale) sc *= p.k_descale[di];
-        if (p.v_descale) vds = p.v_descale[di];
+        const float sc = p.scale * ds_q * ds_k;
         c_mul = has_cap ? p.softcap * kLog2e : sc * kLog2e;
         cap_in = has_cap ? sc / p.softcap : 0.f;
         const int off = it.seqlen_k - it.seqlen_q;
         const int rb = it.mt * 16;                   // first packed row of this work item
-        const int qp_a = off + (rb + g) / rep, qp_b = off + (rb + g + 8) / rep;
+        const int qp_a = off + token_of(rb + g), qp_b = off + token_of(rb + g + 8);
         lo_a = lo_b = it.leftpad;
         hi_a = hi_b = min(it.seqlen_k, it.hi * TN) - 1;   // keys past this split's range are not ours
         if (p.is_causal) { hi_a = min(hi_a, qp_a); hi_b = min(hi_b, qp_b); }
         if (p.window_right >= 0) { hi_a = min(hi_a, qp_a + p.window_right); hi_b = min(hi_b, qp_b + p.window_right); }
         if (p.window_left >= 0) { lo_a = max(lo_a, qp_a - p.window_left); lo_b = max(lo_b, qp_b - p.window_left); }
         // bounds valid for all 16 rows (rows past rows_total included: conservative)
-        const int qp_lo = off + rb / rep, qp_hi = off + (rb + 15) / rep;
+        const int qp_lo = off + token_of(rb), qp_hi = off + token_of(rb + 15);
         lo_max = it.leftpad; hi_min = min(it.seqlen_k, it.hi * TN) - 1;
         if (p.is_causal) hi_min = min(hi_min, qp_lo);
         if (p.window_right >= 0) hi_min = min(hi_min, qp_lo + p.window_right);
         if (p.window_left >= 0) lo_max = max(lo_max, qp_hi - p.window_left);
         m_a = m_b = -INFINITY; l_a = l_b = 0.f;
-#pragma unroll
-        for (int i = 0; i < HDV / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
+        if constexpr (!BAL) clear_o();
       }
 
       if constexpr (BAL) {      // (the queries above are fetched while the first stage is on its way)
@@ -955,8 +999,9 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         bar_consumers<NC>();
         {
           constexpr int CPT = 16 * HDV / (NC * 32);      // output columns per thread: 16 or 8
-          constexpr int GPR = HDV / CPT;                 // threads per row
-          const int Rl = tid / GPR, c0 = (tid % GPR) * CPT;   // row within the tile, first column
+          constexpr int GPR = HDV / CPT;                 // threads per row, side by side: four columns each, CPT / 4 times
+          constexpr int CST = 4 * GPR;                   // (16 columns in a row per thread: four-way bank conflicts)
+          const int Rl = tid / GPR, c0 = (tid % GPR) * 4;     // row within the tile, first column
           const int R = it.mt * 16 + Rl;                     // packed row (token, head)
           const int rows_total = it.seqlen_q * rep;
           float mw[NC], M = -INFINITY;
@@ -972,7 +1017,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
             const float* src = s_o + (wi * 16 + Rl) * SM::kLdO + c0;
 #pragma unroll
             for (int j = 0; j < CPT; j += 4) {
-              const float4 v4 = *reinterpret_cast<const float4*>(src + j);
+              const float4 v4 = *reinterpret_cast<const float4*>(src + j / 4 * CST);
               acc[j] += e * v4.x; acc[j + 1] += e * v4.y; acc[j + 2] += e * v4.z; acc[j + 3] += e * v4.w;
             }
           }
@@ -986,54 +1031,90 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
                 float* po = p.part_o + (slot * p.part_rows + Rl) * HDV + c0;
 #pragma unroll
                 for (int j = 0; j < CPT; j += 4)
-                  *reinterpret_cast<float4*>(po + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+                  *reinterpret_cast<float4*>(po + j / 4 * CST) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
                 if (tid % GPR == 0) reinterpret_cast<float2*>(p.part_ml)[slot * p.part_rows + Rl] = make_float2(M, L);
               }
               bar_consumers<NC>();       // (thread 0's fence then covers the rows of all four warps)
               if (tid == 0) {
-                __threadfence();
+                // (release: the rows of all four warps lie behind the barrier; acquire: the other pieces' rows)
                 unsigned* word = p.arrivals + cur.first;
-                const bool last = atomicAdd(word, 1u) == (unsigned)cur.pieces - 1u;
+                const bool last = atomic_add_acq_rel(word, 1u) == (unsigned)cur.pieces - 1u;
                 if (last) *word = 0u;        // zero again for the next call
-                __threadfence();
                 *s_last = last ? 1 : 0;
               }
               bar_consumers<NC>();
               if (*s_last) {
-                // piece j lies in slot 2 (first + j) + (j == 0).  Weights first, a warp per row and a lane per piece (the
-                // merge area is free: every warp has written its piece); then all threads over (row, 4 columns).  With
-                // every thread reading the pairs by itself, twice and one after the other, 148 pieces took some 20 us.
+                // piece j lies in slot 2 (first + j) + (j == 0).  All threads over (row, 4 columns).  Few pieces: a thread
+                // loads the rows and their pairs together, one trip to L2.  Many: weights first, every pair loaded before any
+                // is used, then a warp per row and a lane per piece (the merge area is free: every warp has written its
+                // piece).  (With every thread reading many pairs by itself, one after the other, 148 pieces took some 20 us;
+                // a warp that took its rows one after the other waited for two trips per row, 6600 cycles for 16 rows.)
                 const int live = min(p.part_rows, rows_total - it.mt * 16), np = cur.pieces;
                 const int64_t s0 = (int64_t)cur.first * 2;
                 const float2* ml = reinterpret_cast<const float2*>(p.part_ml);
-                for (int r = warp; r < live; r += NC) {
-                  float Mx = -INFINITY, Ls = 0.f;
-                  for (int j = lane; j < np; j += 32) Mx = fmaxf(Mx, __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows + r).x);
-#pragma unroll
-                  for (int d = 16; d > 0; d >>= 1) Mx = fmaxf(Mx, __shfl_xor_sync(0xffffffffu, Mx, d));
-                  for (int j = lane; j < np; j += 32) {
-                    const float2 q2 = __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows + r);
-                    const float e = Mx > -INFINITY ? ex2(q2.x - Mx) : 0.f;   // (a piece without visible keys: exactly 0, its rows are 0)
-                    s_o[r * kMaxMerge + j] = e;
-                    Ls += e * q2.y;
+                float2* pairs = reinterpret_cast<float2*>(s_o);      // (maximum, sum), then (weight, sum)
+                if (np > kFewPieces) {
+                  for (int u = tid; u < live * np; u += NC * 32) {
+                    const int j = u / live, r = u - j * live;
+                    pairs[r * kMaxMerge + j] = __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows + r);
                   }
+                  bar_consumers<NC>();
+#pragma unroll 1
+                  for (int r = warp; r < live; r += NC) {
+                    float Mx = -INFINITY, Ls = 0.f;
+                    for (int j = lane; j < np; j += 32) Mx = fmaxf(Mx, pairs[r * kMaxMerge + j].x);
 #pragma unroll
-                  for (int d = 16; d > 0; d >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, d);
-                  if (lane == 0) { s_m[r] = Mx; s_l[r] = Ls; }
+                    for (int d = 16; d > 0; d >>= 1) Mx = fmaxf(Mx, __shfl_xor_sync(0xffffffffu, Mx, d));
+                    for (int j = lane; j < np; j += 32) {
+                      const float2 q2 = pairs[r * kMaxMerge + j];
+                      const float e = Mx > -INFINITY ? ex2(q2.x - Mx) : 0.f;   // (a piece without visible keys: exactly 0, its rows are 0)
+                      pairs[r * kMaxMerge + j].x = e;
+                      Ls += e * q2.y;
+                    }
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, d);
+                    if (lane == 0) { s_m[r] = Mx; s_l[r] = Ls; }
+                  }
+                  bar_consumers<NC>();
                 }
-                bar_consumers<NC>();
+#pragma unroll 1
                 for (int u = tid; u < live * (HDV / 4); u += NC * 32) {
                   const int r = u / (HDV / 4), c4 = (u - r * (HDV / 4)) * 4;
                   const float* pr = p.part_o + (int64_t)r * HDV + c4;
-                  float Mx = s_m[r], Ls = s_l[r];
+                  float Mx, Ls;
                   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                  if (np > kFewPieces) {
+                    Mx = s_m[r]; Ls = s_l[r];
 #pragma unroll 8
-                  for (int j = 0; j < np; ++j) {
-                    const float4 w4 = __ldcg(reinterpret_cast<const float4*>(pr + (s0 + 2 * j + (j == 0)) * p.part_rows * HDV));
-                    const float e = s_o[r * kMaxMerge + j];
-                    v.x += e * w4.x; v.y += e * w4.y; v.z += e * w4.z; v.w += e * w4.w;
+                    for (int j = 0; j < np; ++j) {
+                      const float4 w4 = __ldcg(reinterpret_cast<const float4*>(pr + (s0 + 2 * j + (j == 0)) * p.part_rows * HDV));
+                      const float e = pairs[r * kMaxMerge + j].x;
+                      v.x += e * w4.x; v.y += e * w4.y; v.z += e * w4.z; v.w += e * w4.w;
+                    }
+                  } else {
+                    float2 ml_[kFewPieces];
+                    float4 w4[kFewPieces];
+                    Mx = -INFINITY; Ls = 0.f;
+#pragma unroll
+                    for (int j = 0; j < kFewPieces; ++j) {
+                      ml_[j] = make_float2(-INFINITY, 0.f);
+                      w4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                      if (j < np) {
+                        const int64_t slot = (s0 + 2 * j + (j == 0)) * p.part_rows;
+                        ml_[j] = __ldcg(ml + slot + r);
+                        w4[j] = __ldcg(reinterpret_cast<const float4*>(pr + slot * HDV));
+                      }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kFewPieces; ++j) Mx = fmaxf(Mx, ml_[j].x);
+#pragma unroll
+                    for (int j = 0; j < kFewPieces; ++j) {
+                      const float e = Mx > -INFINITY ? ex2(ml_[j].x - Mx) : 0.f;
+                      Ls += e * ml_[j].y;
+                      v.x += e * w4[j].x; v.y += e * w4[j].y; v.z += e * w4[j].z; v.w += e * w4[j].w;
+                    }
                   }
-                  const int Rg = it.mt * 16 + r, token = Rg / rep, head = it.hk * rep + Rg % rep;
+                  const int Rg = it.mt * 16 + r, token = token_of(Rg), head = it.hk * rep + Rg - token * rep;
                   const int64_t qi = it.q0 + token;
                   float osc = 1.f;
                   if (p.s_aux) {
@@ -1053,14 +1134,14 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
               }
             }
           } else if (R < rows_total) {
-            const int token = R / rep, head = it.hk * rep + R % rep;
+            const int token = token_of(R), head = it.hk * rep + R - token * rep;
             const int64_t qi = it.q0 + token;
             if (!BAL && p.nsplits > 1) {
               const float inv = L > 0.f ? vds / L : 0.f;
               float* op = p.o_part + (((int64_t)it.split * p.total_q + qi) * p.hq + head) * p.hdv + c0;
 #pragma unroll
               for (int j = 0; j < CPT; j += 4)
-                *reinterpret_cast<float4*>(op + j) = make_float4(acc[j] * inv, acc[j + 1] * inv, acc[j + 2] * inv, acc[j + 3] * inv);
+                *reinterpret_cast<float4*>(op + j / 4 * CST) = make_float4(acc[j] * inv, acc[j + 1] * inv, acc[j + 2] * inv, acc[j + 3] * inv);
               if (tid % GPR == 0)
                 p.lse_part[((int64_t)it.split * p.hq + head) * p.total_q + qi] = L > 0.f ? (M + lg2(L)) * kLn2 : -INFINITY;
             } else {
@@ -1077,21 +1158,19 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
                 float* of = reinterpret_cast<float*>(p.out) + qi * p.o_row_stride + (int64_t)head * p.o_head_stride + c0;
 #pragma unroll
                 for (int j = 0; j < CPT; j += 4)
-                  *reinterpret_cast<float4*>(of + j) = make_float4(acc[j] * inv, acc[j + 1] * inv, acc[j + 2] * inv, acc[j + 3] * inv);
+                  *reinterpret_cast<float4*>(of + j / 4 * CST) = make_float4(acc[j] * inv, acc[j + 1] * inv, acc[j + 2] * inv, acc[j + 3] * inv);
               } else {
                 T* op = reinterpret_cast<T*>(p.out) + qi * p.o_row_stride + (int64_t)head * p.o_head_stride + c0;
 #pragma unroll
-                for (int j = 0; j < CPT; j += 8) {
-                  uint4 v;
-                  v.x = pack2<T>(acc[j] * inv, acc[j + 1] * inv);     v.y = pack2<T>(acc[j + 2] * inv, acc[j + 3] * inv);
-                  v.z = pack2<T>(acc[j + 4] * inv, acc[j + 5] * inv); v.w = pack2<T>(acc[j + 6] * inv, acc[j + 7] * inv);
-                  *reinterpret_cast<uint4*>(op + j) = v;
-                }
+                for (int j = 0; j < CPT; j += 4)
+                  *reinterpret_cast<uint2*>(op + j / 4 * CST) =
+                      make_uint2(pack2<T>(acc[j] * inv, acc[j + 1] * inv), pack2<T>(acc[j + 2] * inv, acc[j + 3] * inv));
               }
               if (tid % GPR == 0) p.lse[(int64_t)head * p.total_q + qi] = L > 0.f ? (M + lg2(L)) * kLn2 : -INFINITY;
             }
           }
         }
+        if constexpr (BAL) clear();
         bar_consumers<NC>();   // the scratch area is free again
         if constexpr (BAL) {
           if (lane == 0) mbar_arrive(bar_pc_empty + 8 * (pcnt % kPieces));

@@ -77,6 +77,12 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
   }
 }
 
+__device__ __forceinline__ unsigned atomic_add_acq_rel(unsigned* p, unsigned v) {
+  unsigned old;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+
 // Persistent kernels take work ids from counters[0].  ONE thread of every CTA calls this after the CTA's last
 // ticket: the last CTA of the grid to arrive puts both words back to zero, so the next launch on the stream
 // finds them clean without a memset in between.
