@@ -7,7 +7,7 @@
 //
 //   warp 4      producer: resolves page-table entries (32 at a time, one coalesced load) and streams whole
 //               pages with TMA 2-D boxes over the page pool viewed as [num_pages * page_size, hkv * hd] into a
-//               ring of 32 KB stages (64 keys of 16-bit K+V, or 128 keys of e4m3 K+V; 128-byte swizzle).  The ring runs on across
+//               ring of two stages of 128 keys of K and V (128-byte swizzle).  The ring runs on across
 //               work-item boundaries; each stage carries a small descriptor (work id, first key, flags).  Pages
 //               of 1, 2 or 4 keys are fetched with cp.async, 16 bytes per lane, into the same swizzled layout.
 //   warps 0-3   consumers: each takes a quarter of the stage's keys: S = Q K^T and O += P V with warp-level
@@ -30,13 +30,13 @@ namespace fa {
 namespace dec {
 
 
-constexpr int TN = 64;                 // keys per scheduler block (metadata unit); a stage holds TNS keys
-// Consumer warps per CTA.  A 16-bit cache runs one CTA per SM; an e4m3 cache runs TWO (half-size stages): every
-// consumer warp works on every stage, so one CTA's stage rate is bounded by the latency of one warp's
-// ldmatrix -> widen -> MMA -> softmax -> MMA chain, and with twice the keys per byte that chain, not HBM, was the
-// limit; a second CTA's chain runs beside it.
+constexpr int TN = 64;                 // keys per scheduler block (metadata unit)
+constexpr int kStageKeys = 128;        // keys of a stage of the ring: 32 per consumer warp, two independent chains (see launch_decode_t)
+// Consumer warps per CTA.  Head dims of 128 and more run one CTA per SM over a 16-bit cache; an e4m3 cache and head_dim 64
+// run TWO (half-size stages): every consumer warp works on every stage, so one CTA's stage rate is bounded by the latency
+// of one warp's ldmatrix -> (widen) -> MMA -> softmax -> MMA chain, and with twice the keys per byte that chain, not HBM, was
+// the limit; a second CTA's chain runs beside it.
 constexpr int ncons_for(int) { return 4; }
-constexpr int ctas_per_sm(int esz) { return esz == 1 ? 2 : 1; }
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr int kPieces = 4;             // mailbox slots between the producer and the consumers
@@ -70,10 +70,10 @@ struct DecArgs {
   int class_rows;     // > 0: only sequences with at most this many packed query rows (the short ones of a mixed batch)
 };
 
-template <int ESZ, int NST, int HD, int HDV, int TNS_>
+template <int ESZ, int NST, int HD, int HDV>
 struct Smem {
-  static constexpr int TNS = TNS_;                  // keys per stage (64, or 128: two independent 16-key chains per warp)
-  static constexpr int NC = ncons_for(ESZ);         // consumer warps; 16 keys per warp and stage either way
+  static constexpr int TNS = kStageKeys;
+  static constexpr int NC = ncons_for(ESZ);         // consumer warps
   static constexpr int kKBytes = TNS * HD * ESZ, kVBytes = TNS * HDV * ESZ;
   static constexpr int kStage = kKBytes + kVBytes;
   static constexpr int kRing = NST * kStage;
@@ -304,14 +304,13 @@ __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* sr
 }
 
 // T = MMA element type (bf16 / fp16); KV8 = the cache holds e4m3 bytes.
-template <typename T, bool KV8, int NST, int HD, int HDV, int CPS, int TNS_, bool BAL>
+template <typename T, bool KV8, int NST, int HD, int HDV, int CPS, bool BAL>
 __global__ void __launch_bounds__((ncons_for(KV8 ? 1 : 2) + 1) * 32, CPS)
 fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v) {
   constexpr int ESZ = KV8 ? 1 : 2;
   static_assert(!KV8 || (HD == 128 && HDV == 128), "an e4m3 cache row must fill one 128-byte swizzle row");
   static_assert(HD % 64 == 0 && HDV % 64 == 0, "whole 128-byte column blocks");
-  using SM = Smem<ESZ, NST, HD, HDV, TNS_>;
-  static_assert(!(TNS_ != 64 && !KV8), "the 16-bit consumers take 16 keys per warp and stage");
+  using SM = Smem<ESZ, NST, HD, HDV>;
   // 16-bit cache: m16n8k16 MMA in the cache's type.  e4m3 cache: the bytes are widened to fp16 in registers (exact,
   // one conversion per two elements) and fed to the fp16 m16n8k16 MMA; Q rows are scaled into fp16 range with a
   // per-row factor (undone in the softmax scale), P is fp16.  (The warp-level e4m3 MMA is not used: on sm_100a
@@ -320,7 +319,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   using TM = typename std::conditional<KV8, __half, T>::type;
   constexpr int TNS = SM::TNS;            // keys per stage
   constexpr int NC = SM::NC;
-  constexpr int WK = TNS / NC;            // keys per consumer warp and stage: 16
+  constexpr int WK = TNS / NC;            // keys per consumer warp and stage: 32
   constexpr int NT = WK / 8;              // 8-key MMA column tiles per warp
   const KParams& p = a.kp;
   extern __shared__ unsigned char smem_dyn[];
@@ -847,11 +846,14 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           const uint32_t krow = kb + (uint32_t)(warp * WK + (mat >> 1) * 8 + l7) * 128u;
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks) {
-            uint32_t bfr[4];
             const uint32_t chunk = (uint32_t)((ks * 2 + (mat & 1)) & 7);
-            ldmatrix_x4(bfr, krow + (ks >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
-            mma_16816<TM>(sacc[0], qf[ks], bfr[0], bfr[1]);
-            mma_16816<TM>(sacc[1], qf[ks], bfr[2], bfr[3]);
+#pragma unroll
+            for (int hf = 0; hf < WK / 16; ++hf) {
+              uint32_t bfr[4];
+              ldmatrix_x4(bfr, krow + hf * (16 * 128) + (ks >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
+              mma_16816<TM>(sacc[2 * hf], qf[ks], bfr[0], bfr[1]);
+              mma_16816<TM>(sacc[2 * hf + 1], qf[ks], bfr[2], bfr[3]);
+            }
           }
         } else {
           // e4m3 rows are 128 bytes: one swizzle row per key.  ldmatrix moves 16-byte chunks, so lane (g, tq)
@@ -919,19 +921,22 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         }
         // ---- O += P V ----
         if constexpr (!KV8) {
-          uint32_t pa[4];
-          pa[0] = pack2<TM>(sacc[0][0], sacc[0][1]);
-          pa[1] = pack2<TM>(sacc[0][2], sacc[0][3]);
-          pa[2] = pack2<TM>(sacc[1][0], sacc[1][1]);
-          pa[3] = pack2<TM>(sacc[1][2], sacc[1][3]);
-          const uint32_t vrow = vb + (uint32_t)(warp * WK + (mat & 1) * 8 + l7) * 128u;
 #pragma unroll
-          for (int np = 0; np < HDV / 16; ++np) {
-            uint32_t bfr[4];
-            const uint32_t chunk = (uint32_t)((np * 2 + (mat >> 1)) & 7);
-            ldmatrix_x4_trans(bfr, vrow + (np >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
-            mma_16816<TM>(o[2 * np], pa, bfr[0], bfr[1]);
-            mma_16816<TM>(o[2 * np + 1], pa, bfr[2], bfr[3]);
+          for (int hf = 0; hf < WK / 16; ++hf) {
+            uint32_t pa[4];
+            pa[0] = pack2<TM>(sacc[2 * hf][0], sacc[2 * hf][1]);
+            pa[1] = pack2<TM>(sacc[2 * hf][2], sacc[2 * hf][3]);
+            pa[2] = pack2<TM>(sacc[2 * hf + 1][0], sacc[2 * hf + 1][1]);
+            pa[3] = pack2<TM>(sacc[2 * hf + 1][2], sacc[2 * hf + 1][3]);
+            const uint32_t vrow = vb + (uint32_t)(warp * WK + hf * 16 + (mat & 1) * 8 + l7) * 128u;
+#pragma unroll
+            for (int np = 0; np < HDV / 16; ++np) {
+              uint32_t bfr[4];
+              const uint32_t chunk = (uint32_t)((np * 2 + (mat >> 1)) & 7);
+              ldmatrix_x4_trans(bfr, vrow + (np >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
+              mma_16816<TM>(o[2 * np], pa, bfr[0], bfr[1]);
+              mma_16816<TM>(o[2 * np + 1], pa, bfr[2], bfr[3]);
+            }
           }
         } else {
           // P as the fp16 A operand, one k-step of 16 keys at a time.
@@ -1226,9 +1231,9 @@ static int line_team(int hkv, int ctas) {
   return team;
 }
 
-template <typename T, bool KV8, int NST, int HD, int HDV, bool BAL, int CPS = ctas_per_sm(KV8 ? 1 : 2), int TNS_ = 64>
+template <typename T, bool KV8, int NST, int HD, int HDV, bool BAL, int CPS>
 static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaStream_t stream) {
-  using SM = Smem<KV8 ? 1 : 2, NST, HD, HDV, TNS_>;
+  using SM = Smem<KV8 ? 1 : 2, NST, HD, HDV>;
   DecArgs a;
   a.kp = kp;
   a.total_work = num_work_slots * kp.hkv * kp.nsplits;
@@ -1250,7 +1255,7 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
   CUtensorMap mk, mv;
   if (!make_map(&mk, kp.k, kvdt, rows, (uint64_t)kp.hkv * HD, (uint64_t)kp.k_row_stride, a.box_rows)) return -1;
   if (!make_map(&mv, kp.v, kvdt, rows, (uint64_t)kp.hkv * HDV, (uint64_t)kp.v_row_stride, a.box_rows)) return -1;
-  auto kern = fwd_decode_kernel<T, KV8, NST, HD, HDV, CPS, TNS_, BAL>;
+  auto kern = fwd_decode_kernel<T, KV8, NST, HD, HDV, CPS, BAL>;
   const int smem = (BAL ? SM::kBytesBalanced : SM::kBytes) + 1024;
   static std::atomic<unsigned long long> attr_done{0};   // one bit per device
   int dev = 0;
@@ -1300,12 +1305,16 @@ bool decode_supported(const PlanInput& in) {
 
 template <typename T, bool BAL>
 static int launch_decode_t(const KParams& kp, const Plan& pl, int slots, cudaStream_t stream) {
-  // e4m3 cache: 128-key stages (32 keys = two independent 16-key chains per consumer warp: the chains hide each
-  // other's fixed latencies; 0.80 -> 0.92 of the HBM peak against 64-key stages), two stages, two CTAs per SM
-  if (kp.kv_fp8) return dec::launch_t<T, true, 2, 128, 128, BAL, 2, 128>(kp, pl, slots, stream);
-  if (kp.hd == 64) return dec::launch_t<T, false, 5, 64, 64, BAL, 2>(kp, pl, slots, stream);   // 16 KB stages: two CTAs per SM
-  if (kp.hd == 192) return dec::launch_t<T, false, 4, 192, 128, BAL>(kp, pl, slots, stream);
-  return dec::launch_t<T, false, 5, 128, 128, BAL>(kp, pl, slots, stream);
+  // Two stages of 128 keys everywhere: 32 keys = two independent 16-key chains per consumer warp, which hide each other's
+  // fixed latencies, half the stage hand-offs per byte, and for small pages enough copies per stage for every lane of the
+  // producer.  e4m3 cache: 0.80 -> 0.92 of the HBM peak against 64-key stages (of which more fit).  16-bit caches, against
+  // five stages of 64 keys (four at head_dim 192), in a CUDA graph: 16 sequences of 1024 .. 16384 keys over pages of 64 /
+  // 16 keys 94.6 -> 90.1 / 138 -> 109 us, 24 x 4 queries of head_dim 64 (two row tiles) 79.5 -> 65.3, of head_dim 128
+  // 115 -> 95, of 192 over 16 sequences 101 -> 92, 128 sequences of 1024 .. 32768 keys 1328 -> 1269.
+  if (kp.kv_fp8) return dec::launch_t<T, true, 2, 128, 128, BAL, 2>(kp, pl, slots, stream);
+  if (kp.hd == 64) return dec::launch_t<T, false, 2, 64, 64, BAL, 2>(kp, pl, slots, stream);   // 32 KB stages: two CTAs per SM
+  if (kp.hd == 192) return dec::launch_t<T, false, 2, 192, 128, BAL, 1>(kp, pl, slots, stream);
+  return dec::launch_t<T, false, 2, 128, 128, BAL, 1>(kp, pl, slots, stream);
 }
 
 int launch_decode(const KParams& kp, const Plan& pl, int compute_dtype, cudaStream_t stream) {
