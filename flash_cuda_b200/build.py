@@ -1,7 +1,8 @@
-"""In-tree build of the two shared libraries (no JIT cache, so the built files travel with the tree):
+"""In-tree build of the shared libraries (no JIT cache, so the built files travel with the tree):
 
   flash_cuda_b200/lib/libfa_b200.so     the C-ABI library (include/fa_b200.h): CUDA kernels + planner
   flash_cuda_b200/lib/fa_b200_torch.so  the torch-op boundary (`fwd`, `get_scheduler_metadata`), links the first
+  flash_cuda_b200/lib/fa_b200_direct.so `fwd` as a Python function for calls the dispatcher has nothing to do for, links the second
 
 nvcc cross-compiles for sm_100a without a GPU.  `python -m flash_cuda_b200.build [--force] [-v]`.
 """
@@ -21,6 +22,7 @@ OBJ = os.path.join(LIB, "obj")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 CAPI_SO = os.path.join(LIB, "libfa_b200.so")
 TORCH_SO = os.path.join(LIB, "fa_b200_torch.so")
+DIRECT_SO = os.path.join(LIB, "fa_b200_direct.so")
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
@@ -124,29 +126,45 @@ def build_record() -> dict:
     return rec
 
 
-def build_torch_op(force=False, verbose=False, namespace="_vllm_fa3_C") -> str:
+def _torch_command(source, target, extra):
     import torch
     from torch.utils.cpp_extension import include_paths
 
-    src = os.path.join(CSRC, "torch_op.cpp")
-    stamp = _digest([src, os.path.join(INCLUDE, "fa_b200.h")], namespace + torch.__version__)
-    if not force and not _stale(TORCH_SO, stamp):
-        return TORCH_SO
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-DFA3_LIB_NAME={namespace}",
-           "-DTORCH_API_INCLUDE_EXTENSION_H", "-D_GLIBCXX_USE_CXX11_ABI=1"]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_API_INCLUDE_EXTENSION_H", "-D_GLIBCXX_USE_CXX11_ABI=1"]
     for inc in include_paths() + [sysconfig.get_paths()["include"], os.path.join(CUDA_HOME, "include")]:
         cmd += ["-isystem", inc]
-    cmd += [src, "-o", TORCH_SO, f"-L{LIB}", "-lfa_b200", f"-L{tlib}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
-            "-ltorch_cuda", "-ltorch", f"-L{CUDA_HOME}/lib64", "-lcudart",
-            "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"]
-    _run(cmd, verbose)
+    return cmd + [source, "-o", target, f"-L{LIB}", f"-L{tlib}"] + extra + [
+        "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", f"-L{CUDA_HOME}/lib64", "-lcudart",
+        "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"]
+
+
+def build_torch_op(force=False, verbose=False, namespace="_vllm_fa3_C") -> str:
+    import torch
+
+    src, hdr = os.path.join(CSRC, "torch_op.cpp"), os.path.join(CSRC, "torch_op.h")
+    stamp = _digest([src, hdr, os.path.join(INCLUDE, "fa_b200.h")], namespace + torch.__version__)
+    if not force and not _stale(TORCH_SO, stamp):
+        return TORCH_SO
+    _run(_torch_command(src, TORCH_SO, [f"-DFA3_LIB_NAME={namespace}", "-lfa_b200"]), verbose)
     _write_stamp(TORCH_SO, stamp)
     return TORCH_SO
 
 
+def build_direct(force=False, verbose=False) -> str:
+    import torch
+
+    src, hdr = os.path.join(CSRC, "torch_direct.cpp"), os.path.join(CSRC, "torch_op.h")
+    stamp = _digest([src, hdr], torch.__version__ + sys.version)
+    if not force and not _stale(DIRECT_SO, stamp):
+        return DIRECT_SO
+    _run(_torch_command(src, DIRECT_SO, ["-l:fa_b200_torch.so", "-ltorch_python"]), verbose)
+    _write_stamp(DIRECT_SO, stamp)
+    return DIRECT_SO
+
+
 def build_all(force=False, verbose=False):
-    return build_capi(force, verbose), build_torch_op(force, verbose)
+    return build_capi(force, verbose), build_torch_op(force, verbose), build_direct(force, verbose)
 
 
 def ptxas_report() -> str:

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/fa_b200.h"
+#include "torch_op.h"
 
 #ifndef FA3_LIB_NAME
 #define FA3_LIB_NAME _vllm_fa3_C
@@ -97,9 +98,11 @@ void check_rc(int rc, const char* what) {
               rc == FA_ERR_LAUNCH ? " — " : "", rc == FA_ERR_LAUNCH ? fa_b200_last_cuda_error() : "");
 }
 
-// Mirrors mha_fwd (kernels/fa4_blackwell.cu:10081-10173): same arguments, same return
-// {out, softmax_lse, empty, empty}; unsupported configurations raise with "unsupported" in the text.
-std::vector<at::Tensor> mha_fwd(
+}  // namespace
+
+// What mha_fwd does (kernels/fa4_blackwell.cu:10081-10173), up to the two empty tensors at the end of its result;
+// unsupported configurations raise with "unsupported" in the text.
+std::pair<at::Tensor, at::Tensor> fa_b200::attention(
     at::Tensor q, at::Tensor k, at::Tensor v,
     std::optional<at::Tensor> k_new, std::optional<at::Tensor> v_new, std::optional<at::Tensor> q_v,
     std::optional<at::Tensor> out_,
@@ -323,8 +326,43 @@ std::vector<at::Tensor> mha_fwd(
     if (st != FA_OK) drop_cached_workspace(q, stream.stream());   // its header is no longer clean
     TORCH_CHECK(st == FA_OK, "fa_b200: ", fa_b200_strerror(st), " (detail=", detail, ")");
   }
-  at::Tensor empty = at::empty({0}, q.options().dtype(at::kFloat));
-  return {out, lse, empty, empty};
+  return {out, lse};
+}
+
+namespace {
+
+// Same arguments and return as the reference's {out, softmax_lse, empty, empty}.
+std::vector<at::Tensor> mha_fwd(
+    at::Tensor q, at::Tensor k, at::Tensor v,
+    std::optional<at::Tensor> k_new, std::optional<at::Tensor> v_new, std::optional<at::Tensor> q_v,
+    std::optional<at::Tensor> out_,
+    std::optional<at::Tensor> cu_seqlens_q, std::optional<at::Tensor> cu_seqlens_k,
+    std::optional<at::Tensor> cu_seqlens_k_new,
+    std::optional<at::Tensor> seqused_q, std::optional<at::Tensor> seqused_k,
+    std::optional<int64_t> max_seqlen_q, std::optional<int64_t> max_seqlen_k,
+    std::optional<at::Tensor> page_table, std::optional<at::Tensor> kv_batch_idx,
+    std::optional<at::Tensor> leftpad_k,
+    std::optional<at::Tensor> rotary_cos, std::optional<at::Tensor> rotary_sin,
+    std::optional<at::Tensor> seqlens_rotary,
+    std::optional<at::Tensor> q_descale, std::optional<at::Tensor> k_descale, std::optional<at::Tensor> v_descale,
+    double softmax_scale, bool is_causal, int64_t window_size_left, int64_t window_size_right,
+    double softcap, bool is_rotary_interleaved,
+    std::optional<at::Tensor> scheduler_metadata, int64_t num_splits, std::optional<bool> pack_gqa,
+    int64_t sm_margin,
+    std::optional<at::Tensor> s_aux, int64_t cp_world_size, int64_t cp_rank,
+    std::optional<at::Tensor> cp_tot_seqused_k) {
+  const auto options = q.options().dtype(at::kFloat);
+  auto r = fa_b200::attention(std::move(q), std::move(k), std::move(v), std::move(k_new), std::move(v_new), std::move(q_v), std::move(out_),
+                              std::move(cu_seqlens_q), std::move(cu_seqlens_k), std::move(cu_seqlens_k_new),
+                              std::move(seqused_q), std::move(seqused_k), max_seqlen_q, max_seqlen_k,
+                              std::move(page_table), std::move(kv_batch_idx), std::move(leftpad_k),
+                              std::move(rotary_cos), std::move(rotary_sin), std::move(seqlens_rotary),
+                              std::move(q_descale), std::move(k_descale), std::move(v_descale), softmax_scale,
+                              is_causal, window_size_left, window_size_right, softcap, is_rotary_interleaved,
+                              std::move(scheduler_metadata), num_splits, pack_gqa, sm_margin, std::move(s_aux),
+                              cp_world_size, cp_rank, std::move(cp_tot_seqused_k));
+  at::Tensor empty = at::empty({0}, options);
+  return {std::move(r.first), std::move(r.second), empty, empty};
 }
 
 // Mirrors mha_fwd_get_scheduler_metadata (kernels/fa4_blackwell.cu:10175-10183): same arguments; returns an
