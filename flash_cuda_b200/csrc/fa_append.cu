@@ -256,6 +256,8 @@ constexpr int kWidenBatchMax = 512;
 __global__ void __launch_bounds__(256) widen_plan_kernel(const WidenArgs a) {
   __shared__ int s_blocks[kWidenBatchMax];      // 128-row blocks a sequence needs, then its first block, -1 - that if left out
   __shared__ int s_rows, s_left;
+  wait_for_predecessors();
+  let_successor_start();
   for (int b = threadIdx.x; b < a.batch; b += 256) {
     const int len = widen_len(a, b);
     s_blocks[b] = (a.cu_q[b + 1] - a.cu_q[b]) * a.rep > a.class_rows ? (max(len, 0) + 127) / 128 : 0;
@@ -288,6 +290,8 @@ __global__ void __launch_bounds__(256) widen_plan_kernel(const WidenArgs a) {
 template <typename T>
 __global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {
   constexpr int RB = 8;                       // slab rows per turn (slabs are multiples of 128 rows)
+  wait_for_predecessors();
+  let_successor_start();
   const int rows = a.cu[a.batch];
   const int kc = a.hkv * a.k_chunks, vc = a.hkv * a.v_chunks, rc = kc + vc;
   for (int r0 = blockIdx.x * RB; r0 < rows; r0 += gridDim.x * RB) {
@@ -353,12 +357,11 @@ int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_r
   a.page_size = kp.page_size; a.page_table_stride = kp.page_table_stride;
   a.k_chunks = kp.hd / 16; a.v_chunks = kp.hdv / 16;
   a.leftpad_k = kp.leftpad_k; a.window_left = kp.window_left;
-  widen_plan_kernel<<<1, 256, 0, stream>>>(a);
+  const int rc = launch_overlapped(widen_plan_kernel, 1, 256, 0, stream, a);
+  if (rc != 0) return rc;
   int blocks = (cap_rows + 7) / 8;
   if (blocks > num_sms * 8) blocks = num_sms * 8;
-  if (compute_dtype == FA_DT_FP16) widen_kernel<__half><<<blocks, 256, 0, stream>>>(a);
-  else widen_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(a);
-  return (int)cudaGetLastError();
+  return launch_overlapped(compute_dtype == FA_DT_FP16 ? widen_kernel<__half> : widen_kernel<__nv_bfloat16>, blocks, 256, 0, stream, a);
 }
 
 int launch_depage(const KParams& kp, int kpad, void* k_out, void* v_out, int32_t* cu_out, int num_sms, cudaStream_t stream) {

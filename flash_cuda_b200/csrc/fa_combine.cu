@@ -102,6 +102,8 @@ __global__ void __launch_bounds__(256) combine_kernel(const float* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) merge_parts_kernel(const KParams p, int tile_m, int class_rows, const int32_t* skip) {
   __shared__ int s_parts;
+  wait_for_predecessors();
+  let_successor_start();
   const int qi = blockIdx.x, vec = p.hdv >> 2;
   if (threadIdx.x == 0) {
     int parts = 0;
@@ -136,9 +138,8 @@ int launch_merge_parts(const KParams& kp, int tile_m, int class_rows, const int3
   if (y > 65535) return -1;
   if (kp.total_q <= 0 || y == 0) return 0;
   const dim3 grid((unsigned)kp.total_q, (unsigned)y);
-  if (out_dtype == FA_DT_FP16) merge_parts_kernel<__half><<<grid, 256, 0, stream>>>(kp, tile_m, class_rows, skip);
-  else merge_parts_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(kp, tile_m, class_rows, skip);
-  return (int)cudaGetLastError();
+  return launch_overlapped(out_dtype == FA_DT_FP16 ? merge_parts_kernel<__half> : merge_parts_kernel<__nv_bfloat16>, grid, 256, 0,
+                           stream, kp, tile_m, class_rows, skip);
 }
 
 int launch_combine_strided(const float* o_part, const float* lse_part, int64_t o_split_stride, int64_t lse_split_stride,
@@ -216,6 +217,8 @@ __device__ __forceinline__ bool sched_entry(const SchedArgs& a, int e, int* b_ou
 __global__ void __launch_bounds__(1024) sched_kernel(const SchedArgs a, int32_t* __restrict__ out) {
   extern __shared__ __align__(16) uint32_t s_key[];   // sort keys, sort_n of them (a multiple of four)
   __shared__ int s_valid;
+  wait_for_predecessors();
+  let_successor_start();
   const int E = a.batch * a.max_mtiles;
   const int tid = threadIdx.x, nt = blockDim.x;
   const bool sorted = a.sorted != 0;
@@ -359,8 +362,7 @@ int launch_sched(const FaSchedParams& sp, const Plan& pl, int32_t* out_dev, int3
   a.row_class = row_class; a.class_rows = class_rows; a.class_rep = sp.hkv > 0 ? sp.hq / sp.hkv : 1;
   const size_t smem = a.sorted ? (size_t)a.sort_n * sizeof(uint32_t) : 0;
   const int threads = (a.sorted && a.sort_n < 1024) ? (a.sort_n < 64 ? 64 : a.sort_n) : 1024;
-  sched_kernel<<<1, threads, smem, stream>>>(a, out_dev);
-  return (int)cudaGetLastError();
+  return launch_overlapped(sched_kernel, 1, threads, smem, stream, a, out_dev);
 }
 
 }  // namespace fa

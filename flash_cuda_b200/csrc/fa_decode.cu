@@ -344,6 +344,8 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     s_abort[0] = 0; s_abort[1] = 0;
     mbar_fence_init();
   }
+  wait_for_predecessors();
+  let_successor_start();
   Piece* s_piece = reinterpret_cast<Piece*>(sm + SM::kPieceOff);
   const uint32_t bar_pc_full = base + SM::kPieceBarOff, bar_pc_empty = bar_pc_full + 8 * kPieces;
   volatile int* s_last = reinterpret_cast<volatile int*>(sm + SM::kPieceBarOff + 2 * kPieces * 8);
@@ -1275,8 +1277,7 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
     grid = (int)(spans < ctas / a.team ? spans : ctas / a.team) * a.team;
   }
   if (grid <= 0) return 0;
-  kern<<<grid, (SM::NC + 1) * 32, smem, stream>>>(a, mk, mv);
-  return (int)cudaGetLastError();
+  return launch_overlapped(kern, grid, (SM::NC + 1) * 32, smem, stream, a, mk, mv);
 }
 
 }  // namespace dec

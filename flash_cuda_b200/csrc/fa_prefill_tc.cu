@@ -429,6 +429,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
   }
   if (warp == WARP_MMA) { tmem_alloc(smem_u32(s_tmem), 512); tmem_relinquish(); }
   if (warp == WARP_TMA && lane == 0) { tma_prefetch_desc(&map_q); tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
+  wait_for_predecessors();
+  let_successor_start();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -1545,8 +1547,7 @@ static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t k
   }
   const int grid = a.num_items < pl.num_sms ? a.num_items : pl.num_sms;
   if (grid <= 0) return 0;
-  kern<<<grid, NTHREADS, smem, stream>>>(a, mq, mk, mv, mo);
-  return (int)cudaGetLastError();
+  return launch_overlapped(kern, grid, NTHREADS, smem, stream, a, mq, mk, mv, mo);
 }
 
 template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD>

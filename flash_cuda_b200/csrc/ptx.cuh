@@ -83,6 +83,13 @@ __device__ __forceinline__ unsigned atomic_add_acq_rel(unsigned* p, unsigned v) 
   return old;
 }
 
+// Programmatic dependent launch.  A kernel launched with it (launch_overlapped in fa_internal.h) may start before the
+// kernels in front of it in the stream have ended: `wait_for_predecessors` stands before its first access to memory
+// that they may read or write, and returns once they have ended and their writes are visible.  `let_successor_start`
+// allows the same to whoever comes next, once every CTA of this grid has started.
+__device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Persistent kernels take work ids from counters[0].  ONE thread of every CTA calls this after the CTA's last
 // ticket: the last CTA of the grid to arrive puts both words back to zero, so the next launch on the stream
 // finds them clean without a memset in between.
