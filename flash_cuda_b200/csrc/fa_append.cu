@@ -243,6 +243,8 @@ struct WidenArgs {
   int batch, hkv, rep, class_rows, cap_rows, page_size, page_table_stride, k_chunks, v_chunks;   // 16-byte chunks per head
   const int32_t* leftpad_k;
   int window_left;
+  int32_t* zero;      // workspace header of the kernels behind, or null: `zero_words` words to clear (a memset in front of
+  int zero_words;     // five kernels cost some 10 of 184 us: nothing overlaps with it)
 };
 
 __device__ __forceinline__ int widen_len(const WidenArgs& a, int b) {
@@ -258,6 +260,7 @@ __global__ void __launch_bounds__(256) widen_plan_kernel(const WidenArgs a) {
   __shared__ int s_rows, s_left;
   wait_for_predecessors();
   let_successor_start();
+  for (int i = threadIdx.x; i < a.zero_words; i += 256) a.zero[i] = 0;
   for (int b = threadIdx.x; b < a.batch; b += 256) {
     const int len = widen_len(a, b);
     s_blocks[b] = (a.cu_q[b + 1] - a.cu_q[b]) * a.rep > a.class_rows ? (max(len, 0) + 127) / 128 : 0;
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(256) widen_kernel(const WidenArgs a) {
 }
 
 int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_rows, void* k_out, void* v_out, int32_t* cu,
-                 int32_t* take, int32_t* lens, int num_sms, cudaStream_t stream) {
+                 int32_t* take, int32_t* lens, int32_t* zero, int zero_words, int num_sms, cudaStream_t stream) {
   if (kp.hd % 16 || kp.hdv % 16 || kp.batch <= 0 || kp.batch > kWidenBatchMax) return (int)cudaErrorInvalidValue;
   WidenArgs a;
   a.k = reinterpret_cast<const unsigned char*>(kp.k);
@@ -357,6 +360,7 @@ int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_r
   a.page_size = kp.page_size; a.page_table_stride = kp.page_table_stride;
   a.k_chunks = kp.hd / 16; a.v_chunks = kp.hdv / 16;
   a.leftpad_k = kp.leftpad_k; a.window_left = kp.window_left;
+  a.zero = zero; a.zero_words = zero_words;
   const int rc = launch_overlapped(widen_plan_kernel, 1, 256, 0, stream, a);
   if (rc != 0) return rc;
   int blocks = (cap_rows + 7) / 8;

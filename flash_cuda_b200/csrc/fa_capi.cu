@@ -16,7 +16,7 @@ namespace fa {
 int launch_sched(const FaSchedParams& sp, const Plan& pl, int32_t* out_dev, int32_t* zero_words, cudaStream_t stream,
                  int row_class = 0, int class_rows = 0, const int32_t* skip = nullptr);
 int launch_widen(const KParams& kp, int compute_dtype, int class_rows, int cap_rows, void* k_out, void* v_out, int32_t* cu,
-                 int32_t* take, int32_t* lens, int num_sms, cudaStream_t stream);
+                 int32_t* take, int32_t* lens, int32_t* zero, int zero_words, int num_sms, cudaStream_t stream);
 int launch_selftest_timeout(DeviceStatus* status, long long max_cycles, cudaStream_t stream);
 int launch_append_kv(const FaAppendParams& p, int num_sms, cudaStream_t stream);
 int launch_depage(const KParams& kp, int kpad, void* k_out, void* v_out, int32_t* cu_out, int num_sms, cudaStream_t stream);
@@ -574,13 +574,14 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   // The header (status word, work counters) must be zero when the kernels start.  A caller that keeps it clean
   // (FA_FLAG_WORKSPACE_CLEAN) saves the memset: the kernels leave the counters at zero when they finish.
   const bool clean = (p->flags & FA_FLAG_WORKSPACE_CLEAN) != 0;
-  // (on the decode route without caller metadata the work-list kernel runs first and clears the header itself)
+  // (on the decode route without caller metadata the work-list kernel runs first and clears the header itself, where an
+  // e4m3 cache is widened the kernel that lays out the slabs does)
   const bool balanced = w.part_o_off > 0;
   const bool sched_first = pl.route == FA_ROUTE_DECODE && p->scheduler_metadata == nullptr && !balanced;
-  if (!clean && !sched_first) {
+  if (!clean && !sched_first && !w.widen.on) {
     cudaError_t ce = cudaMemsetAsync(ws, 0, balanced ? kWsHeader : kWsArrivalOff, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(workspace header)");
-  } else if (balanced && !(p->flags & FA_FLAG_WORKSPACE_CLEAN_4K)) {
+  } else if (clean && balanced && !(p->flags & FA_FLAG_WORKSPACE_CLEAN_4K)) {
     // the caller keeps the first 256 bytes only
     cudaError_t ce = cudaMemsetAsync(ws + kWsArrivalOff, 0, kWsHeader - kWsArrivalOff, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(workspace header)");
@@ -688,7 +689,9 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
     int32_t* list = (int32_t*)(ws + w.work2_off);
     KParams kt = kp;
     rc = note_cuda_error(launch_widen(kp, compute_dtype, wp.class_rows, wp.cap_rows, ws + w.wd_k_off, ws + w.wd_v_off, cu,
-                                      take, (int32_t*)(ws + w.wd_lens_off), pl.num_sms, stream), "widening kernel");
+                                      take, (int32_t*)(ws + w.wd_lens_off), clean ? nullptr : (int32_t*)ws,
+                                      clean ? 0 : (balanced ? kWsHeader : kWsArrivalOff) / 4, pl.num_sms, stream),
+                         "widening kernel");
     if (rc == FA_OK)
       rc = note_cuda_error(launch_sched(sp, wp.tc, list, nullptr, stream, wp.class_rows > 0 ? 2 : 0, wp.class_rows, take), "sched_kernel");
     if (rc != FA_OK) return rc;
