@@ -321,6 +321,13 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   constexpr int NC = SM::NC;
   constexpr int WK = TNS / NC;            // keys per consumer warp and stage: 32
   constexpr int NT = WK / 8;              // 8-key MMA column tiles per warp
+  // A warp's 32 keys are two groups of 16, one of each 64-key block of the stage, each with a running maximum of its own
+  // (16-bit cache).  P is rounded to 16 bits, except where it is exactly 1: at a maximum.  With one maximum for 32 keys in
+  // a row half as many weights were exact, the largest among them, and the error against 64 bits was larger: one sequence of
+  // 1000 keys 2.024e-3 instead of 1.987e-3, in fp16 2.54e-4 instead of 2.50e-4.  The second maximum costs 1 % of the time
+  // (16 sequences of 1024 .. 16384 keys, in a graph, 77.2 -> 78.0 us, at most 4 % on short ones).  An e4m3 cache: 32 keys in a row, fp16 P.
+  constexpr int NG = KV8 ? 1 : WK / 16, GT = NT / NG;      // groups, 8-key tiles of each
+  constexpr int kWarpRows = KV8 ? WK : 16, kGroupRows = KV8 ? 16 : TN;   // first rows of warps, and of a warp's 16-key steps
   const KParams& p = a.kp;
   extern __shared__ unsigned char smem_dyn[];
   const uint32_t raw = smem_u32(smem_dyn);
@@ -845,14 +852,14 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
 #pragma unroll
         for (int i = 0; i < NT; ++i) { sacc[i][0] = sacc[i][1] = sacc[i][2] = sacc[i][3] = 0.f; }
         if constexpr (!KV8) {
-          const uint32_t krow = kb + (uint32_t)(warp * WK + (mat >> 1) * 8 + l7) * 128u;
+          const uint32_t krow = kb + (uint32_t)(warp * kWarpRows + (mat >> 1) * 8 + l7) * 128u;
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks) {
             const uint32_t chunk = (uint32_t)((ks * 2 + (mat & 1)) & 7);
 #pragma unroll
             for (int hf = 0; hf < WK / 16; ++hf) {
               uint32_t bfr[4];
-              ldmatrix_x4(bfr, krow + hf * (16 * 128) + (ks >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
+              ldmatrix_x4(bfr, krow + hf * (kGroupRows * 128) + (ks >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
               mma_16816<TM>(sacc[2 * hf], qf[ks], bfr[0], bfr[1]);
               mma_16816<TM>(sacc[2 * hf + 1], qf[ks], bfr[2], bfr[3]);
             }
@@ -879,58 +886,75 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           }
         }
         // ---- mask + online softmax over this warp's keys ----
-        const int kbase = key0 + warp * WK;
-        const bool full = (kbase >= lo_max) && (kbase + WK - 1 <= hi_min);
         const float cm_a = c_mul * (has_cap ? 1.f : qs_a), cm_b = c_mul * (has_cap ? 1.f : qs_b);
         const float ci_a = cap_in * qs_a, ci_b = cap_in * qs_b;
-        float mx_a = -INFINITY, mx_b = -INFINITY;
+        float mx_a[NG], mx_b[NG];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
+        for (int gr = 0; gr < NG; ++gr) {
+          const int kbase = key0 + warp * kWarpRows + gr * kGroupRows;
+          const bool full = (kbase >= lo_max) && (kbase + GT * 8 - 1 <= hi_min);
+          mx_a[gr] = mx_b[gr] = -INFINITY;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float y = sacc[nt][e];
-            if (e >= 2) y = has_cap ? tanh_fast(y * ci_b) * c_mul : y * cm_b;
-            else y = has_cap ? tanh_fast(y * ci_a) * c_mul : y * cm_a;
-            if (!full) {
-              const int kk = kbase + nt * 8 + 2 * tq + (e & 1);
-              const bool okk = e >= 2 ? (kk >= lo_b && kk <= hi_b) : (kk >= lo_a && kk <= hi_a);
-              y = okk ? y : -INFINITY;
+          for (int t = 0; t < GT; ++t) {
+            const int nt = gr * GT + t;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float y = sacc[nt][e];
+              if (e >= 2) y = has_cap ? tanh_fast(y * ci_b) * c_mul : y * cm_b;
+              else y = has_cap ? tanh_fast(y * ci_a) * c_mul : y * cm_a;
+              if (!full) {
+                const int kk = kbase + t * 8 + 2 * tq + (e & 1);
+                const bool okk = e >= 2 ? (kk >= lo_b && kk <= hi_b) : (kk >= lo_a && kk <= hi_a);
+                y = okk ? y : -INFINITY;
+              }
+              sacc[nt][e] = y;
+              if (e >= 2) mx_b[gr] = fmaxf(mx_b[gr], y); else mx_a[gr] = fmaxf(mx_a[gr], y);
             }
-            sacc[nt][e] = y;
-            if (e >= 2) mx_b = fmaxf(mx_b, y); else mx_a = fmaxf(mx_a, y);
           }
-        mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1));
-        mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
-        mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
-        mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
-        const float mn_a = fmaxf(m_a, mx_a), mn_b = fmaxf(m_b, mx_b);
-        const float ms_a = mn_a == -INFINITY ? 0.f : mn_a, ms_b = mn_b == -INFINITY ? 0.f : mn_b;
-        const float corr_a = ex2(m_a - ms_a), corr_b = ex2(m_b - ms_b);
-        m_a = mn_a; m_b = mn_b;
-        float ps_a = 0.f, ps_b = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          sacc[nt][0] = ex2(sacc[nt][0] - ms_a); sacc[nt][1] = ex2(sacc[nt][1] - ms_a);
-          sacc[nt][2] = ex2(sacc[nt][2] - ms_b); sacc[nt][3] = ex2(sacc[nt][3] - ms_b);
-          ps_a += sacc[nt][0] + sacc[nt][1];
-          ps_b += sacc[nt][2] + sacc[nt][3];
         }
-        l_a = l_a * corr_a + ps_a;
-        l_b = l_b * corr_b + ps_b;
-        if (__any_sync(0xffffffffu, corr_a != 1.f || corr_b != 1.f)) {
 #pragma unroll
-          for (int i = 0; i < HDV / 8; ++i) { o[i][0] *= corr_a; o[i][1] *= corr_a; o[i][2] *= corr_b; o[i][3] *= corr_b; }
+        for (int gr = 0; gr < NG; ++gr) {
+          mx_a[gr] = fmaxf(mx_a[gr], __shfl_xor_sync(0xffffffffu, mx_a[gr], 1));
+          mx_a[gr] = fmaxf(mx_a[gr], __shfl_xor_sync(0xffffffffu, mx_a[gr], 2));
+          mx_b[gr] = fmaxf(mx_b[gr], __shfl_xor_sync(0xffffffffu, mx_b[gr], 1));
+          mx_b[gr] = fmaxf(mx_b[gr], __shfl_xor_sync(0xffffffffu, mx_b[gr], 2));
         }
+        float corr_a[NG], corr_b[NG];
+#pragma unroll
+        for (int gr = 0; gr < NG; ++gr) {
+          const float mn_a = fmaxf(m_a, mx_a[gr]), mn_b = fmaxf(m_b, mx_b[gr]);
+          const float ms_a = mn_a == -INFINITY ? 0.f : mn_a, ms_b = mn_b == -INFINITY ? 0.f : mn_b;
+          corr_a[gr] = ex2(m_a - ms_a); corr_b[gr] = ex2(m_b - ms_b);
+          m_a = mn_a; m_b = mn_b;
+          float ps_a = 0.f, ps_b = 0.f;
+#pragma unroll
+          for (int nt = gr * GT; nt < (gr + 1) * GT; ++nt) {
+            sacc[nt][0] = ex2(sacc[nt][0] - ms_a); sacc[nt][1] = ex2(sacc[nt][1] - ms_a);
+            sacc[nt][2] = ex2(sacc[nt][2] - ms_b); sacc[nt][3] = ex2(sacc[nt][3] - ms_b);
+            ps_a += sacc[nt][0] + sacc[nt][1];
+            ps_b += sacc[nt][2] + sacc[nt][3];
+          }
+          l_a = l_a * corr_a[gr] + ps_a;
+          l_b = l_b * corr_b[gr] + ps_b;
+        }
+        auto rescale_o = [&](float ca, float cb) {
+          if (__any_sync(0xffffffffu, ca != 1.f || cb != 1.f)) {
+#pragma unroll
+            for (int i = 0; i < HDV / 8; ++i) { o[i][0] *= ca; o[i][1] *= ca; o[i][2] *= cb; o[i][3] *= cb; }
+          }
+        };
+        if constexpr (KV8) rescale_o(corr_a[0], corr_b[0]);
         // ---- O += P V ----
         if constexpr (!KV8) {
 #pragma unroll
           for (int hf = 0; hf < WK / 16; ++hf) {
+            rescale_o(corr_a[hf], corr_b[hf]);
             uint32_t pa[4];
             pa[0] = pack2<TM>(sacc[2 * hf][0], sacc[2 * hf][1]);
             pa[1] = pack2<TM>(sacc[2 * hf][2], sacc[2 * hf][3]);
             pa[2] = pack2<TM>(sacc[2 * hf + 1][0], sacc[2 * hf + 1][1]);
             pa[3] = pack2<TM>(sacc[2 * hf + 1][2], sacc[2 * hf + 1][3]);
-            const uint32_t vrow = vb + (uint32_t)(warp * WK + hf * 16 + (mat & 1) * 8 + l7) * 128u;
+            const uint32_t vrow = vb + (uint32_t)(warp * kWarpRows + hf * kGroupRows + (mat & 1) * 8 + l7) * 128u;
 #pragma unroll
             for (int np = 0; np < HDV / 16; ++np) {
               uint32_t bfr[4];
@@ -1101,7 +1125,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
                   } else {
                     float2 ml_[kFewPieces];
                     float4 w4[kFewPieces];
-                    Mx = -INFINITY; Ls = 0.f;
+                    Mx = -INFINITY;
 #pragma unroll
                     for (int j = 0; j < kFewPieces; ++j) {
                       ml_[j] = make_float2(-INFINITY, 0.f);
@@ -1117,9 +1141,15 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
 #pragma unroll
                     for (int j = 0; j < kFewPieces; ++j) {
                       const float e = Mx > -INFINITY ? ex2(ml_[j].x - Mx) : 0.f;
-                      Ls += e * ml_[j].y;
+                      ml_[j].y = __fmul_rn(e, ml_[j].y);
                       v.x += e * w4[j].x; v.y += e * w4[j].y; v.z += e * w4[j].z; v.w += e * w4[j].w;
                     }
+                    // (the order in which the warp above adds them: the same bits whichever form merges)
+#pragma unroll
+                    for (int d = kFewPieces / 2; d > 0; d >>= 1)
+#pragma unroll
+                      for (int j = 0; j < d; ++j) ml_[j].y = __fadd_rn(ml_[j].y, ml_[j + d].y);
+                    Ls = ml_[0].y;
                   }
                   const int Rg = it.mt * 16 + r, token = token_of(Rg), head = it.hk * rep + Rg - token * rep;
                   const int64_t qi = it.q0 + token;
