@@ -60,7 +60,7 @@ enum : int { F_FIRST = 1, F_LAST = 2, F_EMPTY = 4 };
 struct DecArgs {
   KParams kp;
   int total_work;     // num_work * hkv * nsplits
-  int box_rows;       // rows per TMA box = min(page_size, 64); 1 in gather mode
+  int box_rows;       // rows per TMA box: min(page_size, 64), 64 of contiguous K/V; 1 in gather mode
   int kv_total_rows;
   int gather;         // pages of 1, 2 or 4 keys: rows are fetched 16 bytes per lane with cp.async
   // balanced kernels (see LineCut)
@@ -249,41 +249,43 @@ struct Piece {
 };
 static_assert(sizeof(Piece) <= 80, "mailbox slot");
 
-// The cp.async producer's copies of one operand (K or V) of a stage: TNS rows of CPR 16-byte chunks, row r from
-// pool row yr[r / 32] of lane r % 32, written where a 128-byte-swizzled TMA box would have put them (column block
-// ch / 8 of the stage, row r, chunk (ch % 8) ^ (r % 8)).
-template <int CPR, int TNS>
-__device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* src0, uint32_t pitch,
-                                          const int (&yr)[TNS / 32], int lane) {
+// The cp.async producer's copies of one operand (K or V) of a 64-key block of a stage: 64 rows of CPR 16-byte chunks, row r
+// from pool row yr[r / 32] of lane r % 32, written where a 128-byte-swizzled TMA box would have put them (column block
+// ch / 8 of the stage, row r, chunk (ch % 8) ^ (r % 8)).  Rows with a negative number are zeros, nothing is read for them;
+// ALL: there are none.
+template <int CPR, int TNS, bool ALL>
+__device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* src0, uint32_t pitch, int y0, int y1, int lane) {
+  constexpr int G = 8;
+  auto copy = [&](uint32_t dst, const unsigned char* src, int y) {
+    cp_async16(dst, src + (uint64_t)(uint32_t)(ALL ? y : max(y, 0)) * pitch, ALL || y >= 0 ? 16u : 0u);
+  };
   if constexpr (32 % CPR == 0) {
     // RPI rows per instruction; row r = i * RPI + hb, and (r & 7) = ((i * RPI) & 7) ^ hb because the low bits of
     // i * RPI are clear: the swizzle term splits into a lane constant and an immediate
-    constexpr int RPI = 32 / CPR;
+    constexpr int RPI = 32 / CPR, N = TN / RPI;
     const int hb = lane / CPR, ch = lane - hb * CPR;
     const uint32_t dl = dst0 + (uint32_t)(ch >> 3) * (TNS * 128) + (uint32_t)hb * 128u;
     const uint32_t xs = (uint32_t)(((ch & 7) ^ hb) << 4);
     const unsigned char* sl = src0 + ch * 16;
     // the row numbers of eight copies are fetched first: a shuffle followed at once by its copy would cost the
     // shuffle's latency per copy (the statements are not reordered)
-    constexpr int G = 8;
-    static_assert((TNS / RPI) % G == 0, "whole groups");
+    static_assert(N % G == 0, "whole groups");
 #pragma unroll
-    for (int i0 = 0; i0 < TNS / RPI; i0 += G) {
+    for (int i0 = 0; i0 < N; i0 += G) {
       int y[G];
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const int i = i0 + g;
-        y[g] = __shfl_sync(0xffffffffu, yr[(i * RPI) >> 5], ((i * RPI) & 31) + hb);
+        y[g] = __shfl_sync(0xffffffffu, (i * RPI) >> 5 ? y1 : y0, ((i * RPI) & 31) + hb);
       }
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const int i = i0 + g;
-        cp_async16(dl + (uint32_t)(i * RPI) * 128u + (xs ^ (uint32_t)(((i * RPI) & 7) << 4)),
-                   sl + (uint64_t)(uint32_t)y[g] * pitch, 16u);
+        copy(dl + (uint32_t)(i * RPI) * 128u + (xs ^ (uint32_t)(((i * RPI) & 7) << 4)), sl, y[g]);
       }
     }
   } else {
-    constexpr int N = TNS * CPR / 32, G = 8;
+    constexpr int N = TN * CPR / 32;
     static_assert(N % G == 0, "whole groups");
 #pragma unroll
     for (int i0 = 0; i0 < N; i0 += G) {
@@ -291,13 +293,12 @@ __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* sr
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const int i = i0 + g, r = (i * 32 + lane) / CPR;
-        y[g] = __shfl_sync(0xffffffffu, yr[(i * 32 / CPR) >> 5], r & 31);
+        y[g] = __shfl_sync(0xffffffffu, (i * 32 / CPR) >> 5 ? y1 : y0, r & 31);
       }
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const int q = (i0 + g) * 32 + lane, r = q / CPR, ch = q - r * CPR;
-        cp_async16(dst0 + (uint32_t)(ch >> 3) * (TNS * 128) + (uint32_t)r * 128u + (uint32_t)(((ch & 7) ^ (r & 7)) << 4),
-                   src0 + (uint64_t)(uint32_t)y[g] * pitch + ch * 16, 16u);
+        copy(dst0 + (uint32_t)(ch >> 3) * (TNS * 128) + (uint32_t)r * 128u + (uint32_t)(((ch & 7) ^ (r & 7)) << 4), src0 + ch * 16, y[g]);
       }
     }
   }
@@ -580,15 +581,14 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         // warp walks the stage's 16-byte chunks in row order, CPR consecutive lanes on one row, and writes them
         // where the swizzled TMA box would have put them.  The TMA unit retires about one copy per 100 cycles
         // whatever its size; these copies go through the load/store path instead (the reference's route for page
-        // size 1, kernels/fa4_blackwell.cu:8936-8947).  Keys beyond the sequence fetch pool row 0 and are masked
-        // by the consumers.
+        // size 1, kernels/fa4_blackwell.cu:8936-8947).  Keys beyond the sequence or the piece are zeros.
         const int32_t* pt = p.page_table + (int64_t)it.b * p.page_table_stride;
         constexpr int RG = TNS / 32;
         auto lookup = [&](int key0, int (&yr)[RG]) {
 #pragma unroll
           for (int u = 0; u < RG; ++u) {
             const int kk = key0 + 32 * u + lane;
-            yr[u] = 0;
+            yr[u] = -1;
             if (kk < it.seqlen_k && kk < key_end) {
               const int lp = kk >> p.page_shift;
               yr[u] = (pt[lp] << p.page_shift) + (kk - (lp << p.page_shift));
@@ -616,8 +616,19 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
             s_info[4 * s] = w; s_info[4 * s + 1] = key0; s_info[4 * s + 2] = flags;
             mbar_arrive(bar_full + 8 * s);
           }
-          copy_rows<HD * ESZ / 16, TNS>(kdst, kb, kpitch, ycur, lane);
-          copy_rows<HDV * ESZ / 16, TNS>(vdst, vb, vpitch, ycur, lane);
+          const int present = min(key_end, it.seqlen_k) - key0;
+#pragma unroll 1
+          for (int h = 0; h < TNS / TN; ++h) {
+            const int y0 = h ? ycur[RG - 2] : ycur[0], y1 = h ? ycur[RG - 1] : ycur[1];
+            const uint32_t off = (uint32_t)(h * TN) * 128u;
+            if (present >= (h + 1) * TN) {
+              copy_rows<HD * ESZ / 16, TNS, true>(kdst + off, kb, kpitch, y0, y1, lane);
+              copy_rows<HDV * ESZ / 16, TNS, true>(vdst + off, vb, vpitch, y0, y1, lane);
+            } else {
+              copy_rows<HD * ESZ / 16, TNS, false>(kdst + off, kb, kpitch, y0, y1, lane);
+              copy_rows<HDV * ESZ / 16, TNS, false>(vdst + off, vb, vpitch, y0, y1, lane);
+            }
+          }
           cp_async_arrive_noinc(bar_full + 8 * s);
           ++cnt;
         }
@@ -1272,15 +1283,14 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
   a.use_list = kp.work != nullptr;
   a.max_mtiles = pl.max_mtiles;
   a.class_rows = kp.class_rows;
-  constexpr int TNS = SM::TNS;
   const bool paged = kp.page_table != nullptr;
   // (the cp.async producer takes any power-of-two page; measured, pages of 8 and 16 keys are faster as TMA boxes:
   // 0.49 / 0.70 of the HBM peak against 0.48 / 0.60)
   a.gather = paged && (kp.page_size == 1 || kp.page_size == 2 || kp.page_size == 4);
-  // rows per TMA box: a whole stage of contiguous K/V, else a page or 64 rows of a larger page.  (Never more than 64
-  // of a page: a stage starts at a multiple of 64 keys - split and window boundaries are in 64-key blocks - so a
-  // 128-row box of a 128-key stage could start in the middle of a page and run into the physically next one.)
-  a.box_rows = a.gather ? 1 : (!paged ? TNS : (kp.page_size < 64 ? kp.page_size : 64));
+  // rows per TMA box: 64, or a smaller page.  A stage starts at a multiple of 64 keys (split, piece and window boundaries are in
+  // 64-key blocks) and may end after its first 64: a 128-row box could run into the physically next page, and over
+  // contiguous K/V it would fetch up to 127 rows of the next sequence, whose weights are zero but whose values may be anything.
+  a.box_rows = a.gather ? 1 : (paged && kp.page_size < TN ? kp.page_size : TN);
   const uint64_t rows = paged ? (uint64_t)kp.num_pages * (uint64_t)kp.page_size : (uint64_t)kp.total_k;
   a.kv_total_rows = (int)rows;
   const int kvdt = KV8 ? FA_DT_FP8_E4M3 : (std::is_same<T, __half>::value ? FA_DT_FP16 : FA_DT_BF16);
