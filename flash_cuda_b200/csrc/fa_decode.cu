@@ -252,10 +252,9 @@ static_assert(sizeof(Piece) <= 80, "mailbox slot");
 // The cp.async producer's copies of one operand (K or V) of a 64-key block of a stage: 64 rows of CPR 16-byte chunks, row r
 // from pool row yr[r / 32] of lane r % 32, written where a 128-byte-swizzled TMA box would have put them (column block
 // ch / 8 of the stage, row r, chunk (ch % 8) ^ (r % 8)).  Rows with a negative number are zeros, nothing is read for them;
-// ALL: there are none.
+// ALL: there are none.  (A block at a time and not a whole stage: the code is unrolled.)
 template <int CPR, int TNS, bool ALL>
 __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* src0, uint32_t pitch, int y0, int y1, int lane) {
-  constexpr int G = 8;
   auto copy = [&](uint32_t dst, const unsigned char* src, int y) {
     cp_async16(dst, src + (uint64_t)(uint32_t)(ALL ? y : max(y, 0)) * pitch, ALL || y >= 0 ? 16u : 0u);
   };
@@ -269,6 +268,7 @@ __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* sr
     const unsigned char* sl = src0 + ch * 16;
     // the row numbers of eight copies are fetched first: a shuffle followed at once by its copy would cost the
     // shuffle's latency per copy (the statements are not reordered)
+    constexpr int G = 8;
     static_assert(N % G == 0, "whole groups");
 #pragma unroll
     for (int i0 = 0; i0 < N; i0 += G) {
@@ -285,21 +285,26 @@ __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* sr
       }
     }
   } else {
-    constexpr int N = TN * CPR / 32;
-    static_assert(N % G == 0, "whole groups");
+    // CPR / 4 instructions cover 8 rows, whose swizzle repeats every 8: a lane keeps row, column and address of that many
+    // copies.  (The compiler had kept those of all 96 copies of a 128-key stage of 24-chunk rows, in registers and then on the
+    // stack: 16 sequences of 1024 .. 16384 keys of head_dim 192, page size 1, 246 -> 151 us; 24 of 200 .. 4000 120 -> 84.)
+    constexpr int P = CPR / 4;
+    static_assert(CPR % 4 == 0, "whole instructions");
+    uint32_t row[P], dst[P], col[P];
 #pragma unroll
-    for (int i0 = 0; i0 < N; i0 += G) {
-      int y[G];
+    for (int i = 0; i < P; ++i) {
+      const uint32_t q = (uint32_t)(i * 32 + lane), r = q / CPR, ch = q - r * CPR;
+      row[i] = r;
+      dst[i] = dst0 + (ch >> 3) * (TNS * 128) + r * 128u + (((ch & 7) ^ r) << 4);
+      col[i] = ch * 16;
+    }
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const int i = i0 + g, r = (i * 32 + lane) / CPR;
-        y[g] = __shfl_sync(0xffffffffu, (i * 32 / CPR) >> 5 ? y1 : y0, r & 31);
-      }
+    for (int r0 = 0; r0 < TN; r0 += 8) {
+      int y[P];
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const int q = (i0 + g) * 32 + lane, r = q / CPR, ch = q - r * CPR;
-        copy(dst0 + (uint32_t)(ch >> 3) * (TNS * 128) + (uint32_t)r * 128u + (uint32_t)(((ch & 7) ^ (r & 7)) << 4), src0 + ch * 16, y[g]);
-      }
+      for (int i = 0; i < P; ++i) y[i] = __shfl_sync(0xffffffffu, r0 >= 32 ? y1 : y0, (r0 & 31) + row[i]);
+#pragma unroll
+      for (int i = 0; i < P; ++i) copy(dst[i] + (uint32_t)r0 * 128u, src0 + col[i], y[i]);
     }
   }
 }
