@@ -57,8 +57,12 @@ const EnvConfig& env_config() {
 // Scratch for fa_b200_fwd, kept per (device, stream) and reused: its 4 KB header is zeroed once when the
 // buffer is made and every call leaves it zero again (FA_FLAG_WORKSPACE_CLEAN), so a call costs neither an
 // allocation nor a memset.  Calls on one stream run one after the other, which is what sharing a buffer needs.
+// Calls under stream capture have a buffer per capture instead: a graph runs on any stream, as often as and in whatever order
+// with other graphs and calls its owner likes, so it shares no buffer with them (the buffer lies in the memory pool of the
+// capture, which lives as long as the graph), and the clearing of the header is one of its nodes.
 // Requests above kCacheLimit are served by a plain allocation instead.
 constexpr int64_t kCacheLimit = 64ll << 20;
+constexpr size_t kHeaderBytes = 4096;
 struct WsKey {
   int device;
   cudaStream_t stream;
@@ -67,25 +71,38 @@ struct WsKey {
 struct WsKeyHash {
   size_t operator()(const WsKey& k) const { return std::hash<const void*>()(k.stream) * 31u + (size_t)k.device; }
 };
+struct Scratch {
+  at::Tensor own;                   // of calls that run at once
+  at::Tensor captured;              // of the stream's latest capture, whose id follows
+  unsigned long long capture = 0;
+};
 std::mutex g_ws_mu;
-std::unordered_map<WsKey, at::Tensor, WsKeyHash> g_ws_cache;
+std::unordered_map<WsKey, Scratch, WsKeyHash> g_ws_cache;
 
 at::Tensor cached_workspace(const at::Tensor& like, cudaStream_t stream, int64_t bytes, bool* clean) {
+  const auto options = like.options().dtype(at::kByte);
   if (bytes > kCacheLimit) {
     *clean = false;
-    return at::empty({bytes}, like.options().dtype(at::kByte));
+    return at::empty({bytes}, options);
   }
-  const WsKey key{(int)like.get_device(), stream};
-  std::lock_guard<std::mutex> lk(g_ws_mu);
-  auto it = g_ws_cache.find(key);
-  if (it == g_ws_cache.end() || it->second.numel() < bytes) {
-    const int64_t cap = std::max<int64_t>(bytes, 1 << 20);
-    at::Tensor t = at::zeros({cap}, like.options().dtype(at::kByte));   // zero-filled on the current stream
-    if (it == g_ws_cache.end()) it = g_ws_cache.emplace(key, t).first;
-    else it->second = t;
-  }
+  const int64_t cap = std::max<int64_t>(bytes, 1 << 20);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long capture = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &capture));
   *clean = true;
-  return it->second;
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  Scratch& s = g_ws_cache[WsKey{(int)like.get_device(), stream}];
+  if (status == cudaStreamCaptureStatusNone) {
+    if (!s.own.defined() || s.own.numel() < bytes) s.own = at::zeros({cap}, options);   // zero-filled on the current stream
+    return s.own;
+  }
+  if (!s.captured.defined() || s.capture != capture || s.captured.numel() < bytes) {
+    at::Tensor t = at::empty({cap}, options);
+    C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, kHeaderBytes, stream));
+    s.captured = std::move(t);
+    s.capture = capture;
+  }
+  return s.captured;
 }
 void drop_cached_workspace(const at::Tensor& like, cudaStream_t stream) {
   std::lock_guard<std::mutex> lk(g_ws_mu);
