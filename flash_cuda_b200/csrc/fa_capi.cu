@@ -34,7 +34,9 @@ bool prefill_tc_layout_ok(const FaFwdParams* p);
 
 static thread_local char g_last_cuda_error[256] = "";
 
+// (clears the runtime's own record of the error as well: whoever looks there next, after a launch of theirs, would find it)
 static int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();
   snprintf(g_last_cuda_error, sizeof(g_last_cuda_error), "%s: %s", what, cudaGetErrorString(e));
   return FA_ERR_LAUNCH;
 }
@@ -52,7 +54,8 @@ static std::mutex g_dev_mu;
 
 static const DevInfo* device_info() {
   int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (dev < 0 || dev >= 64) return nullptr;
   if (g_dev_init[dev].load(std::memory_order_acquire) == 0) {
     std::lock_guard<std::mutex> lk(g_dev_mu);
     if (g_dev_init[dev].load(std::memory_order_relaxed) == 0) {
