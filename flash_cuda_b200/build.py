@@ -151,11 +151,20 @@ def build_torch_op(force=False, verbose=False, namespace="_vllm_fa3_C") -> str:
     return TORCH_SO
 
 
-def build_direct(force=False, verbose=False) -> str:
+def _direct_source():
     import torch
 
     src, hdr = os.path.join(CSRC, "torch_direct.cpp"), os.path.join(CSRC, "torch_op.h")
-    stamp = _digest([src, hdr], torch.__version__ + sys.version)
+    return src, _digest([src, hdr], torch.__version__ + sys.version)
+
+
+def direct_is_current() -> bool:
+    """Whether DIRECT_SO was built from these sources for this Python and this torch, whose C++ interfaces it uses."""
+    return not _stale(DIRECT_SO, _direct_source()[1])
+
+
+def build_direct(force=False, verbose=False) -> str:
+    src, stamp = _direct_source()
     if not force and not _stale(DIRECT_SO, stamp):
         return DIRECT_SO
     _run(_torch_command(src, DIRECT_SO, ["-l:fa_b200_torch.so", "-ltorch_python"]), verbose)

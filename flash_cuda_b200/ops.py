@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import importlib.util
 import os
+import warnings
 
 import torch
 
@@ -16,6 +17,22 @@ from . import build as _build
 NAMESPACE = "_vllm_fa3_C"
 _loaded = False
 _direct = None      # `fwd` of torch_direct.cpp, where it is built
+
+
+def _load_direct(build_if_missing: bool):
+    """`fwd` of torch_direct.cpp, or None with a warning: the op does all it does, some 4 us later per call."""
+    try:
+        if build_if_missing and not os.path.isfile(_build.DIRECT_SO):
+            _build.build_direct()
+        if not _build.direct_is_current():
+            raise ImportError("it is missing, or was built from other sources, or for another Python or torch")
+        spec = importlib.util.spec_from_file_location("fa_b200_direct", _build.DIRECT_SO)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module.fwd
+    except (ImportError, OSError, RuntimeError) as e:
+        warnings.warn(f"flash_cuda_b200: {_build.DIRECT_SO} is not used ({e}); call_fwd goes through the dispatcher")
+        return None
 
 
 def load(build_if_missing: bool = True):
@@ -27,11 +44,7 @@ def load(build_if_missing: bool = True):
                 raise RuntimeError("flash_cuda_b200 extension is not built; run `python -m flash_cuda_b200.build`")
             _build.build_all()
         torch.ops.load_library(_build.TORCH_SO)
-        if os.path.isfile(_build.DIRECT_SO):
-            spec = importlib.util.spec_from_file_location("fa_b200_direct", _build.DIRECT_SO)
-            module = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(module)
-            _direct = module.fwd
+        _direct = _load_direct(build_if_missing)
         _loaded = True
     ns = getattr(torch.ops, NAMESPACE)
     if getattr(ns, "fwd", None) is None:
