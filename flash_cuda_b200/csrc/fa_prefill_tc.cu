@@ -881,17 +881,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       }
       const float c_mul = has_cap ? p.softcap * kLog2e : sc * kLog2e;
       const float cap_in = has_cap ? sc / p.softcap : 0.f;
-      // capped scores on the FMA pipe: c_mul * tanh(cap_in * s) = s * (cap_a[0] + s^2 (cap_a[1] + ..)), see kTanhC
-      float cap_a[4];
-      if constexpr (CAP && !F8) {
-        const float i2 = cap_in * cap_in;
-        cap_a[0] = kTanhC[0] * c_mul * cap_in;
-        cap_a[1] = kTanhC[1] * c_mul * cap_in * i2;
-        cap_a[2] = kTanhC[2] * c_mul * cap_in * i2 * i2;
-        cap_a[3] = kTanhC[3] * c_mul * cap_in * i2 * i2 * i2;
-      }
-      const float cap_s_max = kTanhMax / cap_in;      // largest |s| the polynomial is good for
-      bool cap_poly = CAP && !F8;     // until a block of this item has shown a score beyond that
+      // whether blocks of capped scores may take the polynomial form: until one of this item has shown a score beyond its range.
+      // (Its coefficients carry scale / cap to the sixth power, which under a cap of 3e-8 is infinite and times a score of 0 a NaN; at
+      // the other end the square of the largest score in range is to stay finite.)
+      bool cap_poly = CAP && !F8 && cap_in >= 0x1p-40f && cap_in <= 0x1p16f;
       const int qp = it.seqlen_k - it.seqlen_q + row;
       int lo = it.leftpad, hi = it.seqlen_k - 1;
       if (p.is_causal) hi = min(hi, qp);
@@ -944,9 +937,18 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
                 am[(j >> 1) & 3] = fmax3_abs(am[(j >> 1) & 3], __uint_as_float(sq[j]), __uint_as_float(sq[j + 1]));
               tmem_ld32(tS + ((c + 2) & 3) * 32, sq);     // (the last two: the first quarters again, for the second pass)
             }
+            // c_mul * tanh(cap_in * s) = s * (cap_a[0] + s^2 (cap_a[1] + ..)), see kTanhC
+            float cap_a[4];
+            {
+              const float i2 = cap_in * cap_in;
+              cap_a[0] = kTanhC[0] * c_mul * cap_in;
+              cap_a[1] = kTanhC[1] * c_mul * cap_in * i2;
+              cap_a[2] = kTanhC[2] * c_mul * cap_in * i2 * i2;
+              cap_a[3] = kTanhC[3] * c_mul * cap_in * i2 * i2 * i2;
+            }
             const float amax = fmaxf(fmaxf(am[0], am[1]), fmaxf(am[2], am[3]));
             const float ub = cap_a[0] * amax;              // c_mul * tanh(cap_in * amax) is no larger
-            cap_poly = __all_sync(0xffffffffu, amax <= cap_s_max && ub - m_used <= kFastShift);
+            cap_poly = __all_sync(0xffffffffu, amax * cap_in <= kTanhMax && ub - m_used <= kFastShift);
             tmem_wait_ld32(sp[0]);
             tmem_wait_ld32(sp[1]);
             if (cap_poly) {
