@@ -430,9 +430,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
   if (warp == WARP_MMA) { tmem_alloc(smem_u32(s_tmem), 512); tmem_relinquish(); }
   if (warp == WARP_TMA && lane == 0) { tma_prefetch_desc(&map_q); tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
   wait_for_predecessors();
-  let_successor_start();
   tc_fence_before_sync();
   __syncthreads();
+  // (behind the barrier, so behind the TMEM allocation: a successor that allocates too can then only wait for this CTA's end)
+  let_successor_start();
   tc_fence_after_sync();
   const uint32_t tmem = *s_tmem;
 
