@@ -1550,6 +1550,13 @@ static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t k
   }
   const int grid = a.num_items < pl.num_sms ? a.num_items : pl.num_sms;
   if (grid <= 0) return 0;
+  // Calls in parts wait for what is in front of them: their CTAs, fewer than the SMs, took whichever SMs the merge of the call
+  // before left first.  One chunk of 512 rows over 24500 keys, back to back under the power cap, 208.0 us (206.9 before
+  // launches overlapped, 205.4 so); in a burst 183.8 / 183.1 / 184.0.  (The merge itself overlaps.)
+  if constexpr (PARTS) {
+    kern<<<grid, NTHREADS, smem, stream>>>(a, mq, mk, mv, mo);
+    return (int)cudaGetLastError();
+  }
   return launch_overlapped(kern, grid, NTHREADS, smem, stream, a, mq, mk, mv, mo);
 }
 
