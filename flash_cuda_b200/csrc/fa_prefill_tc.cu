@@ -55,6 +55,7 @@ constexpr int kCapEmuPairs = FA_CAP_EMU_PAIRS;   // of every four pairs in the f
 // ordinary scores, which lie far below the cap, by more than with tanh.approx.
 __device__ constexpr float kTanhC[4] = {0.99999785f, -0.33314040f, 0.13057856f, -0.04092942f};
 constexpr float kTanhMax = 0.6f;
+constexpr float kTanhAtMax = 0.5370496f;   // tanh(0.6)
 constexpr float kRescaleThreshold = 8.0f;   // log2 units
 constexpr float kFastShift = 14.f;         // log2 units: largest probability of a fast block of capped scores
 constexpr float kFastSumLimit = 16384.f;    // 2^14: row sum of a block above which the fast softmax form is redone
@@ -901,7 +902,96 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       const bool two_term = F8 && (it.hi[t] - it.lo[t] <= kTwoTermBlocks);   // tile-uniform; see the P store below
       float m_used = -INFINITY, l = 0.f;
       float lr = 0.f;   // e4m3 only: sum of the ROUNDED probabilities (normalises O); l stays exact for the LSE
+      // The fast form of a capped block (no masked column, a reference point already taken).  tanh is an odd polynomial
+      // on the FMA pipe, which leaves the special-function unit the exp2 alone (tanh and exp2 on that one unit, half of the
+      // exp2 emulated on the FMA pipe, bounded the capped kernel).  First the largest |s| of the row's block: it says
+      // whether the polynomial's range holds and bounds the probabilities by 2^14, as in the plain kernel's fast
+      // form; a block where either fails sends the rest of the item to the general form.  S comes in quarters, the
+      // next one on its way while one is worked on: the registers of a whole row are those that keep the
+      // exponentials' chains apart.  16 sequences of 128 .. 8192 queries, window 4096, cap 30, sinks: 4860 -> 4230 us
+      // sustained (power-limited), 4440 -> 3680 in a burst; with the whole row held and the range checked afterwards,
+      // 4470 sustained; P held back in registers until a check afterwards, 4160 - 4270 but a redo to code for.
+      // It has a loop of its own: both forms in one loop body cost either of them.  4 sequences of 3000 queries, cap 30 / cap 2
+      // (nearly every block beyond the range): 383 / 383 us without this form, 328 / 417 in one body, 322 / 387 in two.
+      auto may_be_fast = [&](int i) {
+        return __all_sync(0xffffffffu, cap_poly && m_used != -INFINITY && i * TN >= lo_max && i * TN + TN - 1 <= hi_min);
+      };
+      auto capped_block = [&]() {
+        // (one-tile kernels: S buffer and barrier pair alternate block by block, see SDB)
+        const uint32_t sb = SDB ? (scnt & 1) : (uint32_t)t;
+        const uint32_t tS = SDB ? tS0 + ((scnt & 1) ? S1_COL : 0u) : tS0;
+        ok = wait_or_abort(bar_s_full + 8 * sb, SDB ? ((scnt >> 1) & 1) : (scnt & 1), s_abort);
+        ++scnt;
+        if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_SOFTMAX); return; }
+        tc_fence_after_sync();
+        uint32_t sp[2][32];
+        tmem_ld32(tS, sp[0]);
+        tmem_ld32(tS + 32, sp[1]);
+        tmem_wait_ld32(sp[0]);
+        tmem_wait_ld32(sp[1]);
+        float am[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t (&sq)[32] = sp[c & 1];
+          if (c >= 2) tmem_wait_ld32(sq);
+#pragma unroll
+          for (int j = 0; j < 32; j += 2)
+            am[(j >> 1) & 3] = fmax3_abs(am[(j >> 1) & 3], __uint_as_float(sq[j]), __uint_as_float(sq[j + 1]));
+          tmem_ld32(tS + ((c + 2) & 3) * 32, sq);     // (the last two: the first quarters again, for the second pass)
+        }
+        // c_mul * tanh(cap_in * s) = s * (cap_a[0] + s^2 (cap_a[1] + ..)), see kTanhC
+        float cap_a[4];
+        {
+          const float i2 = cap_in * cap_in;
+          cap_a[0] = kTanhC[0] * c_mul * cap_in;
+          cap_a[1] = kTanhC[1] * c_mul * cap_in * i2;
+          cap_a[2] = kTanhC[2] * c_mul * cap_in * i2 * i2;
+          cap_a[3] = kTanhC[3] * c_mul * cap_in * i2 * i2 * i2;
+        }
+        const float amax = fmaxf(fmaxf(am[0], am[1]), fmaxf(am[2], am[3]));
+        const float ub = cap_a[0] * amax;              // c_mul * tanh(cap_in * amax) is no larger
+        cap_poly = __all_sync(0xffffffffu, amax * cap_in <= kTanhMax && ub - m_used <= kFastShift);
+        tmem_wait_ld32(sp[0]);
+        tmem_wait_ld32(sp[1]);
+        if (!cap_poly) { --scnt; return; }      // (the general form waits for the same S again, which is there)
+        const float2 nm2 = make_float2(-m_used, -m_used);
+        const float2 a0 = make_float2(cap_a[0], cap_a[0]), a1 = make_float2(cap_a[1], cap_a[1]);
+        const float2 a2 = make_float2(cap_a[2], cap_a[2]), a3 = make_float2(cap_a[3], cap_a[3]);
+        float2 fs[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t (&sq)[32] = sp[c & 1];
+          if (c >= 2) tmem_wait_ld32(sq);
+          uint32_t pk[16];
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float2 x = make_float2(__uint_as_float(sq[j]), __uint_as_float(sq[j + 1]));
+            const float2 x2 = fmul2(x, x);
+            const float2 y = ffma2(x, ffma2(ffma2(ffma2(a3, x2, a2), x2, a1), x2, a0), nm2);
+            const float2 pp = make_float2(ex2(y.x), ex2(y.y));
+            fs[(j >> 1) & 3] = fadd2(fs[(j >> 1) & 3], pp);
+            pk[j >> 1] = pack2<TO>(pp.x, pp.y);
+          }
+          if (c + 2 < 4) tmem_ld32(tS + (c + 2) * 32, sq);
+          tmem_st16(tS + c * 16, pk);               // (columns of quarters that have been read)
+        }
+        const float2 s01 = fadd2(fs[0], fs[1]), s23 = fadd2(fs[2], fs[3]);
+        const float2 s4 = fadd2(s01, s23);
+        l += s4.x + s4.y;
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_p_full + 8 * sb);
+      };
       for (int i = it.lo[t]; i < it.hi[t]; ++i) {
+        if constexpr (CAP && !F8) {
+          while (i < it.hi[t] && may_be_fast(i)) {
+            capped_block();
+            if (!ok) break;
+            i += cap_poly;
+          }
+          if (!ok || i >= it.hi[t]) break;
+        }
         // (one-tile kernels: S buffer and barrier pair alternate block by block, see SDB)
         const uint32_t sb = SDB ? (scnt & 1) : (uint32_t)t;
         const uint32_t tS = SDB ? tS0 + ((scnt & 1) ? S1_COL : 0u) : tS0;
@@ -911,77 +1001,6 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         tc_fence_after_sync();
         const int n0 = i * TN;
         const bool full = (n0 >= lo_max) && (n0 + TN - 1 <= hi_min);
-        // The fast form of a capped block (no masked column, a reference point already taken).  tanh is an odd polynomial
-        // on the FMA pipe, which leaves the special-function unit the exp2 alone (tanh and exp2 on that one unit, half of the
-        // exp2 emulated on the FMA pipe, bounded the capped kernel).  First the largest |s| of the row's block: it says
-        // whether the polynomial's range holds and bounds the probabilities by 2^14, as in the plain kernel's fast
-        // form; a block where either fails sends the rest of the item to the general form.  S comes in quarters, the
-        // next one on its way while one is worked on: the registers of a whole row are those that keep the
-        // exponentials' chains apart.  16 sequences of 128 .. 8192 queries, window 4096, cap 30, sinks: 4860 -> 4230 us
-        // sustained (power-limited), 4440 -> 3680 in a burst; with the whole row held and the range checked afterwards,
-        // 4470 sustained; P held back in registers until a check afterwards, 4160 - 4270 but a redo to code for.
-        bool cap_done = false;
-        if constexpr (CAP && !F8) {
-          if (__all_sync(0xffffffffu, full && cap_poly && m_used != -INFINITY)) {
-            uint32_t sp[2][32];
-            tmem_ld32(tS, sp[0]);
-            tmem_ld32(tS + 32, sp[1]);
-            tmem_wait_ld32(sp[0]);
-            tmem_wait_ld32(sp[1]);
-            float am[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t (&sq)[32] = sp[c & 1];
-              if (c >= 2) tmem_wait_ld32(sq);
-#pragma unroll
-              for (int j = 0; j < 32; j += 2)
-                am[(j >> 1) & 3] = fmax3_abs(am[(j >> 1) & 3], __uint_as_float(sq[j]), __uint_as_float(sq[j + 1]));
-              tmem_ld32(tS + ((c + 2) & 3) * 32, sq);     // (the last two: the first quarters again, for the second pass)
-            }
-            // c_mul * tanh(cap_in * s) = s * (cap_a[0] + s^2 (cap_a[1] + ..)), see kTanhC
-            float cap_a[4];
-            {
-              const float i2 = cap_in * cap_in;
-              cap_a[0] = kTanhC[0] * c_mul * cap_in;
-              cap_a[1] = kTanhC[1] * c_mul * cap_in * i2;
-              cap_a[2] = kTanhC[2] * c_mul * cap_in * i2 * i2;
-              cap_a[3] = kTanhC[3] * c_mul * cap_in * i2 * i2 * i2;
-            }
-            const float amax = fmaxf(fmaxf(am[0], am[1]), fmaxf(am[2], am[3]));
-            const float ub = cap_a[0] * amax;              // c_mul * tanh(cap_in * amax) is no larger
-            cap_poly = __all_sync(0xffffffffu, amax * cap_in <= kTanhMax && ub - m_used <= kFastShift);
-            tmem_wait_ld32(sp[0]);
-            tmem_wait_ld32(sp[1]);
-            if (cap_poly) {
-              const float2 nm2 = make_float2(-m_used, -m_used);
-              const float2 a0 = make_float2(cap_a[0], cap_a[0]), a1 = make_float2(cap_a[1], cap_a[1]);
-              const float2 a2 = make_float2(cap_a[2], cap_a[2]), a3 = make_float2(cap_a[3], cap_a[3]);
-              float2 fs[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                uint32_t (&sq)[32] = sp[c & 1];
-                if (c >= 2) tmem_wait_ld32(sq);
-                uint32_t pk[16];
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                  const float2 x = make_float2(__uint_as_float(sq[j]), __uint_as_float(sq[j + 1]));
-                  const float2 x2 = fmul2(x, x);
-                  const float2 y = ffma2(x, ffma2(ffma2(ffma2(a3, x2, a2), x2, a1), x2, a0), nm2);
-                  const float2 pp = make_float2(ex2(y.x), ex2(y.y));
-                  fs[(j >> 1) & 3] = fadd2(fs[(j >> 1) & 3], pp);
-                  pk[j >> 1] = pack2<TO>(pp.x, pp.y);
-                }
-                if (c + 2 < 4) tmem_ld32(tS + (c + 2) * 32, sq);
-                tmem_st16(tS + c * 16, pk);               // (columns of quarters that have been read)
-              }
-              const float2 s01 = fadd2(fs[0], fs[1]), s23 = fadd2(fs[2], fs[3]);
-              const float2 s4 = fadd2(s01, s23);
-              l += s4.x + s4.y;
-              cap_done = true;
-            }
-          }
-        }
-        if (!cap_done) {
         uint32_t sreg[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, sreg[c]);
@@ -1065,6 +1084,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         // (normal down to 2^-6), so there the reference sits 2^5 BELOW the maximum: p runs up to 2^5..2^8 <= 448
         // and probabilities down to 2^-11 of the maximum keep their three mantissa bits.  Numerator and
         // denominator carry the same factor; the LSE is taken from the reference point and the sum as they are.
+        // (shows most items that leave the polynomial's range in their first block, before the fast form is tried in vain)
+        if constexpr (CAP && !F8) cap_poly = cap_poly && __all_sync(0xffffffffu, !(y_max > kTanhAtMax * c_mul));
         constexpr float kRefShift = F8 ? 5.f : 0.f;
         if (m_used == -INFINITY) {
           m_used = y_max - kRefShift;                 // first block with a visible key (may stay -inf)
@@ -1192,7 +1213,6 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           l += s4.x + s4.y;
         }
         }   // general form
-        }   // not the capped fast form
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
