@@ -530,7 +530,7 @@ def run_ours(args) -> None:
                                lambda p, r: {"workload": "varlen packed causal prefill bf16, 16 sequences 128..8192, Hq=32 Hkv=8 d=128, window 4096, softcap 30, sink",
                                              "unit": "TFLOP/s", "roofline": _tensor_roofline(r["per_gpu"], peaks),
                                              "kernels_per_step": ["fwd_prefill_tc_kernel"], "l2": "inputs (0.7 GB) larger than L2",
-                                             "note": "one tanh and one exp2 per score share the special-function unit"})
+                                             "note": "blocks without masked keys and with scores below 0.6 of the cap: tanh as a polynomial on the FMA pipe"})
 
     # ---- decode workload: bf16 KV cache and e4m3 KV cache ----
     def decode_leg(kv_dtype):

@@ -32,11 +32,7 @@ namespace dec {
 
 constexpr int TN = 64;                 // keys per scheduler block (metadata unit)
 constexpr int kStageKeys = 128;        // keys of a stage of the ring: 32 per consumer warp, two independent chains (see launch_decode_t)
-// Consumer warps per CTA.  Head dims of 128 and more run one CTA per SM over a 16-bit cache; an e4m3 cache and head_dim 64
-// run TWO (half-size stages): every consumer warp works on every stage, so one CTA's stage rate is bounded by the latency
-// of one warp's ldmatrix -> (widen) -> MMA -> softmax -> MMA chain, and with twice the keys per byte that chain, not HBM, was
-// the limit; a second CTA's chain runs beside it.
-constexpr int ncons_for(int) { return 4; }
+constexpr int kConsumers = 4;          // warps; each takes 32 keys of every stage
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr int kPieces = 4;             // mailbox slots between the producer and the consumers
@@ -73,7 +69,7 @@ struct DecArgs {
 template <int ESZ, int NST, int HD, int HDV>
 struct Smem {
   static constexpr int TNS = kStageKeys;
-  static constexpr int NC = ncons_for(ESZ);         // consumer warps
+  static constexpr int NC = kConsumers;         // consumer warps
   static constexpr int kKBytes = TNS * HD * ESZ, kVBytes = TNS * HDV * ESZ;
   static constexpr int kStage = kKBytes + kVBytes;
   static constexpr int kRing = NST * kStage;
@@ -225,7 +221,7 @@ __device__ __forceinline__ int line_len(const WorkItem& it) { return it.valid ? 
 // had read its own a second time, in code that every CTA ran cold.
 __device__ __forceinline__ void keep_entry(int* rec, const WorkItem& it) {
   int4* r4 = reinterpret_cast<int4*>(rec);
-  r4[0] = make_int4(it.b | it.mt << 16, it.q0, it.seqlen_q, it.seqlen_k);      // (b, mt < 160)
+  r4[0] = make_int4(it.b | it.mt << 16, it.q0, it.seqlen_q, it.seqlen_k);      // (b < kBalancedEntriesMax, mt < 4)
   r4[1] = make_int4(it.k0, it.leftpad, it.lo, it.hi);
 }
 __device__ __forceinline__ WorkItem kept_entry(const int* rec) {
@@ -311,7 +307,7 @@ __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* sr
 
 // T = MMA element type (bf16 / fp16); KV8 = the cache holds e4m3 bytes.
 template <typename T, bool KV8, int NST, int HD, int HDV, int CPS, bool BAL>
-__global__ void __launch_bounds__((ncons_for(KV8 ? 1 : 2) + 1) * 32, CPS)
+__global__ void __launch_bounds__((kConsumers + 1) * 32, CPS)
 fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v) {
   constexpr int ESZ = KV8 ? 1 : 2;
   static_assert(!KV8 || (HD == 128 && HDV == 128), "an e4m3 cache row must fill one 128-byte swizzle row");
@@ -1289,8 +1285,9 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
   a.max_mtiles = pl.max_mtiles;
   a.class_rows = kp.class_rows;
   const bool paged = kp.page_table != nullptr;
-  // (the cp.async producer takes any power-of-two page; measured, pages of 8 and 16 keys are faster as TMA boxes:
-  // 0.49 / 0.70 of the HBM peak against 0.48 / 0.60)
+  // (The cp.async producer takes any power-of-two page.  16 sequences of 1024 .. 16384 keys, TMA boxes / cp.async, us in a graph:
+  // pages of 16 keys 48 / 61 at head_dim 64, 90 / 122 at 128, 110 / 148 at 192.  Pages of 8: 55 / 63, 143 / 123, 175 / 149; the line
+  // was drawn with 64-key stages, where boxes were no slower there at 128 either.)
   a.gather = paged && (kp.page_size == 1 || kp.page_size == 2 || kp.page_size == 4);
   // rows per TMA box: 64, or a smaller page.  A stage starts at a multiple of 64 keys (split, piece and window boundaries are in
   // 64-key blocks) and may end after its first 64: a 128-row box could run into the physically next page, and over
@@ -1343,14 +1340,18 @@ bool decode_supported(const PlanInput& in) {
                      (in.kv_dtype != FA_DT_FP8_E4M3 && ((in.hd == 64 && in.hdv == 64) || (in.hd == 192 && in.hdv == 128)));
   if (!hd_ok) return false;
   const int ps = in.page_size;
-  // pages of 8, 16 or 32 keys divide a 64-row stage into whole 1024-byte swizzle atoms; multiples of 64 are whole
-  // stages; pages of 1, 2 or 4 keys are fetched row by row with cp.async
+  // boxes of min(page, 64) rows tile the two 64-key blocks of a stage in whole 1024-byte swizzle atoms, and work starts at
+  // multiples of 64 keys: pages of 8, 16, 32 or a multiple of 64; pages of 1, 2 or 4 keys are fetched row by row with cp.async
   if (!(ps == 0 || ps == 1 || ps == 2 || ps == 4 || ps == 8 || ps == 16 || ps == 32 || ps % 64 == 0)) return false;
   return in.hkv > 0 && in.hq % in.hkv == 0 && in.tc_layout_ok;
 }
 
 template <typename T, bool BAL>
 static int launch_decode_t(const KParams& kp, const Plan& pl, int slots, cudaStream_t stream) {
+  // CTAs per SM: one over a 16-bit cache of head_dim 128 and more; two over an e4m3 cache and at head_dim 64 (half-size
+  // stages): every consumer warp works on every stage, so one CTA's stage rate is bounded by the latency of one warp's ldmatrix
+  // -> (widen) -> MMA -> softmax -> MMA chain, and with twice the keys per byte that chain, not HBM, was the limit; a second
+  // CTA's chain runs beside it.
   // Two stages of 128 keys everywhere: 32 keys = two independent 16-key chains per consumer warp, which hide each other's
   // fixed latencies, half the stage hand-offs per byte, and for small pages enough copies per stage for every lane of the
   // producer.  e4m3 cache: 0.80 -> 0.92 of the HBM peak against 64-key stages (of which more fit).  16-bit caches, against
