@@ -1523,6 +1523,23 @@ static bool producer_is_wide(const KParams& kp) {
   return kp.page_size <= 32 || (KST == VST && kp.page_size <= 64);
 }
 
+// What a call takes with all SMs busy, from the lengths that the host knows: 1.8 us per 128 keys of 256 rows x 256 columns.
+static double expected_us(const KParams& kp, int num_sms) {
+  const double rows = (double)kp.total_q / kp.batch;
+  double keys = kp.max_seqlen_k;
+  if (!kp.page_table && (double)kp.total_k / kp.batch < keys) keys = (double)kp.total_k / kp.batch;
+  if (kp.is_causal) keys -= 0.5 * (rows < keys ? rows : keys);
+  if (kp.window_left >= 0 && kp.window_left + 256.0 < keys) keys = kp.window_left + 256.0;
+  return 1.8 * (kp.total_q / 256.0) * kp.hq * (keys / 128.0) * ((kp.hd + kp.hdv) / 256.0) / num_sms;
+}
+// Calls expected to take longer wait for what is in front of them instead of starting beside it: that saves a gap of some 2 us,
+// but the CTAs then start on whichever SMs the kernel in front leaves first, and that costs longer calls more.  Calls back to
+// back, overlapped / plain, us: 13.5 / 15.9 (2 x 8 heads x 512), 56.3 / 57.2 (3 x 714 rows over 1379 keys), 78.7 / 80.7 (10 x 128 ..
+// 699 rows, 64 heads), 73.0 / 72.2 (e4m3, 2 x 3227, 8 heads); 208.0 / 205.4 (512 rows over 24500 keys, in parts), 545.5 / 543.2 (4 x
+// 4096 x 32 heads), 723 / 725 (2048 rows over 32768 keys, head_dim 192), 1299 / 1282 (3 x 393 rows over 65303 keys), 4142 / 4091
+// (varlen, window, cap).  The first four are expected to take 2, 26, 15 and 31; the others 147 and more.
+constexpr double kOverlapUs = 100.0;
+
 template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD, bool PARTS>
 static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t kv_rows, cudaStream_t stream) {
   using SM = Smem<Elem<T>::kSize, HD, HDV, KST, VST, NTL>;
@@ -1570,10 +1587,7 @@ static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t k
   }
   const int grid = a.num_items < pl.num_sms ? a.num_items : pl.num_sms;
   if (grid <= 0) return 0;
-  // Calls in parts wait for what is in front of them: their CTAs, fewer than the SMs, took whichever SMs the merge of the call
-  // before left first.  One chunk of 512 rows over 24500 keys, back to back under the power cap, 208.0 us (206.9 before
-  // launches overlapped, 205.4 so); in a burst 183.8 / 183.1 / 184.0.  (The merge itself overlaps.)
-  if constexpr (PARTS) {
+  if (expected_us(kp, pl.num_sms) > kOverlapUs) {
     kern<<<grid, NTHREADS, smem, stream>>>(a, mq, mk, mv, mo);
     return (int)cudaGetLastError();
   }
