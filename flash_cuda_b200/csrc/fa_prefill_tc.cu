@@ -439,9 +439,10 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
   const uint32_t tmem = *s_tmem;
 
   // register tiers: the launch gives every thread 168; the MMA/TMA warpgroup hands most of its share to the
-  // two softmax warpgroups, which hold a full 128-wide fp32 score row per thread
+  // two softmax warpgroups, which hold a full 128-wide fp32 score row per thread.  (With 200 + 200 + 104 the softmax loop spilled
+  // 24 bytes at head_dim 128 and 12 at 64; causal 4 x 4096 x 32 heads 549 -> 539 us without that, in a burst 474 -> 467.  2 x 208 + 88 = 3 x 168.)
   if (warp >= 8) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
   if (warp == WARP_TMA) {
     // =========================================== TMA producer ===========================================
     // Two forms, chosen by the host (template argument PROD).  Wide: the whole warp runs the control flow; lane 0 (the
@@ -701,20 +702,20 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       }
     };
     auto issue_qk = [&](int t, uint32_t kslot) { issue_qk_to(t, kslot, t * TN, bar_s_full + 8 * t); };
-    // two_term (e4m3 only): P was written as P_hi (columns 0..31 of S_t) + P_lo (columns 32..63), see the softmax role
+    // two_term (e4m3 only): P was written as P_hi + P_lo, 8 columns of either per 32 keys, see the softmax role
     auto issue_pv = [&](int t, uint32_t vslot, bool first, bool two_term, uint32_t pcol = 0xffffffffu) {
       if (pcol == 0xffffffffu) pcol = t * TN;      // P overlays the S it came from
       const uint64_t vd = vd0 + (uint64_t)(vslot * (SM::kVStage >> 4));
       if (leader) {
 #pragma unroll
         for (int ks = 0; ks < TN / KEL; ++ks)   // KEL keys per step = KEL rows of 128 bytes; P: 8 TMEM columns per step
-          umma_ts<F8>(tmem_u + O_BASE + t * O_STRIDE, tmem_u + pcol + ks * 8, vd + (uint64_t)(ks * ((KEL * 128) >> 4)), idesc_pv,
-                      (!first || ks > 0) ? 1u : 0u);
+          umma_ts<F8>(tmem_u + O_BASE + t * O_STRIDE, tmem_u + pcol + ks * (F8 && two_term ? 16 : 8),
+                      vd + (uint64_t)(ks * ((KEL * 128) >> 4)), idesc_pv, (!first || ks > 0) ? 1u : 0u);
         if constexpr (F8) {
           if (two_term) {
 #pragma unroll
             for (int ks = 0; ks < TN / KEL; ++ks)
-              umma_ts<F8>(tmem_u + O_BASE + t * O_STRIDE, tmem_u + pcol + 32 + ks * 8, vd + (uint64_t)(ks * ((KEL * 128) >> 4)),
+              umma_ts<F8>(tmem_u + O_BASE + t * O_STRIDE, tmem_u + pcol + 8 + ks * 16, vd + (uint64_t)(ks * ((KEL * 128) >> 4)),
                           idesc_pv, 1u);
           }
         }
@@ -841,8 +842,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
     // 256-column O row, and wait at the final barrier
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
   } else {
-    if constexpr (NTL == 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-    else asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    if constexpr (NTL == 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 240;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     // ========================================= softmax + epilogue =======================================
     const int t = warp >> 2;                       // tile of this warpgroup
     const int r = (warp & 3) * 32 + lane;          // row within the tile == TMEM lane
@@ -873,9 +874,9 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       const int row0 = it.pair * (NTL * TM) + t * TM;
       if (row0 >= it.seqlen_q) continue;           // this tile owns no row
       const int row = row0 + r;
-      const int hk = (PARTS ? it.h & kHeadMask : it.h) / p.rep;
       float sc = p.scale, vds = 1.f;
-      {
+      if (p.q_descale || p.k_descale || p.v_descale) {
+        const int hk = (PARTS ? it.h & kHeadMask : it.h) / p.rep;
         const int di = it.b * p.descale_batch_stride + hk * p.descale_head_stride;
         if (p.q_descale) sc *= p.q_descale[di];
         if (p.k_descale) sc *= p.k_descale[di];
@@ -983,7 +984,111 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_p_full + 8 * sb);
       };
-      for (int i = it.lo[t]; i < it.hi[t]; ++i) {
+      // The e4m3 form for a tile whose rows see at most kTwoTermBlocks key blocks in all (256 keys: the first rows of a causal
+      // sequence, short sequences): little averaging over keys hides the 3-bit mantissa of P there, so P is written as two
+      // e4m3 terms, P_hi + P_lo with P_lo = round(P - P_hi), and the MMA warp runs PV over both.  A loop of its own, over
+      // quarters of the row, rolled, with S read from TMEM twice: as a branch of the common block, on the row in registers, it
+      // made that block spill (240 bytes) and its code twice as long.  All e4m3, us: causal 2 x 4096 x 32 heads 256 -> 227, 2 x 2048
+      // not causal 134 -> 122, causal 3 x 700 33.4 -> 27.5; rolled but inside the common block 233, 127 and 28.2.
+      auto two_term_block = [&](int i) {
+        const uint32_t sb = (uint32_t)t, tS = tS0;
+        ok = wait_or_abort(bar_s_full + 8 * sb, scnt & 1, s_abort);
+        ++scnt;
+        if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_SOFTMAX); return; }
+        tc_fence_after_sync();
+        const int n0 = i * TN;
+        float mx = -INFINITY;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t sq[32];
+          tmem_ld32(tS + c * 32, sq);
+          tmem_wait_ld32(sq);
+          const uint32_t seen = bits_between(lo - n0 - c * 32, hi - n0 - c * 32);
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (seen & (1u << j)) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(sq[j]));
+          mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+        }
+        const float y_max = (has_cap && mx != -INFINITY ? tanh_fast(mx * cap_in) : mx) * c_mul;
+        float corr = 1.f;
+        bool rescale = false;
+        constexpr float kRefShift = 5.f;
+        if (m_used == -INFINITY) {
+          m_used = y_max - kRefShift;
+        } else if (y_max > m_used + kRescaleThreshold) {
+          corr = ex2(m_used - (y_max - kRefShift));
+          m_used = y_max - kRefShift;
+          l *= corr;
+          lr *= corr;
+          rescale = true;
+        }
+        if (__any_sync(0xffffffffu, rescale)) {
+#pragma unroll 1
+          for (int c = 0; c < HDV / 32; ++c) {
+            uint32_t o[32];
+            tmem_ld32(tO + c * 32, o);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+            tmem_st32(tO + c * 32, o);
+          }
+        }
+        const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+        const float2 c2 = make_float2(c_mul, c_mul), nm2 = make_float2(neg_m, neg_m);
+        float2 psum[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t sq[32], pk[8], pl[8];
+          tmem_ld32(tS + c * 32, sq);
+          tmem_wait_ld32(sq);
+          const uint32_t seen = bits_between(lo - n0 - c * 32, hi - n0 - c * 32);
+          float lsum = 0.f;
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            float x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              x[u] = __uint_as_float(sq[j + u]);
+              if (has_cap) x[u] = tanh_fast(x[u] * cap_in);
+              if (!(seen >> (j + u) & 1u)) x[u] = -INFINITY;
+            }
+            const float2 y0 = ffma2(make_float2(x[0], x[1]), c2, nm2), y1 = ffma2(make_float2(x[2], x[3]), c2, nm2);
+            const float2 p0 = make_float2(ex2(y0.x), ex2(y0.y)), p1 = make_float2(ex2(y1.x), ex2(y1.y));
+            psum[(j >> 2) & 3] = fadd2(psum[(j >> 2) & 3], fadd2(p0, p1));
+            const uint32_t q4 = pack4_e4m3(p0.x, p0.y, p1.x, p1.y);
+            pk[j >> 2] = q4;
+            const uint32_t h0 = e4m3x2_to_f16x2((uint16_t)(q4 & 0xffffu)), h1 = e4m3x2_to_f16x2((uint16_t)(q4 >> 16));
+            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&h0));
+            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
+            const uint32_t r4 = pack4_e4m3(p0.x - f0.x, p0.y - f0.y, p1.x - f1.x, p1.y - f1.y);
+            pl[j >> 2] = r4;
+            const uint32_t g0 = e4m3x2_to_f16x2((uint16_t)(r4 & 0xffffu)), g1 = e4m3x2_to_f16x2((uint16_t)(r4 >> 16));
+            const float2 e0 = __half22float2(*reinterpret_cast<const __half2*>(&g0));
+            const float2 e1 = __half22float2(*reinterpret_cast<const __half2*>(&g1));
+            lsum += ((f0.x + e0.x) + (f0.y + e0.y)) + ((f1.x + e1.x) + (f1.y + e1.y));
+          }
+          tmem_st8(tS + c * 16, pk);           // (columns of quarters that have been read)
+          tmem_st8(tS + c * 16 + 8, pl);
+          lr += lsum;
+        }
+        const float2 s01 = fadd2(psum[0], psum[1]), s23 = fadd2(psum[2], psum[3]);
+        const float2 s4 = fadd2(s01, s23);
+        l += s4.x + s4.y;
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_p_full + 8 * sb);
+      };
+      int i0 = it.lo[t];
+      if constexpr (F8) {
+        if (two_term) {
+#pragma unroll 1
+          for (; i0 < it.hi[t] && ok; ++i0) two_term_block(i0);
+          if (!ok) break;
+        }
+      }
+      for (int i = i0; i < it.hi[t]; ++i) {
         if constexpr (CAP && !F8) {
           while (i < it.hi[t] && may_be_fast(i)) {
             capped_block();
@@ -1053,14 +1158,15 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
               sreg[c][j] = __float_as_uint(tanh_fast(__uint_as_float(sreg[c][j]) * cap_in));
         }
         if (!full) {
-          const int rlo = lo - n0, rhi = hi - n0;
+          // (a word of visible columns per quarter, a test of one bit per column: two instructions where two comparisons
+          // against the row's limits were three.  Causal, us: 4 x 4096 x 32 heads 539 -> 529, 8 x 512 40 -> 36.)
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 4; ++c) {
+            const uint32_t seen = bits_between(lo - n0 - c * 32, hi - n0 - c * 32);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int col = c * 32 + j;
-              if (col < rlo || col > rhi) sreg[c][j] = 0xff800000u;   // -inf
-            }
+            for (int j = 0; j < 32; ++j)
+              if (!(seen & (1u << j))) sreg[c][j] = 0xff800000u;   // -inf
+          }
         }
         {
           // eight independent chains instead of one 128-deep dependency chain
@@ -1150,7 +1256,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
               tmem_st16(tS + c * 16, pk);
             }
           }
-        } else if (!two_term) {
+        } else {
           // four e4m3 probabilities per TMEM column.  The row sum is taken over the ROUNDED probabilities, so that
           // numerator (P V on the tensor cores) and denominator describe the same weights.
 #pragma unroll
@@ -1172,39 +1278,6 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
             tmem_st8(tS + c * 8, pk);
             const float2 f01 = __half22float2(__hadd2(hs[0], hs[1])), f23 = __half22float2(__hadd2(hs[2], hs[3]));
             lr += (f01.x + f23.x) + (f01.y + f23.y);
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            // A tile whose rows see at most kTwoTermBlocks key blocks in all (256 keys: the first rows of a causal
-            // sequence, short sequences) has little averaging over keys to hide the 3-bit mantissa of P: there P
-            // is written as two e4m3 terms, P_hi + P_lo with P_lo = round(P - P_hi), and the MMA warp runs PV
-            // over both.  Kept apart from the common path above, whose loop body must stay small: the softmax
-            // warps run out of the instruction cache (with this code inside the common loop the e4m3 kernel fell
-            // from 1160 to 767 TFLOP/s).
-            uint32_t pk[8], pl[8];
-            float lsum = 0.f;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float2 y0 = ffma2(make_float2(__uint_as_float(sreg[c][j]), __uint_as_float(sreg[c][j + 1])), c2, nm2);
-              const float2 y1 = ffma2(make_float2(__uint_as_float(sreg[c][j + 2]), __uint_as_float(sreg[c][j + 3])), c2, nm2);
-              const float2 p0 = make_float2(ex2(y0.x), ex2(y0.y)), p1 = make_float2(ex2(y1.x), ex2(y1.y));
-              psum[(j >> 2) & 3] = fadd2(psum[(j >> 2) & 3], fadd2(p0, p1));
-              const uint32_t q4 = pack4_e4m3(p0.x, p0.y, p1.x, p1.y);
-              pk[j >> 2] = q4;
-              const uint32_t h0 = e4m3x2_to_f16x2((uint16_t)(q4 & 0xffffu)), h1 = e4m3x2_to_f16x2((uint16_t)(q4 >> 16));
-              const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&h0));
-              const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
-              const uint32_t r4 = pack4_e4m3(p0.x - f0.x, p0.y - f0.y, p1.x - f1.x, p1.y - f1.y);
-              pl[j >> 2] = r4;
-              const uint32_t g0 = e4m3x2_to_f16x2((uint16_t)(r4 & 0xffffu)), g1 = e4m3x2_to_f16x2((uint16_t)(r4 >> 16));
-              const float2 e0 = __half22float2(*reinterpret_cast<const __half2*>(&g0));
-              const float2 e1 = __half22float2(*reinterpret_cast<const __half2*>(&g1));
-              lsum += ((f0.x + e0.x) + (f0.y + e0.y)) + ((f1.x + e1.x) + (f1.y + e1.y));
-            }
-            tmem_st8(tS + c * 8, pk);
-            tmem_st8(tS + 32 + c * 8, pl);
-            lr += lsum;
           }
         }
         {

@@ -401,6 +401,13 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
   return d;
 }
+// bits lo .. hi of a word (either may lie outside of it): a shift by 32 or more gives zero in PTX
+__device__ __forceinline__ uint32_t bits_between(int lo, int hi) {
+  uint32_t from_lo, above_hi;
+  asm("shl.b32 %0, 0xffffffff, %1;" : "=r"(from_lo) : "r"(max(lo, 0)));
+  asm("shl.b32 %0, 0xffffffff, %1;" : "=r"(above_hi) : "r"(max(hi + 1, 0)));
+  return from_lo & ~above_hi;
+}
 // three-input maximum (one instruction on sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float r;
