@@ -191,6 +191,32 @@ static Plan decode_part_plan(const PlanInput& in, const Plan& pl) {
   return d;
 }
 
+// More than 16 packed rows: the decode kernel may take 32 at a time, which reads the keys half as often.  It has twice the rows to fetch
+// and to merge per piece, one row tile after the other, so it wants long passes: by the key blocks (of 64, from the longest sequence) of a
+// CTA's share when tiles go one at a time.  Time one at a time / two at a time, in a graph, pages of 64 keys (of 16 in brackets, where the TMA
+// copies count as well and half of them go):
+//   head_dim 128 and 192, 24 or 32 rows, 5 blocks 0.71 - 0.77 (0.74 - 0.82), 27 1.02 - 1.11 (1.25 - 1.34), 34 0.96 - 1.03 (1.12 - 1.25), 122 1.25 (1.4),
+//   400 and more 1.3 - 1.4 (1.6 - 1.7); 64 rows, 10 blocks 0.90 - 0.96 (1.09), 54 and 68 1.1 - 1.2 (1.3 - 1.5); 48 rows, whose last pass is half
+//   empty, 41 - 51 0.91 - 1.04 (1.08 - 1.2), 183 1.02 - 1.05 (1.3), 560 1.2 (1.35);
+//   head_dim 64, 24 or 32 rows, 17 blocks 0.62 - 0.68 (0.72), 61 0.98 (1.06), 203 0.97 - 1.0 (1.1), 340 1.28 (1.4); 64 rows, 122 0.83 (0.94), 406 1.2
+//   (1.4); 48 rows, 304 0.94 (1.1), 510 0.99 (1.13).
+// Not with a caller's work list, whose entries are tiles of 16 rows, and not over an e4m3 cache (two CTAs of four warps per SM as
+// well, and no registers for a second tile beside the widening).
+static void wide_decode_rows(Plan* pl, const FaFwdParams* p) {
+  if (pl->err != FA_OK || pl->route != FA_ROUTE_DECODE || p->scheduler_metadata != nullptr || p->kv_dtype == FA_DT_FP8_E4M3) return;
+  const int tiles = pl->max_mtiles;
+  if (tiles < 2) return;
+  const bool small = p->page_table && p->page_size <= 16;
+  const long long share = (long long)p->batch * tiles * p->hkv * ceil_div(p->max_seqlen_k, 64) / decode_line_ctas(p->hd, p->kv_dtype, pl->num_sms);
+  long long least;
+  if (p->hd > 64) least = tiles == 3 && !small ? 128 : 24;
+  else if (small) least = tiles == 2 ? 60 : 160;
+  else least = tiles == 3 ? 1ll << 40 : 256;
+  if (share < least) return;
+  pl->tile_m = 32;
+  pl->max_mtiles = (tiles + 1) / 2;
+}
+
 // The decode kernel cuts the batch's key blocks by itself (LineCut in fa_decode.cu), or runs work items, longest first,
 // with a split count from here.  Measured side by side over batches of 1 .. 100 x 300 .. 20000 keys, equal and ragged, 8 / 1
 // .. 64 / 8 heads (time as items / time balanced, per class of items per CTA):
@@ -224,7 +250,7 @@ struct PartPlan { int rows; size_t ml_bytes, o_bytes; };
 static PartPlan part_plan(const FaFwdParams* p, const Plan& decode_plan) {
   PartPlan pp;
   const long long rows = (long long)p->max_seqlen_q * decode_plan.rows_per_token;
-  pp.rows = rows < 16 ? (int)rows : 16;
+  pp.rows = rows < decode_plan.tile_m ? (int)rows : decode_plan.tile_m;
   const size_t n = (size_t)decode_line_ctas(p->hd, p->kv_dtype, decode_plan.num_sms) * 2 * pp.rows;
   pp.ml_bytes = align_up(n * 8, 256);
   pp.o_bytes = align_up(n * p->hdv * 4, 256);
@@ -526,6 +552,7 @@ size_t fa_b200_fwd_workspace_bytes(const FaFwdParams* p_in) {
   const DevInfo* di = device_info();
   Plan pl = make_plan(plan_input(p, di && di->sms > 0 ? di->sms : 148));
   if (pl.err != FA_OK) return 256;
+  wide_decode_rows(&pl, p);
   return ws_layout(p, pl).total;
 }
 
@@ -557,6 +584,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   PlanInput in = plan_input(p, di->sms);
   Plan pl = make_plan(in);
   if (pl.err != FA_OK) return pl.err;
+  wide_decode_rows(&pl, p);
   WsLayout w = ws_layout(p, pl);
   if (!workspace || ((uintptr_t)workspace % 256)) return FA_ERR_WORKSPACE;
   if (workspace_bytes < w.total)
@@ -765,6 +793,7 @@ int fa_b200_decode_fwd_static(const FaFwdParams* p, fa_stream_t stream) {
   Plan pl = make_plan(plan_input(p, di->sms));
   if (pl.err != FA_OK) return pl.err;
   if (pl.route != FA_ROUTE_DECODE) return FA_ERR_UNSUPPORTED;
+  wide_decode_rows(&pl, p);
   if (ws_layout(p, pl).total > kStaticBytes) return FA_ERR_STATIC_LIMIT;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FA_ERR_NO_DEVICE;

@@ -2,7 +2,7 @@
 //
 // Work item = (batch entry and 16-row tile, kv head, split).  The `rep * q_len` query rows that share one KV head
 // are packed into 16-row MMA tiles: with up to 16 rows every K/V byte is read from HBM once per kv head, with
-// more rows (up to 64) once per tile.  Persistent CTAs
+// more rows (up to 64) once per tile, or once per two tiles (MT = 2).  Persistent CTAs
 // (one per SM) pull work items longest-first from the scheduler metadata through an atomic counter.
 //
 //   warp 4      producer: resolves page-table entries (32 at a time, one coalesced load) and streams whole
@@ -66,10 +66,11 @@ struct DecArgs {
   int class_rows;     // > 0: only sequences with at most this many packed query rows (the short ones of a mixed batch)
 };
 
-template <int ESZ, int NST, int HD, int HDV>
+template <int ESZ, int NST, int HD, int HDV, int MT>
 struct Smem {
   static constexpr int TNS = kStageKeys;
-  static constexpr int NC = kConsumers;         // consumer warps
+  static constexpr int TW = MT > 1 && HD >= 128 ? MT : 1;     // groups of consumer warps, a row tile each (see wide_decode_rows)
+  static constexpr int NC = kConsumers * TW;                  // consumer warps
   static constexpr int kKBytes = TNS * HD * ESZ, kVBytes = TNS * HDV * ESZ;
   static constexpr int kStage = kKBytes + kVBytes;
   static constexpr int kRing = NST * kStage;
@@ -78,10 +79,13 @@ struct Smem {
   static constexpr int kMiscOff = kBarOff + 2 * NST * 8;       // abort flags
   static constexpr int kScrOff = (kMiscOff + 16 + 15) / 16 * 16;
   static constexpr int kLdO = HDV + 4;
-  static constexpr int kScrBytes = NC * 16 * kLdO * 4 + 2 * NC * 16 * 4;
-  static_assert(NC * 16 * kLdO >= 2 * 16 * kMaxMerge, "the merge's pairs lie in the merge area");
+  static constexpr int kScrBytes = kConsumers * 16 * kLdO * 4 + 2 * kConsumers * 16 * 4;
+  static_assert(kConsumers * 16 * kLdO >= 2 * 16 * kMaxMerge, "the merge's pairs lie in the merge area");
   // balanced kernels: piece mailbox with its barriers, then the line's prefix sums
-  static constexpr int kPieceOff = kScrOff + kScrBytes;
+  // two row tiles: the queries as MMA operands, 16 bytes per lane, tile and 16 columns (in registers they would not fit)
+  static constexpr bool kQShared = MT > 1;
+  static constexpr int kQOff = kScrOff + kScrBytes;
+  static constexpr int kPieceOff = kQOff + (kQShared ? MT * (HD / 16) * 512 : 0);
   static constexpr int kPieceBarOff = kPieceOff + kPieces * 80;   // full[kPieces], empty[kPieces], flag
   static constexpr int kPrefOff = kPieceBarOff + 2 * kPieces * 8 + 16;
   static constexpr int kBorderOff = kPrefOff + (kBalancedEntriesMax + 4) * 4;
@@ -177,6 +181,7 @@ __device__ __forceinline__ int entry_of(const int* pref, int E, int groups, int 
 }
 
 // Entry e of the line: a (batch, row tile), all head groups; `hk` and `split` are left at 0.
+template <int MT>
 __device__ __forceinline__ WorkItem line_entry(const DecArgs& a, int e) {
   const KParams& p = a.kp;
   WorkItem it;
@@ -202,12 +207,12 @@ __device__ __forceinline__ WorkItem line_entry(const DecArgs& a, int e) {
   it.seqlen_k = p.seqused_k ? p.seqused_k[it.b] : (p.cu_k[it.b + 1] - p.cu_k[it.b]);
   it.leftpad = p.leftpad_k ? p.leftpad_k[it.b] : 0;
   const int rows = it.seqlen_q * p.rep;
-  if (it.mt * 16 >= rows || (a.class_rows > 0 && rows > a.class_rows)) return it;
+  if (it.mt * (16 * MT) >= rows || (a.class_rows > 0 && rows > a.class_rows)) return it;
   if (a.use_list) {
     if (n_lo < 0 || n_hi < n_lo || (int64_t)n_hi * TN > (int64_t)it.seqlen_k + TN - 1) { it.bad = true; return it; }
   } else {
-    const int off = it.seqlen_k - it.seqlen_q, row0 = it.mt * 16;
-    nblock_range(it.seqlen_k, it.leftpad, off + row0 / p.rep, off + min(it.seqlen_q - 1, (row0 + 15) / p.rep), p.is_causal,
+    const int off = it.seqlen_k - it.seqlen_q, row0 = it.mt * (16 * MT);
+    nblock_range(it.seqlen_k, it.leftpad, off + row0 / p.rep, off + min(it.seqlen_q - 1, (row0 + 16 * MT - 1) / p.rep), p.is_causal,
                  p.window_left, p.window_right, TN, &n_lo, &n_hi);
   }
   it.valid = true;
@@ -306,13 +311,19 @@ __device__ __forceinline__ void copy_rows(uint32_t dst0, const unsigned char* sr
 }
 
 // T = MMA element type (bf16 / fp16); KV8 = the cache holds e4m3 bytes.
-template <typename T, bool KV8, int NST, int HD, int HDV, int CPS, bool BAL>
-__global__ void __launch_bounds__((kConsumers + 1) * 32, CPS)
+// MT = row tiles that one pass over the keys serves.  Two tiles at head_dim 128 and more: a group of four consumer warps for each, on
+// the same stages.  One CTA per SM fits there, so one tile had one warp per scheduler, whose fixed latencies nothing hid (issue
+// slots 19 - 25 % busy); with two tiles in the same four warps instead 90 x 35 rows of head_dim 128 took 380 us, with a group each 288
+// (one tile at a time 360).  At head_dim 64 two CTAs of four warps share an SM already: there a warp serves both tiles, every K and V operand
+// loaded once (groups of warps at one CTA per SM: 24 x 4 x 8 rows 15 % slower).
+template <typename T, bool KV8, int NST, int HD, int HDV, int CPS, bool BAL, int MT>
+__global__ void __launch_bounds__((Smem<KV8 ? 1 : 2, NST, HD, HDV, MT>::NC + 1) * 32, CPS)
 fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v) {
   constexpr int ESZ = KV8 ? 1 : 2;
   static_assert(!KV8 || (HD == 128 && HDV == 128), "an e4m3 cache row must fill one 128-byte swizzle row");
   static_assert(HD % 64 == 0 && HDV % 64 == 0, "whole 128-byte column blocks");
-  using SM = Smem<ESZ, NST, HD, HDV>;
+  static_assert(MT == 1 || !KV8, "two row tiles: 16-bit caches");
+  using SM = Smem<ESZ, NST, HD, HDV, MT>;
   // 16-bit cache: m16n8k16 MMA in the cache's type.  e4m3 cache: the bytes are widened to fp16 in registers (exact,
   // one conversion per two elements) and fed to the fp16 m16n8k16 MMA; Q rows are scaled into fp16 range with a
   // per-row factor (undone in the softmax scale), P is fp16.  (The warp-level e4m3 MMA is not used: on sm_100a
@@ -321,7 +332,9 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   using TM = typename std::conditional<KV8, __half, T>::type;
   constexpr int TNS = SM::TNS;            // keys per stage
   constexpr int NC = SM::NC;
-  constexpr int WK = TNS / NC;            // keys per consumer warp and stage: 32
+  constexpr int KW = kConsumers;          // warps that share a stage's keys
+  constexpr int WK = TNS / KW;            // keys per consumer warp and stage: 32
+  constexpr int IT = MT / SM::TW;         // row tiles of a consumer warp
   constexpr int NT = WK / 8;              // 8-key MMA column tiles per warp
   // A warp's 32 keys are two groups of 16, one of each 64-key block of the stage, each with a running maximum of its own
   // (16-bit cache).  P is rounded to 16 bits, except where it is exactly 1: at a maximum.  With one maximum for 32 keys in
@@ -339,8 +352,8 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   volatile int* s_info = reinterpret_cast<volatile int*>(sm + SM::kInfoOff);   // 4 ints per stage
   volatile int* s_abort = reinterpret_cast<volatile int*>(sm + SM::kMiscOff);
   float* s_o = reinterpret_cast<float*>(sm + SM::kScrOff);
-  float* s_m = s_o + NC * 16 * SM::kLdO;
-  float* s_l = s_m + NC * 16;
+  float* s_m = s_o + KW * 16 * SM::kLdO;
+  float* s_l = s_m + KW * 16;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // (set up by the producer warp: the first threads have the entries of a short line to read)
@@ -366,7 +379,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   bool own = false;      // every triple has teams of its own: a unit of the line is a piece; else a unit is a key block
   if constexpr (BAL) {
     int* s_sum = reinterpret_cast<int*>(s_o);      // the merge area is not in use yet
-    if (tid == NC * 32 + 31) s_sum[30] = __ldcg(&p.status->error) != 0u;      // (one read: the CTA's threads must agree on the plan)
+    if (tid == NC * 32 + 31) s_sum[15] = __ldcg(&p.status->error) != 0u;      // (one read: the CTA's threads must agree on the plan)
     int E = p.batch * a.max_mtiles;
     if (a.use_list) {
       // the list's header must describe this call before any entry is read
@@ -381,14 +394,14 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     constexpr int kMinSpan = min_span(KV8), kCutCost = cut_cost(KV8), kMaxPieces = max_pieces(KV8);
     // ---- lengths: consecutive entries per thread; their sum, number and maximum ----
     constexpr int NTH = (NC + 1) * 32;
-    static_assert(NTH <= kSmallLine, "the prefix sums of a small line end before its records");
+    static_assert(NC + 1 < 15, "words of the warps");
     const int per = (E + NTH - 1) / NTH, e_lo = min(E, tid * per), e_hi = min(E, e_lo + per);
-    small = E <= NTH;
+    small = E <= kSmallLine;     // (the prefix sums of such a line end before its records)
     int sum = 0, num = 0, longest = 0;
     bool bad = false;
 #pragma unroll 1
     for (int e = e_lo; e < e_hi; ++e) {
-      const WorkItem it = line_entry(a, e);
+      const WorkItem it = line_entry<MT>(a, e);
       const int len = line_len(it);
       bad |= it.bad;
       if (small && it.valid) keep_entry(s_pref + kRecordOff + 8 * e, it);
@@ -399,12 +412,12 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     sum = __reduce_add_sync(0xffffffffu, sum);
     num = __reduce_add_sync(0xffffffffu, num);
     longest = __reduce_max_sync(0xffffffffu, longest);
-    if (lane == 0) { s_sum[warp] = sum; s_sum[8 + warp] = num; s_sum[16 + warp] = longest; }
+    if (lane == 0) { s_sum[warp] = sum; s_sum[16 + warp] = num; s_sum[32 + warp] = longest; }
     __syncthreads();
-    const bool whole = s_sum[30] != 0;
+    const bool whole = s_sum[15] != 0;
     sum = num = longest = 0;
 #pragma unroll
-    for (int w = 0; w <= NC; ++w) { sum += s_sum[w]; num += s_sum[8 + w]; longest = max(longest, s_sum[16 + w]); }
+    for (int w = 0; w <= NC; ++w) { sum += s_sum[w]; num += s_sum[16 + w]; longest = max(longest, s_sum[32 + w]); }
     // ---- the plan ----
     groups = p.hkv / a.team;
     const int teams = min((int)gridDim.x / a.team, kMaxBorders - 1);
@@ -423,11 +436,11 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       for (int e = tid >> 3; e < E; e += NTH / 8) n += (s_pref[e] + wd - 1) / wd;
       n += __shfl_xor_sync(0xffffffffu, n, 8);
       n += __shfl_xor_sync(0xffffffffu, n, 16);
-      if (lane < 8) s_sum[32 + warp * 8 + lane] = n;
+      if (lane < 8) s_sum[64 + warp * 8 + lane] = n;
       __syncthreads();
       n = 0;
 #pragma unroll
-      for (int w = 0; w <= NC; ++w) n += s_sum[32 + w * 8 + (lane & 7)];
+      for (int w = 0; w <= NC; ++w) n += s_sum[64 + w * 8 + (lane & 7)];
       const int found = __reduce_min_sync(0xffffffffu, n * groups <= teams ? min(wd, longest) : longest);
       if (found + kCutCost < longest) width = found;
       __syncthreads();       // (every thread has read the lengths that the prefix sums replace)
@@ -447,13 +460,13 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       const int v = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += v;
     }
-    if (lane == 31) s_sum[24 + warp] = incl;
+    if (lane == 31) s_sum[48 + warp] = incl;
     __syncthreads();
     int total = 0, before = incl - mine;
 #pragma unroll
     for (int w = 0; w <= NC; ++w) {
-      if (w < warp) before += s_sum[24 + w];
-      total += s_sum[24 + w];
+      if (w < warp) before += s_sum[48 + w];
+      total += s_sum[48 + w];
     }
 #pragma unroll 1
     for (int e = e_lo; e < e_hi; ++e) s_pref[e] += before;
@@ -522,7 +535,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         while (x >= s_pref[ent + 1] * groups) ++ent;      // (entries without blocks are passed over)
         const int len = s_pref[ent + 1] - s_pref[ent], off = x - s_pref[ent] * groups;
         const int hg = off / len, pos = off - hg * len, n = own ? 1 : min(len - pos, x_end - x);
-        it = small ? kept_entry(s_pref + kRecordOff + 8 * ent) : line_entry(a, ent);
+        it = small ? kept_entry(s_pref + kRecordOff + 8 * ent) : line_entry<MT>(a, ent);
         it.hk = hg * a.team + member;
         int pieces = 1, first = span;      // of this triple, and the span that holds its first piece
         if (own) {
@@ -700,17 +713,25 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
   } else {
     // ============================================ consumers ===========================================
     const int g = lane >> 2, tq = lane & 3;
+    const int kw = SM::TW > 1 ? warp % KW : warp, tw = SM::TW > 1 ? warp / KW : 0;     // its keys of a stage, its row tile
     const int rep = p.rep;
     // R / rep for rows of a sequence: R < 2^21 keeps the rounded product on the right side of every multiple
     const float inv_rep = __frcp_rn((float)rep);
     auto token_of = [&](int R) { return (int)(((float)R + 0.5f) * inv_rep); };
     uint32_t cnt = 0;
     bool ok = true;
-    uint32_t qf[HD / 16][4];   // A operand of 8 k-steps of 16
+    // A operand of 8 k-steps of 16, in registers (one row tile) or in shared memory
+    uint32_t qf[HD / 16][4];
+    const uint32_t sq = base + SM::kQOff + (uint32_t)lane * 16u;
     float qs_a = 1.f, qs_b = 1.f;   // e4m3 Q: 1 / (row quantisation scale), folded into the logit scale
-    float o[HDV / 8][4];
-    float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
-    int lo_a = 0, hi_a = -1, lo_b = 0, hi_b = -1, lo_max = 0, hi_min = -1;
+    float o[IT][HDV / 8][4];
+    float m_a[IT], m_b[IT], l_a[IT], l_b[IT];
+    int lo_a[IT], hi_a[IT], lo_b[IT], hi_b[IT], lo_max[IT], hi_min[IT];
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {
+      m_a[u] = m_b[u] = -INFINITY; l_a[u] = l_b[u] = 0.f;
+      lo_a[u] = lo_b[u] = lo_max[u] = 0; hi_a[u] = hi_b[u] = hi_min[u] = -1;
+    }
     float c_mul = 0.f, cap_in = 0.f, vds = 1.f;
     WorkItem it_reg{};
     uint32_t pcnt = 0;
@@ -720,14 +741,17 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
     // free during the merge (an e4m3 kernel has 168).
     auto clear_o = [&]() {
 #pragma unroll
-      for (int i = 0; i < HDV / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
+      for (int u = 0; u < IT; ++u)
+#pragma unroll
+        for (int i = 0; i < HDV / 8; ++i) { o[u][i][0] = o[u][i][1] = o[u][i][2] = o[u][i][3] = 0.f; }
     };
     auto clear = [&]() {
       clear_o();
 #pragma unroll
       for (int i = 0; i < HD / 16; ++i) { qf[i][0] = qf[i][1] = qf[i][2] = qf[i][3] = 0u; }
     };
-    if constexpr (BAL) clear();
+    if constexpr (BAL && !SM::kQShared) clear();
+    else if constexpr (BAL) clear_o();
     int bal_key = 0, bal_end = 0, bal_flags = F_LAST;     // balanced kernels: position inside the piece
     while (true) {
       const uint32_t s = cnt % NST;
@@ -765,17 +789,42 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         vds = p.v_descale ? p.v_descale[di] : 1.f;
         // Q fragments straight from global memory (rows g and g+8 of the packed tile)
         if constexpr (!KV8) {
+          // A operand of m16n8k16: rows g and g + 8 of a tile, columns ks * 16 + 2 * tq (+ 8)
+          auto row_of = [&](int tile, int rr, bool* live) {
+            const int R = tile * 16 + g + rr * 8;
+            *live = R < rows_total;
+            const int token = *live ? token_of(R) : 0, head = it.hk * rep + (*live ? R - token * rep : 0);
+            return reinterpret_cast<const T*>(p.q) + (int64_t)(it.q0 + token) * p.q_row_stride + (int64_t)head * p.q_head_stride + 2 * tq;
+          };
+          if constexpr (SM::kQShared) {
+            // the warps share them out (nobody reads the previous item's any more: the barriers at its end)
+            constexpr int NQ = MT * (HD / 16) / NC;
+            static_assert(NQ * NC == MT * (HD / 16), "whole fragments per warp");
+            uint32_t x[NQ][4];
 #pragma unroll
-          for (int rr = 0; rr < 2; ++rr) {       // A operand of m16n8k16: columns ks*16 + 2*tq (+8)
-            const int R = it.mt * 16 + g + rr * 8;
-            const bool live = R < rows_total;
-            const int token = live ? token_of(R) : 0, head = it.hk * rep + (live ? R - token * rep : 0);
-            const T* qrow = reinterpret_cast<const T*>(p.q) + (int64_t)(it.q0 + token) * p.q_row_stride +
-                            (int64_t)head * p.q_head_stride + 2 * tq;
+            for (int k = 0; k < NQ; ++k) {
+              const int n = k * NC + warp, u = n / (HD / 16), ks = n - u * (HD / 16);
 #pragma unroll
-            for (int ks = 0; ks < HD / 16; ++ks) {
-              qf[ks][rr] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16) : 0u;
-              qf[ks][rr + 2] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8) : 0u;
+              for (int rr = 0; rr < 2; ++rr) {
+                bool live;
+                const T* qrow = row_of(it.mt * MT + u, rr, &live);
+                x[k][rr] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16) : 0u;
+                x[k][rr + 2] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8) : 0u;
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) st_shared_v4(sq + (uint32_t)(k * NC + warp) * 512u, x[k][0], x[k][1], x[k][2], x[k][3]);
+            bar_consumers<NC>();
+          } else {
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+              bool live;
+              const T* qrow = row_of(it.mt, rr, &live);
+#pragma unroll
+              for (int ks = 0; ks < HD / 16; ++ks) {
+                qf[ks][rr] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16) : 0u;
+                qf[ks][rr + 2] = live ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8) : 0u;
+              }
             }
           }
         } else {
@@ -836,20 +885,24 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         c_mul = has_cap ? p.softcap * kLog2e : sc * kLog2e;
         cap_in = has_cap ? sc / p.softcap : 0.f;
         const int off = it.seqlen_k - it.seqlen_q;
-        const int rb = it.mt * 16;                   // first packed row of this work item
-        const int qp_a = off + token_of(rb + g), qp_b = off + token_of(rb + g + 8);
-        lo_a = lo_b = it.leftpad;
-        hi_a = hi_b = min(it.seqlen_k, it.hi * TN) - 1;   // keys past this split's range are not ours
-        if (p.is_causal) { hi_a = min(hi_a, qp_a); hi_b = min(hi_b, qp_b); }
-        if (p.window_right >= 0) { hi_a = min(hi_a, qp_a + p.window_right); hi_b = min(hi_b, qp_b + p.window_right); }
-        if (p.window_left >= 0) { lo_a = max(lo_a, qp_a - p.window_left); lo_b = max(lo_b, qp_b - p.window_left); }
-        // bounds valid for all 16 rows (rows past rows_total included: conservative)
-        const int qp_lo = off + token_of(rb), qp_hi = off + token_of(rb + 15);
-        lo_max = it.leftpad; hi_min = min(it.seqlen_k, it.hi * TN) - 1;
-        if (p.is_causal) hi_min = min(hi_min, qp_lo);
-        if (p.window_right >= 0) hi_min = min(hi_min, qp_lo + p.window_right);
-        if (p.window_left >= 0) lo_max = max(lo_max, qp_hi - p.window_left);
-        m_a = m_b = -INFINITY; l_a = l_b = 0.f;
+        const int last_key = min(it.seqlen_k, it.hi * TN) - 1;   // keys past this split's range are not ours
+#pragma unroll
+        for (int u = 0; u < IT; ++u) {
+          const int rb = (it.mt * MT + tw + u) * 16;      // first packed row of this tile
+          const int qp_a = off + token_of(rb + g), qp_b = off + token_of(rb + g + 8);
+          lo_a[u] = lo_b[u] = it.leftpad;
+          hi_a[u] = hi_b[u] = last_key;
+          if (p.is_causal) { hi_a[u] = min(hi_a[u], qp_a); hi_b[u] = min(hi_b[u], qp_b); }
+          if (p.window_right >= 0) { hi_a[u] = min(hi_a[u], qp_a + p.window_right); hi_b[u] = min(hi_b[u], qp_b + p.window_right); }
+          if (p.window_left >= 0) { lo_a[u] = max(lo_a[u], qp_a - p.window_left); lo_b[u] = max(lo_b[u], qp_b - p.window_left); }
+          // bounds valid for all 16 rows (rows past rows_total included: conservative)
+          const int qp_lo = off + token_of(rb), qp_hi = off + token_of(rb + 15);
+          lo_max[u] = it.leftpad; hi_min[u] = last_key;
+          if (p.is_causal) hi_min[u] = min(hi_min[u], qp_lo);
+          if (p.window_right >= 0) hi_min[u] = min(hi_min[u], qp_lo + p.window_right);
+          if (p.window_left >= 0) lo_max[u] = max(lo_max[u], qp_hi - p.window_left);
+          m_a[u] = m_b[u] = -INFINITY; l_a[u] = l_b[u] = 0.f;
+        }
         if constexpr (!BAL) clear_o();
       }
 
@@ -857,69 +910,119 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         ok = wait_or_abort(bar_full + 8 * s, (cnt / NST) & 1, s_abort);
         if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_CONSUMER); s_abort[0] = 1; break; }
       }
-      if (!(flags & F_EMPTY)) {
+      // (a group of warps whose row tile has no rows, the last of an odd number, has nothing to add)
+      if (!(flags & F_EMPTY) && (SM::TW == 1 || (it.mt * MT + tw) * 16 < it.seqlen_q * rep)) {
         const uint32_t kb = base + s * SM::kStage, vb = kb + SM::kKBytes;
         const int mat = lane >> 3, l7 = lane & 7;
-        float sacc[NT][4];
+        float sacc[IT][NT][4];
 #pragma unroll
-        for (int i = 0; i < NT; ++i) { sacc[i][0] = sacc[i][1] = sacc[i][2] = sacc[i][3] = 0.f; }
+        for (int u = 0; u < IT; ++u)
+#pragma unroll
+          for (int i = 0; i < NT; ++i) { sacc[u][i][0] = sacc[u][i][1] = sacc[u][i][2] = sacc[u][i][3] = 0.f; }
         if constexpr (!KV8) {
-          const uint32_t krow = kb + (uint32_t)(warp * kWarpRows + (mat >> 1) * 8 + l7) * 128u;
-#pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t krow = kb + (uint32_t)(kw * kWarpRows + (mat >> 1) * 8 + l7) * 128u;
+          uint32_t qx[IT][4];
+          // (the operands of the next step are on their way while this one's MMAs run)
+          uint32_t kf[2][WK / 16][4];
+          auto load_k = [&](int ks, uint32_t (&x)[WK / 16][4]) {
             const uint32_t chunk = (uint32_t)((ks * 2 + (mat & 1)) & 7);
 #pragma unroll
+            for (int hf = 0; hf < WK / 16; ++hf)
+              ldmatrix_x4(x[hf], krow + hf * (kGroupRows * 128) + (ks >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
+          };
+          constexpr bool kAhead = MT > 1;
+          if (kAhead) load_k(0, kf[0]);
+#pragma unroll
+          for (int ks = 0; ks < HD / 16; ++ks) {
+            if (!kAhead) load_k(ks, kf[ks & 1]);
+            else if (ks + 1 < HD / 16) load_k(ks + 1, kf[(ks + 1) & 1]);
+            if constexpr (SM::kQShared) {
+#pragma unroll
+              for (int u = 0; u < IT; ++u) {
+                const uint4 x = ld_shared_v4(sq + (uint32_t)((tw + u) * (HD / 16) + ks) * 512u);
+                qx[u][0] = x.x; qx[u][1] = x.y; qx[u][2] = x.z; qx[u][3] = x.w;
+              }
+            }
+#pragma unroll
             for (int hf = 0; hf < WK / 16; ++hf) {
-              uint32_t bfr[4];
-              ldmatrix_x4(bfr, krow + hf * (kGroupRows * 128) + (ks >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
-              mma_16816<TM>(sacc[2 * hf], qf[ks], bfr[0], bfr[1]);
-              mma_16816<TM>(sacc[2 * hf + 1], qf[ks], bfr[2], bfr[3]);
+              const uint32_t (&bfr)[4] = kf[ks & 1][hf];
+#pragma unroll
+              for (int u = 0; u < IT; ++u) {
+                const uint32_t (&qa)[4] = SM::kQShared ? qx[u] : qf[ks];
+                mma_16816<TM>(sacc[u][2 * hf], qa, bfr[0], bfr[1]);
+                mma_16816<TM>(sacc[u][2 * hf + 1], qa, bfr[2], bfr[3]);
+              }
             }
           }
         } else {
           // e4m3 rows are 128 bytes: one swizzle row per key.  ldmatrix moves 16-byte chunks, so lane (g, tq)
           // receives bytes 4tq..4tq+3 of key g; widened to two fp16 pairs they are the B operand of one k-step.
+          uint32_t kf8[2][4];
+          auto load_k8 = [&](int n, uint32_t (&x)[4]) {
+            const int hf = n / (HD / 32), k32 = n % (HD / 32);
+            const uint32_t chunk = (uint32_t)(k32 * 2 + (mat & 1));
+            ldmatrix_x4(x, kb + (uint32_t)(kw * WK + hf * 16 + (mat >> 1) * 8 + l7) * 128u + ((chunk ^ (uint32_t)l7) << 4));
+          };
+          load_k8(0, kf8[0]);
 #pragma unroll
-          for (int hf = 0; hf < WK / 16; ++hf) {
-            const uint32_t krow = kb + (uint32_t)(warp * WK + hf * 16 + (mat >> 1) * 8 + l7) * 128u;
-#pragma unroll
-            for (int k32 = 0; k32 < HD / 32; ++k32) {
-              uint32_t raw4[4];
-              const uint32_t chunk = (uint32_t)(k32 * 2 + (mat & 1));
-              ldmatrix_x4(raw4, krow + ((chunk ^ (uint32_t)l7) << 4));
+          for (int n = 0; n < WK / 16 * (HD / 32); ++n) {
+            {
+              const int hf = n / (HD / 32), k32 = n % (HD / 32);
+              if (n + 1 < WK / 16 * (HD / 32)) load_k8(n + 1, kf8[(n + 1) & 1]);
+              const uint32_t (&raw4)[4] = kf8[n & 1];
               uint32_t b[4][2];
 #pragma unroll
               for (int m = 0; m < 4; ++m) e4m3x4_to<__half>(raw4[m], b[m][0], b[m][1]);
-              mma_16816<__half>(sacc[2 * hf], qf[2 * k32], b[0][0], b[0][1]);
-              mma_16816<__half>(sacc[2 * hf], qf[2 * k32 + 1], b[1][0], b[1][1]);
-              mma_16816<__half>(sacc[2 * hf + 1], qf[2 * k32], b[2][0], b[2][1]);
-              mma_16816<__half>(sacc[2 * hf + 1], qf[2 * k32 + 1], b[3][0], b[3][1]);
+              mma_16816<__half>(sacc[0][2 * hf], qf[2 * k32], b[0][0], b[0][1]);
+              mma_16816<__half>(sacc[0][2 * hf], qf[2 * k32 + 1], b[1][0], b[1][1]);
+              mma_16816<__half>(sacc[0][2 * hf + 1], qf[2 * k32], b[2][0], b[2][1]);
+              mma_16816<__half>(sacc[0][2 * hf + 1], qf[2 * k32 + 1], b[3][0], b[3][1]);
             }
           }
         }
+        // The next V operands, the first during the softmax, ahead of the MMAs that use them: over an e4m3 cache and with two row tiles, where
+        // the MMAs wait for more than one operand.  e4m3, one row tile, us: 48 sequences of 1024 .. 16384 keys 192.5 -> 188.5, 5 of 100 .. 900
+        // 15.9 -> 15.1; 24 x 4 x 8 rows of head_dim 64 60.7 -> 59.1.  With one row tile over a 16-bit cache 16 sequences took 94 instead of 91.
+        constexpr int VD = MT > 1 || KV8 ? 1 : 0;
+        uint32_t vf[VD + 1][4];
+        auto load_v = [&](int n, uint32_t (&x)[4]) {
+          if constexpr (!KV8) {
+            const int hf = n / (HDV / 16), np = n % (HDV / 16);
+            const uint32_t chunk = (uint32_t)((np * 2 + (mat >> 1)) & 7);
+            ldmatrix_x4_trans(x, vb + (uint32_t)(kw * kWarpRows + hf * kGroupRows + (mat & 1) * 8 + l7) * 128u + (np >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
+          } else {
+            const int hf = n / (HDV / 32), c2 = n % (HDV / 32);
+            ldmatrix_x4_trans(x, vb + (uint32_t)(kw * WK + hf * 16 + (mat & 1) * 8 + l7) * 128u + (((uint32_t)(2 * c2 + (mat >> 1)) ^ (uint32_t)l7) << 4));
+          }
+        };
+#pragma unroll
+        for (int n = 0; n < VD; ++n) load_v(n, vf[n]);
         // ---- mask + online softmax over this warp's keys ----
         const float cm_a = c_mul * (has_cap ? 1.f : qs_a), cm_b = c_mul * (has_cap ? 1.f : qs_b);
         const float ci_a = cap_in * qs_a, ci_b = cap_in * qs_b;
+        float corr_a[IT][NG], corr_b[IT][NG];
+#pragma unroll
+        for (int u = 0; u < IT; ++u) {
         float mx_a[NG], mx_b[NG];
 #pragma unroll
         for (int gr = 0; gr < NG; ++gr) {
-          const int kbase = key0 + warp * kWarpRows + gr * kGroupRows;
-          const bool full = (kbase >= lo_max) && (kbase + GT * 8 - 1 <= hi_min);
+          const int kbase = key0 + kw * kWarpRows + gr * kGroupRows;
+          const bool full = (kbase >= lo_max[u]) && (kbase + GT * 8 - 1 <= hi_min[u]);
           mx_a[gr] = mx_b[gr] = -INFINITY;
 #pragma unroll
           for (int t = 0; t < GT; ++t) {
             const int nt = gr * GT + t;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              float y = sacc[nt][e];
+              float y = sacc[u][nt][e];
               if (e >= 2) y = has_cap ? tanh_fast(y * ci_b) * c_mul : y * cm_b;
               else y = has_cap ? tanh_fast(y * ci_a) * c_mul : y * cm_a;
               if (!full) {
                 const int kk = kbase + t * 8 + 2 * tq + (e & 1);
-                const bool okk = e >= 2 ? (kk >= lo_b && kk <= hi_b) : (kk >= lo_a && kk <= hi_a);
+                const bool okk = e >= 2 ? (kk >= lo_b[u] && kk <= hi_b[u]) : (kk >= lo_a[u] && kk <= hi_a[u]);
                 y = okk ? y : -INFINITY;
               }
-              sacc[nt][e] = y;
+              sacc[u][nt][e] = y;
               if (e >= 2) mx_b[gr] = fmaxf(mx_b[gr], y); else mx_a[gr] = fmaxf(mx_a[gr], y);
             }
           }
@@ -931,49 +1034,54 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           mx_b[gr] = fmaxf(mx_b[gr], __shfl_xor_sync(0xffffffffu, mx_b[gr], 1));
           mx_b[gr] = fmaxf(mx_b[gr], __shfl_xor_sync(0xffffffffu, mx_b[gr], 2));
         }
-        float corr_a[NG], corr_b[NG];
 #pragma unroll
         for (int gr = 0; gr < NG; ++gr) {
-          const float mn_a = fmaxf(m_a, mx_a[gr]), mn_b = fmaxf(m_b, mx_b[gr]);
+          const float mn_a = fmaxf(m_a[u], mx_a[gr]), mn_b = fmaxf(m_b[u], mx_b[gr]);
           const float ms_a = mn_a == -INFINITY ? 0.f : mn_a, ms_b = mn_b == -INFINITY ? 0.f : mn_b;
-          corr_a[gr] = ex2(m_a - ms_a); corr_b[gr] = ex2(m_b - ms_b);
-          m_a = mn_a; m_b = mn_b;
+          corr_a[u][gr] = ex2(m_a[u] - ms_a); corr_b[u][gr] = ex2(m_b[u] - ms_b);
+          m_a[u] = mn_a; m_b[u] = mn_b;
           float ps_a = 0.f, ps_b = 0.f;
 #pragma unroll
           for (int nt = gr * GT; nt < (gr + 1) * GT; ++nt) {
-            sacc[nt][0] = ex2(sacc[nt][0] - ms_a); sacc[nt][1] = ex2(sacc[nt][1] - ms_a);
-            sacc[nt][2] = ex2(sacc[nt][2] - ms_b); sacc[nt][3] = ex2(sacc[nt][3] - ms_b);
-            ps_a += sacc[nt][0] + sacc[nt][1];
-            ps_b += sacc[nt][2] + sacc[nt][3];
+            sacc[u][nt][0] = ex2(sacc[u][nt][0] - ms_a); sacc[u][nt][1] = ex2(sacc[u][nt][1] - ms_a);
+            sacc[u][nt][2] = ex2(sacc[u][nt][2] - ms_b); sacc[u][nt][3] = ex2(sacc[u][nt][3] - ms_b);
+            ps_a += sacc[u][nt][0] + sacc[u][nt][1];
+            ps_b += sacc[u][nt][2] + sacc[u][nt][3];
           }
-          l_a = l_a * corr_a[gr] + ps_a;
-          l_b = l_b * corr_b[gr] + ps_b;
+          l_a[u] = l_a[u] * corr_a[u][gr] + ps_a;
+          l_b[u] = l_b[u] * corr_b[u][gr] + ps_b;
         }
-        auto rescale_o = [&](float ca, float cb) {
+        }
+        auto rescale_o = [&](int u, float ca, float cb) {
           if (__any_sync(0xffffffffu, ca != 1.f || cb != 1.f)) {
 #pragma unroll
-            for (int i = 0; i < HDV / 8; ++i) { o[i][0] *= ca; o[i][1] *= ca; o[i][2] *= cb; o[i][3] *= cb; }
+            for (int i = 0; i < HDV / 8; ++i) { o[u][i][0] *= ca; o[u][i][1] *= ca; o[u][i][2] *= cb; o[u][i][3] *= cb; }
           }
         };
-        if constexpr (KV8) rescale_o(corr_a[0], corr_b[0]);
+        if constexpr (KV8) rescale_o(0, corr_a[0][0], corr_b[0][0]);
         // ---- O += P V ----
         if constexpr (!KV8) {
 #pragma unroll
           for (int hf = 0; hf < WK / 16; ++hf) {
-            rescale_o(corr_a[hf], corr_b[hf]);
-            uint32_t pa[4];
-            pa[0] = pack2<TM>(sacc[2 * hf][0], sacc[2 * hf][1]);
-            pa[1] = pack2<TM>(sacc[2 * hf][2], sacc[2 * hf][3]);
-            pa[2] = pack2<TM>(sacc[2 * hf + 1][0], sacc[2 * hf + 1][1]);
-            pa[3] = pack2<TM>(sacc[2 * hf + 1][2], sacc[2 * hf + 1][3]);
-            const uint32_t vrow = vb + (uint32_t)(warp * kWarpRows + hf * kGroupRows + (mat & 1) * 8 + l7) * 128u;
+            uint32_t pa[IT][4];
+#pragma unroll
+            for (int u = 0; u < IT; ++u) {
+              rescale_o(u, corr_a[u][hf], corr_b[u][hf]);
+              pa[u][0] = pack2<TM>(sacc[u][2 * hf][0], sacc[u][2 * hf][1]);
+              pa[u][1] = pack2<TM>(sacc[u][2 * hf][2], sacc[u][2 * hf][3]);
+              pa[u][2] = pack2<TM>(sacc[u][2 * hf + 1][0], sacc[u][2 * hf + 1][1]);
+              pa[u][3] = pack2<TM>(sacc[u][2 * hf + 1][2], sacc[u][2 * hf + 1][3]);
+            }
 #pragma unroll
             for (int np = 0; np < HDV / 16; ++np) {
-              uint32_t bfr[4];
-              const uint32_t chunk = (uint32_t)((np * 2 + (mat >> 1)) & 7);
-              ldmatrix_x4_trans(bfr, vrow + (np >> 2) * (TNS * 128) + ((chunk ^ (uint32_t)l7) << 4));
-              mma_16816<TM>(o[2 * np], pa, bfr[0], bfr[1]);
-              mma_16816<TM>(o[2 * np + 1], pa, bfr[2], bfr[3]);
+              const int n = hf * (HDV / 16) + np;
+              if (n + VD < WK / 16 * (HDV / 16)) load_v(n + VD, vf[(n + VD) % (VD + 1)]);
+              const uint32_t (&bfr)[4] = vf[n % (VD + 1)];
+#pragma unroll
+              for (int u = 0; u < IT; ++u) {
+                mma_16816<TM>(o[u][2 * np], pa[u], bfr[0], bfr[1]);
+                mma_16816<TM>(o[u][2 * np + 1], pa[u], bfr[2], bfr[3]);
+              }
             }
           }
         } else {
@@ -987,15 +1095,15 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
 #pragma unroll
           for (int hf = 0; hf < WK / 16; ++hf) {
             uint32_t pa[4];
-            pa[0] = pack2<__half>(sacc[2 * hf][0], sacc[2 * hf][1]);
-            pa[1] = pack2<__half>(sacc[2 * hf][2], sacc[2 * hf][3]);
-            pa[2] = pack2<__half>(sacc[2 * hf + 1][0], sacc[2 * hf + 1][1]);
-            pa[3] = pack2<__half>(sacc[2 * hf + 1][2], sacc[2 * hf + 1][3]);
-            const uint32_t vrow = vb + (uint32_t)(warp * WK + hf * 16 + (mat & 1) * 8 + l7) * 128u;
+            pa[0] = pack2<__half>(sacc[0][2 * hf][0], sacc[0][2 * hf][1]);
+            pa[1] = pack2<__half>(sacc[0][2 * hf][2], sacc[0][2 * hf][3]);
+            pa[2] = pack2<__half>(sacc[0][2 * hf + 1][0], sacc[0][2 * hf + 1][1]);
+            pa[3] = pack2<__half>(sacc[0][2 * hf + 1][2], sacc[0][2 * hf + 1][3]);
 #pragma unroll
             for (int c2 = 0; c2 < HDV / 32; ++c2) {
-              uint32_t r4[4];
-              ldmatrix_x4_trans(r4, vrow + (((uint32_t)(2 * c2 + (mat >> 1)) ^ (uint32_t)l7) << 4));
+              const int n = hf * (HDV / 32) + c2;
+              if (n + VD < WK / 16 * (HDV / 32)) load_v(n + VD, vf[(n + VD) % (VD + 1)]);
+              const uint32_t (&r4)[4] = vf[n % (VD + 1)];
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 const int c = 2 * c2 + h;
@@ -1004,8 +1112,8 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
                 asm("prmt.b32 %0, %1, %2, 0x7531;" : "=r"(od) : "r"(r4[2 * h]), "r"(r4[2 * h + 1]));
                 e4m3x4_to<__half>(ev, be0, be1);
                 e4m3x4_to<__half>(od, bo0, bo1);
-                mma_16816<__half>(o[2 * c], pa, be0, be1);
-                mma_16816<__half>(o[2 * c + 1], pa, bo0, bo1);
+                mma_16816<__half>(o[0][2 * c], pa, be0, be1);
+                mma_16816<__half>(o[0][2 * c + 1], pa, bo0, bo1);
               }
             }
           }
@@ -1016,28 +1124,36 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       ++cnt;
 
       if (flags & F_LAST) {
-        // ---- merge the four warps' partial results and write the output rows ----
-        l_a += __shfl_xor_sync(0xffffffffu, l_a, 1); l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
-        l_b += __shfl_xor_sync(0xffffffffu, l_b, 1); l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-        float* so = s_o + warp * 16 * SM::kLdO;
+        // ---- merge the four warps' partial results and write the output rows, a row tile at a time ----
+        bool is_piece = false;
+        if constexpr (BAL) is_piece = cur.pieces > 1;
+#pragma unroll SM::TW > 1 ? 1 : MT
+        for (int ut = 0; ut < MT; ++ut) {
+          const int u = SM::TW > 1 ? 0 : ut;      // (this warp's own number of the tile)
+        if (ut > 0) bar_consumers<NC>();      // (the tile before has left the merge area)
+        if (SM::TW == 1 || tw == ut) {
+        l_a[u] += __shfl_xor_sync(0xffffffffu, l_a[u], 1); l_a[u] += __shfl_xor_sync(0xffffffffu, l_a[u], 2);
+        l_b[u] += __shfl_xor_sync(0xffffffffu, l_b[u], 1); l_b[u] += __shfl_xor_sync(0xffffffffu, l_b[u], 2);
+        float* so = s_o + kw * 16 * SM::kLdO;
         if (!KV8) {
 #pragma unroll
           for (int nt = 0; nt < HDV / 8; ++nt) {
-            *reinterpret_cast<float2*>(so + g * SM::kLdO + nt * 8 + 2 * tq) = make_float2(o[nt][0], o[nt][1]);
-            *reinterpret_cast<float2*>(so + (g + 8) * SM::kLdO + nt * 8 + 2 * tq) = make_float2(o[nt][2], o[nt][3]);
+            *reinterpret_cast<float2*>(so + g * SM::kLdO + nt * 8 + 2 * tq) = make_float2(o[u][nt][0], o[u][nt][1]);
+            *reinterpret_cast<float2*>(so + (g + 8) * SM::kLdO + nt * 8 + 2 * tq) = make_float2(o[u][nt][2], o[u][nt][3]);
           }
         } else {
 #pragma unroll
           for (int c = 0; c < HDV / 16; ++c) {   // undo the even/odd column split of the fp8 V path
             *reinterpret_cast<float4*>(so + g * SM::kLdO + c * 16 + 4 * tq) =
-                make_float4(o[2 * c][0], o[2 * c + 1][0], o[2 * c][1], o[2 * c + 1][1]);
+                make_float4(o[u][2 * c][0], o[u][2 * c + 1][0], o[u][2 * c][1], o[u][2 * c + 1][1]);
             *reinterpret_cast<float4*>(so + (g + 8) * SM::kLdO + c * 16 + 4 * tq) =
-                make_float4(o[2 * c][2], o[2 * c + 1][2], o[2 * c][3], o[2 * c + 1][3]);
+                make_float4(o[u][2 * c][2], o[u][2 * c + 1][2], o[u][2 * c][3], o[u][2 * c + 1][3]);
           }
         }
         if (tq == 0) {
-          s_m[warp * 16 + g] = m_a; s_m[warp * 16 + g + 8] = m_b;
-          s_l[warp * 16 + g] = l_a; s_l[warp * 16 + g + 8] = l_b;
+          s_m[kw * 16 + g] = m_a[u]; s_m[kw * 16 + g + 8] = m_b[u];
+          s_l[kw * 16 + g] = l_a[u]; s_l[kw * 16 + g + 8] = l_b[u];
+        }
         }
         bar_consumers<NC>();
         {
@@ -1045,16 +1161,16 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
           constexpr int GPR = HDV / CPT;                 // threads per row, side by side: four columns each, CPT / 4 times
           constexpr int CST = 4 * GPR;                   // (16 columns in a row per thread: four-way bank conflicts)
           const int Rl = tid / GPR, c0 = (tid % GPR) * 4;     // row within the tile, first column
-          const int R = it.mt * 16 + Rl;                     // packed row (token, head)
+          const int R = (it.mt * MT + ut) * 16 + Rl;                     // packed row (token, head)
           const int rows_total = it.seqlen_q * rep;
-          float mw[NC], M = -INFINITY;
+          float mw[KW], M = -INFINITY;
 #pragma unroll
-          for (int wi = 0; wi < NC; ++wi) { mw[wi] = s_m[wi * 16 + Rl]; M = fmaxf(M, mw[wi]); }
+          for (int wi = 0; wi < KW; ++wi) { mw[wi] = s_m[wi * 16 + Rl]; M = fmaxf(M, mw[wi]); }
           float L = 0.f, acc[CPT];
 #pragma unroll
           for (int j = 0; j < CPT; ++j) acc[j] = 0.f;
 #pragma unroll
-          for (int wi = 0; wi < NC; ++wi) {
+          for (int wi = 0; wi < KW; ++wi) {
             const float e = mw[wi] == -INFINITY ? 0.f : ex2(mw[wi] - M);
             L += e * s_l[wi * 16 + Rl];
             const float* src = s_o + (wi * 16 + Rl) * SM::kLdO + c0;
@@ -1064,122 +1180,16 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
               acc[j] += e * v4.x; acc[j + 1] += e * v4.y; acc[j + 2] += e * v4.z; acc[j + 3] += e * v4.w;
             }
           }
-          bool is_piece = false;
-          if constexpr (BAL) is_piece = cur.pieces > 1;
           if (BAL && is_piece) {
             if constexpr (BAL) {
               // one piece: rows as they are, with their maximum and sum; the CTA that arrives last merges
               const int64_t slot = (int64_t)cur.number * 2 + cur.head;
-              if (R < rows_total && Rl < p.part_rows) {
-                float* po = p.part_o + (slot * p.part_rows + Rl) * HDV + c0;
+              if (R < rows_total && ut * 16 + Rl < p.part_rows) {
+                float* po = p.part_o + (slot * p.part_rows + ut * 16 + Rl) * HDV + c0;
 #pragma unroll
                 for (int j = 0; j < CPT; j += 4)
                   *reinterpret_cast<float4*>(po + j / 4 * CST) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-                if (tid % GPR == 0) reinterpret_cast<float2*>(p.part_ml)[slot * p.part_rows + Rl] = make_float2(M, L);
-              }
-              bar_consumers<NC>();       // (thread 0's fence then covers the rows of all four warps)
-              if (tid == 0) {
-                // (release: the rows of all four warps lie behind the barrier; acquire: the other pieces' rows)
-                unsigned* word = p.arrivals + cur.first;
-                const bool last = atomic_add_acq_rel(word, 1u) == (unsigned)cur.pieces - 1u;
-                if (last) *word = 0u;        // zero again for the next call
-                *s_last = last ? 1 : 0;
-              }
-              bar_consumers<NC>();
-              if (*s_last) {
-                // piece j lies in slot 2 (first + j) + (j == 0).  All threads over (row, 4 columns).  Few pieces: a thread
-                // loads the rows and their pairs together, one trip to L2.  Many: weights first, every pair loaded before any
-                // is used, then a warp per row and a lane per piece (the merge area is free: every warp has written its
-                // piece).  (With every thread reading many pairs by itself, one after the other, 148 pieces took some 20 us;
-                // a warp that took its rows one after the other waited for two trips per row, 6600 cycles for 16 rows.)
-                const int live = min(p.part_rows, rows_total - it.mt * 16), np = cur.pieces;
-                const int64_t s0 = (int64_t)cur.first * 2;
-                const float2* ml = reinterpret_cast<const float2*>(p.part_ml);
-                float2* pairs = reinterpret_cast<float2*>(s_o);      // (maximum, sum), then (weight, sum)
-                if (np > kFewPieces) {
-                  for (int u = tid; u < live * np; u += NC * 32) {
-                    const int j = u / live, r = u - j * live;
-                    pairs[r * kMaxMerge + j] = __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows + r);
-                  }
-                  bar_consumers<NC>();
-#pragma unroll 1
-                  for (int r = warp; r < live; r += NC) {
-                    float Mx = -INFINITY, Ls = 0.f;
-                    for (int j = lane; j < np; j += 32) Mx = fmaxf(Mx, pairs[r * kMaxMerge + j].x);
-#pragma unroll
-                    for (int d = 16; d > 0; d >>= 1) Mx = fmaxf(Mx, __shfl_xor_sync(0xffffffffu, Mx, d));
-                    for (int j = lane; j < np; j += 32) {
-                      const float2 q2 = pairs[r * kMaxMerge + j];
-                      const float e = Mx > -INFINITY ? ex2(q2.x - Mx) : 0.f;   // (a piece without visible keys: exactly 0, its rows are 0)
-                      pairs[r * kMaxMerge + j].x = e;
-                      Ls += e * q2.y;
-                    }
-#pragma unroll
-                    for (int d = 16; d > 0; d >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, d);
-                    if (lane == 0) { s_m[r] = Mx; s_l[r] = Ls; }
-                  }
-                  bar_consumers<NC>();
-                }
-#pragma unroll 1
-                for (int u = tid; u < live * (HDV / 4); u += NC * 32) {
-                  const int r = u / (HDV / 4), c4 = (u - r * (HDV / 4)) * 4;
-                  const float* pr = p.part_o + (int64_t)r * HDV + c4;
-                  float Mx, Ls;
-                  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                  if (np > kFewPieces) {
-                    Mx = s_m[r]; Ls = s_l[r];
-#pragma unroll 8
-                    for (int j = 0; j < np; ++j) {
-                      const float4 w4 = __ldcg(reinterpret_cast<const float4*>(pr + (s0 + 2 * j + (j == 0)) * p.part_rows * HDV));
-                      const float e = pairs[r * kMaxMerge + j].x;
-                      v.x += e * w4.x; v.y += e * w4.y; v.z += e * w4.z; v.w += e * w4.w;
-                    }
-                  } else {
-                    float2 ml_[kFewPieces];
-                    float4 w4[kFewPieces];
-                    Mx = -INFINITY;
-#pragma unroll
-                    for (int j = 0; j < kFewPieces; ++j) {
-                      ml_[j] = make_float2(-INFINITY, 0.f);
-                      w4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                      if (j < np) {
-                        const int64_t slot = (s0 + 2 * j + (j == 0)) * p.part_rows;
-                        ml_[j] = __ldcg(ml + slot + r);
-                        w4[j] = __ldcg(reinterpret_cast<const float4*>(pr + slot * HDV));
-                      }
-                    }
-#pragma unroll
-                    for (int j = 0; j < kFewPieces; ++j) Mx = fmaxf(Mx, ml_[j].x);
-#pragma unroll
-                    for (int j = 0; j < kFewPieces; ++j) {
-                      const float e = Mx > -INFINITY ? ex2(ml_[j].x - Mx) : 0.f;
-                      ml_[j].y = __fmul_rn(e, ml_[j].y);
-                      v.x += e * w4[j].x; v.y += e * w4[j].y; v.z += e * w4[j].z; v.w += e * w4[j].w;
-                    }
-                    // (the order in which the warp above adds them: the same bits whichever form merges)
-#pragma unroll
-                    for (int d = kFewPieces / 2; d > 0; d >>= 1)
-#pragma unroll
-                      for (int j = 0; j < d; ++j) ml_[j].y = __fadd_rn(ml_[j].y, ml_[j + d].y);
-                    Ls = ml_[0].y;
-                  }
-                  const int Rg = it.mt * 16 + r, token = token_of(Rg), head = it.hk * rep + Rg - token * rep;
-                  const int64_t qi = it.q0 + token;
-                  float osc = 1.f;
-                  if (p.s_aux) {
-                    const float ys = p.s_aux[head] * kLog2e, mn = fmaxf(Mx, ys);
-                    osc = Mx == -INFINITY ? 0.f : ex2(Mx - mn);
-                    Ls = Ls * osc + ex2(ys - mn);
-                    Mx = mn;
-                  }
-                  const float inv = Ls > 0.f ? osc * vds / Ls : 0.f;
-                  T* op = reinterpret_cast<T*>(p.out) + qi * p.o_row_stride + (int64_t)head * p.o_head_stride + c4;
-                  uint2 w2;
-                  w2.x = pack2<T>(v.x * inv, v.y * inv);
-                  w2.y = pack2<T>(v.z * inv, v.w * inv);
-                  *reinterpret_cast<uint2*>(op) = w2;
-                  if (c4 == 0) p.lse[(int64_t)head * p.total_q + qi] = Ls > 0.f ? (Mx + lg2(Ls)) * kLn2 : -INFINITY;
-                }
+                if (tid % GPR == 0) reinterpret_cast<float2*>(p.part_ml)[slot * p.part_rows + ut * 16 + Rl] = make_float2(M, L);
               }
             }
           } else if (R < rows_total) {
@@ -1219,7 +1229,122 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
             }
           }
         }
-        if constexpr (BAL) clear();
+        }
+        if constexpr (BAL) {
+          if (is_piece) {
+          bar_consumers<NC>();       // (thread 0's fence then covers the rows of all four warps)
+          if (tid == 0) {
+            // (release: the rows of all four warps lie behind the barrier; acquire: the other pieces' rows)
+            unsigned* word = p.arrivals + cur.first;
+            const bool last = atomic_add_acq_rel(word, 1u) == (unsigned)cur.pieces - 1u;
+            if (last) *word = 0u;        // zero again for the next call
+            *s_last = last ? 1 : 0;
+          }
+          bar_consumers<NC>();
+          if (*s_last) {
+            // piece j lies in slot 2 (first + j) + (j == 0).  All threads over (row, 4 columns).  Few pieces: a thread
+            // loads the rows and their pairs together, one trip to L2.  Many: weights first, every pair loaded before any
+            // is used, then a warp per row and a lane per piece (the merge area is free: every warp has written its
+            // piece).  (With every thread reading many pairs by itself, one after the other, 148 pieces took some 20 us;
+            // a warp that took its rows one after the other waited for two trips per row, 6600 cycles for 16 rows.)
+            const int rows_total = it.seqlen_q * rep, np = cur.pieces;
+            const int all_live = min(p.part_rows, rows_total - it.mt * (16 * MT));
+            const int64_t s0 = (int64_t)cur.first * 2;
+            const float2* ml = reinterpret_cast<const float2*>(p.part_ml);
+            float2* pairs = reinterpret_cast<float2*>(s_o);      // (maximum, sum), then (weight, sum)
+            for (int r0 = 0; r0 < (MT > 1 ? all_live : 1); r0 += 16) {      // (a row tile at a time)
+            if (r0 > 0) bar_consumers<NC>();
+            const int live = MT > 1 ? min(16, all_live - r0) : all_live;
+            if (np > kFewPieces) {
+              for (int u = tid; u < live * np; u += NC * 32) {
+                const int j = u / live, r = u - j * live;
+                pairs[r * kMaxMerge + j] = __ldcg(ml + (s0 + 2 * j + (j == 0)) * p.part_rows + r0 + r);
+              }
+              bar_consumers<NC>();
+#pragma unroll 1
+              for (int r = warp; r < live; r += NC) {
+                float Mx = -INFINITY, Ls = 0.f;
+                for (int j = lane; j < np; j += 32) Mx = fmaxf(Mx, pairs[r * kMaxMerge + j].x);
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) Mx = fmaxf(Mx, __shfl_xor_sync(0xffffffffu, Mx, d));
+                for (int j = lane; j < np; j += 32) {
+                  const float2 q2 = pairs[r * kMaxMerge + j];
+                  const float e = Mx > -INFINITY ? ex2(q2.x - Mx) : 0.f;   // (a piece without visible keys: exactly 0, its rows are 0)
+                  pairs[r * kMaxMerge + j].x = e;
+                  Ls += e * q2.y;
+                }
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, d);
+                if (lane == 0) { s_m[r] = Mx; s_l[r] = Ls; }
+              }
+              bar_consumers<NC>();
+            }
+#pragma unroll 1
+            for (int u = tid; u < live * (HDV / 4); u += NC * 32) {
+              const int r = u / (HDV / 4), c4 = (u - r * (HDV / 4)) * 4;
+              const float* pr = p.part_o + (int64_t)(r0 + r) * HDV + c4;
+              float Mx, Ls;
+              float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (np > kFewPieces) {
+                Mx = s_m[r]; Ls = s_l[r];
+#pragma unroll 8
+                for (int j = 0; j < np; ++j) {
+                  const float4 w4 = __ldcg(reinterpret_cast<const float4*>(pr + (s0 + 2 * j + (j == 0)) * p.part_rows * HDV));
+                  const float e = pairs[r * kMaxMerge + j].x;
+                  v.x += e * w4.x; v.y += e * w4.y; v.z += e * w4.z; v.w += e * w4.w;
+                }
+              } else {
+                float2 ml_[kFewPieces];
+                float4 w4[kFewPieces];
+                Mx = -INFINITY;
+#pragma unroll
+                for (int j = 0; j < kFewPieces; ++j) {
+                  ml_[j] = make_float2(-INFINITY, 0.f);
+                  w4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                  if (j < np) {
+                    const int64_t slot = (s0 + 2 * j + (j == 0)) * p.part_rows;
+                    ml_[j] = __ldcg(ml + slot + r0 + r);
+                    w4[j] = __ldcg(reinterpret_cast<const float4*>(pr + slot * HDV));
+                  }
+                }
+#pragma unroll
+                for (int j = 0; j < kFewPieces; ++j) Mx = fmaxf(Mx, ml_[j].x);
+#pragma unroll
+                for (int j = 0; j < kFewPieces; ++j) {
+                  const float e = Mx > -INFINITY ? ex2(ml_[j].x - Mx) : 0.f;
+                  ml_[j].y = __fmul_rn(e, ml_[j].y);
+                  v.x += e * w4[j].x; v.y += e * w4[j].y; v.z += e * w4[j].z; v.w += e * w4[j].w;
+                }
+                // (the order in which the warp above adds them: the same bits whichever form merges)
+#pragma unroll
+                for (int d = kFewPieces / 2; d > 0; d >>= 1)
+#pragma unroll
+                  for (int j = 0; j < d; ++j) ml_[j].y = __fadd_rn(ml_[j].y, ml_[j + d].y);
+                Ls = ml_[0].y;
+              }
+              const int Rg = it.mt * (16 * MT) + r0 + r, token = token_of(Rg), head = it.hk * rep + Rg - token * rep;
+              const int64_t qi = it.q0 + token;
+              float osc = 1.f;
+              if (p.s_aux) {
+                const float ys = p.s_aux[head] * kLog2e, mn = fmaxf(Mx, ys);
+                osc = Mx == -INFINITY ? 0.f : ex2(Mx - mn);
+                Ls = Ls * osc + ex2(ys - mn);
+                Mx = mn;
+              }
+              const float inv = Ls > 0.f ? osc * vds / Ls : 0.f;
+              T* op = reinterpret_cast<T*>(p.out) + qi * p.o_row_stride + (int64_t)head * p.o_head_stride + c4;
+              uint2 w2;
+              w2.x = pack2<T>(v.x * inv, v.y * inv);
+              w2.y = pack2<T>(v.z * inv, v.w * inv);
+              *reinterpret_cast<uint2*>(op) = w2;
+              if (c4 == 0) p.lse[(int64_t)head * p.total_q + qi] = Ls > 0.f ? (Mx + lg2(Ls)) * kLn2 : -INFINITY;
+            }
+            }
+          }
+          }
+        }
+        if constexpr (BAL && !SM::kQShared) clear();
+        else if constexpr (BAL) clear_o();
         bar_consumers<NC>();   // the scratch area is free again
         if constexpr (BAL) {
           if (lane == 0) mbar_arrive(bar_pc_empty + 8 * (pcnt % kPieces));
@@ -1275,9 +1400,9 @@ static int line_team(int hkv, int ctas) {
   return team;
 }
 
-template <typename T, bool KV8, int NST, int HD, int HDV, bool BAL, int CPS>
-static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaStream_t stream) {
-  using SM = Smem<KV8 ? 1 : 2, NST, HD, HDV>;
+template <typename T, bool KV8, int NST, int HD, int HDV, bool BAL, int CPS, int MT>
+static int launch_tiles(const KParams& kp, const Plan& pl, int num_work_slots, cudaStream_t stream) {
+  using SM = Smem<KV8 ? 1 : 2, NST, HD, HDV, MT>;
   DecArgs a;
   a.kp = kp;
   a.total_work = num_work_slots * kp.hkv * kp.nsplits;
@@ -1299,7 +1424,7 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
   CUtensorMap mk, mv;
   if (!make_map(&mk, kp.k, kvdt, rows, (uint64_t)kp.hkv * HD, (uint64_t)kp.k_row_stride, a.box_rows)) return -1;
   if (!make_map(&mv, kp.v, kvdt, rows, (uint64_t)kp.hkv * HDV, (uint64_t)kp.v_row_stride, a.box_rows)) return -1;
-  auto kern = fwd_decode_kernel<T, KV8, NST, HD, HDV, CPS, BAL>;
+  auto kern = fwd_decode_kernel<T, KV8, NST, HD, HDV, CPS, BAL, MT>;
   const int smem = (BAL ? SM::kBytesBalanced : SM::kBytes) + 1024;
   static std::atomic<unsigned long long> attr_done{0};   // one bit per device
   int dev = 0;
@@ -1320,6 +1445,14 @@ static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaS
   }
   if (grid <= 0) return 0;
   return launch_overlapped(kern, grid, (SM::NC + 1) * 32, smem, stream, a, mk, mv);
+}
+
+template <typename T, bool KV8, int NST, int HD, int HDV, bool BAL, int CPS>
+static int launch_t(const KParams& kp, const Plan& pl, int num_work_slots, cudaStream_t stream) {
+  if constexpr (!KV8) {
+    if (pl.tile_m == 32) return launch_tiles<T, KV8, NST, HD, HDV, BAL, CPS, 2>(kp, pl, num_work_slots, stream);
+  }
+  return launch_tiles<T, KV8, NST, HD, HDV, BAL, CPS, 1>(kp, pl, num_work_slots, stream);
 }
 
 }  // namespace dec

@@ -148,6 +148,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int x
       : "memory");
 }
 
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
 // 3-D tiled store shared -> global (bulk async group of the issuing thread).  x * elem_size must be a multiple of
 // 16 bytes and no coordinate may be negative; elements outside the tensor are not written.
 __device__ __forceinline__ void tma_store_3d(const void* map, uint32_t src, int x, int y, int z) {
