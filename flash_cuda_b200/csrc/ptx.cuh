@@ -156,6 +156,13 @@ __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
+// 32 bytes to a 32-byte aligned address: one store of a whole sector (sm_100)
+__device__ __forceinline__ void st_global_32(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f,
+                                             uint32_t g, uint32_t h) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h) : "memory");
+}
+
 // 3-D tiled store shared -> global (bulk async group of the issuing thread).  x * elem_size must be a multiple of
 // 16 bytes and no coordinate may be negative; elements outside the tensor are not written.
 __device__ __forceinline__ void tma_store_3d(const void* map, uint32_t src, int x, int y, int z) {
