@@ -335,7 +335,7 @@ static WidenPlan widen_plan(const FaFwdParams* p, const PlanInput& in, const Pla
 // 8 parts 224), since every part pays for filling its pipeline and for its fp32 rows.  `classed`: the short sequences of
 // the batch are another kernel's.
 static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, bool classed) {
-  TcCut t{1, 0, 0};
+  TcCut t{1, 0, 0, 1, 1, 1};
   if (pl.route != FA_ROUTE_PREFILL_TC || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 || p->total_q <= 0) return t;
   if (p->hdv % 4 || (long long)p->hq * p->hdv > (1ll << 25)) return t;
   if ((long long)p->batch * p->hq * pl.max_mtiles * 16 > 0x7fffffff) return t;
@@ -347,9 +347,14 @@ static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, b
     if (n_long < seqs) { rows -= seqs - n_long; seqs = n_long; }
   }
   const long long per_seq = (rows + seqs - 1) / seqs, n = p->hq * seqs * ((per_seq + pl.tile_m - 1) / pl.tile_m);
-  long long most = pl.num_sms / n;
-  if (most > 16) most = 16;
-  if (most < 2) return t;
+  const long long spare = n > 0 ? pl.num_sms % n : 0;      // SMs that equal parts leave idle
+  long long even = pl.num_sms / n;
+  if (even < 1) return t;
+  if (even > 16) even = 16;
+  // (512 rows over 24500 keys, 64 items: leads of 4 / 9, tails of 1 / 9; us without / with tails, sustained and in a burst: 201.6 / 200.8, 182.5 /
+  // 181.9; 96 items over 12000 keys 166.7 / 150.5; 40 over 20000 108.0 / 102.4; 128 of head_dim 192 over 32768 719.6 / 698.0, 710 / 663)
+  const bool tails = even < 16 && spare > 0;
+  if (even < 2 && !tails) return t;
   // (max_seqlen_k may be a loose bound: a packed K/V says how many keys a sequence has on average; the kernel cuts an
   // item by its true keys)
   double keys = p->max_seqlen_k;
@@ -364,9 +369,17 @@ static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, b
   t.block_ns = (int)(1800.0 * (p->hd + p->hdv) / 256.0 * pl.tile_m / 256.0);
   t.part_ns = (int)((double)rows * p->hq * p->hdv * 8.0 / 4.0e3);
   const size_t part_bytes = (size_t)p->total_q * p->hq * (p->hdv + 1) * 4;
-  while (most > 1 && most * part_bytes > ((size_t)128 << 20)) --most;
-  t.most = (int)most;
-  t.most = tc_item_parts((int)blocks, t);
+  while (even > 1 && even * part_bytes > ((size_t)128 << 20)) --even;
+  t.even = t.most = (int)even;
+  if (tails && even == pl.num_sms / n && (even + 1) * part_bytes <= ((size_t)128 << 20)) {
+    // each idle SM takes `per` tails one after the other while the others run one leading part
+    const long long per = (n + spare - 1) / spare;
+    t.most = (int)even + 1;
+    t.lead_num = (int)per;
+    t.lead_den = (int)(per * even + 1);
+  }
+  const int parts = tc_item_parts((int)blocks, t);
+  if (parts <= t.even) { t.most = parts; t.even = parts < t.even ? parts : t.even; }
   return t;
 }
 
@@ -408,7 +421,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = fal
     w.o_bytes = align_up((size_t)nsplits * p->total_q * p->hq * p->hdv * 4, 256);
     off += w.o_bytes;
   };
-  w.cut = TcCut{1, 0, 0};
+  w.cut = TcCut{1, 0, 0, 1, 1, 1};
   if (pl.route == FA_ROUTE_GENERAL && !plain) {
     const PlanInput in = plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0));
     w.widen = widen_plan(p, in, pl);
@@ -643,7 +656,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   kp.q_fp8 = p->q_dtype == FA_DT_FP8_E4M3; kp.kv_fp8 = p->kv_dtype == FA_DT_FP8_E4M3;
   kp.is_causal = in.is_causal; kp.window_left = in.window_left; kp.window_right = in.window_right;
   kp.nsplits = pl.nsplits;
-  kp.tc_cut = TcCut{1, 0, 0};
+  kp.tc_cut = TcCut{1, 0, 0, 1, 1, 1};
   kp.out_f32 = p->out_dtype == FA_DT_FP32;
   kp.work_expect = SchedExpect{p->batch, pl.nsplits, pl.tile_m, pl.tile_n, pl.max_mtiles, pl.rows_per_token, pl.route};
   kp.scale = p->softmax_scale; kp.softcap = p->softcap;

@@ -17,19 +17,29 @@ constexpr int kWsArrivalOff = 256;
 constexpr int kWsArrivalWords = (kWsHeader - kWsArrivalOff) / 4;
 constexpr int kBalancedEntriesMax = 2048;   // (sequence, row tile) entries a balanced decode call may have
 
-// Tensor-core prefill in key-range parts: into how many parts (at most `most`) an item of that many key blocks is cut.
-// The least of blocks / c blocks of block_ns each plus what c parts cost: 5.5 us, and part_ns for writing one as fp32
-// and reading it back; uncut where that saves less than a tenth.  Asked on the host with what it knows of the key count,
+// Tensor-core prefill in key-range parts: into how many parts an item of that many key blocks is cut.  Either up to `even` equal ones,
+// or `even` of lead_num / lead_den of the item each and a shorter one, the tail (even + 1 parts): equal parts leave SMs idle
+// unless the items divide their number, and several tails after one another are what those SMs are given.  The least of the blocks of the
+// longest part, block_ns each, plus what parts cost: 5.5 us, and part_ns for writing one as fp32 and reading it back; uncut where
+// that saves less than a tenth (a twentieth by tails).  Asked on the host with what it knows of the key count,
 // which may be no more than a loose bound, and on the device with the true range, by the attention kernel and the merge
 // behind it: integers, so that both get the same answer.
-struct TcCut { int most, block_ns, part_ns; };
+struct TcCut { int most, block_ns, part_ns, even, lead_num, lead_den; };      // most: parts at most, even or even + 1
+__host__ __device__ inline int tc_lead_blocks(int blocks, const TcCut& t) {
+  return (int)(((long long)blocks * t.lead_num + t.lead_den - 1) / t.lead_den);
+}
 __host__ __device__ inline int tc_item_parts(int blocks, const TcCut& t) {
   const long long whole = (long long)blocks * t.block_ns;
   long long best = whole * 9 / 10;
   int parts = 1;
-  for (int c = 2; c <= t.most && c * 2 <= blocks; ++c) {
+  for (int c = 2; c <= t.even && c * 2 <= blocks; ++c) {
     const long long cost = whole / c + 5500 + (long long)c * t.part_ns;
     if (cost < best) { best = cost; parts = c; }
+  }
+  if (t.most > t.even && t.most * 4 <= blocks) {
+    const int lead = tc_lead_blocks(blocks, t);
+    const long long cost = (long long)lead * t.block_ns + 5500 + (long long)t.most * t.part_ns;
+    if (cost < (parts > 1 ? best : whole * 19 / 20) && lead * t.even < blocks) parts = t.most;
   }
   return parts;
 }
@@ -131,6 +141,14 @@ __host__ __device__ inline void split_range(int lo, int hi, int s, int nsplits, 
   int a = lo + s * per, b = lo + (s + 1) * per;
   *slo = a < hi ? a : hi;
   *shi = b < hi ? b : hi;
+}
+
+// Part `part` of `parts` of an item's key blocks [lo, hi).
+__host__ __device__ inline void tc_part_range(int lo, int hi, int part, int parts, const TcCut& t, int* plo, int* phi) {
+  if (parts <= t.even) { split_range(lo, hi, part, parts, plo, phi); return; }
+  const int lead = tc_lead_blocks(hi - lo, t);
+  *plo = lo + part * lead;
+  *phi = part < t.even ? *plo + lead : hi;
 }
 
 // Launch of a kernel that may start while its predecessor in the stream still runs (see wait_for_predecessors in ptx.cuh):

@@ -212,7 +212,7 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
       it.h |= kWhole << kPartShift;
     } else {
       int plo, phi;
-      split_range(it.ulo, it.uhi, part, parts, &plo, &phi);
+      tc_part_range(it.ulo, it.uhi, part, parts, p.tc_cut, &plo, &phi);
       it.ulo = 0x7fffffff;
       it.uhi = 0;
 #pragma unroll

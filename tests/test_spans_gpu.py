@@ -130,3 +130,30 @@ def test_wide_queries_over_more_keys_than_the_slabs_hold(cuda_device):
     torch.testing.assert_close(lse, gen_lse, atol=1e-3, rtol=1e-4)
 
 
+
+
+TAILS = {    # items that do not divide the SMs: leading parts and a shorter one.  One, two and nine leads (by 148 SMs).
+    "one_lead": ([(700, 6000)], dict(hq=32, hkv=8, hd=128, page_size=64)),
+    "two_leads": ([(260, 7000), (200, 6500)], dict(hq=20, hkv=4, hd=128, page_size=16, sink=True)),
+    "nine_leads": ([(300, 20000)], dict(hq=8, hkv=2, hd=64, page_size=0)),
+    "hd192": ([(500, 7000)], dict(hq=24, hkv=24, hd=192, hdv=128, page_size=64, leftpad=[100])),
+    "window": ([(640, 9000)], dict(hq=32, hkv=4, hd=128, page_size=128, window_left=7000)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(TAILS))
+def test_prefill_with_tails(name, cuda_device):
+    """The whole call against the uncut form, every 37th row of two heads against the oracle."""
+    reqs, kw = TAILS[name]
+    p = W.make_problem("tails_" + name, reqs, dtype="bf16", seed=95, **kw)
+    out, lse = _run(p, cuda_device, 2e-2, check_ref=False)
+    whole, whole_lse = _run(p, cuda_device, 2e-2, check_ref=False, num_splits=1)
+    assert not torch.equal(lse, whole_lse)                     # the call was cut
+    assert (out.float() - whole.float()).abs().max().item() <= 2 ** -7
+    torch.testing.assert_close(lse, whole_lse, atol=1e-4, rtol=1e-5)
+    again, again_lse = _run(p, cuda_device, 2e-2, check_ref=False)
+    assert torch.equal(out, again) and torch.equal(lse, again_lse)
+    rows, heads = list(range(0, p.q.shape[0], 37)), [0, p.q.shape[1] - 1]
+    want, want_lse = ref_attention(p.q, p.k, p.v, q_rows=rows, heads=heads, **p.oracle_kw())
+    assert (out.float().cpu() - want)[rows][:, heads].abs().max().item() <= 2e-2
+    torch.testing.assert_close(lse.cpu()[heads][:, rows], want_lse[heads][:, rows], atol=5e-3, rtol=1e-2)
