@@ -38,12 +38,15 @@ constexpr float kLn2 = 0.6931471805599453f;
 constexpr int kPieces = 4;             // mailbox slots between the producer and the consumers
 // Balanced kernels, see LineCut (key blocks, about 0.65 us each with all SMs busy):
 // (an e4m3 cache: a stage holds two blocks and a block passes in half the time, so cuts are dearer in blocks; with
-// pieces of 2 blocks and 63 of them a head over 5000 / 20000 keys took 25 / 36 us against 19 / 28 as split work items)
+// pieces of 2 blocks and 63 of them a head over 5000 / 20000 keys took 25 / 36 us against 19 / 28 as split work items).  Again with 128-key
+// stages, a short start and short merges, us in a graph: a cut over e4m3 at 6 blocks instead of 10, 5 sequences of 100 .. 900 keys 15.1 ->
+// 11.5, 24 of 500 .. 3000 30.4 -> 28.9; borders that move by 4 blocks instead of 8, 14 of 1000 .. 8000 e4m3 37.6 -> 36.6, bf16 53.1 -> 51.8; pieces
+// of 2 over e4m3 (3 of 2000 12.5 -> 13.9), kCrossCost of 6 (6 of 700 .. 9000 29.2 -> 32.3) and more pieces (1 of 9000 15.3 -> 16.0) lose.
 constexpr int min_span(bool kv8) { return kv8 ? 4 : 2; }       // a piece has at least so many
-constexpr int cut_cost(bool kv8) { return kv8 ? 10 : 6; }      // what cutting a triple costs the CTAs that share it: rows out, fence, atomic, merge
+constexpr int kCutCost = 6;            // what cutting a triple costs the CTAs that share it: rows out, fence, atomic, merge
 constexpr int max_pieces(bool kv8) { return kv8 ? 24 : 64; }   // pieces of a triple at most ...
 constexpr int kCrossCost = 12;         // what a CTA pays for a span that begins and ends inside triples
-constexpr int kSnap = 8;               // a span border this close to the end of a triple moves there
+constexpr int kSnap = 4;               // a span border this close to the end of a triple moves there
 constexpr int kMaxLinePieces = 96;     // ... and where spans cross sequences (what one CTA merges)
 constexpr int kMaxMerge = 104;         // (those, and a few more where borders moved)
 constexpr int kFewPieces = 8;          // ... of which a thread loads so many at once
@@ -151,7 +154,7 @@ __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
 //
 // Where the line is cut.  Only the kernel knows the lengths, so every CTA plans the same from them:
 //   - no more (row tile, head group) triples than teams: each triple gets teams of its own, ceil(blocks / width) of them
-//     with the smallest width that the teams suffice for, unless that saves less than the cut costs (cut_cost: nothing
+//     with the smallest width that the teams suffice for, unless that saves less than the cut costs (kCutCost: nothing
 //     of up to 8 blocks is cut).  No CTA then works on two triples: with equal spans over the line two sequences of 300
 //     keys took 17.7 us, since nearly every CTA had two halves to open, write out and merge.
 //   - otherwise, or where the lengths are so uneven that this leaves the longest piece above the line's mean by more than
@@ -391,7 +394,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
       for (int i = 0; i < kPieces; ++i) { mbar_init(bar_pc_full + 8 * i, 1); mbar_init(bar_pc_empty + 8 * i, NC); }
       mbar_fence_init();
     }
-    constexpr int kMinSpan = min_span(KV8), kCutCost = cut_cost(KV8), kMaxPieces = max_pieces(KV8);
+    constexpr int kMinSpan = min_span(KV8), kMaxPieces = max_pieces(KV8);
     // ---- lengths: consecutive entries per thread; their sum, number and maximum ----
     constexpr int NTH = (NC + 1) * 32;
     static_assert(NC + 1 < 15, "words of the warps");
@@ -1127,7 +1130,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         // ---- merge the four warps' partial results and write the output rows, a row tile at a time ----
         bool is_piece = false;
         if constexpr (BAL) is_piece = cur.pieces > 1;
-#pragma unroll SM::TW > 1 ? 1 : MT
+#pragma unroll SM::TW > 1 ? 1 : 2
         for (int ut = 0; ut < MT; ++ut) {
           const int u = SM::TW > 1 ? 0 : ut;      // (this warp's own number of the tile)
         if (ut > 0) bar_consumers<NC>();      // (the tile before has left the merge area)
