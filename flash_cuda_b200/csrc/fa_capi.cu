@@ -28,6 +28,7 @@ int launch_decode(const KParams& kp, const Plan& pl, int compute_dtype, cudaStre
 int launch_prefill_tc(const KParams& kp, const Plan& pl, int compute_dtype, cudaStream_t stream);
 bool prefill_tc_supported(const PlanInput& in);
 bool prefill_tc_single_tile(int hd, int hdv);
+bool tc_shared_supported(const PlanInput& in);
 bool decode_supported(const PlanInput& in);
 int decode_line_ctas(int hd, int kv_dtype, int num_sms);
 bool prefill_tc_layout_ok(const FaFwdParams* p);
@@ -334,8 +335,8 @@ static WidenPlan widen_plan(const FaFwdParams* p, const PlanInput& in, const Pla
 // wave of shorter parts lost what it was to balance (those 64 items: whole 322 us, 2 parts 191, 3 parts 251, 4 parts 201,
 // 8 parts 224), since every part pays for filling its pipeline and for its fp32 rows.  `classed`: the short sequences of
 // the batch are another kernel's.
-static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, bool classed) {
-  TcCut t{1, 0, 0, 1, 1, 1};
+static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, bool classed, bool listed) {
+  TcCut t = kTcUncut;
   if (pl.route != FA_ROUTE_PREFILL_TC || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 || p->total_q <= 0) return t;
   if (p->hdv % 4 || (long long)p->hq * p->hdv > (1ll << 25)) return t;
   if ((long long)p->batch * p->hq * pl.max_mtiles * 16 > 0x7fffffff) return t;
@@ -353,7 +354,7 @@ static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, b
   if (even > 16) even = 16;
   // (512 rows over 24500 keys, 64 items: leads of 4 / 9, tails of 1 / 9; us without / with tails, sustained and in a burst: 201.6 / 200.8, 182.5 /
   // 181.9; 96 items over 12000 keys 166.7 / 150.5; 40 over 20000 108.0 / 102.4; 128 of head_dim 192 over 32768 719.6 / 698.0, 710 / 663)
-  const bool tails = even < 16 && spare > 0;
+  const bool tails = even < 16 && spare > 0 && pl.num_sms < 255;
   if (even < 2 && !tails) return t;
   // (max_seqlen_k may be a loose bound: a packed K/V says how many keys a sequence has on average; the kernel cuts an
   // item by its true keys)
@@ -361,25 +362,49 @@ static TcCut tc_cut(const FaFwdParams* p, const PlanInput& in, const Plan& pl, b
   if (!p->page_table && (double)p->total_k / p->batch < keys) keys = (double)p->total_k / p->batch;
   if (p->page_table && (double)p->num_pages * p->page_size < keys) keys = (double)p->num_pages * p->page_size;
   double blocks = (keys - (in.is_causal ? 0.5 * (p->max_seqlen_q < keys ? p->max_seqlen_q : keys) : 0.0)) / 128.0;
+  double longest = keys / 128.0;      // blocks of the item that sees most
   if (in.window_left >= 0 && (in.is_causal || in.window_right >= 0)) {
     const double w = (in.window_left + (in.window_right > 0 ? in.window_right : 0) + pl.tile_m) / 128.0 + 1.0;
     if (w < blocks) blocks = w;
+    if (w < longest) longest = w;
   }
   // 1.8 us per key block of 2 x 128 rows at 256 columns; 8 bytes per row and column of a part through memory
-  t.block_ns = (int)(1800.0 * (p->hd + p->hdv) / 256.0 * pl.tile_m / 256.0);
-  t.part_ns = (int)((double)rows * p->hq * p->hdv * 8.0 / 4.0e3);
+  t.block_ns = (uint16_t)(1800.0 * (p->hd + p->hdv) / 256.0 * pl.tile_m / 256.0);
+  t.part_ns = (int32_t)((double)rows * p->hq * p->hdv * 8.0 / 4.0e3);
   const size_t part_bytes = (size_t)p->total_q * p->hq * (p->hdv + 1) * 4;
   while (even > 1 && even * part_bytes > ((size_t)128 << 20)) --even;
-  t.even = t.most = (int)even;
+  t.even = t.most = (uint8_t)even;
   if (tails && even == pl.num_sms / n && (even + 1) * part_bytes <= ((size_t)128 << 20)) {
     // each idle SM takes `per` tails one after the other while the others run one leading part
     const long long per = (n + spare - 1) / spare;
-    t.most = (int)even + 1;
-    t.lead_num = (int)per;
-    t.lead_den = (int)(per * even + 1);
+    t.most = (uint8_t)(even + 1);
+    t.lead_num = (uint8_t)per;          // (n * even SMs at most, and per <= n)
+    t.lead_den = (uint8_t)(per * even + 1);
   }
   const int parts = tc_item_parts((int)blocks, t);
-  if (parts <= t.even) { t.most = parts; t.even = parts < t.even ? parts : t.even; }
+  // Items of 128 rows whose key blocks the two tiles of the kernel share: half of the longest item's blocks one after the other, and
+  // nothing to merge through memory.  A block then serves 128 rows instead of 256, so the pace is that of its loads: 15 % slower
+  // over contiguous K/V, 30 % over pages of 128 keys and more.  Over pages of 64 (twice the copies) it is 75 % slower, over smaller ones that
+  // stay where they are more: not taken there.  Whole or in parts / shared, us in a graph: 2 x 512 rows x 8 heads 12.9 / 10.3, 512 rows x 32 heads causal 13.7 / 11.4, 2300 rows
+  // x 8 heads 35.0 / 22.7, 512 rows over 3000 keys 40.1 / 27.9 (pages of 128 41.4 / 33.1, of 64 43.4 / 42.3), 500 over 8000 74.6 / 70.2 (75 / 77, 81 / 101),
+  // 512 over 24500 195.6 / 201 (pages of 64 199 / 291).
+  const long long tiles = p->hq * seqs * ((per_seq + 127) / 128);
+  if (!listed && tiles <= pl.num_sms && tc_shared_supported(in)) {
+    size_t kb, vb;
+    int kpad;
+    const bool packed = !p->page_table || depage_plan(p, pl, &kpad, &kb, &vb);
+    const int pace = packed ? 115 : p->page_size >= 128 ? 130 : 0, n_longest = (int)(longest + 0.99);
+    const long long half = (long long)((n_longest + 1) / 2) * t.block_ns * pace / 100 + 700;
+    const long long other = parts <= 1        ? (long long)n_longest * t.block_ns
+                            : parts <= t.even ? (long long)n_longest * t.block_ns / parts + 5500 + (long long)parts * t.part_ns
+                                              : (long long)tc_lead_blocks(n_longest, t) * t.block_ns + 5500 + (long long)parts * t.part_ns;
+    if (pace && half < other) {
+      t.most = t.even = 1;
+      t.shared = 1;
+      return t;
+    }
+  }
+  if (parts <= t.even) t.most = t.even = (uint8_t)parts;
   return t;
 }
 
@@ -421,7 +446,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = fal
     w.o_bytes = align_up((size_t)nsplits * p->total_q * p->hq * p->hdv * 4, 256);
     off += w.o_bytes;
   };
-  w.cut = TcCut{1, 0, 0, 1, 1, 1};
+  w.cut = kTcUncut;
   if (pl.route == FA_ROUTE_GENERAL && !plain) {
     const PlanInput in = plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0));
     w.widen = widen_plan(p, in, pl);
@@ -436,7 +461,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = fal
       w.work2_bytes = align_up((size_t)sched_len(w.widen.tc, p->batch) * 4, 256);
       off += w.work2_bytes;
       if (w.widen.class_rows > 0) carve_parts(decode_part_plan(in, pl));
-      w.cut = tc_cut(p, in, w.widen.tc, w.widen.class_rows > 0);
+      w.cut = tc_cut(p, in, w.widen.tc, w.widen.class_rows > 0, true);
       if (w.cut.most > 1) carve_splits(w.cut.most);
       w.wd_k_off = off;
       off += align_up((size_t)w.widen.cap_rows * p->hkv * p->hd * 2, 256);
@@ -487,7 +512,7 @@ static WsLayout ws_layout(const FaFwdParams* p, const Plan& pl, bool plain = fal
     }
   }
   if (pl.route == FA_ROUTE_PREFILL_TC && !plain)
-    w.cut = tc_cut(p, plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0)), pl, w.work2_bytes > 0);
+    w.cut = tc_cut(p, plan_input(p, pl.num_sms + (p->sm_margin > 0 ? p->sm_margin : 0)), pl, w.work2_bytes > 0, w.work2_bytes > 0 || p->scheduler_metadata != nullptr);
   if (pl.nsplits > 1 || w.cut.most > 1) carve_splits(pl.nsplits > 1 ? pl.nsplits : w.cut.most);
   w.total = off;
   return w;
@@ -656,7 +681,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   kp.q_fp8 = p->q_dtype == FA_DT_FP8_E4M3; kp.kv_fp8 = p->kv_dtype == FA_DT_FP8_E4M3;
   kp.is_causal = in.is_causal; kp.window_left = in.window_left; kp.window_right = in.window_right;
   kp.nsplits = pl.nsplits;
-  kp.tc_cut = TcCut{1, 0, 0, 1, 1, 1};
+  kp.tc_cut = kTcUncut;
   kp.out_f32 = p->out_dtype == FA_DT_FP32;
   kp.work_expect = SchedExpect{p->batch, pl.nsplits, pl.tile_m, pl.tile_n, pl.max_mtiles, pl.rows_per_token, pl.route};
   kp.scale = p->softmax_scale; kp.softcap = p->softcap;
@@ -678,8 +703,8 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   // the tensor-core kernel over `kt`, in key-range parts with their merge where the plan says so; `class_rows` and `skip`
   // say which sequences are other kernels'
   auto run_prefill = [&](KParams kt, const Plan& plt, int class_rows, const int32_t* skip) -> int {
+    kt.tc_cut = w.cut;
     if (w.cut.most > 1) {
-      kt.tc_cut = w.cut;
       kt.whole_out = kt.out; kt.whole_lse = kt.lse; kt.whole_s_aux = kt.s_aux;
       kt.whole_row_stride = kt.o_row_stride; kt.whole_head_stride = kt.o_head_stride;
       kt.out = ws + w.o_off; kt.lse = (float*)(ws + w.lse_off); kt.out_f32 = 1; kt.s_aux = nullptr;

@@ -24,7 +24,15 @@ constexpr int kBalancedEntriesMax = 2048;   // (sequence, row tile) entries a ba
 // that saves less than a tenth (a twentieth by tails).  Asked on the host with what it knows of the key count,
 // which may be no more than a loose bound, and on the device with the true range, by the attention kernel and the merge
 // behind it: integers, so that both get the same answer.
-struct TcCut { int most, block_ns, part_ns, even, lead_num, lead_den; };      // most: parts at most, even or even + 1
+// (12 bytes: with 28 the decode kernel's parameters passed 768 bytes, and calls of 9 us took 0.15 us longer)
+struct TcCut {
+  int32_t part_ns;
+  uint16_t block_ns;
+  uint8_t most, even;               // parts at most: even or even + 1
+  uint8_t lead_num, lead_den;       // both at most the number of SMs and one
+  uint8_t shared;                   // no parts: items of 128 rows whose key blocks the two tiles of the kernel share
+};
+constexpr TcCut kTcUncut{0, 0, 1, 1, 1, 1, 0};
 __host__ __device__ inline int tc_lead_blocks(int blocks, const TcCut& t) {
   return (int)(((long long)blocks * t.lead_num + t.lead_den - 1) / t.lead_den);
 }

@@ -132,9 +132,9 @@ struct alignas(16) Item {
 static_assert(sizeof(Item) == 64, "mailbox slot");
 constexpr int kPartShift = 24, kHeadMask = (1 << kPartShift) - 1, kWhole = 127;
 
-template <int NTL, bool PARTS>
+template <int NTL, bool PARTS, bool KS>
 __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_entry) {
-  constexpr int kItemRows = NTL * TM;
+  constexpr int kItemRows = KS ? TM : NTL * TM;
   const KParams& p = a.kp;
   Item it;
   it.w = w;
@@ -195,7 +195,7 @@ __device__ __forceinline__ Item decode_item(const TcArgs& a, int w, bool* bad_en
   it.uhi = 0;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int row0 = it.pair * kItemRows + t * TM;
+    const int row0 = it.pair * kItemRows + (KS ? 0 : t * TM);      // (KS: both tiles are the same rows)
     it.lo[t] = it.hi[t] = 0;
     if (it.valid && row0 < it.seqlen_q && t < NTL) {
       const int rmax = min(it.seqlen_q - 1, row0 + TM - 1);
@@ -356,7 +356,10 @@ __device__ __forceinline__ void copy_tile_rows(uint32_t dst0, const unsigned cha
 // PROD: the form of the TMA producer: 0 = contiguous K/V, lane 0 alone; 1 = paged, lane 0 alone; 2 = paged, the whole
 // warp (see the TMA role).  Template arguments rather than run-time flags for the same reason as CAP: code that a
 // launch never runs still moved the time of the code it does run by a few per cent.
-template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD, bool PARTS>
+// KS: an item is one tile of 128 rows, and the two tiles of the kernel share its key blocks, the even ones and the odd ones, each with a softmax
+// and an accumulator of its own, merged at the end in registers.  Where items are few the time of a call is the chain of blocks of one
+// item, which this halves: see tc_cut for when.
+template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD, bool PARTS, bool KS>
 __global__ void __launch_bounds__(NTHREADS, 1)
 fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -404,6 +407,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
   // PV -> QK -> softmax -> PV to max(PV -> load of the single V stage, softmax) -> PV.  Buffers alternate block by
   // block across items; buffer b has s_full / p_full barrier b (the second tile's, unused in these kernels).
   constexpr bool SDB = NTL == 1;
+  static_assert(!KS || (NTL == 2 && MERGE_KV && !CAP && !PARTS && !F8), "the form with shared key blocks");
+  constexpr int kItemRows = KS ? TM : NTL * TM;
   constexpr uint32_t S1_COL = 384;                       // second S buffer: behind O (128 + up to 256 columns)
   static_assert(!SDB || NTL * TN + HDV <= S1_COL, "O must end before the second S buffer");
   Item* s_item = reinterpret_cast<Item*>(sm + SM::kItemOff);   // [2]
@@ -413,7 +418,8 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    for (int t = 0; t < 2; ++t) { mbar_init(bar_q_full + 8 * t, 1); mbar_init(bar_q_empty + 8 * t, 1); }
+    // (KS: the pair of tile 1 guards the maxima and sums that its warps hand to those of tile 0, in its Q buffer)
+    for (int t = 0; t < 2; ++t) { mbar_init(bar_q_full + 8 * t, KS && t ? 4 : 1); mbar_init(bar_q_empty + 8 * t, KS && t ? 4 : 1); }
     for (int s = 0; s < KST; ++s) mbar_init(bar_k_empty + 8 * s, 1);
     // (rows copied with cp.async: a tile completes on one arrival per producer lane when its copies have landed, plus
     // lane 0's own)
@@ -502,7 +508,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
             first_ticket = false;
             if (w >= num_items) { it.w = kEndOfWork; break; }
             bool bad = false;
-            it = decode_item<NTL, PARTS>(a, w, &bad);   // sequence bounds are read from global memory once per item
+            it = decode_item<NTL, PARTS, KS>(a, w, &bad);   // sequence bounds are read from global memory once per item
             if (bad) { report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_TMA); num_items = 0; it.w = kEndOfWork; break; }
             if (it.valid) break;
           }
@@ -535,7 +541,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
 #pragma unroll
             for (int cb = 0; cb < HD / EPB; ++cb)
               tma_load_3d(sQ + t * (TM * HD * ESZ) + cb * (TM * 128), &map_q, cb * EPB, PARTS ? it.h & kHeadMask : it.h,
-                          it.q0 + it.pair * (NTL * TM) + t * TM, bar_q_full + 8 * t);
+                          it.q0 + it.pair * kItemRows + t * TM, bar_q_full + 8 * t);
           }
           return true;
         };
@@ -570,6 +576,54 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         };
         // K of the first block has a barrier of its own; every later K tile arrives together with the V tile of
         // the block before it (the MMA warp needs both at the same point), so the consumer waits once per block
+        if constexpr (KS) {
+          // K of the first two blocks together, then V of a block with K of the block two behind it, whose QK follows its PV
+          // (pool rows three blocks ahead: a block's loads have half the time that they have where both tiles work on it)
+          PageRows r0 = {{0, 0, 0, 0}}, r1 = r0, r2 = r0, r3 = r0;
+          const bool two = it.ulo + 1 < it.uhi;
+          if (paged) {
+            r0 = page_rows(a, it.ulo, it.b, it.seqlen_k, lane, pj0, pjs);
+            if (two) r1 = page_rows(a, it.ulo + 1, it.b, it.seqlen_k, lane, pj0, pjs);
+            if (it.ulo + 2 < it.uhi) r2 = page_rows(a, it.ulo + 2, it.b, it.seqlen_k, lane, pj0, pjs);
+          }
+          const uint32_t s0 = kr.slot;
+          ok = lead_wait(bar_k_empty + 8 * s0, kr.phase ^ 1u);
+          if (!ok) { if (leader) report_error(p.status, DEV_ERR_TIMEOUT, ROLE_TMA); break; }
+          kr.advance();
+          const uint32_t s1 = kr.slot;
+          if (two) {
+            ok = lead_wait(bar_k_empty + 8 * s1, kr.phase ^ 1u);
+            if (!ok) { if (leader) report_error(p.status, DEV_ERR_TIMEOUT, ROLE_TMA); break; }
+            kr.advance();
+          }
+          open_bar(bar_k0_full, two ? 2 * SM::kKStage : SM::kKStage);
+          load_tile(&map_k, HD, sK + s0 * SM::kKStage, it.ulo, bar_k0_full, r0);
+          if (two) load_tile(&map_k, HD, sK + s1 * SM::kKStage, it.ulo + 1, bar_k0_full, r1);
+          close_bar(bar_k0_full);
+          ++k0cnt;
+          ++qcnt;
+          for (int nb = it.ulo; nb < it.uhi; ++nb) {
+            const bool nxt = nb + 2 < it.uhi;
+            const uint32_t vs = vr.slot, ks = kr.slot;
+            if (paged && nb + 3 < it.uhi) r3 = page_rows(a, nb + 3, it.b, it.seqlen_k, lane, pj0, pjs);
+            ok = lead_wait(bar_v_empty + 8 * vs, vr.phase ^ 1u);
+            if (ok && nxt) ok = lead_wait(bar_k_empty + 8 * ks, kr.phase ^ 1u);
+            if (!ok) { if (leader) report_error(p.status, DEV_ERR_TIMEOUT, ROLE_TMA); break; }
+            open_bar(bar_v_full + 8 * vs, SM::kVStage + (nxt ? SM::kKStage : 0));
+            load_tile(&map_v, HDV, sV + vs * SM::kVStage, nb, bar_v_full + 8 * vs, r0);
+            vr.advance();
+            if (nxt) {
+              load_tile(&map_k, HD, sK + ks * SM::kKStage, nb + 2, bar_v_full + 8 * vs, r2);
+              kr.advance();
+            }
+            close_bar(bar_v_full + 8 * vs);
+            r0 = r1;
+            r1 = r2;
+            r2 = r3;
+            if (nb == max(it.ulo, it.uhi - kFetchAhead)) it_next = fetch_and_publish();
+          }
+          continue;
+        }
         PageRows rows_cur = {{0, 0, 0, 0}};
         if (paged) rows_cur = page_rows(a, it.ulo, it.b, it.seqlen_k, lane, pj0, pjs);
         {
@@ -633,7 +687,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       if (leader) {
         if (qcnt > 0) {
           wait_or_abort(bar_q_full, (qcnt - 1) & 1, s_abort + 1 /* never set: pure time limit */);
-          if constexpr (NTL == 2) wait_or_abort(bar_q_full + 8, (qcnt - 1) & 1, s_abort + 1);
+          if constexpr (NTL == 2 && !KS) wait_or_abort(bar_q_full + 8, (qcnt - 1) & 1, s_abort + 1);
         }
         if constexpr (MERGE_KV) {
           if (k0cnt > 0) wait_or_abort(bar_k0_full, (k0cnt - 1) & 1, s_abort + 1);
@@ -692,7 +746,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
 
     // S of tile t into TMEM column `col`, completion on `bar`
     auto issue_qk_to = [&](int t, uint32_t kslot, uint32_t col, uint32_t bar) {
-      const uint64_t qd = qd0 + (uint64_t)(t * ((TM * HD * ESZ) >> 4));
+      const uint64_t qd = qd0 + (uint64_t)((KS ? 0 : t) * ((TM * HD * ESZ) >> 4));
       const uint64_t kd = kd0 + (uint64_t)(kslot * (SM::kKStage >> 4));
       if (leader) {
 #pragma unroll
@@ -783,6 +837,51 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         }
         continue;
       }
+      if constexpr (KS) {
+        // block j belongs to tile j & 1.  Order QK(0) QK(1) | PV(j) QK(j + 2): the QK that follows a PV is the same tile's.
+        const int n = uhi - ulo;
+        wait_tile(bar_k0_full, k0cnt & 1);
+        ++k0cnt;
+        wait(bar_q_full, qcnt & 1);
+        ++qcnt;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (t < n) {
+            issue_qk(t, kr.slot);
+            if (t + 1 == n || (t == 1 && n == 2)) commit(bar_q_empty);      // the item's last QK
+            commit(bar_k_empty + 8 * kr.slot);
+            kr.advance();
+          }
+        }
+        for (int j0 = 0; j0 < n; j0 += 2) {
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            const int j = j0 + t;
+            if (j < n) {
+              const uint32_t vs = vr.slot;
+              wait_tile(bar_v_full + 8 * vs, vr.phase);      // V of this block, and K of the block two behind it
+              if (j0 == 0) {
+                wait(bar_o_empty + 8 * t, (oecnt[t] & 1) ^ 1);
+                ++oecnt[t];
+              }
+              wait(bar_p_full + 8 * t, pcnt[t] & 1);
+              tc_fence_after_sync();
+              issue_pv(t, vs, j0 == 0, false);
+              ++pcnt[t];
+              if (j + 2 >= n) commit(bar_o_full + 8 * t);
+              commit(bar_v_empty + 8 * vs);
+              vr.advance();
+              if (j + 2 < n) {
+                issue_qk(t, kr.slot);
+                if (j + 3 == n) commit(bar_q_empty);
+                commit(bar_k_empty + 8 * kr.slot);
+                kr.advance();
+              }
+            }
+          }
+        }
+        continue;
+      }
       // prologue: QK of the first block
       {
         const uint32_t ks = kr.slot;
@@ -854,7 +953,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
     const uint32_t tS0 = tmem + lane_base + t * TN;
     const uint32_t tO = tmem + lane_base + O_BASE + t * O_STRIDE;
     constexpr bool has_cap = CAP;
-    uint32_t scnt = 0, ocnt = 0;
+    uint32_t scnt = 0, ocnt = 0, ocnt1 = 0, xcnt = 0;      // (the last two: KS)
     bool ok = true;
 
     uint32_t wcnt = 0;
@@ -874,7 +973,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
     };
     for (Item it = next_work(); it.w != kEndOfWork && ok; it = next_work()) {
       if (!it.valid) continue;
-      const int row0 = it.pair * (NTL * TM) + t * TM;
+      const int row0 = it.pair * kItemRows + (KS ? 0 : t * TM);
       if (row0 >= it.seqlen_q) continue;           // this tile owns no row
       const int row = row0 + r;
       float sc = p.scale, vds = 1.f;
@@ -1083,7 +1182,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_p_full + 8 * sb);
       };
-      int i0 = it.lo[t];
+      int i0 = it.lo[t] + (KS ? t : 0);
       if constexpr (F8) {
         if (two_term) {
 #pragma unroll 1
@@ -1091,7 +1190,7 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           if (!ok) break;
         }
       }
-      for (int i = i0; i < it.hi[t]; ++i) {
+      for (int i = i0; i < it.hi[t]; i += KS ? 2 : 1) {
         if constexpr (CAP && !F8) {
           while (i < it.hi[t] && may_be_fast(i)) {
             capped_block();
@@ -1298,6 +1397,19 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
       if (CAP && kCapEmuPairs > 0 && m_used == -INFINITY) l = 0.f;   // the cubic never returns exactly 0
 
       // ---- epilogue of this tile ----
+      if constexpr (KS) {
+        // (a row's maximum and sum of the odd blocks go to the thread of tile 0 that has the same row)
+        const uint32_t xch = sQ + TM * HD * ESZ + (uint32_t)r * 8u;
+        if (t == 1) {
+          ok = wait_or_abort(bar_q_empty + 8, (xcnt & 1) ^ 1, s_abort);
+          ++xcnt;
+          if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_EPILOGUE); break; }
+          asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(xch), "f"(m_used), "f"(l) : "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_q_full + 8);
+          continue;
+        }
+      }
       if constexpr (HDV <= 128) {
         // The whole O row goes to registers first and O_t is released at once: the MMA warp may start the next
         // item's first PV while this thread is still normalising and storing.
@@ -1319,6 +1431,42 @@ fwd_prefill_tc_kernel(const __grid_constant__ TcArgs a, const __grid_constant__ 
           for (int c = 0; c < HDV / 32; ++c)
   #pragma unroll
             for (int j = 0; j < 32; ++j) o[c][j] = 0u;
+        }
+        if constexpr (KS) {
+          ok = wait_or_abort(bar_q_full + 8, xcnt & 1, s_abort);
+          ++xcnt;
+          if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_EPILOGUE); break; }
+          float m1, l1;
+          asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(m1), "=f"(l1) : "r"(sQ + TM * HD * ESZ + (uint32_t)r * 8u) : "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_q_empty + 8);
+          if (it.hi[0] - it.lo[0] > 1) {
+            const float m = fmaxf(m_used, m1);
+            const float w0 = m_used == -INFINITY ? 0.f : ex2(m_used - m), w1 = m1 == -INFINITY ? 0.f : ex2(m1 - m);
+            m_used = m;
+            l = l * w0 + l1 * w1;
+            ok = wait_or_abort(bar_o_full + 8, ocnt1 & 1, s_abort);
+            ++ocnt1;
+            if (!ok) { report_error(p.status, DEV_ERR_TIMEOUT, ROLE_EPILOGUE); break; }
+            tc_fence_after_sync();
+            const float2 a2 = make_float2(w0, w0), b2 = make_float2(w1, w1);
+#pragma unroll
+            for (int c = 0; c < HDV / 32; ++c) {
+              uint32_t o1[32];
+              tmem_ld32(tO + O_STRIDE + c * 32, o1);
+              tmem_wait_ld32(o1);
+#pragma unroll
+              for (int j = 0; j < 32; j += 2) {
+                const float2 y = ffma2(make_float2(__uint_as_float(o[c][j]), __uint_as_float(o[c][j + 1])), a2,
+                                       fmul2(make_float2(__uint_as_float(o1[j]), __uint_as_float(o1[j + 1])), b2));
+                o[c][j] = __float_as_uint(y.x);
+                o[c][j + 1] = __float_as_uint(y.y);
+              }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_o_empty + 8);
+          }
         }
         float m_fin = m_used, l_fin = l, osc = 1.f;
         float l_norm = F8 ? lr : l;          // what O is divided by
@@ -1647,12 +1795,12 @@ static double expected_us(const KParams& kp, int num_sms) {
 // (varlen, window, cap).  The first four are expected to take 2, 26, 15 and 31; the others 147 and more.
 constexpr double kOverlapUs = 100.0;
 
-template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD, bool PARTS>
+template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD, bool PARTS, bool KS = false>
 static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t kv_rows, cudaStream_t stream) {
   using SM = Smem<Elem<T>::kSize, HD, HDV, KST, VST, NTL>;
   TcArgs a;
   a.kp = kp;
-  a.item_rows = NTL * TM;
+  a.item_rows = KS ? TM : NTL * TM;
   a.max_pairs = (kp.max_seqlen_q + a.item_rows - 1) / a.item_rows;
   a.num_items = kp.batch * kp.hq * a.max_pairs * kp.tc_cut.most;
   a.use_list = kp.work != nullptr;
@@ -1681,7 +1829,7 @@ static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t k
                     (uint64_t)kp.o_row_stride, 32))
       a.stage_out = 1;
   }
-  auto kern = fwd_prefill_tc_kernel<T, HD, HDV, KST, VST, NTL, CAP, PROD, PARTS>;
+  auto kern = fwd_prefill_tc_kernel<T, HD, HDV, KST, VST, NTL, CAP, PROD, PARTS, KS>;
   int smem = SM::kBytes + 1024;
   if (smem < 120 * 1024) smem = 120 * 1024;   // one CTA per SM: the CTA owns all 512 TMEM columns
   static std::atomic<unsigned long long> attr_done{0};   // one bit per device
@@ -1703,6 +1851,9 @@ static int launch_parts(const KParams& kp, const Plan& pl, int dtype, uint64_t k
 
 template <typename T, int HD, int HDV, int KST, int VST, int NTL, bool CAP, int PROD>
 static int launch_prod(const KParams& kp, const Plan& pl, int dtype, uint64_t kv_rows, cudaStream_t stream) {
+  if constexpr (NTL == 2 && KST == VST && !CAP && !Elem<T>::kF8 && PROD != 2) {
+    if (kp.tc_cut.shared) return launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, false, true>(kp, pl, dtype, kv_rows, stream);
+  }
   return kp.tc_cut.most > 1 ? launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, true>(kp, pl, dtype, kv_rows, stream)
                           : launch_parts<T, HD, HDV, KST, VST, NTL, CAP, PROD, false>(kp, pl, dtype, kv_rows, stream);
 }
@@ -1726,6 +1877,11 @@ static int launch_impl(const KParams& kp, const Plan& pl, int dtype, uint64_t kv
 // back to back) are checked at launch: fa_b200_fwd re-plans onto the general route when they do not hold.
 // Head dims whose O accumulator leaves TMEM room for one query tile only (work items of 128 rows).
 bool prefill_tc_single_tile(int hd, int hdv) { return (hd == 256 && hdv == 256) || (hd == 192 && hdv == 192); }
+
+// The form with shared key blocks: two tiles per kernel, rings of equal depth, no soft cap, 16-bit.
+bool tc_shared_supported(const PlanInput& in) {
+  return in.q_dtype != FA_DT_FP8_E4M3 && !in.has_softcap && ((in.hd == 64 && in.hdv == 64) || (in.hd == 128 && in.hdv == 128) || (in.hd == 96 && in.hdv == 96));
+}
 
 bool prefill_tc_supported(const PlanInput& in) {
   if (in.q_dtype != in.kv_dtype) return false;

@@ -1,0 +1,65 @@
+"""Prefill with few items: tiles of 128 rows whose key blocks are shared by the two softmax groups of a CTA (even and odd blocks),
+against the CPU oracle with the benchmark's tolerances (2e-2, LSE 5e-3 and 1e-2) and against the form in which a group has a row
+tile of its own (num_splits = 1; one rounding to 16 bits of |values| < 4, P rounded against another maximum)."""
+import pytest
+import torch
+
+from flash_cuda_b200 import capi, workloads as W
+from oracle.ref_attention import ref_attention
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(p, dev):
+    d = p.to(dev)
+    kw = dict(d.capi_kw(), route=capi.FA_ROUTE_PREFILL_TC)
+    out, lse, _ = capi.fwd(d.q, d.k, d.v, check=True, **kw)
+    whole, whole_lse, _ = capi.fwd(d.q, d.k, d.v, check=True, num_splits=1, **kw)
+    want, want_lse = ref_attention(p.q, p.k, p.v, **p.oracle_kw())
+    assert (out.float().cpu() - want).abs().max().item() <= 2e-2, p.name
+    fin = torch.isfinite(want_lse)
+    assert torch.equal(torch.isfinite(lse.cpu()), fin), p.name
+    torch.testing.assert_close(lse.cpu()[fin], want_lse[fin], atol=5e-3, rtol=1e-2)
+    assert (out.float() - whole.float()).abs().max().item() <= 2 ** -6 + 2 ** -8
+    torch.testing.assert_close(lse[fin], whole_lse[fin], atol=1e-4, rtol=1e-5)
+    return out, lse, whole, whole_lse
+
+
+@pytest.mark.parametrize("hd,dtype", [(64, "fp16"), (96, "bf16"), (128, "bf16"), (128, "fp16")])
+@pytest.mark.parametrize("keys", [1, 127, 128, 129, 256, 257, 384, 500, 1300])       # 1 .. 11 blocks, odd and even
+@pytest.mark.parametrize("page", [0, 16, 64, 128])
+def test_numbers_of_blocks(page, keys, hd, dtype, cuda_device):
+    p = W.make_problem("shared", [(130, keys), (min(keys, 70), keys), (1, 900)], hq=4, hkv=2, hd=hd, dtype=dtype, page_size=page, causal=False, seed=601)
+    _check(p, cuda_device)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("name,reqs,kw", [
+    ("causal", [(700, 700), (257, 900), (5, 5), (128, 128)], {}),
+    ("window", [(300, 1500), (200, 200)], dict(window_left=200)),
+    ("two_sided", [(300, 1000)], dict(window_left=100, window_right=150, causal=False)),
+    ("sink_leftpad", [(200, 900), (140, 600)], dict(sink=True, leftpad=[300, 599])),
+    ("empty", [(150, 0), (0, 300), (129, 800), (20, 7)], dict(sink=True)),
+    ("hidden_rows", [(600, 300)], {}),          # queries before the first key see nothing
+])
+def test_masks(name, reqs, kw, hd, cuda_device):
+    p = W.make_problem("shared_" + name, reqs, hq=6, hkv=2, hd=hd, page_size=0, seed=602, **kw)
+    _check(p, cuda_device)
+
+
+def test_scores_that_grow_in_one_half_only(cuda_device):
+    """Keys of the odd blocks are forty times as large, then of the even ones: the two maxima lie far apart, either way."""
+    for odd in (0, 1):
+        p = W.make_problem("shared", [(200, 1100)], hq=4, hkv=2, hd=128, page_size=0, causal=False, seed=603)
+        p.k[(torch.arange(1100) // 128) % 2 == odd] *= 40.0
+        _check(p, cuda_device)
+
+
+def test_it_is_another_form(cuda_device):
+    p = W.make_problem("shared", [(512, 512)] * 2, hq=8, hkv=8, hd=128, page_size=0, causal=False, seed=604)
+    _, lse, _, whole_lse = _check(p, cuda_device)
+    assert not torch.equal(lse, whole_lse)
+    d = p.to(cuda_device)
+    first = capi.fwd(d.q, d.k, d.v, check=True, **d.capi_kw())[:2]
+    again = capi.fwd(d.q, d.k, d.v, check=True, **d.capi_kw())[:2]
+    assert all(torch.equal(a, b) for a, b in zip(first, again))
