@@ -1,0 +1,39 @@
+"""All-e4m3 prefill of tiles that see one or two key blocks (P as two e4m3 terms, a loop of its own) and of tiles just beyond (one term),
+with every kind of mask, against the CPU oracle.  Output tolerance 6e-2, the benchmark's for e4m3; LSE 5e-3 and 1e-2, with a cap of 20 besides
+2^-11 of it (tanh.approx)."""
+import pytest
+import torch
+
+from flash_cuda_b200 import capi, workloads as W
+from oracle.ref_attention import ref_attention
+
+pytestmark = pytest.mark.gpu
+REQS = {"one_block": [(1, 1), (65, 65), (128, 128), (7, 100)], "two_blocks": [(130, 256), (129, 200), (256, 256), (100, 129)],
+        "three_blocks": [(200, 300), (300, 300), (90, 384)], "keyless": [(80, 0), (0, 40), (129, 140)]}
+
+
+@pytest.mark.parametrize("name", sorted(REQS))
+@pytest.mark.parametrize("kw", [dict(), dict(causal=False), dict(window_left=50), dict(window_left=20, window_right=31, causal=False),
+                                dict(softcap=20.0), dict(sink=True, softcap=20.0, window_left=90)],
+                         ids=["causal", "full", "window", "two_sided", "cap", "cap_sink_window"])
+@pytest.mark.parametrize("page", [0, 64])
+def test_tiles_of_few_blocks(name, kw, page, cuda_device):
+    p = W.make_problem("two_term", REQS[name], hq=4, hkv=2, hd=128, dtype="fp8", page_size=page, seed=701, **kw)
+    d = p.to(cuda_device)
+    out, lse, _ = capi.fwd(d.q, d.k, d.v, check=True, **d.capi_kw())
+    want, want_lse = ref_attention(p.q, p.k, p.v, **p.oracle_kw())
+    assert (out.float().cpu() - want).abs().max().item() <= 6e-2
+    fin = torch.isfinite(want_lse)
+    assert torch.equal(torch.isfinite(lse.cpu()), fin)
+    torch.testing.assert_close(lse.cpu()[fin], want_lse[fin], atol=5e-3 + kw.get("softcap", 0.0) * 2 ** -11, rtol=1e-2)
+
+
+def test_leftpad(cuda_device):
+    p = W.make_problem("two_term", [(70, 256), (128, 250), (20, 129)], hq=4, hkv=2, hd=128, dtype="fp8", page_size=64, leftpad=[130, 100, 128], seed=702)
+    d = p.to(cuda_device)
+    out, lse, _ = capi.fwd(d.q, d.k, d.v, check=True, **d.capi_kw())
+    want, want_lse = ref_attention(p.q, p.k, p.v, **p.oracle_kw())
+    assert (out.float().cpu() - want).abs().max().item() <= 6e-2
+    fin = torch.isfinite(want_lse)
+    assert torch.equal(torch.isfinite(lse.cpu()), fin)
+    torch.testing.assert_close(lse.cpu()[fin], want_lse[fin], atol=5e-3, rtol=1e-2)
