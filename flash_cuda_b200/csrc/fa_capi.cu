@@ -201,10 +201,12 @@ static Plan decode_part_plan(const PlanInput& in, const Plan& pl) {
 //   empty, 41 - 51 0.91 - 1.04 (1.08 - 1.2), 183 1.02 - 1.05 (1.3), 560 1.2 (1.35);
 //   head_dim 64, 24 or 32 rows, 17 blocks 0.62 - 0.68 (0.72), 61 0.98 (1.06), 203 0.97 - 1.0 (1.1), 340 1.28 (1.4); 64 rows, 122 0.83 (0.94), 406 1.2
 //   (1.4); 48 rows, 304 0.94 (1.1), 510 0.99 (1.13).
-// Not with a caller's work list, whose entries are tiles of 16 rows, and not over an e4m3 cache (two CTAs of four warps per SM as
-// well, and no registers for a second tile beside the widening).
+// A caller's work list keeps its entries of 16 rows, which the kernel joins (join_row_tiles).  Sequences of 2048 .. 16384 keys, us one
+// at a time / two at a time with a list: 16 of 32 rows over pages of 16, head_dim 128 256 / 157, 64 234 / 161; 64 of 32 rows over pages
+// of 64, 648 / 494 and 566 / 474; 16 of 32 rows with head_dim 192, pages of 16, 626 / 379.  Not over an e4m3 cache: two CTAs of four warps per SM as
+// well, and no registers for a second tile beside the widening.
 static void wide_decode_rows(Plan* pl, const FaFwdParams* p) {
-  if (pl->err != FA_OK || pl->route != FA_ROUTE_DECODE || p->scheduler_metadata != nullptr || p->kv_dtype == FA_DT_FP8_E4M3) return;
+  if (pl->err != FA_OK || pl->route != FA_ROUTE_DECODE || p->kv_dtype == FA_DT_FP8_E4M3) return;
   const int tiles = pl->max_mtiles;
   if (tiles < 2) return;
   const bool small = p->page_table && p->page_size <= 16;
@@ -230,7 +232,8 @@ static void wide_decode_rows(Plan* pl, const FaFwdParams* p) {
 // Never with a split count of the caller's (1 = one pass per sequence, whatever else is in the batch), for fp32 partials,
 // or where the scan over the lengths, which every CTA makes, would have more than 2048 entries (13 per thread).
 static bool balanced_decode(const FaFwdParams* p, const Plan& decode_plan, bool mixed = false) {
-  const long long entries = (long long)p->batch * decode_plan.max_mtiles, items = entries * p->hkv;
+  const long long tiles = (long long)p->batch * decode_plan.max_mtiles, items = tiles * p->hkv;
+  const long long entries = p->scheduler_metadata && decode_plan.tile_m > 16 ? 2 * tiles : tiles;      // (a list keeps one per 16 rows)
   const int ctas = decode_line_ctas(p->hd, p->kv_dtype, decode_plan.num_sms);
   if (decode_plan.route != FA_ROUTE_DECODE || p->num_splits > 0 || p->out_dtype == FA_DT_FP32 ||
       entries > kBalancedEntriesMax || items * (p->max_seqlen_k / 64 + 2) >= (1ll << 30) || ctas > kWsArrivalWords)
@@ -622,6 +625,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   PlanInput in = plan_input(p, di->sms);
   Plan pl = make_plan(in);
   if (pl.err != FA_OK) return pl.err;
+  const Plan listed = pl;      // what a caller's work list was made for
   wide_decode_rows(&pl, p);
   WsLayout w = ws_layout(p, pl);
   if (!workspace || ((uintptr_t)workspace % 256)) return FA_ERR_WORKSPACE;
@@ -636,7 +640,7 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   // unread rather than refused.
   const bool md_read = pl.route == FA_ROUTE_DECODE || pl.route == FA_ROUTE_PREFILL_TC;
   if (md_read && p->scheduler_metadata && p->scheduler_metadata_len > 0 &&
-      p->scheduler_metadata_len != sched_len(pl, p->batch))
+      p->scheduler_metadata_len != sched_len(listed, p->batch))
     return FA_ERR_BAD_METADATA;
 
   char* ws = (char*)workspace;
@@ -683,7 +687,8 @@ int fa_b200_fwd(const FaFwdParams* p_in, void* workspace, size_t workspace_bytes
   kp.nsplits = pl.nsplits;
   kp.tc_cut = kTcUncut;
   kp.out_f32 = p->out_dtype == FA_DT_FP32;
-  kp.work_expect = SchedExpect{p->batch, pl.nsplits, pl.tile_m, pl.tile_n, pl.max_mtiles, pl.rows_per_token, pl.route};
+  const Plan& lp = p->scheduler_metadata ? listed : pl;
+  kp.work_expect = SchedExpect{p->batch, lp.nsplits, lp.tile_m, lp.tile_n, lp.max_mtiles, lp.rows_per_token, lp.route};
   kp.scale = p->softmax_scale; kp.softcap = p->softcap;
   if (balanced) {
     kp.part_ml = (float*)(ws + w.part_ml_off); kp.part_o = (float*)(ws + w.part_o_off);

@@ -107,8 +107,20 @@ struct WorkItem {
   bool bad;     // the entry names a batch or a key range that this problem does not have
 };
 
+// A caller's list has an entry for every 16 rows.  Where a pass takes 32 (wide_decode_rows) the entry of the even tile stands for both,
+// over the keys that either sees, and the odd one's is passed over once it has been checked.
+__device__ __forceinline__ void join_row_tiles(const KParams& p, WorkItem* it) {
+  if (p.work_expect.tile_m != 16) return;
+  if (it->mt & 1) { it->valid = false; return; }
+  const int off = it->seqlen_k - it->seqlen_q, row0 = it->mt * 16;
+  nblock_range(it->seqlen_k, it->leftpad, off + row0 / p.rep, off + min(it->seqlen_q - 1, (row0 + 31) / p.rep), p.is_causal,
+               p.window_left, p.window_right, TN, &it->lo, &it->hi);
+  it->mt >>= 1;
+}
+
 // Entry e of the work list -> work item.  The list may come from the caller: an entry is used only if its batch
 // index and key-block range lie inside this problem (else `bad`, and nothing is dereferenced with it).
+template <int MT>
 __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
   WorkItem it;
   const int per_entry = p.hkv * p.nsplits;
@@ -131,7 +143,9 @@ __device__ __forceinline__ WorkItem decode_work(const KParams& p, int w) {
     it.leftpad = p.leftpad_k ? p.leftpad_k[it.b] : 0;
     const int n_lo = ent[2], n_hi = ent[3];
     if (n_lo < 0 || n_hi < n_lo || (int64_t)n_hi * TN > (int64_t)it.seqlen_k + TN - 1) { it.valid = false; it.bad = true; return it; }
-    split_range(n_lo, n_hi, it.split, p.nsplits, &it.lo, &it.hi);
+    it.lo = n_lo; it.hi = n_hi;
+    if constexpr (MT > 1) join_row_tiles(p, &it);
+    split_range(it.lo, it.hi, it.split, p.nsplits, &it.lo, &it.hi);
   }
   return it;
 }
@@ -210,7 +224,7 @@ __device__ __forceinline__ WorkItem line_entry(const DecArgs& a, int e) {
   it.seqlen_k = p.seqused_k ? p.seqused_k[it.b] : (p.cu_k[it.b + 1] - p.cu_k[it.b]);
   it.leftpad = p.leftpad_k ? p.leftpad_k[it.b] : 0;
   const int rows = it.seqlen_q * p.rep;
-  if (it.mt * (16 * MT) >= rows || (a.class_rows > 0 && rows > a.class_rows)) return it;
+  if (it.mt * (MT > 1 && a.use_list ? p.work_expect.tile_m : 16 * MT) >= rows || (a.class_rows > 0 && rows > a.class_rows)) return it;
   if (a.use_list) {
     if (n_lo < 0 || n_hi < n_lo || (int64_t)n_hi * TN > (int64_t)it.seqlen_k + TN - 1) { it.bad = true; return it; }
   } else {
@@ -220,6 +234,9 @@ __device__ __forceinline__ WorkItem line_entry(const DecArgs& a, int e) {
   }
   it.valid = true;
   it.lo = n_lo; it.hi = n_hi;
+  if constexpr (MT > 1) {
+    if (a.use_list) join_row_tiles(p, &it);
+  }
   return it;
 }
 // Blocks of one head group of an entry; an entry whose rows see no key counts as one, so that some CTA writes its rows.
@@ -573,7 +590,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         if (!first_ticket) w = __shfl_sync(0xffffffffu, w, 0);
         first_ticket = false;
         if (w >= total_work) break;
-        it = decode_work(p, w);
+        it = decode_work<MT>(p, w);
         if (it.bad) {
           if (lane == 0) report_error(p.status, DEV_ERR_BAD_INDEX, ROLE_PRODUCER);
           break;
@@ -785,7 +802,7 @@ fwd_decode_kernel(const DecArgs a, const __grid_constant__ CUtensorMap map_k, co
         key0 = s_info[4 * s + 1]; flags = s_info[4 * s + 2];
       }
       if (flags & F_FIRST) {
-        if constexpr (!BAL) it_reg = decode_work(p, wid);
+        if constexpr (!BAL) it_reg = decode_work<MT>(p, wid);
         const int rows_total = it.seqlen_q * rep;
         const int di = it.b * p.descale_batch_stride + it.hk * p.descale_head_stride;
         const float ds_q = p.q_descale ? p.q_descale[di] : 1.f, ds_k = p.k_descale ? p.k_descale[di] : 1.f;
@@ -1410,7 +1427,7 @@ static int launch_tiles(const KParams& kp, const Plan& pl, int num_work_slots, c
   a.kp = kp;
   a.total_work = num_work_slots * kp.hkv * kp.nsplits;
   a.use_list = kp.work != nullptr;
-  a.max_mtiles = pl.max_mtiles;
+  a.max_mtiles = kp.work ? kp.work_expect.max_mtiles : pl.max_mtiles;     // (a caller's list: tiles of 16 rows)
   a.class_rows = kp.class_rows;
   const bool paged = kp.page_table != nullptr;
   // (The cp.async producer takes any power-of-two page.  16 sequences of 1024 .. 16384 keys, TMA boxes / cp.async, us in a graph:
@@ -1502,7 +1519,7 @@ static int launch_decode_t(const KParams& kp, const Plan& pl, int slots, cudaStr
 
 int launch_decode(const KParams& kp, const Plan& pl, int compute_dtype, cudaStream_t stream) {
   // every (batch, m_tile) slot of the metadata may hold a work entry
-  const int slots = kp.batch * pl.max_mtiles;
+  const int slots = kp.batch * (kp.work ? kp.work_expect.max_mtiles : pl.max_mtiles);
   if (kp.part_o != nullptr)
     return compute_dtype != FA_DT_FP16 ? launch_decode_t<__nv_bfloat16, true>(kp, pl, slots, stream)
                                        : launch_decode_t<__half, true>(kp, pl, slots, stream);
